@@ -9,7 +9,9 @@
 //   ℓ = mean_b (o0 - t0)^2 + mean_b [softplus(o1) - t1 o1]
 // (o0: the log-response prediction, o1: the logit of the pole-proximity score).
 //
-// One strided GEMM serves the three products of a layer:
+// Networks whose layers are at most 256 wide run fused (ytf_mlp_fused.cuh): one kernel for the
+// forward pass, one for the input gradients, one for all weight gradients. Wider ones take one
+// strided GEMM per product of a layer:
 //   forward  Z[b][o]  = Σ_i H[b][i] W[o][i] + bias[o]   (then GELU)
 //   input    dH[b][i] = Σ_o dZ[b][o] W[o][i]
 //   weights  dW[o][i] = Σ_b dZ[b][o] H[b][i]
@@ -32,6 +34,7 @@
 #include <vector>
 
 #include "../../include/ytf.h"
+#include "ytf_mlp_fused.cuh"
 #include "ytf_tcgen05.cuh"
 
 namespace ytf {
@@ -291,10 +294,17 @@ struct ytf_mlp {
   // activations for the largest batch seen: Z_l and H_l per layer, gradients, loss terms
   long cap = 0;
   std::vector<float*> Z, H, dZ, dH;
-  float *T = nullptr, *lb = nullptr, *X = nullptr;
-  unsigned* tc_err = nullptr;      // set by a tensor-core GEMM whose commit wait ran out
-  float* part = nullptr;           // K-slice sums of split GEMMs
+  float *T = nullptr, *lb = nullptr;
+  // inputs and outputs of the largest forward-only batch from host memory (fused networks)
+  long cap_io = 0;
+  float *Xin = nullptr, *Yout = nullptr;
+  unsigned* tc_err = nullptr;      // page-locked: set by a kernel whose tensor-core wait ran out
+  float* part = nullptr;           // K-slice sums of split GEMMs, batch-slice sums of the gradients
   size_t part_cap = 0;
+  bool fused = false;              // every layer at most 256 wide (ytf_mlp_fused.cuh)
+  uint8_t* img = nullptr;          // packed BF16 weights: forward images, then transposed ones
+  std::vector<size_t> img_f, img_b;
+  int nsm = 148;
   std::string err;
   ~ytf_mlp() {
     cudaFree(p); cudaFree(g); cudaFree(m); cudaFree(v); cudaFree(wb);
@@ -302,7 +312,8 @@ struct ytf_mlp {
     for (auto* q : H) cudaFree(q);
     for (auto* q : dZ) cudaFree(q);
     for (auto* q : dH) cudaFree(q);
-    cudaFree(T); cudaFree(lb); cudaFree(X); cudaFree(tc_err); cudaFree(part);
+    cudaFree(T); cudaFree(lb); cudaFree(Xin); cudaFree(Yout); cudaFree(part); cudaFree(img);
+    if (tc_err) cudaFreeHost(tc_err);
   }
 };
 
@@ -366,14 +377,16 @@ int ensure(ytf_mlp* net, long B) {
   for (auto* q : net->H) cudaFree(q);
   for (auto* q : net->dZ) cudaFree(q);
   for (auto* q : net->dH) cudaFree(q);
-  cudaFree(net->T); cudaFree(net->lb); cudaFree(net->X);
+  cudaFree(net->T); cudaFree(net->lb);
+  net->T = net->lb = nullptr;
+  net->cap = 0;
   const int L = (int)net->sizes.size() - 1;
   net->Z.assign(L + 1, nullptr); net->H.assign(L + 1, nullptr);
   net->dZ.assign(L + 1, nullptr); net->dH.assign(L + 1, nullptr);
   for (int l = 0; l <= L; ++l) {
     const size_t bytes = sizeof(float) * B * net->sizes[l];
     MCK(cudaMalloc(&net->H[l], bytes));
-    MCK(cudaMalloc(&net->dH[l], bytes));
+    if (!net->fused) MCK(cudaMalloc(&net->dH[l], bytes));
     if (l > 0) {
       MCK(cudaMalloc(&net->Z[l], bytes));
       MCK(cudaMalloc(&net->dZ[l], bytes));
@@ -381,9 +394,150 @@ int ensure(ytf_mlp* net, long B) {
   }
   MCK(cudaMalloc(&net->T, sizeof(float) * 2 * B));
   MCK(cudaMalloc(&net->lb, sizeof(float) * B));
-  MCK(cudaMalloc(&net->X, sizeof(float) * B * net->sizes[0]));
   net->cap = B;
   return YTF_OK;
+}
+
+// staging of a forward-only batch from host memory
+int ensure_io(ytf_mlp* net, long B) {
+  if (B <= net->cap_io) return YTF_OK;
+  cudaFree(net->Xin); cudaFree(net->Yout);
+  net->Xin = net->Yout = nullptr;
+  net->cap_io = 0;
+  MCK(cudaMalloc(&net->Xin, sizeof(float) * B * net->sizes[0]));
+  MCK(cudaMalloc(&net->Yout, sizeof(float) * B * net->sizes.back()));
+  net->cap_io = B;
+  return YTF_OK;
+}
+
+int round16(int n) { return (n + 15) / 16 * 16; }
+
+// the weight images of the fused kernels from the current parameters
+int pack_weights(ytf_mlp* net, bool back) {
+  const int L = (int)net->sizes.size() - 1;
+  Pack pk;
+  pk.n = 0;
+  pk.total = 0;
+  for (int trans = 0; trans <= (back ? 1 : 0); ++trans)
+    for (int l = 1 + trans; l <= L; ++l) {  // the first layer's input gradient is not formed
+      PackLayer& q = pk.l[pk.n++];
+      q.W = net->p + net->woff[l - 1];
+      q.img = net->img + (trans ? net->img_b[l - 1] : net->img_f[l - 1]);
+      q.in = net->sizes[l - 1];
+      q.out = net->sizes[l];
+      q.trans = trans;
+      q.Np = round16(trans ? q.in : q.out);
+      q.kblocks = ((trans ? q.out : q.in) + FKB - 1) / FKB;
+      q.first = pk.total;
+      pk.total += (long)q.Np * q.kblocks * (FKB / 8);
+    }
+  k_mlp_pack<<<(unsigned)((pk.total + 255) / 256), 256, 0, net->stream>>>(pk);
+  MCK(cudaGetLastError());
+  return YTF_OK;
+}
+
+// forward pass of B device rows X into `out`; `keep`: Z_l and H_l of the inner layers for the backward pass
+int forward_fused(ytf_mlp* net, long B, const float* X, float* out, bool keep) {
+  const int L = (int)net->sizes.size() - 1;
+  Chain c;
+  std::memset(&c, 0, sizeof(c));
+  c.L = L;
+  c.B = B;
+  c.X = X;
+  c.out = out;
+  c.err = net->tc_err;
+  for (int l = 1; l <= L; ++l) {
+    ChainLayer& q = c.l[l - 1];
+    q.img = net->img + net->img_f[l - 1];
+    q.K = net->sizes[l - 1];
+    q.N = net->sizes[l];
+    q.ksteps = round16(q.K) / 16;
+    q.Np = round16(q.N);
+    q.bias = net->p + net->boff[l - 1];
+    if (keep && l < L) { q.Z = net->Z[l]; q.H = net->H[l]; }
+  }
+  MCK(cudaFuncSetAttribute(k_mlp_chain<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chain_smem()));
+  const long tiles = (B + FM - 1) / FM;
+  k_mlp_chain<false><<<(unsigned)std::min<long>(tiles, net->nsm), FDRAIN + 32, chain_smem(), net->stream>>>(c);
+  MCK(cudaGetLastError());
+  return YTF_OK;
+}
+
+// gradients into g from the inputs in X, the kept activations, the outputs in H[L] and the targets in T
+int backward_fused(ytf_mlp* net, long B, const float* X) {
+  const int L = (int)net->sizes.size() - 1;
+  Chain c;
+  std::memset(&c, 0, sizeof(c));
+  c.L = L - 1;
+  c.backward = 1;
+  c.B = B;
+  c.o = net->H[L];
+  c.T = net->T;
+  c.dout = net->dZ[L];
+  c.lb = net->lb;
+  c.err = net->tc_err;
+  for (int l = L; l >= 2; --l) {  // dZ_{l-1} = (dZ_l W_l) GELU'(Z_{l-1})
+    ChainLayer& q = c.l[L - l];
+    q.img = net->img + net->img_b[l - 1];
+    q.K = net->sizes[l];
+    q.N = net->sizes[l - 1];
+    q.ksteps = round16(q.K) / 16;
+    q.Np = round16(q.N);
+    q.Z = net->Z[l - 1];
+    q.H = net->dZ[l - 1];
+  }
+  MCK(cudaFuncSetAttribute(k_mlp_chain<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chain_smem()));
+  const long tiles = (B + FM - 1) / FM;
+  k_mlp_chain<true><<<(unsigned)std::min<long>(tiles, net->nsm), FDRAIN + 32, chain_smem(), net->stream>>>(c);
+  MCK(cudaGetLastError());
+  Dw d;
+  std::memset(&d, 0, sizeof(d));
+  d.L = L;
+  d.B = B;
+  d.nparam = net->nparam;
+  d.g = net->g;
+  d.err = net->tc_err;
+  int mtiles = 0;
+  for (int l = 1; l <= L; ++l) mtiles += (net->sizes[l] + FM - 1) / FM;
+  // batch slices of at least 64 samples that fill the SMs once (one CTA per SM: 192 KB of operands)
+  const long want = std::max(1, net->nsm / mtiles);
+  d.slice = std::max(64L, ((B + want - 1) / want + 63) / 64 * 64);
+  d.slices = (int)((B + d.slice - 1) / d.slice);
+  const size_t need = (size_t)d.slices * net->nparam;
+  if (need > net->part_cap) {
+    cudaFree(net->part);
+    net->part = nullptr;
+    net->part_cap = 0;
+    MCK(cudaMalloc(&net->part, sizeof(float) * need));
+    net->part_cap = need;
+  }
+  d.part = net->part;
+  for (int l = 1; l <= L; ++l) {
+    DwLayer& q = d.l[l - 1];
+    q.dZ = net->dZ[l];
+    q.H = l == 1 ? X : net->H[l - 1];
+    q.M = net->sizes[l];
+    q.N = net->sizes[l - 1];
+    q.Np = round16(q.N);
+    q.mtiles = (q.M + FM - 1) / FM;
+    q.first = d.blocks;
+    q.poff = net->woff[l - 1];
+    q.boff = net->boff[l - 1];
+    d.blocks += q.mtiles * d.slices;
+  }
+  MCK(cudaFuncSetAttribute(k_mlp_dw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dw_smem()));
+  k_mlp_dw<<<d.blocks, DW_THREADS, dw_smem(), net->stream>>>(d);
+  MCK(cudaGetLastError());
+  k_mlp_dw_sum<<<(unsigned)((net->nparam + 255) / 256), 256, 0, net->stream>>>(net->nparam, d.slices, d.part, d.g);
+  MCK(cudaGetLastError());
+  return YTF_OK;
+}
+
+// after a synchronisation: a tensor-core wait that ran out in the work before it
+int check_waits(ytf_mlp* net) {
+  if (!*net->tc_err) return YTF_OK;
+  *net->tc_err = 0;
+  return mfail(net, YTF_ERR_CUDA, "ytf_mlp: a tensor-core pipeline wait timed out");
 }
 
 // forward pass of B samples already in H[0]
@@ -424,6 +578,18 @@ int backward(ytf_mlp* net, int B) {
   return YTF_OK;
 }
 
+// loss terms into lb and gradients into g of the batch in H[0], T
+int loss_and_gradients(ytf_mlp* net, int B) {
+  int rc;
+  if (!net->fused) {
+    if ((rc = forward(net, B))) return rc;
+    return backward(net, B);
+  }
+  if ((rc = pack_weights(net, true)) || (rc = forward_fused(net, B, net->H[0], net->H[net->sizes.size() - 1], true)))
+    return rc;
+  return backward_fused(net, B, net->H[0]);
+}
+
 }  // namespace
 
 extern "C" {
@@ -460,11 +626,27 @@ int ytf_mlp_create(int device, int nlayers, const int* sizes, unsigned long long
   int rc = YTF_OK;
   if (cudaMalloc(&net->p, 4 * o) != cudaSuccess || cudaMalloc(&net->g, 4 * o) != cudaSuccess ||
       cudaMalloc(&net->m, 4 * o) != cudaSuccess || cudaMalloc(&net->v, 4 * o) != cudaSuccess ||
-      cudaMalloc(&net->wb, 2 * o) != cudaSuccess || cudaMalloc(&net->tc_err, sizeof(unsigned)) != cudaSuccess)
+      cudaMalloc(&net->wb, 2 * o) != cudaSuccess ||
+      cudaHostAlloc(&net->tc_err, sizeof(unsigned), cudaHostAllocDefault) != cudaSuccess)
     rc = YTF_ERR_NOMEM;
+  else
+    *net->tc_err = 0;
+  cudaDeviceGetAttribute(&net->nsm, cudaDevAttrMultiProcessorCount, device);
+  net->fused = nlayers <= FMAXL;
+  for (int l = 0; l <= nlayers; ++l) net->fused = net->fused && sizes[l] <= FW;
+  if (!rc && net->fused) {
+    size_t bytes = 0;
+    for (int trans = 0; trans < 2; ++trans)
+      for (int l = 1; l <= nlayers; ++l) {
+        const int rows = trans ? sizes[l - 1] : sizes[l], k = trans ? sizes[l] : sizes[l - 1];
+        (trans ? net->img_b : net->img_f).push_back(bytes);
+        bytes += 2ul * round16(rows) * 64 * ((k + FKB - 1) / FKB);
+      }
+    if (cudaMalloc(&net->img, bytes) != cudaSuccess) rc = YTF_ERR_NOMEM;
+  }
   if (!rc && (cudaMemcpy(net->p, h.data(), 4 * o, cudaMemcpyHostToDevice) != cudaSuccess ||
               cudaMemset(net->m, 0, 4 * o) != cudaSuccess || cudaMemset(net->v, 0, 4 * o) != cudaSuccess ||
-              cudaMemset(net->g, 0, 4 * o) != cudaSuccess || cudaMemset(net->tc_err, 0, sizeof(unsigned)) != cudaSuccess))
+              cudaMemset(net->g, 0, 4 * o) != cudaSuccess))
     rc = YTF_ERR_CUDA;
   if (rc) { delete net; return rc; }
   *out = net;
@@ -499,16 +681,26 @@ int ytf_mlp_forward(ytf_mlp* net, int B, const float* X, float* out, int on_devi
   if (!net || B < 0 || (B > 0 && (!X || !out))) return YTF_ERR_ARG;
   if (B == 0) return YTF_OK;
   MCK(cudaSetDevice(net->device));
-  int rc = ensure(net, B);
-  if (rc) return rc;
+  int rc;
   const size_t xb = sizeof(float) * B * net->sizes[0];
+  if (net->fused) {
+    if (!on_device && (rc = ensure_io(net, B))) return rc;
+    if (!on_device) MCK(cudaMemcpyAsync(net->Xin, X, xb, cudaMemcpyHostToDevice, net->stream));
+    float* y = on_device ? out : net->Yout;
+    if ((rc = pack_weights(net, false)) || (rc = forward_fused(net, B, on_device ? X : net->Xin, y, false))) return rc;
+    if (!on_device) MCK(cudaMemcpyAsync(out, y, sizeof(float) * 2 * B, cudaMemcpyDeviceToHost, net->stream));
+    MCK(cudaStreamSynchronize(net->stream));
+    return check_waits(net);
+  }
+  rc = ensure(net, B);
+  if (rc) return rc;
   MCK(cudaMemcpyAsync(net->H[0], X, xb, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, net->stream));
   if ((rc = forward(net, B))) return rc;
   const int L = (int)net->sizes.size() - 1;
   MCK(cudaMemcpyAsync(out, net->H[L], sizeof(float) * 2 * B, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                       net->stream));
   MCK(cudaStreamSynchronize(net->stream));
-  return YTF_OK;
+  return check_waits(net);
 }
 
 int ytf_mlp_gradients(ytf_mlp* net, int B, const float* X, const float* T, float* grad, float* loss, int on_device) {
@@ -519,7 +711,7 @@ int ytf_mlp_gradients(ytf_mlp* net, int B, const float* X, const float* T, float
   const auto kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   MCK(cudaMemcpyAsync(net->H[0], X, sizeof(float) * B * net->sizes[0], kind, net->stream));
   MCK(cudaMemcpyAsync(net->T, T, sizeof(float) * 2 * B, kind, net->stream));
-  if ((rc = forward(net, B)) || (rc = backward(net, B))) return rc;
+  if ((rc = loss_and_gradients(net, B))) return rc;
   if (grad) MCK(cudaMemcpyAsync(grad, net->g, 4 * net->nparam, cudaMemcpyDeviceToHost, net->stream));
   if (loss) {
     std::vector<float> lb(B);
@@ -530,7 +722,7 @@ int ytf_mlp_gradients(ytf_mlp* net, int B, const float* X, const float* T, float
     *loss = (float)(s / B);
   }
   MCK(cudaStreamSynchronize(net->stream));
-  return YTF_OK;
+  return check_waits(net);
 }
 
 int ytf_mlp_train(ytf_mlp* net, long n, const float* X, const float* T, int batch, int steps, float lr,
@@ -549,7 +741,7 @@ int ytf_mlp_train(ytf_mlp* net, long n, const float* X, const float* T, int batc
     k_gather<<<(unsigned)((cnt + 255) / 256), 256, 0, net->stream>>>(batch, d, n, seed, net->step, X, T, net->H[0],
                                                                       net->T);
     if (cudaGetLastError() != cudaSuccess) { cudaFree(dl); return mfail(net, YTF_ERR_CUDA, "gather launch"); }
-    if ((rc = forward(net, batch)) || (rc = backward(net, batch))) { cudaFree(dl); return rc; }
+    if ((rc = loss_and_gradients(net, batch))) { cudaFree(dl); return rc; }
     net->step += 1;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - std::pow(b1, (float)net->step), c2 = 1.f - std::pow(b2, (float)net->step);
@@ -566,7 +758,7 @@ int ytf_mlp_train(ytf_mlp* net, long n, const float* X, const float* T, int batc
   }
   cudaFree(dl);
   MCK(cudaStreamSynchronize(net->stream));
-  return YTF_OK;
+  return check_waits(net);
 }
 
 }  // extern "C"
