@@ -1,0 +1,64 @@
+"""1D synthesis at the edges of its tiles (32- and 128-row, 32- and 64-column FP64 tiles, k slices of
+16 and 64 nodes, the four-lane slice sums from 8 slices on) and at ragged pixel sets, against the
+FP64 oracle: FP64 to 1e-10 and int8x3 to 1e-6 relative, as the parity tests hold them."""
+import numpy as np
+import pytest
+
+from helpers import config1_like_stack, relerr
+
+pytestmark = pytest.mark.gpu
+
+W = 2 * np.pi
+
+
+def _rule(n, kmax=6 * W):
+    x, w = np.polynomial.legendre.leggauss(min(n, 8))
+    panels = max(1, n // 8)
+    e = np.linspace(0.0, kmax, panels + 1)
+    h = 0.5 * np.diff(e)
+    k = (0.5 * (e[1:] + e[:-1])[:, None] + h[:, None] * x).ravel()
+    wt = (h[:, None] * w).ravel()
+    return np.append(k, [])[:n], np.append(wt, [])[:n]
+
+
+def _case(n, nr, nz, even):
+    k, w = _rule(n)
+    rng = np.random.default_rng(n + nr + nz)
+    z = np.linspace(0.02, 0.31, nz) if even else np.sort(rng.uniform(0.02, 0.31, nz))
+    return k, w, np.geomspace(0.01, 3.0, nr), z
+
+
+@pytest.mark.parametrize("n,nr,nz,even", [(1, 1, 1, True), (7, 33, 3, False), (17, 31, 17, True), (65, 129, 2, False),
+                                          (264, 8, 4, True), (4104, 251, 61, True), (8200, 129, 33, False)])
+@pytest.mark.parametrize("terms", ["all", "scattered"])
+def test_1d_synthesis_shapes(oracle, n, nr, nz, even, terms):
+    from yellowthinfilms_b200 import api
+    st = config1_like_stack()
+    k, w, rho, z = _case(n, nr, nz, even)
+    gc = api.build_cavity_transfer_1d(st, W, 1, k, w, obs_layers=[1, 2])
+    oc = oracle.build_cavity_transfer_1d(st, W, 1, k, w, obs_layers=[1, 2])
+    Go = oracle.closed_form_G(oc, 1, 0.03, z, rho, [0.0], terms=terms)
+    assert relerr(api.closed_form_G(gc, 1, 0.03, z, rho, [0.0], terms=terms), Go) < 1e-10
+    assert relerr(api.closed_form_G(gc, 1, 0.03, z, rho, [0.0], terms=terms, precision="int8x3"), Go) < 1e-6
+    if terms == "all":  # another layer's field, a pixel patch off the axis
+        x, y = np.linspace(-0.4, 0.5, 5), np.linspace(-0.3, 0.2, 3)
+        G2 = oracle.closed_form_G(oc, 2, 0.03, z / 4, x, y)
+        assert relerr(api.closed_form_G(gc, 2, 0.03, z / 4, x, y), G2) < 1e-10
+        G8 = api.closed_form_G_batch([(gc, 2, 0.03, z / 4, x, y)], precision="int8x3")[0]
+        assert relerr(G8, G2) < 1e-6
+
+
+def test_1d_general_columns_without_the_symmetry_check(oracle):
+    """A gyrotropic stack on a 1D rule (check_symmetry=False): every coefficient column in use."""
+    from helpers import FOUNDATION_STACKS
+    from yellowthinfilms_b200 import api
+    st = FOUNDATION_STACKS[4][1]  # gyrotropic: x and y sources couple
+    k, w, rho, z = _case(264, 33, 5, True)
+    gc = api.build_cavity_transfer_1d(st, W, 1, k, w, obs_layers=[1], check_symmetry=False)
+    oc = oracle.build_cavity_transfer_1d(st, W, 1, k, w, obs_layers=[1])
+    Go = oracle.closed_form_G(oc, 1, 0.03, z, rho, [0.1], terms="scattered")
+    assert np.abs(Go[..., 1, 0]).max() > 1e-6 * np.abs(Go).max()
+    assert relerr(api.closed_form_G(gc, 1, 0.03, z, rho, [0.1], terms="scattered"), Go) < 1e-10
+    assert relerr(api.closed_form_G(gc, 1, 0.03, z, rho, [0.1], terms="scattered", precision="int8x3"), Go) < 1e-6
+    G8 = api.closed_form_G_batch([(gc, 1, 0.03, z, rho, [0.1])] * 2, precision="int8x3")
+    assert relerr(G8[1], oracle.closed_form_G(oc, 1, 0.03, z, rho, [0.1])) < 1e-6

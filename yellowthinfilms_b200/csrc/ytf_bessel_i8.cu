@@ -58,17 +58,6 @@ __device__ __forceinline__ double j2_from(double x, double J0, double J1) {
   return (2.0 / x) * J1 - J0;
 }
 
-// J_0, J_1 (j01_real below: the CUDA math library under x = 25, the asymptotic pair above),
-// J_2 from them
-__device__ __forceinline__ void j01_real(double x, double& J0, double& J1);
-__device__ __forceinline__ double bessel_j012(int order, double x) {
-  double J0, J1;
-  j01_real(x, J0, J1);
-  if (order == 0) return J0;
-  if (order == 1) return J1;
-  return j2_from(x, J0, J1);
-}
-
 // J_0(x) and J_1(x) for x >= 25 (absolute error below 1e-12): Hankel's asymptotic expansions
 // (A&S 9.2.5, 9.2.9, 9.2.10), J_n(x) = sqrt(2 / (π x)) (P_n cos χ_n - Q_n sin χ_n) with
 // χ_n = x - (2n + 1) π / 4, five terms each of P_n and Q_n in y = 1/x (the coefficient of y^m
@@ -177,69 +166,9 @@ __device__ __forceinline__ double col_scale(unsigned long long bits) {
   return (m > 0.0 && isfinite(m)) ? BI_SCALE / m : 0.0;
 }
 
-// per (slice, column) max |C| as IEEE bits (Inf for a non-finite entry); 256 threads, every
-// thread of the block calls it
-__device__ __forceinline__ void bcolmax_body(const BesselI8& p, int col, int z) {
-  const long k0 = (long)z * p.kchunk, k1 = min(p.K, k0 + p.kchunk);
-  const float* c = p.C + (long)col * p.K;
-  double m = 0.0;
-  for (long k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
-    const double v = c[k];
-    m = isfinite(v) ? fmax(m, fabs(v)) : __longlong_as_double(0x7ff0000000000000LL);
-  }
-  __shared__ double red[256];
-  red[threadIdx.x] = m;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + w]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) p.colmax[(long)z * p.N + col] = (unsigned long long)__double_as_longlong(red[0]);
-}
-__global__ void __launch_bounds__(256) k_bcolmax(BesselI8 p) { bcolmax_body(p, blockIdx.x, blockIdx.y); }
-
-// one thread per (column tile, row slot, slice, 16-node group): 16 bytes of each digit plane
-// one thread per 4 consecutive nodes of a column slot (one 32-bit word of each digit plane):
-// adjacent threads read adjacent 32-byte runs of C
-__device__ __forceinline__ void bimg_real_body(const BesselI8& p, long t) {
-  const long words = p.kchunk / 4;
-  const long total = (long)p.ntile_n * p.Np * p.nchunk * words;
-  if (t >= total) return;
-  const long wq = t % words;
-  long rest = t / words;
-  const int z = (int)(rest % p.nchunk);
-  rest /= p.nchunk;
-  const int slot = (int)(rest % p.Np);
-  const int ct = (int)(rest / p.Np);
-  const int col = ct * p.ctile + slot;
-  const bool cv = slot < p.ctile && col < p.N;
-  const double sB = cv ? col_scale(p.colmax[(long)z * p.N + col]) : 0.0;
-  const long g = wq / 4;
-  const int q = (int)(wq % 4);
-  uint32_t b[3][4];
-#pragma unroll
-  for (int h = 0; h < 4; ++h) {
-    const long k = (long)z * p.kchunk + 16 * g + 4 * q + h;
-    const double v = (cv && k < p.K) ? (double)p.C[(long)col * p.K + k] : 0.0;
-    uint32_t d0, d1, d2;
-    digits3b(__double2int_rn(v * sB), d0, d1, d2);
-    b[0][h] = d0; b[1][h] = d1; b[2][h] = d2;
-  }
-  const long nstage = p.kchunk / BI_NODES;
-  const int s = (int)(g / 4), kb = (int)(g % 4) * 16;
-  const size_t sbytes = 3ul * (size_t)p.Np * 64;
-  uint8_t* blk = p.Bimg + (((size_t)ct * p.nchunk + z) * nstage + s) * sbytes;
-#pragma unroll
-  for (int pl = 0; pl < 3; ++pl)
-    *reinterpret_cast<uint32_t*>(blk + (size_t)pl * p.Np * 64 + plane_off(slot, kb) + 4 * q) =
-        b[pl][0] | (b[pl][1] << 8) | (b[pl][2] << 16) | (b[pl][3] << 24);
-}
-__global__ void k_bimg_real(BesselI8 p) { bimg_real_body(p, (long)blockIdx.x * blockDim.x + threadIdx.x); }
-
-// the same digit images with the (slice, column) maxima taken in the same kernel: one block of
-// 256 threads per (column tile, 8-slot row group, node slice). Thread (j, r8) = (tid >> 3,
+// the coefficient digit images and their (slice, column) maxima: one block of 256 threads per (column tile, 8-slot row group, node slice). Thread (j, r8) = (tid >> 3,
 // tid & 7) takes column slot 8 rg + r8 and the slice's 16-node groups j, j + 32, ...: a first
-// pass reduces max |C| (IEEE bits into colmax, as k_bcolmax: a non-finite entry counts as Inf),
+// pass reduces max |C| (IEEE bits into colmax: a non-finite entry counts as Inf),
 // a second pass reads the same bytes again (from L2) and writes the digits. Each thread reads
 // 64 consecutive bytes of its column per group; a warp (four groups x eight slots) writes each
 // digit plane's 512-byte block of a stage whole. Blocks: ntile_n x (Np / 8) x nchunk.
@@ -319,49 +248,8 @@ __device__ __forceinline__ void bimg_slice_body(const BesselI8& p, long b) {
   }
 }
 
-// one thread per (radius tile, row, slice, 16-node group): J_n(k ρ) straight into digits
-__global__ void k_aimg_bessel(BesselI8 p) {
-  const long groups = p.kchunk / 16;
-  long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long total = (long)p.ntile_m * BI_M * p.nchunk * groups;
-  if (t >= total) return;
-  const long g = t % groups;
-  long rest = t / groups;
-  const int z = (int)(rest % p.nchunk);
-  rest /= p.nchunk;
-  const int row = (int)(rest % BI_M);
-  const int mt = (int)(rest / BI_M);
-  const int r = mt * BI_M + row;
-  const bool rv = r < p.M;
-  const double rho = rv ? p.rho[r] : 0.0;
-  const double sA = BI_SCALE / j_env(p.kmin[z] * rho);
-  uint32_t w[3][4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    uint32_t b[3][4];
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      const long k = (long)z * p.kchunk + 16 * g + 4 * q + h;
-      const double v = (rv && k < p.K) ? bessel_j012(p.order, p.kr[k] * rho) : 0.0;
-      uint32_t d0, d1, d2;
-      digits3b(__double2int_rn(v * sA), d0, d1, d2);
-      b[0][h] = d0; b[1][h] = d1; b[2][h] = d2;
-    }
-#pragma unroll
-    for (int pl = 0; pl < 3; ++pl) w[pl][q] = b[pl][0] | (b[pl][1] << 8) | (b[pl][2] << 16) | (b[pl][3] << 24);
-  }
-  const long nstage = p.kchunk / BI_NODES;
-  const int s = (int)(g / 4), kb = (int)(g % 4) * 16;
-  const size_t sbytes = 3ul * BI_M * 64;
-  uint8_t* blk = p.Aimg + (((size_t)mt * p.nchunk + z) * nstage + s) * sbytes;
-#pragma unroll
-  for (int pl = 0; pl < 3; ++pl)
-    *reinterpret_cast<uint4*>(blk + (size_t)pl * BI_M * 64 + plane_off(row, kb)) =
-        make_uint4(w[pl][0], w[pl][1], w[pl][2], w[pl][3]);
-}
-
-// k_aimg_bessel for all three orders at once: J_0 and J_1 once per (ρ, k), J_2 from them
-// (series below |x| = 1, recurrence above, as bessel_j012), three images in the same layout.
+// the J_n(k ρ) digit images of all three orders: J_0 and J_1 once per (ρ, k), J_2 from them (series
+// below |x| = 1, recurrence above), three images in the same layout.
 // One thread per 4 consecutive nodes of a radius (one 32-bit word of each digit plane): the
 // FP64 Bessel chains are latency-bound, so short chains and many threads.
 __device__ __forceinline__ void aimg_bessel3_body(const BesselI8& p, long t, uint8_t* __restrict__ A0,
@@ -572,27 +460,26 @@ __device__ __forceinline__ void gemm_i8_img_body(const BesselI8& p, int mt, int 
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BI_TMEM_COLS) : "memory");
   }
 }
-__global__ void __launch_bounds__(BI_THREADS, 1) k_gemm_i8_img(BesselI8 p) {
+// up to six entries by value; entry i's blocks start at first[i]
+struct BesselI8Set {
+  int n;
+  long first[6];
+  BesselI8 e[6];
+};
+__global__ void __launch_bounds__(BI_THREADS, 1) k_gemm_i8_img(const __grid_constant__ BesselI8Set set) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  gemm_i8_img_body(p, blockIdx.x, blockIdx.y, blockIdx.z, smem);
+  int i = 0;
+  while (i + 1 < set.n && set.first[i + 1] <= (long)blockIdx.x) ++i;
+  const BesselI8& p = set.e[i];
+  const long b = blockIdx.x - set.first[i];
+  const int mt = (int)(b % p.ntile_m);
+  const long rest = b / p.ntile_m;
+  gemm_i8_img_body(p, mt, (int)(rest % p.ntile_n), (int)(rest / p.ntile_n), smem);
 }
-
-// P[r][c] = Σ_z partial[z][c][r] through a 32 x 32 shared-memory transpose
-__global__ void k_reduce_transpose(int M, int N, int nz, const double* __restrict__ part, double* __restrict__ P) {
-  __shared__ double tile[32][33];
-  const int r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
-  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-    const int c = c0 + j, r = r0 + threadIdx.x;
-    double s = 0.0;
-    if (c < N && r < M)
-      for (int z = 0; z < nz; ++z) s += part[((long)z * N + c) * M + r];
-    tile[j][threadIdx.x] = s;
-  }
-  __syncthreads();
-  for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-    const int r = r0 + j, c = c0 + threadIdx.x;
-    if (r < M && c < N) P[(long)r * N + c] = tile[threadIdx.x][j];
-  }
+__global__ void __launch_bounds__(256) k_bimg_real(const __grid_constant__ BesselI8Set set) {
+  int i = 0;
+  while (i + 1 < set.n && set.first[i + 1] <= (long)blockIdx.x) ++i;
+  bimg_slice_body(set.e[i], blockIdx.x - set.first[i]);
 }
 
 // per (order, slice, radius): max(|Re J|, |Im J|) over the slice's nodes (1 where it is 0)
@@ -673,31 +560,43 @@ cudaError_t launch_jtable_images(const BesselI8& bp, const double* Jtab, double*
   return cudaGetLastError();
 }
 
-cudaError_t launch_bessel_i8(const BesselI8& p, double* P, cudaStream_t s) {
-  if (p.M <= 0 || p.N <= 0 || p.K <= 0) return cudaSuccess;
-  if ((!p.kmin && !p.rowscale) || p.kchunk % BI_NODES != 0 || p.kchunk > 16384 || p.Np % 16 != 0 || p.Np > BI_ACC_STRIDE || p.Np < p.ctile ||
-      (long)p.nchunk * p.kchunk < p.K)
-    return cudaErrorInvalidValue;
-  cudaError_t e;
-  k_bcolmax<<<dim3((unsigned)p.N, (unsigned)p.nchunk), 256, 0, s>>>(p);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  {
-    const long total = (long)p.ntile_n * p.Np * p.nchunk * (p.kchunk / 4);
-    k_bimg_real<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(p);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+static bool entry_ok(const BesselI8& p) {
+  return (p.kmin || p.rowscale) && p.kchunk % BI_NODES == 0 && p.kchunk <= 16384 && p.Np % 16 == 0 &&
+         p.Np <= BI_ACC_STRIDE && p.Np >= p.ctile && (long)p.nchunk * p.kchunk >= p.K && p.ldc % 4 == 0;
+}
+
+cudaError_t launch_bimg(const BesselI8* e, int n, cudaStream_t s) {
+  BesselI8Set set;
+  set.n = n;
+  long blocks = 0;
+  for (int i = 0; i < n; ++i) {
+    if (!entry_ok(e[i])) return cudaErrorInvalidValue;
+    set.e[i] = e[i];
+    set.first[i] = blocks;
+    blocks += (long)e[i].ntile_n * (e[i].Np / 8) * e[i].nchunk;
   }
-  if (!p.aimg_ready) {
-    const long total = (long)p.ntile_m * BI_M * p.nchunk * (p.kchunk / 16);
-    k_aimg_bessel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(p);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if (blocks <= 0) return cudaSuccess;
+  k_bimg_real<<<(unsigned)blocks, 256, 0, s>>>(set);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_gemm_i8(const BesselI8* e, int n, cudaStream_t s) {
+  BesselI8Set set;
+  set.n = n;
+  long blocks = 0;
+  int Np = 0;
+  for (int i = 0; i < n; ++i) {
+    if (!entry_ok(e[i])) return cudaErrorInvalidValue;
+    set.e[i] = e[i];
+    set.first[i] = blocks;
+    blocks += (long)e[i].ntile_m * e[i].ntile_n * e[i].nchunk;
+    Np = e[i].Np > Np ? e[i].Np : Np;
   }
-  const size_t sm = bessel_i8_smem(p.Np);
-  if ((e = cudaFuncSetAttribute(k_gemm_i8_img, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)) != cudaSuccess)
-    return e;
-  k_gemm_i8_img<<<dim3((unsigned)p.ntile_m, (unsigned)p.ntile_n, (unsigned)p.nchunk), BI_THREADS, sm, s>>>(p);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  k_reduce_transpose<<<dim3((unsigned)((p.M + 31) / 32), (unsigned)((p.N + 31) / 32)), dim3(32, 8), 0, s>>>(
-      p.M, p.N, p.nchunk, p.partial, P);
+  if (blocks <= 0) return cudaSuccess;
+  const size_t sm = bessel_i8_smem(Np);
+  cudaError_t err = cudaFuncSetAttribute(k_gemm_i8_img, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (err != cudaSuccess) return err;
+  k_gemm_i8_img<<<(unsigned)blocks, BI_THREADS, sm, s>>>(set);
   return cudaGetLastError();
 }
 

@@ -1564,202 +1564,147 @@ static int synth_setup(ytf_ctx* ctx, const ytf_cache* c, int obs_layer, double z
   return YTF_OK;
 }
 
-// P_n (n = 0, 1, 2; 26 nz real columns x nr radii) of the 1D synthesis over the nodes of sp.c:
-// the per-node coefficient columns (k_coef1d) and the three order contractions -- complex J_n
-// with FP64 GEMMs on a deformed contour, the int8x3 tensor-core pipeline, or FP64 GEMMs
-static int synth1d_P(ytf_ctx* ctx, const SynthParams& sp, int nz, int nr, const double* drho, int precision, int nsm,
-                     const GreenBatch* gb, double* P0, double* P1, double* P2) {
-  const long nk = sp.c.n;
-  WS(amp1, double2, "g_amp", (size_t)12 * nk);
-  const bool i8 = precision == YTF_PREC_INT8X3;
-  // FP64 coefficient columns for the FP64 contractions, FP32 ones for the int8x3 digits
-  double *C0 = nullptr, *C1 = nullptr, *C2 = nullptr;
-  float *F0 = nullptr, *F1 = nullptr, *F2 = nullptr;
-  if (i8) {
-    WS(Cf, float, "g_Cf", (size_t)C1D_RT * nz * nk);
-    F0 = Cf; F1 = Cf + (size_t)C1D_OFF1 * nz * nk; F2 = Cf + (size_t)C1D_OFF2 * nz * nk;
-    CK(LAUNCH("k_coef1d", launch_coef1d_amp(sp, amp1, F0, F1, F2, ctx->stream)));
-  } else {
-    WS(C, double, "g_C", (size_t)C1D_RT * nz * nk);
-    C0 = C; C1 = C + (size_t)C1D_OFF1 * nz * nk; C2 = C + (size_t)C1D_OFF2 * nz * nk;
-    CK(LAUNCH("k_coef1d", launch_coef1d_amp(sp, amp1, C0, C1, C2, ctx->stream)));
+// the slice partials of a 1D synthesis, per order: part[o] [nchunk][N_o][nr], and on a deformed contour
+// the Im J contraction's part_im[o]
+struct Parts1D {
+  int N[3];
+  int nchunk;
+  double* part[3];
+  double* part_im[3];
+};
+
+// the order contractions of the 1D synthesis over the nodes of sp.c: the per-node coefficient columns
+// (k_coef1d), the Bessel tables or digit images, and one launch for every contraction (two per
+// order, Re J and Im J, on a deformed contour), in FP64 or on the int8 tensor cores
+static int synth1d_parts(ytf_ctx* ctx, const SynthParams& sp, int nz, int nr, const double* drho, int precision, int nsm,
+                         const GreenBatch* gb, Parts1D& out) {
+  const long nk = sp.c.n, ld = (nk + 3) / 4 * 4;  // rows on 16 bytes
+  const bool i8 = precision == YTF_PREC_INT8X3, cplx = sp.c.kri != nullptr;
+  const int np = cplx ? 2 : 1;
+  std::memset(&out, 0, sizeof(out));
+  const int R[3] = {C1D_R0, C1D_R1, C1D_R2};
+  size_t coff[3], ncol = 0;
+  for (int o = 0; o < 3; ++o) {
+    out.N[o] = R[o] * nz;
+    coff[o] = ncol * ld;
+    ncol += out.N[o];
   }
-    if (sp.c.kri && i8) {
-      // nodes on a deformed contour, int8 tensor cores: the complex J_n(kρ ρ) tables (FP64),
-      // their real and imaginary parts as digit images fixed point per (order, slice, radius)
-      // relative to the slice's largest part, two int8x3 contractions per order against the
-      // FP32 coefficient columns (Re J and Im J), then the complex combine as the FP64 path
-      const float* Cn8[3] = {F0, F1, F2};
-      double* Pn8[3] = {P0, P1, P2};
-      const int Nn8[3] = {C1D_R0 * nz, C1D_R1 * nz, C1D_R2 * nz};
-      unsigned* err = gb ? gb->err : nullptr;
-      if (!err) {
-        WS(e1, unsigned, "g_tc_err", 1);
-        err = e1;
-        CK(cudaMemsetAsync(err, 0, sizeof(unsigned), ctx->stream));
-      }
-      WS(Jc, double, "g_Jc", 6 * (size_t)nr * nk);
-      CK(LAUNCH("k_bessel_c", launch_bessel_c(sp.c.kr, sp.c.kri, nk, drho, nr, Jc, ctx->stream)));
-      long kchunk;
-      {
-        const int ct0 = bessel_i8_ctile(Nn8[0]);
-        const long tiles = (long)((nr + 127) / 128) * ((Nn8[0] + ct0 - 1) / ct0);
-        const long want = std::max(1L, (long)nsm / tiles);
-        kchunk = (nk + want - 1) / want;
-        kchunk = std::min(16384L, std::max(64L, ((kchunk + 63) / 64) * 64));
-      }
-      const int nchunk = (int)((nk + kchunk - 1) / kchunk);
-      const size_t nst = (size_t)(kchunk / 64);
-      const size_t abytes = (size_t)((nr + 127) / 128) * nchunk * nst * bessel_i8_stage_bytes_a();
-      WS(Ai, uint8_t, "g_bic_a", 6 * abytes);
-      WS(rs, double, "g_bic_rs", 3 * (size_t)nchunk * nr);
-      uint8_t* imgs[6];
-      for (int i = 0; i < 6; ++i) imgs[i] = Ai + i * abytes;
-      BesselI8 lay;
-      std::memset(&lay, 0, sizeof(lay));
-      lay.M = nr; lay.K = nk; lay.ntile_m = (nr + 127) / 128; lay.kchunk = kchunk; lay.nchunk = nchunk;
-      CK(LAUNCH("k_bessel_i8", launch_jtable_images(lay, Jc, rs, imgs, ctx->stream)));
-      const size_t pab = (size_t)nr * C1D_RMAX * nz;
-      WS(Pab, double, "g_Pab", 2 * pab);
+  auto carve = [&](double* part, size_t nchunk) {
+    size_t off = 0;
+    for (int q = 0; q < np; ++q)
       for (int o = 0; o < 3; ++o) {
-        BesselI8 bp;
-        std::memset(&bp, 0, sizeof(bp));
-        bp.M = nr; bp.N = Nn8[o]; bp.K = nk; bp.order = o;
-        bp.ctile = bessel_i8_ctile(bp.N);
-        bp.Np = ((bp.ctile + 15) / 16) * 16;
-        bp.ntile_n = (bp.N + bp.ctile - 1) / bp.ctile;
-        bp.ntile_m = (nr + 127) / 128;
-        bp.kchunk = kchunk;
-        bp.nchunk = nchunk;
-        WS(Bi, uint8_t, "g_bi_b", (size_t)bp.ntile_n * bp.nchunk * nst * bessel_i8_stage_bytes_b(bp.Np));
-        WS(cm, unsigned long long, "g_bi_cmax", (size_t)bp.nchunk * bp.N);
-        WS(pt, double, "g_bi_part", (size_t)bp.nchunk * bp.N * nr);
-        bp.kr = sp.c.kr; bp.rho = drho; bp.C = Cn8[o]; bp.ldc = nk;
-        bp.Bimg = Bi; bp.colmax = cm; bp.partial = pt; bp.err = err;
-        bp.wait_limit = ctx->wait_limit;
-        bp.aimg_ready = 1;
-        bp.rowscale = rs + (size_t)o * nchunk * nr;
-        for (int part = 0; part < 2; ++part) {
-          bp.Aimg = imgs[2 * o + part];
-          CK(LAUNCH("k_bessel_i8", launch_bessel_i8(bp, Pab + (size_t)part * pab, ctx->stream)));
-        }
-        CK(LAUNCH("k_combine_complex", launch_combine_complex(nr, Nn8[o], Pab, Pab + pab, Pn8[o], ctx->stream)));
+        (q ? out.part_im : out.part)[o] = part + off;
+        off += nchunk * out.N[o] * nr;
       }
-      if (!gb) {
-        unsigned herr = 0;
-        CK(cudaMemcpyAsync(&herr, err, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        if (herr) return fail(ctx, YTF_ERR_CUDA, "closed_form_G: a tensor-core pipeline wait timed out");
-      }
-      return YTF_OK;
-    }
-    if (sp.c.kri) {
-      // nodes on a deformed contour: complex J_n(kρ ρ) tables, two FP64 GEMMs per order
-      // (Re J and Im J against the real/imaginary coefficient columns), then the complex combine
-      WS(Jc, double, "g_Jc", 6 * (size_t)nr * nk);
-      CK(LAUNCH("k_bessel_c", launch_bessel_c(sp.c.kr, sp.c.kri, nk, drho, nr, Jc, ctx->stream)));
-      const double* Cn[3] = {C0, C1, C2};
-      double* Pn[3] = {P0, P1, P2};
-      const int Nn[3] = {C1D_R0 * nz, C1D_R1 * nz, C1D_R2 * nz};
-      const size_t pab = (size_t)nr * C1D_RMAX * nz;
-      WS(Pab, double, "g_Pab", 2 * pab);
+  };
+  WS(amp1, double2, "g_amp", (size_t)12 * nk);
+  if (!i8) {
+    WS(C, double, "g_C", ncol * ld);
+    CK(LAUNCH("k_coef1d", launch_coef1d_amp(sp, amp1, C, ld, ctx->stream)));
+    const size_t plane = (size_t)nr * ld;
+    WS(J, double, "g_J", 3 * np * plane);
+    if (cplx) CK(LAUNCH("k_bessel_c", launch_bessel_c(sp.c.kr, sp.c.kri, nk, drho, nr, ld, J, ctx->stream)));
+    else CK(LAUNCH("k_bessel", launch_bessel(sp.c.kr, nk, drho, nr, ld, J, J + plane, J + 2 * plane, ctx->stream)));
+    Gemm64 g;
+    std::memset(&g, 0, sizeof(g));
+    g.M = nr; g.K = nk; g.lda = ld; g.ldb = ld;
+    for (int q = 0; q < np; ++q)
       for (int o = 0; o < 3; ++o) {
-        long tiles = (long)((nr + 127) / 128) * ((Nn[o] + 127) / 128);
-        long want = (2L * nsm + tiles - 1) / tiles;
-        int sp0 = dgemm_splits((int)nk, (int)std::max(1L, std::min(want, std::max(1L, nk / 256))));
-        WS(Pp, double, "g_partial", (size_t)sp0 * nr * Nn[o]);
-        for (int part = 0; part < 2; ++part) {
-          const double* Jp = Jc + (size_t)(2 * o + part) * nr * nk;
-          CK(LAUNCH("k_dgemm_nt", launch_dgemm_nt(nr, Nn[o], (int)nk, Jp, Cn[o], Pp, sp0, ctx->stream)));
-          CK(LAUNCH("k_reduce_splits", launch_reduce_splits((long)nr * Nn[o], sp0, Pp,
-                                                            Pab + (size_t)part * pab, ctx->stream)));
-        }
-        CK(LAUNCH("k_combine_complex", launch_combine_complex(nr, Nn[o], Pab, Pab + pab, Pn[o], ctx->stream)));
+        Gemm64Entry& e = g.e[g.n++];
+        e.A = J + (size_t)(np * o + q) * plane;
+        e.B = C + coff[o];
+        e.N = out.N[o];
       }
-      return YTF_OK;
-    }
-    if (i8) {
-      // int8 tensor cores: J_n(kρ) and the coefficient columns as fixed-point digit images,
-      // exact INT32 accumulation, FP64 sum of the node slices into P_n
-      const float* Cn8[3] = {F0, F1, F2};
-      double* Pn8[3] = {P0, P1, P2};
-      const int Nn8[3] = {C1D_R0 * nz, C1D_R1 * nz, C1D_R2 * nz};
-      unsigned* err = gb ? gb->err : nullptr;
-      if (!err) {
-        WS(e1, unsigned, "g_tc_err", 1);
-        err = e1;
-        CK(cudaMemsetAsync(err, 0, sizeof(unsigned), ctx->stream));
-      }
-      // one node slicing for the three orders (that of order 0, the widest), so the J_n
-      // digit images of all three come from one Bessel evaluation per (ρ, k)
-      long kchunk;
-      {
-        const int ct0 = bessel_i8_ctile(Nn8[0]);
-        const long tiles = (long)((nr + 127) / 128) * ((Nn8[0] + ct0 - 1) / ct0);
-        const long want = std::max(1L, (long)nsm / tiles);
-        kchunk = (nk + want - 1) / want;
-        kchunk = std::min(16384L, std::max(64L, ((kchunk + 63) / 64) * 64));
-      }
-      const int nchunk = (int)((nk + kchunk - 1) / kchunk);
-      const size_t nst = (size_t)(kchunk / 64);
-      const size_t abytes = (size_t)((nr + 127) / 128) * nchunk * nst * bessel_i8_stage_bytes_a();
-      WS(A0i, uint8_t, "g_bi_a0", abytes);
-      WS(A1i, uint8_t, "g_bi_a1", abytes);
-      WS(A2i, uint8_t, "g_bi_a2", abytes);
-      uint8_t* Aord[3] = {A0i, A1i, A2i};
-      WS(kminb, double, "g_bi_kmin", nchunk);
-      CK(LAUNCH("k_bessel_i8", launch_slice_kmin(sp.c.kr, nk, kchunk, nchunk, kminb, ctx->stream)));
-      for (int o = 0; o < 3; ++o) {
-        BesselI8 bp;
-        std::memset(&bp, 0, sizeof(bp));
-        bp.M = nr; bp.N = Nn8[o]; bp.K = nk; bp.order = o;
-        bp.ctile = bessel_i8_ctile(bp.N);
-        bp.Np = ((bp.ctile + 15) / 16) * 16;
-        bp.ntile_n = (bp.N + bp.ctile - 1) / bp.ctile;
-        bp.ntile_m = (nr + 127) / 128;
-        bp.kchunk = kchunk;
-        bp.nchunk = nchunk;
-        WS(Bi, uint8_t, "g_bi_b", (size_t)bp.ntile_n * bp.nchunk * nst * bessel_i8_stage_bytes_b(bp.Np));
-        WS(cm, unsigned long long, "g_bi_cmax", (size_t)bp.nchunk * bp.N);
-        WS(pt, double, "g_bi_part", (size_t)bp.nchunk * bp.N * nr);
-        bp.kr = sp.c.kr; bp.rho = drho; bp.C = Cn8[o]; bp.ldc = nk;
-        bp.Aimg = Aord[o]; bp.Bimg = Bi; bp.colmax = cm; bp.partial = pt; bp.err = err;
-        bp.wait_limit = ctx->wait_limit;
-        bp.kmin = kminb;
-        if (o == 0) CK(LAUNCH("k_bessel_i8", launch_bessel_i8_aimg3(bp, A0i, A1i, A2i, ctx->stream)));
-        bp.aimg_ready = 1;
-        CK(LAUNCH("k_bessel_i8", launch_bessel_i8(bp, Pn8[o], ctx->stream)));
-      }
-      if (!gb) {
-        unsigned herr = 0;
-        CK(cudaMemcpyAsync(&herr, err, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        if (herr) return fail(ctx, YTF_ERR_CUDA, "closed_form_G: a tensor-core pipeline wait timed out");
-      }
-      return YTF_OK;
-    }
-    WS(J, double, "g_J", 3 * (size_t)nr * nk);
-    double *J0 = J, *J1 = J + (size_t)nr * nk, *J2 = J + 2 * (size_t)nr * nk;
-    CK(LAUNCH("k_bessel", launch_bessel(sp.c.kr, nk, drho, nr, J0, J1, J2, ctx->stream)));
-    auto splits_for = [&](int M, int N) {
-      long tiles = (long)((M + 127) / 128) * ((N + 127) / 128);
-      long want = (2L * nsm + tiles - 1) / tiles;
-      long maxs = std::max(1L, nk / 256);
-      return (int)std::max(1L, std::min(want, maxs));
-    };
-    const int Nn[3] = {C1D_R0 * nz, C1D_R1 * nz, C1D_R2 * nz};
-    const int sps[3] = {splits_for(nr, Nn[0]), splits_for(nr, Nn[1]), splits_for(nr, Nn[2])};
-    size_t part = 0;
-    for (int o = 0; o < 3; ++o) part = std::max(part, (size_t)sps[o] * nr * Nn[o]);
-    WS(Pp, double, "g_partial", part);
-    const double* Jn[3] = {J0, J1, J2};
-    const double* Cn[3] = {C0, C1, C2};
-    double* Pn[3] = {P0, P1, P2};
+    out.nchunk = gemm64_plan(g);
+    WS(Pp, double, "g_partial", np * ncol * (size_t)out.nchunk * nr);
+    carve(Pp, out.nchunk);
+    for (int q = 0; q < np; ++q)
+      for (int o = 0; o < 3; ++o) g.e[3 * q + o].out = (q ? out.part_im : out.part)[o];
+    CK(LAUNCH("k_dgemm_nt", launch_gemm64(g, ctx->stream)));
+    return YTF_OK;
+  }
+  // int8 tensor cores: J_n and the coefficient columns as fixed-point digit images, exact INT32
+  // accumulation per node slice. Real nodes: J digits relative to an envelope, straight from the
+  // Bessel evaluation; a deformed contour: from the FP64 tables of complex J_n, relative to the
+  // slice's largest real or imaginary part.
+  unsigned* err = gb ? gb->err : nullptr;
+  if (!err) {
+    WS(e1, unsigned, "g_tc_err", 1);
+    err = e1;
+    CK(cudaMemsetAsync(err, 0, sizeof(unsigned), ctx->stream));
+  }
+  WS(Cf, float, "g_Cf", ncol * ld);
+  CK(LAUNCH("k_coef1d", launch_coef1d_amp(sp, amp1, Cf, ld, ctx->stream)));
+  // one node slicing for the three orders: its length sets the digits' scales, and follows the
+  // tiles of the widest order's general columns
+  long kchunk;
+  {
+    const int N0 = C1D_R0 * nz, ct0 = bessel_i8_ctile(N0);
+    const long tiles = (long)((nr + 127) / 128) * ((N0 + ct0 - 1) / ct0);
+    const long want = std::max(1L, (long)nsm / tiles);
+    kchunk = (nk + want - 1) / want;
+    kchunk = std::min(16384L, std::max(64L, ((kchunk + 63) / 64) * 64));
+  }
+  const int nchunk = (int)((nk + kchunk - 1) / kchunk);
+  const size_t nst = (size_t)(kchunk / 64);
+  const size_t abytes = (size_t)((nr + 127) / 128) * nchunk * nst * bessel_i8_stage_bytes_a();
+  WS(Ai, uint8_t, "g_bi_a", 3 * np * abytes);
+  out.nchunk = nchunk;
+  WS(Pp, double, "g_partial", np * ncol * (size_t)nchunk * nr);
+  carve(Pp, nchunk);
+  WS(cm, unsigned long long, "g_bi_cmax", ncol * (size_t)nchunk);
+  BesselI8 be[6];
+  std::memset(be, 0, sizeof(be));
+  size_t bbytes = 0, boff[3];
+  unsigned long long* cmo = cm;
+  for (int o = 0; o < 3; ++o) {
+    BesselI8& bp = be[o];
+    bp.M = nr; bp.N = out.N[o]; bp.K = nk; bp.order = o;
+    bp.ctile = bessel_i8_ctile(bp.N);
+    bp.Np = ((bp.ctile + 15) / 16) * 16;
+    bp.ntile_n = (bp.N + bp.ctile - 1) / bp.ctile;
+    bp.ntile_m = (nr + 127) / 128;
+    bp.kchunk = kchunk;
+    bp.nchunk = nchunk;
+    bp.kr = sp.c.kr; bp.rho = drho; bp.C = Cf + coff[o]; bp.ldc = ld;
+    bp.colmax = cmo;
+    cmo += (size_t)nchunk * bp.N;
+    bp.partial = out.part[o];
+    bp.Aimg = Ai + (size_t)np * o * abytes;
+    bp.err = err;
+    bp.wait_limit = ctx->wait_limit;
+    boff[o] = bbytes;
+    bbytes += (size_t)bp.ntile_n * nchunk * nst * bessel_i8_stage_bytes_b(bp.Np);
+  }
+  WS(Bi, uint8_t, "g_bi_b", bbytes);
+  for (int o = 0; o < 3; ++o) be[o].Bimg = Bi + boff[o];
+  if (cplx) {
+    WS(Jc, double, "g_J", 6 * (size_t)nr * nk);
+    CK(LAUNCH("k_bessel_c", launch_bessel_c(sp.c.kr, sp.c.kri, nk, drho, nr, nk, Jc, ctx->stream)));
+    WS(rs, double, "g_bic_rs", 3 * (size_t)nchunk * nr);
+    uint8_t* imgs[6];
+    for (int i = 0; i < 6; ++i) imgs[i] = Ai + i * abytes;
+    CK(LAUNCH("k_bessel_i8", launch_jtable_images(be[0], Jc, rs, imgs, ctx->stream)));
     for (int o = 0; o < 3; ++o) {
-      int sp_ = dgemm_splits((int)nk, sps[o]);
-      CK(LAUNCH("k_dgemm_nt", launch_dgemm_nt(nr, Nn[o], (int)nk, Jn[o], Cn[o], Pp, sp_, ctx->stream)));
-      CK(LAUNCH("k_reduce_splits", launch_reduce_splits((long)nr * Nn[o], sp_, Pp, Pn[o], ctx->stream)));
+      be[o].rowscale = rs + (size_t)o * nchunk * nr;
+      be[3 + o] = be[o];
+      be[3 + o].Aimg = imgs[2 * o + 1];
+      be[3 + o].partial = out.part_im[o];
     }
+  } else {
+    WS(kminb, double, "g_bi_kmin", nchunk);
+    for (int o = 0; o < 3; ++o) be[o].kmin = kminb;
+    CK(LAUNCH("k_bessel_i8", launch_slice_kmin(sp.c.kr, nk, kchunk, nchunk, kminb, ctx->stream)));
+    CK(LAUNCH("k_bessel_i8", launch_bessel_i8_aimg3(be[0], be[0].Aimg, be[1].Aimg, be[2].Aimg, ctx->stream)));
+  }
+  CK(LAUNCH("k_bessel_i8", launch_bimg(be, 3, ctx->stream)));
+  CK(LAUNCH("k_bessel_i8", launch_gemm_i8(be, 3 * np, ctx->stream)));
+  if (!gb) {
+    unsigned herr = 0;
+    CK(cudaMemcpyAsync(&herr, err, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (herr) return fail(ctx, YTF_ERR_CUDA, "closed_form_G: a tensor-core pipeline wait timed out");
+  }
   return YTF_OK;
 }
 
@@ -1857,31 +1802,40 @@ static int green_impl(ytf_ctx* ctx, const ytf_cache* c, int obs_layer, double zs
       drho = urho;
       drmap = urmap;
     }
-    WS(P, double, "g_P", (size_t)C1D_RT * nz * nr);
-    double *P0 = P, *P1 = P + (size_t)C1D_OFF1 * nz * nr, *P2 = P + (size_t)C1D_OFF2 * nz * nr;
+    Asm1D as;
+    std::memset(&as, 0, sizeof(as));
+    as.nx = nx; as.ny = ny; as.nz = nz; as.nr = nr;
+    as.xs = dxs; as.ys = dys; as.rmap = drmap; as.G = G;
+    Parts1D pt;
     if (nk <= SYNTH1D_NODE_CHUNK) {
-      if ((rc = synth1d_P(ctx, sp, nz, nr, drho, precision, nsm, gb, P0, P1, P2))) return rc;
+      if ((rc = synth1d_parts(ctx, sp, nz, nr, drho, precision, nsm, gb, pt))) return rc;
+      as.nchunk = pt.nchunk;
+      for (int o = 0; o < 3; ++o) { as.part[o] = pt.part[o]; as.part_im[o] = pt.part_im[o]; }
     } else {
       // G is linear in the node sum: the rule in passes of at most SYNTH1D_NODE_CHUNK nodes,
-      // their P_n summed (the reference sums closed_form_G over node chunks the same way,
+      // their order sums added (the reference sums closed_form_G over node chunks the same way,
       // chunked_2d, mod_ClosedFormGrid.jl:449-467)
       const size_t np = (size_t)C1D_RT * nz * nr;
-      WS(Pacc, double, "g_Pacc", np);
-      WS(Pc, double, "g_Pchunk", np);
+      const int nq = sp.c.kri ? 2 : 1;
+      WS(Pacc, double, "g_Pacc", nq * np);
       WS(cbuf, double2, "g_chunk_cache", (size_t)48 * SYNTH1D_NODE_CHUNK);
-      CK(cudaMemsetAsync(Pacc, 0, sizeof(double) * np, ctx->stream));
       for (long b0 = 0; b0 < nk; b0 += SYNTH1D_NODE_CHUNK) {
         const long nb = std::min(SYNTH1D_NODE_CHUNK, nk - b0);
         SynthParams spc = sp;
         if ((rc = node_chunk_view(ctx, sp.c, b0, nb, cbuf, spc.c))) return rc;
-        if ((rc = synth1d_P(ctx, spc, nz, nr, drho, precision, nsm, gb, Pc, Pc + (size_t)C1D_OFF1 * nz * nr,
-                            Pc + (size_t)C1D_OFF2 * nz * nr)))
-          return rc;
-        CK(LAUNCH("k_add", launch_add(np, Pc, Pacc, ctx->stream)));
+        if ((rc = synth1d_parts(ctx, spc, nz, nr, drho, precision, nsm, gb, pt))) return rc;
+        size_t off = 0;
+        for (int q = 0; q < nq; ++q)
+          for (int o = 0; o < 3; ++o) {
+            CK(LAUNCH("k_sum_slices", launch_sum_slices((long)pt.N[o] * nr, pt.nchunk, (q ? pt.part_im : pt.part)[o],
+                                                        Pacc + off, b0 > 0, ctx->stream)));
+            (q ? as.part_im : as.part)[o] = Pacc + off;
+            off += (size_t)pt.N[o] * nr;
+          }
       }
-      CK(cudaMemcpyAsync(P, Pacc, sizeof(double) * np, cudaMemcpyDeviceToDevice, ctx->stream));
+      as.nchunk = 1;
     }
-    CK(LAUNCH("k_assemble1d", launch_assemble1d(nx, ny, nz, dxs, dys, drmap, nr, P0, P1, P2, G, ctx->stream)));
+    CK(LAUNCH("k_assemble1d", launch_assemble1d(as, ctx->stream)));
   } else {
     int ncol = 9 * nz;
     WS(S, double2, "g_S", (size_t)ncol * c->n);
@@ -2239,12 +2193,12 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
       it.amp = (double2*)(base + L.off_amp);
       it.C = (float*)(base + L.off_C);
       it.ldc = L.ldc;
-      it.nx = d[i].nx; it.ny = d[i].ny; it.nr = L.nr;
-      it.xs = dc + o[i] + d[i].nz;
-      it.ys = dc + o[i] + d[i].nz + d[i].nx;
-      it.rmap = dm + omap[i];
-      it.G = d[i].out_is_device ? (double2*)d[i].out : (double2*)(base + L.off_G);
-      it.nchunk = L.nchunk;
+      it.a.nx = d[i].nx; it.a.ny = d[i].ny; it.a.nz = L.nz; it.a.nr = L.nr;
+      it.a.xs = dc + o[i] + d[i].nz;
+      it.a.ys = dc + o[i] + d[i].nz + d[i].nx;
+      it.a.rmap = dm + omap[i];
+      it.a.G = d[i].out_is_device ? (double2*)d[i].out : (double2*)(base + L.off_G);
+      it.a.nchunk = L.nchunk;
       it.kchunk = L.kchunk;
       {  // evenly spaced heights (to 4 ulp of the progression): rows by recurrence
         const double* zv = d[i].z_obs;
@@ -2255,12 +2209,12 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
         for (int r = 0; r < m && even; ++r) even = std::fabs(zv[r] - (zv[0] + r * dz)) <= tol;
         it.dz = even ? dz : 0.0;
       }
-      for (int od = 0; od < 3; ++od) it.part[od] = (const double*)(base + L.off_pt[od]);
+      for (int od = 0; od < 3; ++od) it.a.part[od] = (const double*)(base + L.off_pt[od]);
       const long nkb = (L.nk + 127) / 128;
       f_ref[q] = nref; nref += nkb;
       f_coef[q] = ncoef; ncoef += nkb * ((L.nz + COEF1D_ZB_GROUP - 1) / COEF1D_ZB_GROUP);
       f_aimg[q] = naimg; naimg += ((long)L.ntm * 128 * L.nchunk * (L.kchunk / 4) + 255) / 256;
-      f_asm[q] = nasm; nasm += ((long)d[i].nx * d[i].ny * L.nz + 127) / 128;
+      f_asm[q] = nasm; nasm += asm1d_blocks(it.a);
       f_kmin[q] = nkmin; nkmin += L.nchunk;
       const size_t coff[3] = {0, (size_t)C1D_OFF1 * L.nz * L.ldc, (size_t)C1D_OFF2 * L.nz * L.ldc};
       for (int od = 0; od < 3; ++od) {
@@ -2280,7 +2234,6 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
         bp.partial = (double*)(base + L.off_pt[od]);
         bp.err = err;
         bp.wait_limit = ctx->wait_limit;
-        bp.aimg_ready = 1;
         bp.kmin = (double*)(base + L.off_kmin);
         const int e = 3 * q + od;
         f_bimg[e] = nbimg;

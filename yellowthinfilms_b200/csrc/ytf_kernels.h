@@ -133,26 +133,54 @@ constexpr int C1D_OFF1 = C1D_R0, C1D_OFF2 = C1D_R0 + C1D_R1, C1D_RT = C1D_R0 + C
 constexpr int C1D_RMAX = C1D_R1;  // the widest order
 
 // 1D Jacobi-Anger synthesis
-cudaError_t launch_coef1d(const SynthParams& p, double* C0, double* C1, double* C2, cudaStream_t s);
-// the same through per-node reflected amplitudes in amp ([12][n] complex scratch)
-cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, double* C0, double* C1, double* C2, cudaStream_t s);
+// coefficient columns through per-node reflected amplitudes in amp ([12][n] complex scratch), rows
+// ldc apart
+cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, double* C, long ldc, cudaStream_t s);
 // the same columns rounded to FP32 (the int8x3 contraction's input)
-cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, float* C0, float* C1, float* C2, cudaStream_t s);
-cudaError_t launch_bessel_c(const double* kr, const double* kri, long nk, const double* rho, int nr, double* J,
+cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, float* C, long ldc, cudaStream_t s);
+// J_n tables, rows ld apart
+cudaError_t launch_bessel_c(const double* kr, const double* kri, long nk, const double* rho, int nr, long ld, double* J,
                             cudaStream_t s);
-cudaError_t launch_combine_complex(long M, int N2, const double* A, const double* B, double* P, cudaStream_t s);
 cudaError_t launch_bessel_eval(long n, int order, const double* zr, const double* zi, double* outr, double* outi,
                                cudaStream_t s);
-cudaError_t launch_bessel(const double* kr, long nk, const double* rho, int nr, double* J0, double* J1, double* J2,
-                          cudaStream_t s);
-int dgemm_splits(int K, int splits);  // effective split count of launch_dgemm_nt
-cudaError_t launch_dgemm_nt(int M, int N, int K, const double* A, const double* B, double* partial, int splits,
-                            cudaStream_t s);
-cudaError_t launch_reduce_splits(long len, int splits, const double* partial, double* C, cudaStream_t s);
-// acc[i] += x[i], i < len
-cudaError_t launch_add(long len, const double* x, double* acc, cudaStream_t s);
-cudaError_t launch_assemble1d(int nx, int ny, int nz, const double* xs, const double* ys, const int* rmap, int nr,
-                              const double* P0, const double* P1, const double* P2, double2* G, cudaStream_t s);
+cudaError_t launch_bessel(const double* kr, long nk, const double* rho, int nr, long ld, double* J0, double* J1,
+                          double* J2, cudaStream_t s);
+// up to six FP64 contractions over the same M rows and K columns in one launch; lda and ldb even,
+// operands on 16 bytes
+struct Gemm64Entry {
+  const double* A;   // [M][lda]
+  const double* B;   // [N][ldb]
+  double* out;       // [splits][N][M]
+  int N;
+  int first;         // first block (set by the launcher)
+};
+struct Gemm64 {
+  int n, M;
+  long K, lda, ldb;
+  int splits;        // k slices (gemm64_plan)
+  long kchunk;
+  Gemm64Entry e[6];
+};
+int gemm64_plan(Gemm64& p);  // sets kchunk and splits from n, M, K and the entries' N
+cudaError_t launch_gemm64(Gemm64 p, cudaStream_t s);
+// acc[i] = (add ? acc[i] : 0) + Σ_z part[z][i], i < len, z < nz in order
+cudaError_t launch_sum_slices(long len, int nz, const double* part, double* acc, int add, cudaStream_t s);
+// slice sums and pixel assembly of one 1D synthesis
+struct Asm1D {
+  int nx, ny, nz, nr;
+  const double* xs;          // device
+  const double* ys;
+  const int* rmap;           // [nx ny] pixel -> radius index
+  int nchunk;                // slices
+  const double* part[3];     // [nchunk][N_o][nr] of order o
+  const double* part_im[3];  // the Im J contraction on a deformed contour, else NULL
+  double2* G;                // [nx][ny][nz][3][3] (Julia's column-major layout)
+};
+// lanes per (pixel, height): four from 8 slices on (256 radii x 64 heights x 22 slices of a contour:
+// 51 us against 71 us with one thread's serial chain of slices), one below
+__host__ __device__ inline int asm1d_split(int nchunk) { return nchunk >= 8 ? 4 : 1; }
+inline long asm1d_blocks(const Asm1D& a) { return ((long)a.nx * a.ny * a.nz * asm1d_split(a.nchunk) + 127) / 128; }
+cudaError_t launch_assemble1d(const Asm1D& a, cudaStream_t s);
 // 2D direct lateral synthesis
 // colmax (optional, zeroed by the caller): [n / kchunk][9 nz] IEEE bits of max(|Re|, |Im|);
 // amp (optional scratch, [12][n] complex): the two-kernel form (k_reflect2d, k_strengths_rows)
@@ -252,14 +280,13 @@ struct BesselI8 {
   const double* kr;  // [K]
   const double* rho; // [M]
   const float* C;    // [N][ldc] coefficient columns (FP32)
-  long ldc;          // row stride of C: K on the per-item path; K rounded up to 4 (16-byte rows) in groups
+  long ldc;          // row stride of C: K rounded up to 4 (16-byte rows)
   uint8_t* Aimg;     // [ntile_m][nchunk][kchunk/64][3][128 x 64 B]
   uint8_t* Bimg;     // [ntile_n][nchunk][kchunk/64][3][Np x 64 B]
   unsigned long long* colmax;  // [nchunk][N]
   double* partial;   // [nchunk][N][M]
   unsigned* err;
   long wait_limit;   // polls of each bounded pipeline wait before it gives up
-  int aimg_ready;    // Aimg already holds this order's J_n digits (launch_bessel_i8_aimg3)
   double* kmin;      // [nchunk] smallest node of each slice (the J digits' scale, launch_slice_kmin)
   const double* rowscale;  // [nchunk][M] the J digits' scale per (slice, radius) when set (digits
                            // rint(J 8355000 / rowscale)); else j_env(kmin[z] ρ_r)
@@ -282,7 +309,10 @@ size_t bessel_i8_stage_bytes_a();
 size_t bessel_i8_stage_bytes_b(int Np);
 size_t bessel_i8_smem(int Np);
 int bessel_i8_ctile(int N);
-cudaError_t launch_bessel_i8(const BesselI8& p, double* P, cudaStream_t s);
+// the coefficient digit images with their slice maxima, and the contractions, of up to six entries in
+// one launch each (a deformed contour's real and imaginary J share an order's coefficient images)
+cudaError_t launch_bimg(const BesselI8* e, int n, cudaStream_t s);
+cudaError_t launch_gemm_i8(const BesselI8* e, int n, cudaStream_t s);
 
 // ------------------------------------------------------------------------------------
 // Grouped 1D int8x3 synthesis: the items of a batch (each a 1D cache of real nodes with its
@@ -296,15 +326,9 @@ struct Synth1DItem {
   double2* amp;            // [12][nk] reflected amplitudes
   float* C;                // [26 nz][ldc] coefficient columns: orders 0, 1, 2 at rows 0, 10 nz, 18 nz
   long ldc;                // row stride of C: nk rounded up to 4, so every row starts on 16 bytes
-  int nx, ny, nr;          // pixel grid, distinct radii
-  const double* xs;        // [nx] device
-  const double* ys;        // [ny] device
-  const int* rmap;         // [nx ny] pixel -> radius index
-  double2* G;              // [nx][ny][nz][3][3] output (Julia's column-major layout)
-  int nchunk;              // node slices of the contraction
+  Asm1D a;                 // pixel grid, radii, slice partials, output
   long kchunk;             // nodes per slice (a multiple of 64)
   double dz;               // spacing of evenly spaced heights (to 4 ulp), else 0
-  const double* part[3];   // [nchunk][N_o][nr] slice partials of order o (N_0 = 10 nz, N_1 = N_2 = 8 nz)
 };
 // every stage of the group, in order, on stream s; `it`/`bp` and the `first_*` tables are
 // device arrays (bp: 3 entries per item, orders 0, 1, 2; bp[3i] also carries the layout of

@@ -197,25 +197,6 @@ __device__ __forceinline__ void unpack_order_sums(F0 P0, F1 P1, F2 P2, cd g0[5],
   g2[3] = -g2[0];
 }
 
-__global__ void __launch_bounds__(128) k_coef1d(SynthParams p, double* C0, double* C1, double* C2) {
-  long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  int zi = blockIdx.y;
-  const CacheView& c = p.c;
-  if (k >= c.n) return;
-  const long n = c.n;
-  cd Af[2][3], Ab[2][3];
-  reflected_amp(p, k, Af, Ab);
-  cd c0[5], c1[4], c2[4];
-  coef1d_row(p, k, p.zo[zi], Af, Ab, c0, c1, c2);
-  store_coef_row(C0, C1, C2, n, k, zi, c0, c1, c2);
-}
-
-cudaError_t launch_coef1d(const SynthParams& p, double* C0, double* C1, double* C2, cudaStream_t s) {
-  dim3 grid((unsigned)((p.c.n + 127) / 128), (unsigned)p.nz);
-  k_coef1d<<<grid, 128, 0, s>>>(p, C0, C1, C2);
-  return cudaGetLastError();
-}
-
 // J_0, J_1, J_2 of a real argument: CUDA's j0/j1, J2 by its power series below |x| = 1 and the
 // three-term recurrence above
 __device__ __forceinline__ void bessel_j012(double x, double& a0, double& a1, double& a2) {
@@ -234,13 +215,14 @@ __device__ __forceinline__ void bessel_j012(double x, double& a0, double& a1, do
   }
 }
 
-// Bessel tables J_n(k ρ), n = 0, 1, 2; row r = radius, k contiguous
-__global__ void k_bessel(const double* kr, long nk, const double* rho, int nr, double* J0, double* J1, double* J2) {
+// Bessel tables J_n(k ρ), n = 0, 1, 2; row r = radius, k contiguous, rows ld apart
+__global__ void k_bessel(const double* kr, long nk, const double* rho, int nr, long ld, double* J0, double* J1,
+                         double* J2) {
   long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
   int r = blockIdx.y;
   if (k >= nk) return;
   double x = kr[k] * rho[r];
-  long o = (long)r * nk + k;
+  long o = (long)r * ld + k;
   double a0, a1, a2;
   bessel_j012(x, a0, a1, a2);
   J0[o] = a0;
@@ -249,7 +231,7 @@ __global__ void k_bessel(const double* kr, long nk, const double* rho, int nr, d
 }
 
 // J_n(kρ ρ) of complex nodes (deformed contour): real and imaginary tables of each order
-__global__ void k_bessel_c(const double* kr, const double* kri, long nk, const double* rho, int nr, double* J) {
+__global__ void k_bessel_c(const double* kr, const double* kri, long nk, const double* rho, int nr, long ld, double* J) {
   long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
   int r = blockIdx.y;
   if (k >= nk) return;
@@ -260,35 +242,17 @@ __global__ void k_bessel_c(const double* kr, const double* kri, long nk, const d
   } else {
     bessel_j012_c(z, a0, a1, a2);
   }
-  const long o = (long)r * nk + k, plane = (long)nr * nk;
+  const long o = (long)r * ld + k, plane = (long)nr * ld;
   J[o] = a0.x; J[plane + o] = a0.y;
   J[2 * plane + o] = a1.x; J[3 * plane + o] = a1.y;
   J[4 * plane + o] = a2.x; J[5 * plane + o] = a2.y;
 }
 
-cudaError_t launch_bessel_c(const double* kr, const double* kri, long nk, const double* rho, int nr, double* J,
+cudaError_t launch_bessel_c(const double* kr, const double* kri, long nk, const double* rho, int nr, long ld, double* J,
                             cudaStream_t s) {
   if (nk <= 0 || nr <= 0) return cudaSuccess;
   dim3 grid((unsigned)((nk + 127) / 128), (unsigned)nr);
-  k_bessel_c<<<grid, 128, 0, s>>>(kr, kri, nk, rho, nr, J);
-  return cudaGetLastError();
-}
-
-// complex J times the real/imag column pairs: P[r][2c] = A[2c] - B[2c+1], P[r][2c+1] = A[2c+1] + B[2c]
-// with A = Re J · C^T and B = Im J · C^T
-__global__ void k_combine_complex(long M, int N2, const double* A, const double* B, double* P) {
-  long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= M * (N2 / 2)) return;
-  const long r = t / (N2 / 2), c = t % (N2 / 2);
-  const long o = r * N2 + 2 * c;
-  P[o] = A[o] - B[o + 1];
-  P[o + 1] = A[o + 1] + B[o];
-}
-
-cudaError_t launch_combine_complex(long M, int N2, const double* A, const double* B, double* P, cudaStream_t s) {
-  const long tot = M * (N2 / 2);
-  if (tot <= 0) return cudaSuccess;
-  k_combine_complex<<<(unsigned)((tot + 255) / 256), 256, 0, s>>>(M, N2, A, B, P);
+  k_bessel_c<<<grid, 128, 0, s>>>(kr, kri, nk, rho, nr, ld, J);
   return cudaGetLastError();
 }
 
@@ -315,109 +279,170 @@ cudaError_t launch_bessel_eval(long n, int order, const double* zr, const double
   return cudaGetLastError();
 }
 
-cudaError_t launch_bessel(const double* kr, long nk, const double* rho, int nr, double* J0, double* J1, double* J2,
-                          cudaStream_t s) {
+cudaError_t launch_bessel(const double* kr, long nk, const double* rho, int nr, long ld, double* J0, double* J1,
+                          double* J2, cudaStream_t s) {
   dim3 grid((unsigned)((nk + 127) / 128), (unsigned)nr);
-  k_bessel<<<grid, 128, 0, s>>>(kr, nk, rho, nr, J0, J1, J2);
+  k_bessel<<<grid, 128, 0, s>>>(kr, nk, rho, nr, ld, J0, J1, J2);
   return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------------------------
-// FP64 GEMM C[M][N] = A[M][K] · B[N][K]^T (both operands K-contiguous), split-K with a
-// deterministic reduction. 128x128 tile, 8 k per stage, 8x8 outputs per thread.
+// FP64 contractions out[split][n][m] = Σ_k A[m][k] B[n][k] (both operands k-contiguous), up to six
+// of them (the Bessel orders; real and imaginary J on a contour) in one grid, each cut into
+// column tiles, row tiles and k slices; the pixel assembly sums the slices in order. FP64
+// tensor-core instructions (mma m8n8k4: one operand load serves 8 rows or columns, where the
+// scalar FMA tile it replaces was bound by its shared-memory loads and its load-compute-load
+// barriers), a ring of 16-k stages filled by cp.async, warps of 32 x 32 or 16 x 16 outputs. Rows of
+// a stage are 20 doubles apart, so the 4 x 4 operand words of a half-warp fall in distinct banks.
+// Bound: the FP64 pipe (37 TFLOP/s) on large sets; the latency of the k chain on small ones, hence
+// the 32 x 32 tile there, which gives more slices.
 // ------------------------------------------------------------------------------------
-constexpr int GT = 128, GK = 8;
-__global__ void __launch_bounds__(256) k_dgemm_nt(int M, int N, int K, const double* __restrict__ A,
-                                                  const double* __restrict__ B, double* __restrict__ Cp, int kchunk) {
-  __shared__ double As[GK][GT];
-  __shared__ double Bs[GK][GT];
-  const int bm = blockIdx.y * GT, bn = blockIdx.x * GT, sp = blockIdx.z;
-  const long k0 = (long)sp * kchunk;
-  const long k1 = min((long)K, k0 + kchunk);
-  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-  double acc[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0;
-  for (long kk = k0; kk < k1; kk += GK) {
-    // 128x8 tile of A and of B: 1024 elements each, 4 per thread; k fastest in memory
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      int idx = tid + 256 * e;
-      int row = idx / GK, col = idx % GK;
-      long kg = kk + col;
-      int ra = bm + row, rb = bn + row;
-      As[col][row] = (ra < M && kg < k1) ? A[(long)ra * K + kg] : 0.0;
-      Bs[col][row] = (rb < N && kg < k1) ? B[(long)rb * K + kg] : 0.0;
+__device__ __forceinline__ void cp16(uint32_t dst, const double* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c0), "+d"(c1)
+               : "d"(a), "d"(b));
+}
+
+constexpr int G64_K = 16, G64_LD = 20, G64_STAGES = 3;
+
+// BM x BN tile, WT x WT outputs per warp
+template <int BM, int BN, int WT>
+__global__ void __launch_bounds__(32 * (BM / WT) * (BN / WT)) k_gemm64(const __grid_constant__ Gemm64 p) {
+  constexpr int WN = BN / WT, NT = 32 * (BM / WT) * WN, F = WT / 8;
+  extern __shared__ __align__(16) double g64[];
+  constexpr int STAGE = (BM + BN) * G64_LD;
+  int e = 0;
+  while (e + 1 < p.n && p.e[e + 1].first <= (int)blockIdx.x) ++e;
+  const Gemm64Entry& E = p.e[e];
+  const int ntm = (p.M + BM - 1) / BM, ntn = (E.N + BN - 1) / BN;
+  const int u = (int)blockIdx.x - E.first;
+  const int bm = (u % ntm) * BM, bn = (u / ntm % ntn) * BN, sp = u / (ntm * ntn);
+  const long k0 = (long)sp * p.kchunk, k1 = min(p.K, k0 + p.kchunk);
+  const int nst = k1 > k0 ? (int)((k1 - k0 + G64_K - 1) / G64_K) : 0;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wm = (warp / WN) * WT, wn = (warp % WN) * WT;
+  const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(g64);
+  // one stage: (BM + BN) rows of 16 doubles, 8 copies of 16 bytes per row; rows past the operand
+  // and k past the slice are zero-filled
+  auto fill = [&](int st) {
+    const long kk = k0 + (long)st * G64_K;
+    const uint32_t base = sbase + (uint32_t)((st % G64_STAGES) * STAGE) * 8u;
+    for (int t = tid; t < (BM + BN) * 8; t += NT) {
+      const int row = t >> 3, c = 2 * (t & 7);
+      const bool isa = row < BM;
+      const int g = isa ? bm + row : bn + row - BM;
+      const bool in = isa ? g < p.M : g < E.N;
+      const long left = k1 - kk - c;
+      const int bytes = in ? (left >= 2 ? 16 : left == 1 ? 8 : 0) : 0;
+      const double* src = isa ? E.A + (bytes ? (long)g * p.lda + kk + c : 0) : E.B + (bytes ? (long)g * p.ldb + kk + c : 0);
+      cp16(base + (uint32_t)(row * G64_LD + c) * 8u, src, bytes);
     }
-    __syncthreads();
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  double acc[F][F][2];
 #pragma unroll
-    for (int t = 0; t < GK; ++t) {
-      double a[8], b[8];
+  for (int i = 0; i < F; ++i)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) a[i] = As[t][ty + 16 * i];
+    for (int j = 0; j < F; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) b[j] = Bs[t][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
+  for (int s = 0; s < G64_STAGES - 1; ++s) {
+    if (s < nst) fill(s);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  double* C = Cp + (long)sp * M * N;
+  for (int s = 0; s < nst; ++s) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(G64_STAGES - 2) : "memory");
+    __syncthreads();
+    if (s + G64_STAGES - 1 < nst) fill(s + G64_STAGES - 1);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+    const double* A = g64 + (s % G64_STAGES) * STAGE + (wm + (lane >> 2)) * G64_LD + (lane & 3);
+    const double* B = g64 + (s % G64_STAGES) * STAGE + (BM + wn + (lane >> 2)) * G64_LD + (lane & 3);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    int r = bm + ty + 16 * i;
-    if (r >= M) continue;
+    for (int q = 0; q < G64_K; q += 4) {
+      double a[F], b[F];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      int cc = bn + tx + 16 * j;
-      if (cc < N) C[(long)r * N + cc] = acc[i][j];
+      for (int i = 0; i < F; ++i) {
+        a[i] = A[8 * i * G64_LD + q];
+        b[i] = B[8 * i * G64_LD + q];
+      }
+#pragma unroll
+      for (int i = 0; i < F; ++i)
+#pragma unroll
+        for (int j = 0; j < F; ++j) mma_f64(acc[i][j][0], acc[i][j][1], a[i], b[j]);
     }
+  }
+  double* out = E.out + (long)sp * E.N * p.M;
+#pragma unroll
+  for (int i = 0; i < F; ++i) {
+    const int m = bm + wm + 8 * i + (lane >> 2);
+    if (m >= p.M) continue;
+#pragma unroll
+    for (int j = 0; j < F; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int n = bn + wn + 8 * j + 2 * (lane & 3) + h;
+        if (n < E.N) out[(long)n * p.M + m] = acc[i][j][h];
+      }
   }
 }
 
-__global__ void k_reduce_splits(long len, int splits, const double* __restrict__ P, double* __restrict__ C) {
-  long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= len) return;
-  double s = 0.0;
-  for (int k = 0; k < splits; ++k) s += P[(long)k * len + i];
-  C[i] = s;
+// 128 x 64 tiles once they give 148 CTAs (2.0 against 2.4 us per GFLOP at 251 x 61 heights x 4081
+// nodes with 32 x 32 ones); below that 32 x 32 tiles, whose shorter warps and finer slices shorten
+// the k chain (8 radii x 4 heights x 256 nodes: 5 against 11 us)
+static bool gemm64_large(const Gemm64& p) {
+  long t = 0;
+  for (int i = 0; i < p.n; ++i) t += (long)((p.M + 127) / 128) * ((p.e[i].N + 63) / 64);
+  return t * std::max(1L, p.K / 256) >= 148;
 }
 
-int dgemm_splits(int K, int splits) {
-  int kchunk = (K + splits - 1) / splits;
-  kchunk = ((kchunk + GK - 1) / GK) * GK;
-  if (kchunk <= 0) return 1;
-  return std::max(1, (K + kchunk - 1) / kchunk);
+int gemm64_plan(Gemm64& p) {
+  const bool big = gemm64_large(p);
+  const int bm = big ? 128 : 32, bn = big ? 64 : 32;
+  long tiles = 0;
+  for (int i = 0; i < p.n; ++i) tiles += (long)((p.M + bm - 1) / bm) * ((p.e[i].N + bn - 1) / bn);
+  // k slices that fill the SMs (two 128 x 64 or four 32 x 32 CTAs each), at least 64 nodes long
+  const long want = std::max(1L, std::min((148L * (big ? 2 : 4)) / std::max(1L, tiles), p.K / 64));
+  p.kchunk = ((p.K + want - 1) / want + G64_K - 1) / G64_K * G64_K;
+  if (p.kchunk <= 0) p.kchunk = G64_K;
+  p.splits = (int)std::max(1L, (p.K + p.kchunk - 1) / p.kchunk);
+  return p.splits;
 }
 
-cudaError_t launch_dgemm_nt(int M, int N, int K, const double* A, const double* B, double* partial, int splits,
-                            cudaStream_t s) {
-  if (M <= 0 || N <= 0) return cudaSuccess;
-  splits = dgemm_splits(K, splits);
-  int kchunk = (K + splits - 1) / splits;
-  kchunk = ((kchunk + GK - 1) / GK) * GK;
-  dim3 grid((unsigned)((N + GT - 1) / GT), (unsigned)((M + GT - 1) / GT), (unsigned)splits);
-  k_dgemm_nt<<<grid, 256, 0, s>>>(M, N, K, A, B, partial, kchunk);
+cudaError_t launch_gemm64(Gemm64 p, cudaStream_t s) {
+  if (p.M <= 0 || p.n <= 0) return cudaSuccess;
+  if ((p.lda | p.ldb) & 1) return cudaErrorInvalidValue;
+  const bool big = gemm64_large(p);
+  const int bm = big ? 128 : 32, bn = big ? 64 : 32;
+  int blocks = 0;
+  for (int i = 0; i < p.n; ++i) {
+    p.e[i].first = blocks;
+    blocks += ((p.M + bm - 1) / bm) * ((p.e[i].N + bn - 1) / bn) * p.splits;
+  }
+  const int smem = G64_STAGES * (bm + bn) * G64_LD * 8;
+  if (big) {
+    cudaError_t e = cudaFuncSetAttribute(k_gemm64<128, 64, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    k_gemm64<128, 64, 32><<<blocks, 256, smem, s>>>(p);
+  } else {
+    k_gemm64<32, 32, 16><<<blocks, 128, smem, s>>>(p);
+  }
   return cudaGetLastError();
 }
 
-__global__ void k_add(long len, const double* __restrict__ x, double* __restrict__ acc) {
-  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (long)gridDim.x * blockDim.x) acc[i] += x[i];
+// acc[i] = (add ? acc[i] : 0) + Σ_z part[z][i], z in order
+__global__ void k_sum_slices(long len, int nz, const double* __restrict__ part, double* __restrict__ acc, int add) {
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (long)gridDim.x * blockDim.x) {
+    double s = 0.0;
+    for (int z = 0; z < nz; ++z) s += part[(long)z * len + i];
+    acc[i] = add ? acc[i] + s : s;
+  }
 }
 
-cudaError_t launch_add(long len, const double* x, double* acc, cudaStream_t s) {
+cudaError_t launch_sum_slices(long len, int nz, const double* part, double* acc, int add, cudaStream_t s) {
   if (len <= 0) return cudaSuccess;
-  k_add<<<(unsigned)std::min<long>((len + 255) / 256, 148L * 8), 256, 0, s>>>(len, x, acc);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_reduce_splits(long len, int splits, const double* partial, double* C, cudaStream_t s) {
-  if (len <= 0) return cudaSuccess;
-  k_reduce_splits<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(len, splits, partial, C);
+  k_sum_slices<<<(unsigned)std::min<long>((len + 255) / 256, 148L * 16), 256, 0, s>>>(len, nz, part, acc, add);
   return cudaGetLastError();
 }
 
@@ -505,28 +530,76 @@ __device__ __forceinline__ void assemble1d_pixel(double x, double y, const cd g0
     }
 }
 
-__global__ void k_assemble1d(int nx, int ny, int nz, const double* xs, const double* ys, const int* rmap, int nr,
-                             const double* P0, const double* P1, const double* P2, double2* G) {
-  long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  long npix = (long)nx * ny;
-  if (t >= npix * nz) return;
-  long pix = t % npix;
-  int zi = (int)(t / npix);
-  int i = (int)(pix % nx), j = (int)(pix / nx);
-  int r = rmap[pix];
-  const long n0 = (long)C1D_R0 * nz, n1 = (long)C1D_R1 * nz, n2 = (long)C1D_R2 * nz;
-  cd g0[5], g1[4], g2[4];
-  unpack_order_sums([&](int c) { const long o = (long)r * n0 + 2L * (zi * 3 + c); return cd{P0[o], P0[o + 1]}; },
-                    [&](int c) { const long o = (long)r * n1 + 2L * (zi * 4 + c); return cd{P1[o], P1[o + 1]}; },
-                    [&](int c) { const long o = (long)r * n2 + 2L * (zi * 2 + c); return cd{P2[o], P2[o + 1]}; },
-                    g0, g1, g2);
-  assemble1d_pixel(xs[i], ys[j], g0, g1, g2, pix, npix, zi, nz, G);
+// acc[j] = Σ_z p[z N M + j M], j < R, z = first, first + step, ...: the slices of one (radius, height)'s R
+// real columns in order, all columns of a slice in flight together; with step 4 (ASM_SPLIT) the
+// lanes 8 apart hold four interleaved parts of the slices, added at the end
+template <int R>
+__device__ __forceinline__ void sum_columns(const double* __restrict__ p, long M, long NM, int nchunk, int first, int step,
+                                            double acc[R]) {
+#pragma unroll
+  for (int j = 0; j < R; ++j) acc[j] = 0.0;
+  p += first * NM;
+#pragma unroll 2
+  for (int z = first; z < nchunk; z += step, p += step * NM)
+#pragma unroll
+    for (int j = 0; j < R; ++j) acc[j] += __ldg(p + j * M);
+  if (step > 1)
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 8);
+      acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 16);
+    }
+}
+// the order's complex columns of one (radius, height); on a deformed contour part holds Re J · C^T and
+// part_im Im J · C^T of the real and imaginary columns
+template <int R>
+__device__ __forceinline__ void order_columns(const Asm1D& a, int o, int zi, int r, int first, int step, cd g[R / 2]) {
+  const long M = a.nr, NM = (long)R * a.nz * M, off = (long)R * zi * M + r;
+  double x[R];
+  sum_columns<R>(a.part[o] + off, M, NM, a.nchunk, first, step, x);
+#pragma unroll
+  for (int c = 0; c < R / 2; ++c) g[c] = cd{x[2 * c], x[2 * c + 1]};
+  if (a.part_im[o]) {
+    sum_columns<R>(a.part_im[o] + off, M, NM, a.nchunk, first, step, x);
+#pragma unroll
+    for (int c = 0; c < R / 2; ++c) g[c] = cd{g[c].x - x[2 * c + 1], g[c].y + x[2 * c]};
+  }
 }
 
-cudaError_t launch_assemble1d(int nx, int ny, int nz, const double* xs, const double* ys, const int* rmap, int nr,
-                              const double* P0, const double* P1, const double* P2, double2* G, cudaStream_t s) {
-  long tot = (long)nx * ny * nz;
-  k_assemble1d<<<(unsigned)((tot + 127) / 128), 128, 0, s>>>(nx, ny, nz, xs, ys, rmap, nr, P0, P1, P2, G);
+// one thread per (pixel, height), or four lanes of one warp (asm1d_split): the order sums of the pixel's
+// radius, then the pixel assembly. Blocks of 128 threads; b: the block within the item.
+__device__ __forceinline__ void assemble1d_body(const Asm1D& a, long b) {
+  const long npix = (long)a.nx * a.ny;
+  const int nz = a.nz, step = asm1d_split(a.nchunk);
+  const int lane = threadIdx.x & 31;
+  const int first = step > 1 ? lane >> 3 : 0;
+  long t = step > 1 ? (b * 4 + (threadIdx.x >> 5)) * 8 + (lane & 7) : b * 128 + threadIdx.x;
+  const bool live = t < npix * nz;
+  if (!live) {
+    if (step == 1) return;
+    t = 0;  // the warp's shuffles need every lane
+  }
+  const long pix = t % npix;
+  const int zi = (int)(t / npix);
+  const int ix = (int)(pix % a.nx), iy = (int)(pix / a.nx);
+  const int r = a.rmap[pix];
+  cd s0[C1D_R0 / 2], s1[C1D_R1 / 2], s2[C1D_R2 / 2], g0[5], g1[4], g2[4];
+  order_columns<C1D_R0>(a, 0, zi, r, first, step, s0);
+  order_columns<C1D_R1>(a, 1, zi, r, first, step, s1);
+  order_columns<C1D_R2>(a, 2, zi, r, first, step, s2);
+  if (!live || first > 0) return;
+  unpack_order_sums([&](int c) { return s0[c]; }, [&](int c) { return s1[c]; }, [&](int c) { return s2[c]; }, g0, g1, g2);
+  assemble1d_pixel(a.xs[ix], a.ys[iy], g0, g1, g2, pix, npix, zi, nz, a.G);
+}
+
+__global__ void __launch_bounds__(128) k_assemble1d(const __grid_constant__ Asm1D a) {
+  assemble1d_body(a, blockIdx.x);
+}
+
+cudaError_t launch_assemble1d(const Asm1D& a, cudaStream_t s) {
+  const long blocks = asm1d_blocks(a);
+  if (blocks <= 0) return cudaSuccess;
+  k_assemble1d<<<(unsigned)blocks, 128, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -610,7 +683,7 @@ constexpr int COEF1D_ZB = 4;
 // fixed-point scale) and whose coefficient columns are then half the memory traffic
 template <class T>
 __global__ void __launch_bounds__(128) k_coef1d_amp(SynthParams p, const double2* __restrict__ amp, T* C0, T* C1,
-                                                     T* C2) {
+                                                     T* C2, long cst) {
   const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const long n = p.c.n;
   if (k >= n) return;
@@ -627,25 +700,26 @@ __global__ void __launch_bounds__(128) k_coef1d_amp(SynthParams p, const double2
   for (int zi = z0; zi < z1; ++zi) {
     cd c0[5], c1[4], c2[4];
     coef1d_row(p, k, p.zo[zi], Af, Ab, c0, c1, c2);
-    store_coef_row(C0, C1, C2, n, k, zi, c0, c1, c2);
+    store_coef_row(C0, C1, C2, cst, k, zi, c0, c1, c2);
   }
 }
 
+// the order-0 rows at C, orders 1 and 2 behind them
 template <class T>
-static cudaError_t coef1d_amp_impl(const SynthParams& p, double2* amp, T* C0, T* C1, T* C2, cudaStream_t s) {
+static cudaError_t coef1d_amp_impl(const SynthParams& p, double2* amp, T* C, long ldc, cudaStream_t s) {
   if (p.c.n <= 0 || p.nz <= 0) return cudaSuccess;
   k_reflect2d<<<(unsigned)((p.c.n + 127) / 128), 128, 0, s>>>(p, amp);
   k_coef1d_amp<T><<<dim3((unsigned)((p.c.n + 127) / 128), (unsigned)((p.nz + COEF1D_ZB - 1) / COEF1D_ZB)), 128, 0, s>>>(
-      p, amp, C0, C1, C2);
+      p, amp, C, C + (size_t)C1D_OFF1 * p.nz * ldc, C + (size_t)C1D_OFF2 * p.nz * ldc, ldc);
   return cudaGetLastError();
 }
 
-cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, double* C0, double* C1, double* C2, cudaStream_t s) {
-  return coef1d_amp_impl<double>(p, amp, C0, C1, C2, s);
+cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, double* C, long ldc, cudaStream_t s) {
+  return coef1d_amp_impl<double>(p, amp, C, ldc, s);
 }
 
-cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, float* C0, float* C1, float* C2, cudaStream_t s) {
-  return coef1d_amp_impl<float>(p, amp, C0, C1, C2, s);
+cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, float* C, long ldc, cudaStream_t s) {
+  return coef1d_amp_impl<float>(p, amp, C, ldc, s);
 }
 
 // per node of a k_strengths_rows block: 12 amplitudes, the obs-layer basis (16), sf, sb (6 each),
@@ -1310,37 +1384,10 @@ cudaError_t launch_reflect_coef_group(const Synth1DGroup& g, int stage, cudaStre
   return cudaGetLastError();
 }
 
-// one thread per (pixel, height) of an item: P_n(r, c) = Σ_z part_n[z][c][r] (slices in
-// order, as k_reduce_transpose), then assemble1d_pixel
 __global__ void __launch_bounds__(128) k_assemble1d_group(const Synth1DItem* __restrict__ items,
                                                           const long* __restrict__ first, int ni) {
   const int i = group_entry(first, ni, blockIdx.x);
-  const Synth1DItem& it = items[i];
-  const long npix = (long)it.nx * it.ny;
-  const int nz = it.sp.nz;
-  const long t = (long)(blockIdx.x - first[i]) * blockDim.x + threadIdx.x;
-  if (t >= npix * nz) return;
-  const long pix = t % npix;
-  const int zi = (int)(t / npix);
-  const int ix = (int)(pix % it.nx), iy = (int)(pix / it.nx);
-  const int r = it.rmap[pix];
-  const long M = it.nr;
-  const int nch = it.nchunk;
-  const long N0 = (long)C1D_R0 * nz, N1 = (long)C1D_R1 * nz, N2 = (long)C1D_R2 * nz;
-  // the slices' partials summed in order, as k_reduce_transpose
-  auto sum = [&](const double* part, long N, long c) {
-    double re = 0.0, im = 0.0;
-    for (int z = 0; z < nch; ++z) {
-      re += part[((long)z * N + c) * M + r];
-      im += part[((long)z * N + c + 1) * M + r];
-    }
-    return cd{re, im};
-  };
-  cd g0[5], g1[4], g2[4];
-  unpack_order_sums([&](int c) { return sum(it.part[0], N0, 2L * (zi * 3 + c)); },
-                    [&](int c) { return sum(it.part[1], N1, 2L * (zi * 4 + c)); },
-                    [&](int c) { return sum(it.part[2], N2, 2L * (zi * 2 + c)); }, g0, g1, g2);
-  assemble1d_pixel(it.xs[ix], it.ys[iy], g0, g1, g2, pix, npix, zi, nz, it.G);
+  assemble1d_body(items[i].a, blockIdx.x - first[i]);
 }
 
 cudaError_t launch_assemble1d_group(const Synth1DGroup& g, cudaStream_t s) {
