@@ -62,3 +62,25 @@ def test_1d_general_columns_without_the_symmetry_check(oracle):
     assert relerr(api.closed_form_G(gc, 1, 0.03, z, rho, [0.1], terms="scattered", precision="int8x3"), Go) < 1e-6
     G8 = api.closed_form_G_batch([(gc, 1, 0.03, z, rho, [0.1])] * 2, precision="int8x3")
     assert relerr(G8[1], oracle.closed_form_G(oc, 1, 0.03, z, rho, [0.1])) < 1e-6
+
+
+@pytest.mark.parametrize("d,z,obs,terms", [(17.0, np.linspace(0.0, 16.9, 9), 1, "direct"),
+                                           (17.0, np.geomspace(0.01, 16.9, 7), 1, "direct"),
+                                           (0.33, np.linspace(-4.0, 0.07, 20), 2, "all"),
+                                           (0.33, np.linspace(-4.0, 0.3, 20), 1, "scattered")])
+def test_1d_heights_past_the_phase_recurrence(oracle, d, z, obs, terms):
+    """Exponents below -600 (a 17 λ air layer, its direct term: the rows' own exponentials) and above
+    80 (heights below the layer: the general columns' clamped phases)."""
+    from helpers import lay
+    from yellowthinfilms_b200 import api
+    from yellowthinfilms_b200.materials import IsotropicMaterial
+    st = config1_like_stack()
+    st[0] = lay(IsotropicMaterial(1.0), d)
+    k, w, rho, _ = _case(264, 9, 3, True)
+    gc = api.build_cavity_transfer_1d(st, W, 1, k, w, obs_layers=[1, 2])
+    oc = oracle.build_cavity_transfer_1d(st, W, 1, k, w, obs_layers=[1, 2])
+    Go = oracle.closed_form_G(oc, obs, 0.03, z, rho, [0.0], terms=terms)
+    G = api.closed_form_G(gc, obs, 0.03, z, rho, [0.0], terms=terms)
+    assert relerr(G, Go) < 1e-10
+    for i in range(len(z)):  # every height on its own scale
+        assert relerr(G[:, :, i], Go[:, :, i]) < 1e-9 or np.linalg.norm(Go[:, :, i]) < 1e-280

@@ -79,6 +79,7 @@ struct ytf_cache {
   int nL, src, nobs;
   int obs[MAXL];
   bool is2d = false, rotation = false;
+  bool sym = false;  // 1D cache of a stack whose TE and TM decouple (tm_te_decoupled)
   int Nk = 0, Np = 1;
   long n = 0;
   double omega = 0, d_src = 0;
@@ -238,6 +239,28 @@ std::string obs_str(const int* obs, int n) {
 }
 
 bool closed_form(const LayerDev& L) { return (L.ekind == 0 || L.ekind == 1) && L.mkind == 0; }
+
+// TE and TM waves of a φ = 0 node do not mix: closed-form modes in every layer, and no ε_xz, ε_yz in
+// the source projection or the mode fields
+bool tm_te_decoupled(const std::vector<LayerDev>& host) {
+  for (const LayerDev& L : host) {
+    if (!closed_form(L)) return false;
+    for (int e : {2, 5, 6, 7})  // (3,1), (3,2), (1,3), (2,3) of the column-major ε
+      if (L.eps[2 * e] != 0.0 || L.eps[2 * e + 1] != 0.0) return false;
+  }
+  return true;
+}
+
+// spacing of evenly spaced heights (to 4 ulp of the progression), else 0
+double even_spacing(const double* z, int m) {
+  if (m < 2) return 0.0;
+  const double dz = (z[m - 1] - z[0]) / (m - 1);
+  if (!std::isfinite(dz) || dz == 0.0) return 0.0;
+  const double tol = 4 * 2.220446049250313e-16 * std::max(std::fabs(z[0]), std::fabs(z[m - 1]));
+  for (int r = 0; r < m; ++r)
+    if (!(std::fabs(z[r] - (z[0] + r * dz)) <= tol)) return 0.0;
+  return dz;
+}
 
 // a layer's Berreman matrix is finite at every node: finite ε and μ with ε33 ≠ 0 and μ33 ≠ 0
 // (_berreman_core divides by both, mod_ModeSolver.jl:134-135)
@@ -663,6 +686,7 @@ int prepare_cache(ytf_ctx* ctx, const ytf_stack* st, bool is2d, double omega, in
   c->omega = omega;
   c->is2d = is2d;
   c->rotation = *use_rot;
+  c->sym = !is2d && tm_te_decoupled(st->host);
   c->Nk = nk;
   c->Np = is2d ? nphi : 1;
   c->n = is2d ? (long)nk * nphi : nk;
@@ -1550,6 +1574,7 @@ static int synth_setup(ytf_ctx* ctx, const ytf_cache* c, int obs_layer, double z
   v.T = c->d_T + (size_t)oi * 16 * c->n;
   v.Qf = c->d_Qf; v.Qb = c->d_Qb; v.sf = c->d_sf; v.sb = c->d_sb;
   v.basis = c->d_basis + (size_t)oi * 16 * c->n;
+  sp.sym = c->sym;
   sp.same = same;
   switch (terms) {
     case YTF_TERMS_ALL: sp.uf_F = sp.ub_F = sp.uf_B = sp.ub_B = 1.0; sp.with_direct = same; break;
@@ -1576,16 +1601,15 @@ struct Parts1D {
 // the order contractions of the 1D synthesis over the nodes of sp.c: the per-node coefficient columns
 // (k_coef1d), the Bessel tables or digit images, and one launch for every contraction (two per
 // order, Re J and Im J, on a deformed contour), in FP64 or on the int8 tensor cores
-static int synth1d_parts(ytf_ctx* ctx, const SynthParams& sp, int nz, int nr, const double* drho, int precision, int nsm,
-                         const GreenBatch* gb, Parts1D& out) {
+static int synth1d_parts(ytf_ctx* ctx, const SynthParams& sp, int nz, double dz, int nr, const double* drho, int precision,
+                         int nsm, const GreenBatch* gb, Parts1D& out) {
   const long nk = sp.c.n, ld = (nk + 3) / 4 * 4;  // rows on 16 bytes
   const bool i8 = precision == YTF_PREC_INT8X3, cplx = sp.c.kri != nullptr;
   const int np = cplx ? 2 : 1;
   std::memset(&out, 0, sizeof(out));
-  const int R[3] = {C1D_R0, C1D_R1, C1D_R2};
   size_t coff[3], ncol = 0;
   for (int o = 0; o < 3; ++o) {
-    out.N[o] = R[o] * nz;
+    out.N[o] = c1d_rows(sp.sym, o) * nz;
     coff[o] = ncol * ld;
     ncol += out.N[o];
   }
@@ -1597,10 +1621,10 @@ static int synth1d_parts(ytf_ctx* ctx, const SynthParams& sp, int nz, int nr, co
         off += nchunk * out.N[o] * nr;
       }
   };
-  WS(amp1, double2, "g_amp", (size_t)12 * nk);
+  WS(amp1, double2, "g_amp", (size_t)c1d_amp_rows(sp.sym, sp.with_direct) * nk);
   if (!i8) {
     WS(C, double, "g_C", ncol * ld);
-    CK(LAUNCH("k_coef1d", launch_coef1d_amp(sp, amp1, C, ld, ctx->stream)));
+    CK(LAUNCH("k_coef1d", launch_coef1d_amp(sp, amp1, C, ld, dz, ctx->stream)));
     const size_t plane = (size_t)nr * ld;
     WS(J, double, "g_J", 3 * np * plane);
     if (cplx) CK(LAUNCH("k_bessel_c", launch_bessel_c(sp.c.kr, sp.c.kri, nk, drho, nr, ld, J, ctx->stream)));
@@ -1634,7 +1658,7 @@ static int synth1d_parts(ytf_ctx* ctx, const SynthParams& sp, int nz, int nr, co
     CK(cudaMemsetAsync(err, 0, sizeof(unsigned), ctx->stream));
   }
   WS(Cf, float, "g_Cf", ncol * ld);
-  CK(LAUNCH("k_coef1d", launch_coef1d_amp(sp, amp1, Cf, ld, ctx->stream)));
+  CK(LAUNCH("k_coef1d", launch_coef1d_amp(sp, amp1, Cf, ld, dz, ctx->stream)));
   // one node slicing for the three orders: its length sets the digits' scales, and follows the
   // tiles of the widest order's general columns
   long kchunk;
@@ -1804,18 +1828,20 @@ static int green_impl(ytf_ctx* ctx, const ytf_cache* c, int obs_layer, double zs
     }
     Asm1D as;
     std::memset(&as, 0, sizeof(as));
+    as.sym = sp.sym;
     as.nx = nx; as.ny = ny; as.nz = nz; as.nr = nr;
     as.xs = dxs; as.ys = dys; as.rmap = drmap; as.G = G;
     Parts1D pt;
+    const double dz = even_spacing(z_obs, nz);
     if (nk <= SYNTH1D_NODE_CHUNK) {
-      if ((rc = synth1d_parts(ctx, sp, nz, nr, drho, precision, nsm, gb, pt))) return rc;
+      if ((rc = synth1d_parts(ctx, sp, nz, dz, nr, drho, precision, nsm, gb, pt))) return rc;
       as.nchunk = pt.nchunk;
       for (int o = 0; o < 3; ++o) { as.part[o] = pt.part[o]; as.part_im[o] = pt.part_im[o]; }
     } else {
       // G is linear in the node sum: the rule in passes of at most SYNTH1D_NODE_CHUNK nodes,
       // their order sums added (the reference sums closed_form_G over node chunks the same way,
       // chunked_2d, mod_ClosedFormGrid.jl:449-467)
-      const size_t np = (size_t)C1D_RT * nz * nr;
+      const size_t np = (size_t)(c1d_rows(sp.sym, 0) + c1d_rows(sp.sym, 1) + c1d_rows(sp.sym, 2)) * nz * nr;
       const int nq = sp.c.kri ? 2 : 1;
       WS(Pacc, double, "g_Pacc", nq * np);
       WS(cbuf, double2, "g_chunk_cache", (size_t)48 * SYNTH1D_NODE_CHUNK);
@@ -1823,7 +1849,7 @@ static int green_impl(ytf_ctx* ctx, const ytf_cache* c, int obs_layer, double zs
         const long nb = std::min(SYNTH1D_NODE_CHUNK, nk - b0);
         SynthParams spc = sp;
         if ((rc = node_chunk_view(ctx, sp.c, b0, nb, cbuf, spc.c))) return rc;
-        if ((rc = synth1d_parts(ctx, spc, nz, nr, drho, precision, nsm, gb, pt))) return rc;
+        if ((rc = synth1d_parts(ctx, spc, nz, dz, nr, drho, precision, nsm, gb, pt))) return rc;
         size_t off = 0;
         for (int q = 0; q < nq; ++q)
           for (int o = 0; o < 3; ++o) {
@@ -1991,7 +2017,9 @@ struct Group1DLayout {
 
 static size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
-static Group1DLayout group1d_layout(int item, long nk, int nz, int nr, long npix, bool host_out, long slice) {
+static Group1DLayout group1d_layout(int item, const SynthParams& sp, int nz, int nr, long npix, bool host_out,
+                                    long slice) {
+  const long nk = sp.c.n;
   Group1DLayout L;
   std::memset(&L, 0, sizeof(L));
   L.item = item; L.nk = nk; L.nz = nz; L.nr = nr;
@@ -2004,11 +2032,11 @@ static Group1DLayout group1d_layout(int item, long nk, int nz, int nr, long npix
   const size_t nst = (size_t)(kchunk / 64);
   size_t off = 0;
   auto take = [&](size_t b) { size_t o = off; off += align256(b); return o; };
-  L.off_amp = take(sizeof(double2) * 12 * (size_t)nk);
+  L.off_amp = take(sizeof(double2) * c1d_amp_rows(sp.sym, sp.with_direct) * (size_t)nk);
   L.ldc = (nk + 3) / 4 * 4;
-  L.off_C = take(sizeof(float) * C1D_RT * (size_t)nz * L.ldc);
+  for (int o = 0; o < 3; ++o) L.N[o] = c1d_rows(sp.sym, o) * nz;
+  L.off_C = take(sizeof(float) * (size_t)(L.N[0] + L.N[1] + L.N[2]) * L.ldc);
   for (int o = 0; o < 3; ++o) {
-    L.N[o] = (o == 0 ? C1D_R0 : o == 1 ? C1D_R1 : C1D_R2) * nz;
     L.ctile[o] = bessel_i8_ctile(L.N[o]);
     L.Np[o] = ((L.ctile[o] + 15) / 16) * 16;
     L.ntn[o] = (L.N[o] + L.ctile[o] - 1) / L.ctile[o];
@@ -2032,8 +2060,7 @@ static Group1DLayout group1d_layout(int item, long nk, int nz, int nr, long npix
 struct Group1DDesc {
   size_t off_it, off_bp, off_first, bytes;
   int ni;
-  long grid[7];
-
+  long grid[9];
 };
 
 static bool group1d_eligible(const ytf_ctx* ctx, const ytf_green_desc& g) {
@@ -2100,7 +2127,7 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
     if (!cand.empty() && ctas / (double)slice < 2.0 * nsm)
       slice = std::max(64L, std::min(slice, (long)(ctas / (2.0 * nsm)) / 64 * 64));
     for (int i : cand)
-      lay.push_back(group1d_layout(i, d[i].cache->n, d[i].nz, (int)ur[i].size(), (long)d[i].nx * d[i].ny,
+      lay.push_back(group1d_layout(i, gsp[i], d[i].nz, (int)ur[i].size(), (long)d[i].nx * d[i].ny,
                                    !d[i].out_is_device, slice));
     std::stable_sort(lay.begin(), lay.end(), [](const Group1DLayout& a, const Group1DLayout& b) { return a.nk > b.nk; });
   }
@@ -2132,7 +2159,7 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
     D.off_bp = D.off_it + align256(sizeof(Synth1DItem) * ni);
     D.off_first = D.off_bp + align256(sizeof(BesselI8) * 3 * ni);
     D.bytes = align256(sizeof(Synth1DItem) * ni) + align256(sizeof(BesselI8) * 3 * ni) +
-              align256(sizeof(long) * (5 * (size_t)(ni + 1) + 2 * (size_t)(3 * ni + 1)));
+              align256(sizeof(long) * (7 * (size_t)(ni + 1) + 2 * (size_t)(3 * ni + 1)));
 
     desc_bytes += D.bytes;
   }
@@ -2178,9 +2205,11 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
     long* f_aimg = f_coef + (ni + 1);
     long* f_asm = f_aimg + (ni + 1);
     long* f_kmin = f_asm + (ni + 1);
-    long* f_bimg = f_kmin + (ni + 1);
+    long* f_rsym = f_kmin + (ni + 1);
+    long* f_csym = f_rsym + (ni + 1);
+    long* f_bimg = f_csym + (ni + 1);
     long* f_gemm = f_bimg + (3 * ni + 1);
-    long nref = 0, ncoef = 0, naimg = 0, nasm = 0, nbimg = 0, ngemm = 0, nkmin = 0;
+    long nref = 0, ncoef = 0, naimg = 0, nasm = 0, nbimg = 0, ngemm = 0, nkmin = 0, nrsym = 0, ncsym = 0;
     for (int q = 0; q < ni; ++q) {
       const size_t j = groups[g].first + q;
       const Group1DLayout& L = lay[j];
@@ -2193,6 +2222,7 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
       it.amp = (double2*)(base + L.off_amp);
       it.C = (float*)(base + L.off_C);
       it.ldc = L.ldc;
+      it.a.sym = it.sp.sym;
       it.a.nx = d[i].nx; it.a.ny = d[i].ny; it.a.nz = L.nz; it.a.nr = L.nr;
       it.a.xs = dc + o[i] + d[i].nz;
       it.a.ys = dc + o[i] + d[i].nz + d[i].nx;
@@ -2200,23 +2230,18 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
       it.a.G = d[i].out_is_device ? (double2*)d[i].out : (double2*)(base + L.off_G);
       it.a.nchunk = L.nchunk;
       it.kchunk = L.kchunk;
-      {  // evenly spaced heights (to 4 ulp of the progression): rows by recurrence
-        const double* zv = d[i].z_obs;
-        const int m = d[i].nz;
-        const double dz = m > 1 ? (zv[m - 1] - zv[0]) / (m - 1) : 0.0;
-        const double tol = 4 * 2.220446049250313e-16 * std::max(std::fabs(zv[0]), std::fabs(zv[m - 1]));
-        bool even = m > 1 && std::isfinite(dz) && dz != 0.0;
-        for (int r = 0; r < m && even; ++r) even = std::fabs(zv[r] - (zv[0] + r * dz)) <= tol;
-        it.dz = even ? dz : 0.0;
-      }
+      it.dz = even_spacing(d[i].z_obs, d[i].nz);  // rows by recurrence
       for (int od = 0; od < 3; ++od) it.a.part[od] = (const double*)(base + L.off_pt[od]);
       const long nkb = (L.nk + 127) / 128;
-      f_ref[q] = nref; nref += nkb;
-      f_coef[q] = ncoef; ncoef += nkb * ((L.nz + COEF1D_ZB_GROUP - 1) / COEF1D_ZB_GROUP);
+      const bool sym = it.sp.sym != 0;
+      f_ref[q] = nref; nref += sym ? 0 : nkb;
+      f_coef[q] = ncoef; ncoef += sym ? 0 : nkb * ((L.nz + COEF1D_ZB_GROUP - 1) / COEF1D_ZB_GROUP);
+      f_rsym[q] = nrsym; nrsym += sym ? nkb : 0;
+      f_csym[q] = ncsym; ncsym += sym ? nkb * ((L.nz + COEF_SYM_ZB - 1) / COEF_SYM_ZB) : 0;
       f_aimg[q] = naimg; naimg += ((long)L.ntm * 128 * L.nchunk * (L.kchunk / 4) + 255) / 256;
       f_asm[q] = nasm; nasm += asm1d_blocks(it.a);
       f_kmin[q] = nkmin; nkmin += L.nchunk;
-      const size_t coff[3] = {0, (size_t)C1D_OFF1 * L.nz * L.ldc, (size_t)C1D_OFF2 * L.nz * L.ldc};
+      const size_t coff[3] = {0, (size_t)L.N[0] * L.ldc, (size_t)(L.N[0] + L.N[1]) * L.ldc};
       for (int od = 0; od < 3; ++od) {
         BesselI8& bp = hbp[3 * q + od];
         std::memset(&bp, 0, sizeof(bp));
@@ -2242,9 +2267,10 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
       }
     }
     f_ref[ni] = nref; f_coef[ni] = ncoef; f_aimg[ni] = naimg; f_asm[ni] = nasm; f_kmin[ni] = nkmin;
+    f_rsym[ni] = nrsym; f_csym[ni] = ncsym;
     f_bimg[3 * ni] = nbimg; f_gemm[3 * ni] = ngemm;
-    const long grid[7] = {nref, ncoef, naimg, nbimg, ngemm, nasm, nkmin};
-    for (int k = 0; k < 7; ++k) D.grid[k] = grid[k];
+    const long grid[9] = {nref, ncoef, naimg, nbimg, ngemm, nasm, nkmin, nrsym, ncsym};
+    for (int k = 0; k < 9; ++k) D.grid[k] = grid[k];
   }
   CK(cudaMemcpyAsync(dc, h, total_bytes, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemsetAsync(err, 0, sizeof(unsigned), ctx->stream));
@@ -2262,9 +2288,11 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
     G.first_aimg = df + 2 * (ni + 1);
     G.first_asm = df + 3 * (ni + 1);
     G.first_kmin = df + 4 * (ni + 1);
-    G.first_bimg = df + 5 * (ni + 1);
+    G.first_rsym = df + 5 * (ni + 1);
+    G.first_csym = df + 6 * (ni + 1);
+    G.first_bimg = df + 7 * (ni + 1);
     G.first_gemm = G.first_bimg + (3 * ni + 1);
-    for (int k = 0; k < 7; ++k) G.grid[k] = D.grid[k];
+    for (int k = 0; k < 9; ++k) G.grid[k] = D.grid[k];
     CK(LAUNCH("k_reflect2d", launch_reflect_coef_group(G, 0, ctx->stream)));
     CK(LAUNCH("k_coef1d", launch_reflect_coef_group(G, 1, ctx->stream)));
     CK(LAUNCH("k_aimg_bessel3", launch_bessel_i8_group(G, 0, ctx->stream)));

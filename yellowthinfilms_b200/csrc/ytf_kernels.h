@@ -113,6 +113,7 @@ struct CacheView {
 
 struct SynthParams {
   CacheView c;
+  int sym;           // 1D: TE and TM decouple (c1d_rows, the symmetric coefficient columns)
   int same;          // obs layer == source layer
   int with_direct;   // add the same-layer direct term
   double uf_F, ub_F, uf_B, ub_B;  // seed masks of the reflected amplitudes (terms)
@@ -129,15 +130,25 @@ struct SynthParams {
 // exactly (the same products summed in swapped order, or negated: bit for bit); the pixel
 // assembly restores them. Real columns per height of orders 0, 1, 2 and the orders' offsets.
 constexpr int C1D_R0 = 6, C1D_R1 = 8, C1D_R2 = 4;
-constexpr int C1D_OFF1 = C1D_R0, C1D_OFF2 = C1D_R0 + C1D_R1, C1D_RT = C1D_R0 + C1D_R1 + C1D_R2;
-constexpr int C1D_RMAX = C1D_R1;  // the widest order
+constexpr int C1D_OFF1 = C1D_R0, C1D_OFF2 = C1D_R0 + C1D_R1;
+// In a stack of isotropic and uniaxial layers (ε_xz = ε_yz = 0) the two modes of a φ = 0 node are TE
+// (E_y only, driven by the y moment) and TM (E_x, E_z, driven by the x and z moments), so the
+// coefficients yx, zy and yz are identically zero and 5 columns are left, order 0: xx zz, order 1: zx
+// xz, order 2: xx. Per (node, height) they are sums of ten products of a height-independent factor
+// (k_reflect_sym) with a mode's phase.
+constexpr int C1S_R0 = 4, C1S_R1 = 4, C1S_R2 = 2;
+constexpr int C1S_AMP = 14, C1S_AMP_DIRECT = 24;  // complex rows of the factors, with the direct term's
+__host__ __device__ inline int c1d_rows(int sym, int order) {
+  return order == 0 ? (sym ? C1S_R0 : C1D_R0) : order == 1 ? (sym ? C1S_R1 : C1D_R1) : (sym ? C1S_R2 : C1D_R2);
+}
+inline int c1d_amp_rows(int sym, int with_direct) { return !sym ? 12 : with_direct ? C1S_AMP_DIRECT : C1S_AMP; }
 
 // 1D Jacobi-Anger synthesis
-// coefficient columns through per-node reflected amplitudes in amp ([12][n] complex scratch), rows
-// ldc apart
-cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, double* C, long ldc, cudaStream_t s);
+// coefficient columns through per-node amplitudes or factors in amp ([c1d_amp_rows][n] complex
+// scratch), rows ldc apart; dz: the spacing of evenly spaced heights, else 0
+cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, double* C, long ldc, double dz, cudaStream_t s);
 // the same columns rounded to FP32 (the int8x3 contraction's input)
-cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, float* C, long ldc, cudaStream_t s);
+cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, float* C, long ldc, double dz, cudaStream_t s);
 // J_n tables, rows ld apart
 cudaError_t launch_bessel_c(const double* kr, const double* kri, long nk, const double* rho, int nr, long ld, double* J,
                             cudaStream_t s);
@@ -167,6 +178,7 @@ cudaError_t launch_gemm64(Gemm64 p, cudaStream_t s);
 cudaError_t launch_sum_slices(long len, int nz, const double* part, double* acc, int add, cudaStream_t s);
 // slice sums and pixel assembly of one 1D synthesis
 struct Asm1D {
+  int sym;
   int nx, ny, nz, nr;
   const double* xs;          // device
   const double* ys;
@@ -323,8 +335,8 @@ cudaError_t launch_gemm_i8(const BesselI8* e, int n, cudaStream_t s);
 // ------------------------------------------------------------------------------------
 struct Synth1DItem {
   SynthParams sp;          // the item's node data (real nodes), term masks, heights (device)
-  double2* amp;            // [12][nk] reflected amplitudes
-  float* C;                // [26 nz][ldc] coefficient columns: orders 0, 1, 2 at rows 0, 10 nz, 18 nz
+  double2* amp;            // [c1d_amp_rows][nk] reflected amplitudes, or factors (sym)
+  float* C;                // coefficient columns [c1d_rows nz][ldc] of orders 0, 1, 2 in turn
   long ldc;                // row stride of C: nk rounded up to 4, so every row starts on 16 bytes
   Asm1D a;                 // pixel grid, radii, slice partials, output
   long kchunk;             // nodes per slice (a multiple of 64)
@@ -333,7 +345,7 @@ struct Synth1DItem {
 // every stage of the group, in order, on stream s; `it`/`bp` and the `first_*` tables are
 // device arrays (bp: 3 entries per item, orders 0, 1, 2; bp[3i] also carries the layout of
 // item i's J_n images). Host copies (ni, grid sizes) come in `grid`: {reflect, coef, aimg,
-// bimg, gemm, assemble, slice minima}.
+// bimg, gemm, assemble, slice minima, factors, symmetric coef}.
 struct Synth1DGroup {
   int ni;
   const Synth1DItem* it;
@@ -345,7 +357,9 @@ struct Synth1DGroup {
   const long* first_gemm;      // [3 ni + 1]
   const long* first_asm;       // [ni + 1]
   const long* first_kmin;      // [ni + 1]
-  long grid[7];
+  const long* first_rsym;      // [ni + 1] symmetric items' factors and columns (first_reflect and
+  const long* first_csym;      // [ni + 1] first_coef count the other items)
+  long grid[9];
 };
 // the entry whose block range holds block b: the last e with first[e] <= b (first ascending)
 __device__ __forceinline__ int group_entry(const long* first, int ne, long b) {
@@ -364,6 +378,7 @@ cudaError_t launch_reflect_coef_group(const Synth1DGroup& g, int stage, cudaStre
 cudaError_t launch_bessel_i8_group(const Synth1DGroup& g, int stage, cudaStream_t s);
 cudaError_t launch_assemble1d_group(const Synth1DGroup& g, cudaStream_t s);    // slice sum + pixel assembly
 constexpr int COEF1D_ZB_GROUP = 8;   // heights per thread of the grouped coefficient kernel
+constexpr int COEF_SYM_ZB = 16;      // and of the symmetric one
 
 // Gauss-Legendre panels -> nodes/weights, bit-exact with the CPU restatement
 cudaError_t launch_gl_nodes(int npanels, const double* pa, const double* pb, const int* sing_side, const double* xi,

@@ -583,12 +583,25 @@ __device__ __forceinline__ void assemble1d_body(const Asm1D& a, long b) {
   const int zi = (int)(t / npix);
   const int ix = (int)(pix % a.nx), iy = (int)(pix / a.nx);
   const int r = a.rmap[pix];
-  cd s0[C1D_R0 / 2], s1[C1D_R1 / 2], s2[C1D_R2 / 2], g0[5], g1[4], g2[4];
-  order_columns<C1D_R0>(a, 0, zi, r, first, step, s0);
-  order_columns<C1D_R1>(a, 1, zi, r, first, step, s1);
-  order_columns<C1D_R2>(a, 2, zi, r, first, step, s2);
+  cd g0[5], g1[4], g2[4];
+  if (a.sym) {
+    cd s0[C1S_R0 / 2], s1[C1S_R1 / 2], s2[C1S_R2 / 2];
+    order_columns<C1S_R0>(a, 0, zi, r, first, step, s0);
+    order_columns<C1S_R1>(a, 1, zi, r, first, step, s1);
+    order_columns<C1S_R2>(a, 2, zi, r, first, step, s2);
+    const cd z{0.0, 0.0};
+    g0[0] = g0[3] = s0[0]; g0[1] = g0[2] = z; g0[4] = s0[1];
+    g1[0] = s1[0]; g1[2] = s1[1]; g1[1] = g1[3] = z;
+    g2[0] = s2[0]; g2[3] = -s2[0]; g2[1] = g2[2] = z;
+  } else {
+    cd s0[C1D_R0 / 2], s1[C1D_R1 / 2], s2[C1D_R2 / 2];
+    order_columns<C1D_R0>(a, 0, zi, r, first, step, s0);
+    order_columns<C1D_R1>(a, 1, zi, r, first, step, s1);
+    order_columns<C1D_R2>(a, 2, zi, r, first, step, s2);
+    unpack_order_sums([&](int c) { return s0[c]; }, [&](int c) { return s1[c]; }, [&](int c) { return s2[c]; }, g0, g1,
+                      g2);
+  }
   if (!live || first > 0) return;
-  unpack_order_sums([&](int c) { return s0[c]; }, [&](int c) { return s1[c]; }, [&](int c) { return s2[c]; }, g0, g1, g2);
   assemble1d_pixel(a.xs[ix], a.ys[iy], g0, g1, g2, pix, npix, zi, nz, a.G);
 }
 
@@ -704,22 +717,208 @@ __global__ void __launch_bounds__(128) k_coef1d_amp(SynthParams p, const double2
   }
 }
 
+// ------------------------------------------------------------------------------------
+// The symmetric columns (c1d_rows). Factors per node, rows of n (W = i w / 2π, a = the amplitude of
+// the moment, e = the mode field, k the node, f / b the forward and backward wave):
+//   0, 1  T: -(i/2) W a_y e_y k of TE      2, 3  P: -(i/2) W a_x e_x k of TM
+//   4, 5  W a_x e_z k of TM                6, 7  W a_z e_x k             8, 9  -i W a_z e_z k
+//   10-13 kz of TE f, TE b, TM f, TM b     14-23 the direct term's T, P, ... (f above the source, b below)
+// and per height, g the branch phases: xx of order 0 = Σ T g + Σ P g, of order 2 = Σ T g - Σ P g,
+// zx = Σ (4, 5) g, xz = Σ (6, 7) g, zz = Σ (8, 9) g. About 60 FP64 operations per (node, height),
+// against 350 for the nine general columns from the amplitudes, and 10 stored columns against 18:
+// 325k nodes x 64 heights took 1083 us and take 278 us (bound by the 832 MB of columns written, 127 us
+// at the copy rate, and the FP64 pipe).
+// ------------------------------------------------------------------------------------
+__device__ __forceinline__ void reflect_sym_body(const SynthParams& p, long k, double2* amp) {
+  const CacheView& c = p.c;
+  const long n = c.n;
+  cd Af[2][3], Ab[2][3];
+  reflected_amp(p, k, Af, Ab);
+  const cd W = cd{0.0, 1.0 / (2.0 * 3.14159265358979323846)} * cd{c.wr[k], c.wri ? c.wri[k] : 0.0};
+  const cd kx{c.kr[k], c.kri ? c.kri[k] : 0.0};
+  // which of the two modes is TE: the one with the larger E_y (the other's is zero)
+  const bool te1 = norm2(ldc(c.basis, 3, n, k)) + norm2(ldc(c.basis, 9, n, k)) >
+                   norm2(ldc(c.basis, 2, n, k)) + norm2(ldc(c.basis, 8, n, k));
+  const int te = te1 ? 1 : 0, tm = 1 - te;
+  auto put = [&](int row, cd v) { amp[(long)row * n + k] = make_double2(v.x, v.y); };
+  const cd half{0.0, -0.5};
+#pragma unroll
+  for (int br = 0; br < 2; ++br) {
+    const cd ey = ldc(c.basis, (br == 0 ? 2 : 8) + te, n, k);
+    const cd ex = ldc(c.basis, (br == 0 ? 0 : 6) + tm, n, k), ez = ldc(c.basis, (br == 0 ? 4 : 10) + tm, n, k);
+    auto factors = [&](int row, cd ax, cd ay, cd az) {
+      const cd wx = fin0(W * ax) * kx, wy = fin0(W * ay) * kx, wz = fin0(W * az) * kx;
+      put(row + br, half * (wy * ey));
+      put(row + 2 + br, half * (wx * ex));
+      put(row + 4 + br, wx * ez);
+      put(row + 6 + br, wz * ex);
+      put(row + 8 + br, cd{0.0, -1.0} * (wz * ez));
+    };
+    const cd(*A)[3] = br == 0 ? Af : Ab;
+    factors(0, te1 ? A[0][0] : A[1][0], te1 ? A[1][1] : A[0][1], te1 ? A[0][2] : A[1][2]);
+    if (p.with_direct) {
+      const double2* sd = br == 0 ? c.sf : c.sb;
+      const bool v = c.valid[k];
+      const cd z{0.0, 0.0};
+      factors(C1S_AMP, v ? ldc(sd, tm, n, k) : z, v ? ldc(sd, te + 2, n, k) : z, v ? ldc(sd, tm + 4, n, k) : z);
+    }
+    put(10 + br, ldc(c.basis, (br == 0 ? 12 : 14) + te, n, k));
+    put(12 + br, ldc(c.basis, (br == 0 ? 12 : 14) + tm, n, k));
+  }
+}
+__global__ void __launch_bounds__(128) k_reflect_sym(SynthParams p, double2* __restrict__ amp) {
+  const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < p.c.n) reflect_sym_body(p, k, amp);
+}
+
+// e^{a + i b}, out of line: the exact phases are the rare case of the recurrence over the heights
+__device__ __noinline__ cd cexp_call(double a, double b) { return cexp(cd{a, b}); }
+__device__ __forceinline__ cd phase_call(cd kz, double z) { return cexp_call(-kz.y * z, kz.x * z); }
+
+template <class T>
+__device__ __forceinline__ void store_sym_row(T* C0, T* C1, T* C2, long cst, long k, int zi, const cd c[5]) {
+  const long r4 = 4L * zi, r2 = 2L * zi;
+  C0[r4 * cst + k] = (T)c[0].x; C0[(r4 + 1) * cst + k] = (T)c[0].y;
+  C0[(r4 + 2) * cst + k] = (T)c[1].x; C0[(r4 + 3) * cst + k] = (T)c[1].y;
+  C1[r4 * cst + k] = (T)c[2].x; C1[(r4 + 1) * cst + k] = (T)c[2].y;
+  C1[(r4 + 2) * cst + k] = (T)c[3].x; C1[(r4 + 3) * cst + k] = (T)c[3].y;
+  C2[r2 * cst + k] = (T)c[4].x; C2[(r2 + 1) * cst + k] = (T)c[4].y;
+}
+
+// rows whose phases or factors leave the fast path's range: the general columns' arithmetic with its
+// clamps, out of line
+template <class T>
+__device__ __noinline__ void coef_sym_exact(const SynthParams& p, long k, int z0, int z1, T* C0, T* C1, T* C2, long cst) {
+  cd Af[2][3], Ab[2][3];
+  reflected_amp(p, k, Af, Ab);
+  for (int zi = z0; zi < z1; ++zi) {
+    cd c0[5], c1[4], c2[4];
+    coef1d_row(p, k, p.zo[zi], Af, Ab, c0, c1, c2);
+    const cd c[5] = {c0[0], c0[4], c1[0], c1[2], c2[0]};
+    store_sym_row(C0, C1, C2, cst, k, zi, c);
+  }
+}
+
+// rows z0 .. z1 - 1 of one node. Evenly spaced heights (dz != 0): each branch phase by one complex
+// product per row, e^{i kz (z + dz)} = e^{i kz z} e^{i kz dz}, where every exponent stays in
+// [-600, 80] (no underflowed start, no overflow); other heights: one exponential per branch and row.
+template <class T>
+__device__ __forceinline__ void coef_sym_rows(const SynthParams& p, const double2* amp, long k, int z0, int z1, double dz,
+                                              T* C0, T* C1, T* C2, long cst) {
+  const long n = p.c.n;
+  cd F[10], kz[4];  // kz: TE f, TE b, TM f, TM b
+#pragma unroll
+  for (int i = 0; i < 10; ++i) F[i] = ldc(amp, i, n, k);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) kz[i] = ldc(amp, 10 + i, n, k);
+  double zlo = p.zo[z0], zhi = zlo;
+  for (int zi = z0 + 1; zi < z1; ++zi) { zlo = fmin(zlo, p.zo[zi]); zhi = fmax(zhi, p.zo[zi]); }
+  double big = 0.0, lo = 0.0, hi = 0.0;
+#pragma unroll
+  for (int i = 0; i < 10; ++i) big += fabs(F[i].x) + fabs(F[i].y);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    big += fabs(kz[i].x) * (fabs(zlo) + fabs(zhi));
+    const double s = i & 1 ? p.d_obs : 0.0;
+    const double a = -kz[i].y * (zlo - s), b = -kz[i].y * (zhi - s);
+    lo = fmin(lo, fmin(a, b));
+    hi = fmax(hi, fmax(a, b));
+    if (p.with_direct) {  // ζ > 0 forward, ζ < 0 backward: the far end of the rows on that side
+      const double zeta = i & 1 ? fmin(zlo - p.zpos, 0.0) : fmax(zhi - p.zpos, 0.0);
+      lo = fmin(lo, -kz[i].y * zeta);
+      hi = fmax(hi, -kz[i].y * zeta);
+    }
+    big += fabs(kz[i].y);
+  }
+  if (p.with_direct)
+    for (int i = C1S_AMP; i < C1S_AMP_DIRECT; ++i) { const cd v = ldc(amp, i, n, k); big += fabs(v.x) + fabs(v.y); }
+  if (!(big < 1e200 && hi <= 80.0)) {  // also any NaN
+    coef_sym_exact(p, k, z0, z1, C0, C1, C2, cst);
+    return;
+  }
+  const bool rec = dz != 0.0 && lo >= -600.0;
+  cd step[4], g[4], gd[2];
+  if (rec)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) step[i] = phase_call(kz[i], dz);
+  int side = 0;  // of the source: +1 above, -1 below, where gd holds the last row's direct phases
+  for (int zi = z0; zi < z1; ++zi) {
+    const double z = p.zo[zi];
+    if (rec && zi > z0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) g[i] = g[i] * step[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) g[i] = phase_call(kz[i], i & 1 ? z - p.d_obs : z);
+    }
+    cd t = F[0] * g[0], q = F[2] * g[2];
+    cd c[5];
+    t += F[1] * g[1];
+    q += F[3] * g[3];
+    c[2] = F[4] * g[2];
+    c[2] += F[5] * g[3];
+    c[3] = F[6] * g[2];
+    c[3] += F[7] * g[3];
+    c[1] = F[8] * g[2];
+    c[1] += F[9] * g[3];
+    if (p.with_direct) {
+      const double zeta = z - p.zpos;
+      const int now = zeta > 0 ? 1 : zeta < 0 ? -1 : 0, br = now < 0 ? 1 : 0;
+      if (now != 0) {
+        if (rec && now == side) {
+          gd[0] = gd[0] * (br ? step[1] : step[0]);
+          gd[1] = gd[1] * (br ? step[3] : step[2]);
+        } else {
+          gd[0] = phase_call(br ? kz[1] : kz[0], zeta);
+          gd[1] = phase_call(br ? kz[3] : kz[2], zeta);
+        }
+        t += ldc(amp, C1S_AMP + br, n, k) * gd[0];
+        q += ldc(amp, C1S_AMP + 2 + br, n, k) * gd[1];
+        c[2] += ldc(amp, C1S_AMP + 4 + br, n, k) * gd[1];
+        c[3] += ldc(amp, C1S_AMP + 6 + br, n, k) * gd[1];
+        c[1] += ldc(amp, C1S_AMP + 8 + br, n, k) * gd[1];
+      }
+      side = now;
+    }
+    c[0] = t + q;
+    c[4] = t - q;
+    store_sym_row(C0, C1, C2, cst, k, zi, c);
+  }
+}
+
+template <class T>
+__global__ void __launch_bounds__(128, 4) k_coef_sym(SynthParams p, const double2* __restrict__ amp, T* C0, T* C1, T* C2,
+                                                     long cst, double dz) {
+  const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= p.c.n) return;
+  const int z0 = blockIdx.y * COEF_SYM_ZB;
+  coef_sym_rows(p, amp, k, z0, min(p.nz, z0 + COEF_SYM_ZB), dz, C0, C1, C2, cst);
+}
+
 // the order-0 rows at C, orders 1 and 2 behind them
 template <class T>
-static cudaError_t coef1d_amp_impl(const SynthParams& p, double2* amp, T* C, long ldc, cudaStream_t s) {
+static cudaError_t coef1d_amp_impl(const SynthParams& p, double2* amp, T* C, long ldc, double dz, cudaStream_t s) {
   if (p.c.n <= 0 || p.nz <= 0) return cudaSuccess;
+  if (p.sym) {
+    const unsigned nb = (unsigned)((p.c.n + 127) / 128);
+    T* C1 = C + (size_t)C1S_R0 * p.nz * ldc;
+    k_reflect_sym<<<nb, 128, 0, s>>>(p, amp);
+    k_coef_sym<T><<<dim3(nb, (unsigned)((p.nz + COEF_SYM_ZB - 1) / COEF_SYM_ZB)), 128, 0, s>>>(
+        p, amp, C, C1, C1 + (size_t)C1S_R1 * p.nz * ldc, ldc, dz);
+    return cudaGetLastError();
+  }
   k_reflect2d<<<(unsigned)((p.c.n + 127) / 128), 128, 0, s>>>(p, amp);
   k_coef1d_amp<T><<<dim3((unsigned)((p.c.n + 127) / 128), (unsigned)((p.nz + COEF1D_ZB - 1) / COEF1D_ZB)), 128, 0, s>>>(
       p, amp, C, C + (size_t)C1D_OFF1 * p.nz * ldc, C + (size_t)C1D_OFF2 * p.nz * ldc, ldc);
   return cudaGetLastError();
 }
 
-cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, double* C, long ldc, cudaStream_t s) {
-  return coef1d_amp_impl<double>(p, amp, C, ldc, s);
+cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, double* C, long ldc, double dz, cudaStream_t s) {
+  return coef1d_amp_impl<double>(p, amp, C, ldc, dz, s);
 }
 
-cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, float* C, long ldc, cudaStream_t s) {
-  return coef1d_amp_impl<float>(p, amp, C, ldc, s);
+cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, float* C, long ldc, double dz, cudaStream_t s) {
+  return coef1d_amp_impl<float>(p, amp, C, ldc, dz, s);
 }
 
 // per node of a k_strengths_rows block: 12 amplitudes, the obs-layer basis (16), sf, sb (6 each),
@@ -1290,9 +1489,6 @@ __device__ __noinline__ void coef_rows_direct(const Synth1DItem& it, long k, int
   }
 }
 
-// e^{a + i b}, out of line: the exact phases are the rare case of the recurrence below
-__device__ __noinline__ cd cexp_call(double a, double b) { return cexp(cd{a, b}); }
-
 // blocks of an item: ceil(n / 128) node blocks x ceil(nz / COEF1D_ZB_GROUP) height blocks,
 // node block fastest. For
 // the scattered terms at evenly spaced heights (it.dz != 0) the branch phases of a thread's
@@ -1377,8 +1573,31 @@ __global__ void __launch_bounds__(128, 3) k_coef1d_group(const Synth1DItem* __re
   }
 }
 
+__global__ void __launch_bounds__(128) k_reflect_sym_group(const Synth1DItem* __restrict__ items,
+                                                           const long* __restrict__ first, int ni) {
+  const int i = group_entry(first, ni, blockIdx.x);
+  const long k = (long)(blockIdx.x - first[i]) * blockDim.x + threadIdx.x;
+  if (k < items[i].sp.c.n) reflect_sym_body(items[i].sp, k, items[i].amp);
+}
+// node block fastest, as k_coef1d_group
+__global__ void __launch_bounds__(128, 4) k_coef_sym_group(const Synth1DItem* __restrict__ items,
+                                                           const long* __restrict__ first, int ni) {
+  const int i = group_entry(first, ni, blockIdx.x);
+  const Synth1DItem& it = items[i];
+  const SynthParams& p = it.sp;
+  const long nkb = (p.c.n + 127) / 128, b = blockIdx.x - first[i];
+  const long k = (b % nkb) * 128 + threadIdx.x;
+  if (k >= p.c.n) return;
+  const int z0 = (int)(b / nkb) * COEF_SYM_ZB;
+  float* C1 = it.C + (long)C1S_R0 * p.nz * it.ldc;
+  coef_sym_rows(p, it.amp, k, z0, min(p.nz, z0 + COEF_SYM_ZB), it.dz, it.C, C1, C1 + (long)C1S_R1 * p.nz * it.ldc,
+                it.ldc);
+}
+
 cudaError_t launch_reflect_coef_group(const Synth1DGroup& g, int stage, cudaStream_t s) {
   if (g.ni <= 0) return cudaSuccess;
+  if (stage == 0 && g.grid[7] > 0) k_reflect_sym_group<<<(unsigned)g.grid[7], 128, 0, s>>>(g.it, g.first_rsym, g.ni);
+  if (stage == 1 && g.grid[8] > 0) k_coef_sym_group<<<(unsigned)g.grid[8], 128, 0, s>>>(g.it, g.first_csym, g.ni);
   if (stage == 0 && g.grid[0] > 0) k_reflect2d_group<<<(unsigned)g.grid[0], 128, 0, s>>>(g.it, g.first_reflect, g.ni);
   if (stage == 1 && g.grid[1] > 0) k_coef1d_group<<<(unsigned)g.grid[1], 128, 0, s>>>(g.it, g.first_coef, g.ni);
   return cudaGetLastError();
