@@ -84,3 +84,19 @@ def test_1d_heights_past_the_phase_recurrence(oracle, d, z, obs, terms):
     assert relerr(G, Go) < 1e-10
     for i in range(len(z)):  # every height on its own scale
         assert relerr(G[:, :, i], Go[:, :, i]) < 1e-9 or np.linalg.norm(Go[:, :, i]) < 1e-280
+
+
+def test_bessel_pair_of_the_images():
+    """J_0, J_1 of the digit images: the Taylor rows to 4 units of 1 (their rounding) below 25, at row
+    edges and centres, the asymptotic pair to 1e-12 from 25 on, odd and even for negative x."""
+    from scipy.special import j0, j1
+    from yellowthinfilms_b200 import api
+    e = np.arange(26.0)
+    x = np.concatenate([[0.0], np.linspace(0, 25, 5001)[:-1], e[1:] - 1e-14 * e[1:], e[:-1] + 0.5])
+    a, b = api.bessel_j01(np.concatenate([x, -x]))
+    tol = 4 * 2.3e-16 + 4e-16  # and the reference's own error
+    assert np.abs(a - np.tile(j0(x), 2)).max() <= tol
+    assert np.abs(b - np.concatenate([j1(x), -j1(x)])).max() <= tol
+    x = np.concatenate([np.linspace(25, 60, 3001), np.geomspace(60, 1e5, 3001)])
+    a, b = api.bessel_j01(x)
+    assert np.abs(a - j0(x)).max() <= 1e-12 and np.abs(b - j1(x)).max() <= 1e-12

@@ -470,7 +470,7 @@ def rule_panels(stack, omega, source_layer, h_min, rho_max=0.0, target_decay=25.
 
 def bessel_j01(x, ctx: Optional[Context] = None):
     """(J_0(x), J_1(x)) of real x as the int8x3 1D synthesis evaluates them
-    (ytf_bessel_j01: the CUDA library below |x| = 25, Hankel's asymptotic pair above)."""
+    (ytf_bessel_j01: Taylor rows below |x| = 25, Hankel's asymptotic pair above)."""
     ctx = ctx or default_context()
     x = _f64(x)
     a, b = np.zeros(len(x)), np.zeros(len(x))

@@ -16,6 +16,7 @@
 // INT32 headroom: |level-2 sum| ≤ (127·128 + 128·128 + 128·127) K ≤ 48896 · 16384 < 2^30.
 #include "ytf_complex.cuh"
 #include "ytf_kernels.h"
+#include "ytf_bessel_tab.cuh"
 #include "ytf_tcgen05.cuh"
 
 namespace ytf {
@@ -39,36 +40,56 @@ int bessel_i8_ctile(int N) {
   return (N + nt - 1) / nt;
 }
 
-// J_2 from J_0, J_1: its power series below |x| = 1 (A&S 9.1.10; exact 0 at x = 0; the term
-// ratio -h²/((m + 1)(m + 3)) with the reciprocals as constants) and the three-term recurrence
-// above (A&S 9.1.27)
-__device__ __forceinline__ double j2_from(double x, double J0, double J1) {
-  if (fabs(x) < 1.0) {
-    constexpr double inv[12] = {1.0 / 3, 1.0 / 8, 1.0 / 15, 1.0 / 24, 1.0 / 35, 1.0 / 48,
-                                1.0 / 63, 1.0 / 80, 1.0 / 99, 1.0 / 120, 1.0 / 143, 1.0 / 168};
+// J_2 from J_0, J_1 at x >= 0, y = 1 / x: its power series below x = 1 (A&S 9.1.10; exact 0 at x = 0;
+// 9 terms, the first left out below 1e-18) and the three-term recurrence above (A&S 9.1.27)
+__device__ __forceinline__ double j2_from(double x, double y, double J0, double J1) {
+  if (x < 1.0) {
+    // (h2 / 2) Σ_m (-h2)^m 2 / (m! (m + 2)!), h2 = x² / 4
     const double h2 = 0.25 * x * x;
-    double t = 0.5 * h2, s = t;
-#pragma unroll
-    for (int m = 0; m < 12; ++m) {
-      t *= -h2 * inv[m];
-      s += t;
-    }
-    return s;
+    double s = 1.0 / (40320.0 * 1814400.0);
+    s = fma(s, h2, -1.0 / (5040.0 * 181440.0));
+    s = fma(s, h2, 1.0 / (720.0 * 20160.0));
+    s = fma(s, h2, -1.0 / (120.0 * 2520.0));
+    s = fma(s, h2, 1.0 / (24.0 * 360.0));
+    s = fma(s, h2, -1.0 / (6.0 * 60.0));
+    s = fma(s, h2, 1.0 / (2.0 * 12.0));
+    s = fma(s, h2, -1.0 / 3.0);
+    s = fma(s, h2, 1.0);
+    return 0.5 * h2 * s;
   }
-  return (2.0 / x) * J1 - J0;
+  return fma(2.0 * y, J1, -J0);
+}
+
+// J_0(x), J_1(x) for 0 <= x < 25 from the Taylor rows (tab: JTAB, or a copy of it in shared memory): one
+// Horner pass for the value and the derivative, 31 FP64 operations for both orders, |error| <= 2e-16.
+// The math library's j0 and j1 take their own argument ranges apart in every warp: 4096 radii x 65536
+// nodes, 64% of them below 25: 3183 us with them, 1395 us in the present image kernel.
+__device__ __forceinline__ void j01_small(double x, const double* __restrict__ tab, double& J0, double& J1) {
+  const int i = min(max((int)x, 0), JTAB_N - 1);
+  const double d = x - ((double)i + 0.5);
+  const double* c = tab + i * JTAB_M;
+  double p = c[JTAB_M - 1], q = 0.0;
+#pragma unroll
+  for (int m = JTAB_M - 2; m >= 0; --m) {
+    q = fma(q, d, p);
+    p = fma(p, d, c[m]);
+  }
+  J0 = p;
+  J1 = -q;
 }
 
 // J_0(x) and J_1(x) for x >= 25 (absolute error below 1e-12): Hankel's asymptotic expansions
 // (A&S 9.2.5, 9.2.9, 9.2.10), J_n(x) = sqrt(2 / (π x)) (P_n cos χ_n - Q_n sin χ_n) with
 // χ_n = x - (2n + 1) π / 4, five terms each of P_n and Q_n in y = 1/x (the coefficient of y^m
 // is ±a_m / 8^m, a_m = Π_{j<=m} (4n² - (2j - 1)²) / m!). Both orders share one phase
-// (χ_1 = χ_0 - π/2): cos x and sin x from a Cody-Waite reduction by π/2 (a three-part
-// constant whose first two parts carry 33 bits, so n π/2 is exact for n < 2^20) and Taylor
-// polynomials on |r| <= π/4 (to r^17 and r^18), then cos χ_0 = (cos x + sin x)/√2 and
-// sin χ_0 = (sin x - cos x)/√2. The library's j0 and j1 evaluate each order with its own phase.
+// (χ_1 = χ_0 - π/2): χ_0 = r + n π/2, |r| <= π/4, by a Cody-Waite reduction of x by (n + 1/2) π/2 (a
+// three-part constant whose first two parts carry 33 bits, so its products are exact for n < 2^19)
+// and Taylor polynomials for sin r and cos r (to r^17 and r^18). The library's j0 and j1 evaluate each
+// order with its own phase.
 constexpr double J_ASYM_MIN = 25.0;
-__device__ __forceinline__ void j01_large(double x, double& J0, double& J1) {
-  const double y = 1.0 / x, y2 = y * y;
+// y = 1 / x, a = sqrt(2 / (π x)) (products of per-node and per-radius factors in the image kernel)
+__device__ __forceinline__ void j01_large(double x, double y, double a, double& J0, double& J1) {
+  const double y2 = y * y;
   const double p0 = fma(fma(fma(fma(6.074042001273483, y2, -0.5725014209747314), y2, 0.112152099609375), y2,
                             -0.0703125), y2, 1.0);
   const double q0 = y * fma(fma(fma(fma(-24.380529699556064, y2, 1.7277275025844574), y2, -0.22710800170898438), y2,
@@ -77,11 +98,12 @@ __device__ __forceinline__ void j01_large(double x, double& J0, double& J1) {
                             0.1171875), y2, 1.0);
   const double q1 = y * fma(fma(fma(fma(27.248827311268542, y2, -1.993531733751297), y2, 0.2775764465332031), y2,
                                 -0.1025390625), y2, 0.375);
-  // x = n π/2 + r, |r| <= π/4
-  const double n = rint(x * 0.6366197723675814);
-  double r = fma(-n, 1.5707963267341256, x);
-  r = fma(-n, 6.077100506303966e-11, r);
-  r = fma(-n, 2.0222662487959506e-21, r);
+  // x - π/4 = n π/2 + r, |r| <= π/4; nm holds n in its low bits
+  const double nm = fma(x, 0.6366197723675814, 6755399441055744.0 - 0.5);
+  const double m = (nm - 6755399441055744.0) + 0.5;
+  double r = fma(-m, 1.5707963267341256, x);
+  r = fma(-m, 6.077100506303966e-11, r);
+  r = fma(-m, 2.0222662487959506e-21, r);
   const double r2 = r * r;
   double sr = fma(fma(fma(fma(fma(fma(fma(2.8114572543455206e-15, r2, -7.647163731819816e-13), r2,
                                           1.6059043836821613e-10), r2, -2.505210838544172e-08), r2,
@@ -93,23 +115,24 @@ __device__ __forceinline__ void j01_large(double x, double& J0, double& J1) {
                                   -2.755731922398589e-07), r2, 2.48015873015873e-05), r2, -0.001388888888888889), r2,
                   0.041666666666666664), r2, -0.5);
   cr = fma(r2, cr, 1.0);
-  const int q = (int)((long long)n & 3);
-  const double sx = q == 0 ? sr : q == 1 ? cr : q == 2 ? -sr : -cr;
-  const double cx = q == 0 ? cr : q == 1 ? -sr : q == 2 ? -cr : sr;
-  const double c0 = (cx + sx) * 0.7071067811865476, s0 = (sx - cx) * 0.7071067811865476;
-  const double a = 0.7978845608028654 * sqrt(y);
+  // quadrant n: swap for odd n, signs from bit 1 of n (sine) and of n + 1 (cosine)
+  const int q = __double2loint(nm);
+  const double ss = q & 1 ? cr : sr, cc = q & 1 ? sr : cr;
+  const double s0 = __hiloint2double(__double2hiint(ss) ^ ((q & 2) << 30), __double2loint(ss));
+  const double c0 = __hiloint2double(__double2hiint(cc) ^ (((q + 1) & 2) << 30), __double2loint(cc));
   J0 = a * (p0 * c0 - q0 * s0);
   J1 = a * (p1 * s0 + q1 * c0);
 }
-// J_0, J_1 as the int8x3 J images take them: the asymptotic pair from x = 25, the library below
+// J_0, J_1 as the int8x3 J images take them: the asymptotic pair from x = 25, the Taylor rows below
 __device__ __forceinline__ void j01_real(double x, double& J0, double& J1) {
-  if (fabs(x) >= J_ASYM_MIN) {
-    j01_large(fabs(x), J0, J1);
-    if (x < 0) J1 = -J1;  // J_1 is odd
+  const double ax = fabs(x);
+  if (ax >= J_ASYM_MIN) {
+    const double y = 1.0 / ax;
+    j01_large(ax, y, 0.7978845608028654 * sqrt(y), J0, J1);
   } else {
-    J0 = j0(x);
-    J1 = j1(x);
+    j01_small(ax, JTAB, J0, J1);
   }
+  if (x < 0) J1 = -J1;  // J_1 is odd
 }
 
 __global__ void k_bessel_j01(const double* __restrict__ x, long n, double* __restrict__ J0, double* __restrict__ J1) {
@@ -248,65 +271,128 @@ __device__ __forceinline__ void bimg_slice_body(const BesselI8& p, long b) {
   }
 }
 
-// the J_n(k ρ) digit images of all three orders: J_0 and J_1 once per (ρ, k), J_2 from them (series
-// below |x| = 1, recurrence above), three images in the same layout.
-// One thread per 4 consecutive nodes of a radius (one 32-bit word of each digit plane): the
-// FP64 Bessel chains are latency-bound, so short chains and many threads.
-__device__ __forceinline__ void aimg_bessel3_body(const BesselI8& p, long t, uint8_t* __restrict__ A0,
+// ------------------------------------------------------------------------------------
+// The J_n(k ρ) digit images of all three orders: J_0 and J_1 once per (ρ, k), J_2 from them. A block
+// takes one 64-node stage of p.arows rows of a radius tile: thread (w, r) = (tid & 15, tid >> 4) nodes
+// 4 w .. 4 w + 3 of rows r, r + 16, ..., so that 1/k and 1/sqrt(k) are formed once per thread, 1/ρ,
+// sqrt(2/(π ρ)) and the row's digit scale once per row, and a pair needs no division and no root. Where
+// a warp's pairs all lie on one side of x = 25 a thread's four run side by side. The
+// fixed-point value comes from one FMA: v sA + 1.5 2^52 + 0x808080 holds rint(v sA) + 0x808080 in its
+// low word, whose bytes are the three digits with their sign bits flipped; four nodes' words transpose
+// into one word per digit plane by byte permutes.
+//   Bound: the FP64 pipe (59% busy; about 40 operations per pair below x = 25 and 60 above) and the wait
+// between dependent ones. 325k nodes x 256 radii: 491 us; with 64-bit index divisions, library j0 and
+// j1, a division and a root per pair and FP64-to-integer conversions, 1363 us; this form with 32-row
+// blocks and one pair after the other, 806 us.
+// ------------------------------------------------------------------------------------
+constexpr double AI_MAGIC = 6755399441055744.0 + 8421504.0;  // 1.5 2^52 + 0x808080
+
+// rows per block: a whole tile (the per-thread reciprocals then serve 32 pairs) once the stages alone
+// give each SM eight blocks, a quarter of it below
+int bessel_i8_arows(long stages) { return stages >= 8 * 148 ? BI_M : BI_M / 4; }
+long bessel_i8_aimg_blocks(const BesselI8& p) {
+  return (long)p.ntile_m * (BI_M / p.arows) * p.nchunk * (p.kchunk / BI_NODES);
+}
+
+__device__ __forceinline__ void aimg_bessel3_body(const BesselI8& p, long b, uint8_t* __restrict__ A0,
                                                   uint8_t* __restrict__ A1, uint8_t* __restrict__ A2) {
-  const long words = p.kchunk / 4;
-  const long total = (long)p.ntile_m * BI_M * p.nchunk * words;
-  if (t >= total) return;
-  const long wq = t % words;
-  long rest = t / words;
-  const int z = (int)(rest % p.nchunk);
-  rest /= p.nchunk;
-  const int row = (int)(rest % BI_M);
-  const int mt = (int)(rest / BI_M);
-  const int r = mt * BI_M + row;
-  const bool rv = r < p.M;
-  const double rho = rv ? p.rho[r] : 0.0;
-  const double sA = BI_SCALE / j_env(p.kmin[z] * rho);
-  const long g = wq / 4;
-  const int q = (int)(wq % 4);
-  uint32_t b[3][3][4];  // [order][plane][node]
+  __shared__ double tab[JTAB_N * JTAB_M];
+  __shared__ double rho_s[BI_M], rrho_s[BI_M], srho_s[BI_M], scale_s[BI_M];
+  const int tid = threadIdx.x;
+  const int nst = (int)(p.kchunk / BI_NODES);
+  const int arows = p.arows;
+  // stage fastest, then the slice, the row group, the radius tile
+  const unsigned ub = (unsigned)b;
+  const int s = (int)(ub % (unsigned)nst);
+  const unsigned u1 = ub / (unsigned)nst;
+  const int z = (int)(u1 % (unsigned)p.nchunk);
+  const unsigned u2 = u1 / (unsigned)p.nchunk;
+  const unsigned rgroups = (unsigned)(BI_M / arows);
+  const int rb = (int)(u2 % rgroups), mt = (int)(u2 / rgroups);
+  for (int i = tid; i < JTAB_N * JTAB_M; i += 256) tab[i] = JTAB[i];
+  if (tid < arows) {
+    const int r = mt * BI_M + rb * arows + tid;
+    const double rho = r < p.M ? p.rho[r] : 0.0, ar = fabs(rho);
+    rho_s[tid] = rho;
+    rrho_s[tid] = 1.0 / ar;
+    srho_s[tid] = 0.7978845608028654 * sqrt(1.0 / ar);
+    scale_s[tid] = BI_SCALE / j_env(p.kmin[z] * rho);
+  }
+  const int w = tid & 15, rr = tid >> 4;
+  const long k0 = (long)z * p.kchunk + (long)s * BI_NODES + 4 * w;
+  double kv[4], rk[4], sk[4];
 #pragma unroll
   for (int h = 0; h < 4; ++h) {
-    const long k = (long)z * p.kchunk + 16 * g + 4 * q + h;
-    double v[3] = {0.0, 0.0, 0.0};
-    if (rv && k < p.K) {
-      const double x = p.kr[k] * rho;
-      j01_real(x, v[0], v[1]);
-      v[2] = j2_from(x, v[0], v[1]);
+    kv[h] = k0 + h < p.K ? p.kr[k0 + h] : 0.0;
+    rk[h] = 1.0 / fabs(kv[h]);
+    sk[h] = sqrt(rk[h]);
+  }
+  __syncthreads();
+  const size_t off = (((size_t)mt * p.nchunk + z) * nst + s) * (3ul * BI_M * 64);
+  uint8_t* out[3] = {A0 + off, A1 + off, A2 + off};
+#pragma unroll 1
+  for (int i = 0; i < arows / 16; ++i) {
+    const int lr = rr + 16 * i, row = rb * arows + lr;
+    const bool rv = mt * BI_M + row < p.M;
+    const double rho = rho_s[lr], rrho = rrho_s[lr], srho = srho_s[lr], sA = scale_s[lr];
+    double x[4], v0[4], v1[4], v2[4];
+    bool small = true, large = true, over1 = true;
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      x[h] = fabs(kv[h] * rho);
+      small = small && !(x[h] >= J_ASYM_MIN);
+      large = large && x[h] >= J_ASYM_MIN;
+      over1 = over1 && x[h] >= 1.0;
     }
+    if (__all_sync(0xffffffffu, large)) {
+#pragma unroll
+      for (int h = 0; h < 4; ++h) j01_large(x[h], rk[h] * rrho, sk[h] * srho, v0[h], v1[h]);
+    } else if (__all_sync(0xffffffffu, small)) {
+#pragma unroll
+      for (int h = 0; h < 4; ++h) j01_small(x[h], tab, v0[h], v1[h]);
+    } else {
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        if (x[h] >= J_ASYM_MIN) j01_large(x[h], rk[h] * rrho, sk[h] * srho, v0[h], v1[h]);
+        else j01_small(x[h], tab, v0[h], v1[h]);
+      }
+    }
+    if (__all_sync(0xffffffffu, over1)) {
+#pragma unroll
+      for (int h = 0; h < 4; ++h) v2[h] = fma(2.0 * (rk[h] * rrho), v1[h], -v0[h]);
+    } else {
+#pragma unroll
+      for (int h = 0; h < 4; ++h) v2[h] = j2_from(x[h], rk[h] * rrho, v0[h], v1[h]);
+    }
+    uint32_t U[3][4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const bool live = rv && k0 + h < p.K;
+      const double s1 = kv[h] * rho < 0 ? -sA : sA;  // J_1 is odd
+      U[0][h] = (uint32_t)__double2loint(fma(live ? v0[h] : 0.0, sA, AI_MAGIC));
+      U[1][h] = (uint32_t)__double2loint(fma(live ? v1[h] : 0.0, s1, AI_MAGIC));
+      U[2][h] = (uint32_t)__double2loint(fma(live ? v2[h] : 0.0, sA, AI_MAGIC));
+    }
+    const uint32_t at = plane_off(row, 4 * w);
 #pragma unroll
     for (int o = 0; o < 3; ++o) {
-      uint32_t d0, d1, d2;
-      digits3b(__double2int_rn(v[o] * sA), d0, d1, d2);
-      b[o][0][h] = d0; b[o][1][h] = d1; b[o][2][h] = d2;
+      const uint32_t l01 = __byte_perm(U[o][0], U[o][1], 0x5140), l23 = __byte_perm(U[o][2], U[o][3], 0x5140);
+      const uint32_t h01 = __byte_perm(U[o][0], U[o][1], 0x0062), h23 = __byte_perm(U[o][2], U[o][3], 0x0062);
+      uint8_t* dst = out[o] + at;
+      *reinterpret_cast<uint32_t*>(dst) = __byte_perm(h01, h23, 0x5410) ^ 0x80808080u;
+      *reinterpret_cast<uint32_t*>(dst + BI_M * 64) = __byte_perm(l01, l23, 0x7632) ^ 0x80808080u;
+      *reinterpret_cast<uint32_t*>(dst + 2 * BI_M * 64) = __byte_perm(l01, l23, 0x5410) ^ 0x80808080u;
     }
   }
-  const long nstage = p.kchunk / BI_NODES;
-  const int s = (int)(g / 4), kb = (int)(g % 4) * 16;
-  const size_t sbytes = 3ul * BI_M * 64;
-  const size_t off = (((size_t)mt * p.nchunk + z) * nstage + s) * sbytes;
-  uint8_t* out[3] = {A0 + off, A1 + off, A2 + off};
-#pragma unroll
-  for (int o = 0; o < 3; ++o)
-#pragma unroll
-    for (int pl = 0; pl < 3; ++pl)
-      *reinterpret_cast<uint32_t*>(out[o] + (size_t)pl * BI_M * 64 + plane_off(row, kb) + 4 * q) =
-          b[o][pl][0] | (b[o][pl][1] << 8) | (b[o][pl][2] << 16) | (b[o][pl][3] << 24);
 }
-__global__ void __launch_bounds__(256) k_aimg_bessel3(BesselI8 p, uint8_t* __restrict__ A0, uint8_t* __restrict__ A1,
-                                                       uint8_t* __restrict__ A2) {
-  aimg_bessel3_body(p, (long)blockIdx.x * blockDim.x + threadIdx.x, A0, A1, A2);
+__global__ void __launch_bounds__(256, 3) k_aimg_bessel3(const __grid_constant__ BesselI8 p, uint8_t* __restrict__ A0,
+                                                      uint8_t* __restrict__ A1, uint8_t* __restrict__ A2) {
+  aimg_bessel3_body(p, blockIdx.x, A0, A1, A2);
 }
 
 cudaError_t launch_bessel_i8_aimg3(const BesselI8& p, uint8_t* A0, uint8_t* A1, uint8_t* A2, cudaStream_t s) {
   if (p.M <= 0 || p.K <= 0) return cudaSuccess;
-  const long total = (long)p.ntile_m * BI_M * p.nchunk * (p.kchunk / 4);
-  k_aimg_bessel3<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(p, A0, A1, A2);
+  k_aimg_bessel3<<<(unsigned)bessel_i8_aimg_blocks(p), 256, 0, s>>>(p, A0, A1, A2);
   return cudaGetLastError();
 }
 
@@ -605,12 +691,11 @@ cudaError_t launch_gemm_i8(const BesselI8* e, int n, cudaStream_t s) {
 // e = 3 i + o holds item i's order-o parameters; its J_n images share item i's node slicing
 // (bp[3 i] gives the layout), so one Bessel evaluation per (ρ, k) serves the three orders.
 // ------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_aimg_bessel3_group(const BesselI8* __restrict__ bp, const long* __restrict__ first,
+__global__ void __launch_bounds__(256, 3) k_aimg_bessel3_group(const BesselI8* __restrict__ bp, const long* __restrict__ first,
                                                           int ni) {
   const int i = group_entry(first, ni, blockIdx.x);
   const BesselI8& p = bp[3 * i];
-  aimg_bessel3_body(p, (long)(blockIdx.x - first[i]) * blockDim.x + threadIdx.x, bp[3 * i].Aimg, bp[3 * i + 1].Aimg,
-                    bp[3 * i + 2].Aimg);
+  aimg_bessel3_body(p, (long)blockIdx.x - first[i], bp[3 * i].Aimg, bp[3 * i + 1].Aimg, bp[3 * i + 2].Aimg);
 }
 
 // nchunk blocks per item: the slices' smallest nodes (bp[3 i].kmin, shared by the orders)

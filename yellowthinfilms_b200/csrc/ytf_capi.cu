@@ -1690,6 +1690,7 @@ static int synth1d_parts(ytf_ctx* ctx, const SynthParams& sp, int nz, double dz,
     bp.ntile_m = (nr + 127) / 128;
     bp.kchunk = kchunk;
     bp.nchunk = nchunk;
+    bp.arows = bessel_i8_arows((long)bp.ntile_m * nchunk * nst);
     bp.kr = sp.c.kr; bp.rho = drho; bp.C = Cf + coff[o]; bp.ldc = ld;
     bp.colmax = cmo;
     cmo += (size_t)nchunk * bp.N;
@@ -2210,6 +2211,9 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
     long* f_bimg = f_csym + (ni + 1);
     long* f_gemm = f_bimg + (3 * ni + 1);
     long nref = 0, ncoef = 0, naimg = 0, nasm = 0, nbimg = 0, ngemm = 0, nkmin = 0, nrsym = 0, ncsym = 0;
+    long stages = 0;  // of the group's J images
+    for (size_t j = groups[g].first; j < groups[g].second; ++j) stages += (long)lay[j].ntm * lay[j].nchunk * (lay[j].kchunk / 64);
+    const int arows = bessel_i8_arows(stages);
     for (int q = 0; q < ni; ++q) {
       const size_t j = groups[g].first + q;
       const Group1DLayout& L = lay[j];
@@ -2238,7 +2242,6 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
       f_coef[q] = ncoef; ncoef += sym ? 0 : nkb * ((L.nz + COEF1D_ZB_GROUP - 1) / COEF1D_ZB_GROUP);
       f_rsym[q] = nrsym; nrsym += sym ? nkb : 0;
       f_csym[q] = ncsym; ncsym += sym ? nkb * ((L.nz + COEF_SYM_ZB - 1) / COEF_SYM_ZB) : 0;
-      f_aimg[q] = naimg; naimg += ((long)L.ntm * 128 * L.nchunk * (L.kchunk / 4) + 255) / 256;
       f_asm[q] = nasm; nasm += asm1d_blocks(it.a);
       f_kmin[q] = nkmin; nkmin += L.nchunk;
       const size_t coff[3] = {0, (size_t)L.N[0] * L.ldc, (size_t)(L.N[0] + L.N[1]) * L.ldc};
@@ -2260,6 +2263,8 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
         bp.err = err;
         bp.wait_limit = ctx->wait_limit;
         bp.kmin = (double*)(base + L.off_kmin);
+        bp.arows = arows;
+        if (od == 0) { f_aimg[q] = naimg; naimg += bessel_i8_aimg_blocks(bp); }
         const int e = 3 * q + od;
         f_bimg[e] = nbimg;
         nbimg += (long)bp.ntile_n * (bp.Np / 8) * bp.nchunk;

@@ -299,6 +299,7 @@ struct BesselI8 {
   double* partial;   // [nchunk][N][M]
   unsigned* err;
   long wait_limit;   // polls of each bounded pipeline wait before it gives up
+  int arows;         // rows per block of the J image kernel (bessel_i8_arows)
   double* kmin;      // [nchunk] smallest node of each slice (the J digits' scale, launch_slice_kmin)
   const double* rowscale;  // [nchunk][M] the J digits' scale per (slice, radius) when set (digits
                            // rint(J 8355000 / rowscale)); else j_env(kmin[z] ρ_r)
@@ -310,13 +311,15 @@ struct BesselI8 {
 // nchunk
 cudaError_t launch_jtable_images(const BesselI8& bp, const double* Jtab, double* rowscale, uint8_t* const img[6],
                                  cudaStream_t s);
-// J_0(x), J_1(x) as the int8x3 1D synthesis evaluates them (library below 25, asymptotic above)
+// J_0(x), J_1(x) as the int8x3 1D synthesis evaluates them (Taylor rows below 25, asymptotic above)
 cudaError_t launch_bessel_j01(const double* x, long n, double* J0, double* J1, cudaStream_t s);
 // kmin[z] = min over slice z of kr (a slice of kchunk nodes, the last one up to K)
 cudaError_t launch_slice_kmin(const double* kr, long K, long kchunk, int nchunk, double* kmin, cudaStream_t s);
 // the J_0, J_1, J_2 digit images of all three orders in one pass (one Bessel evaluation per
 // (ρ, k)); p gives the shared layout (M, K, ntile_m, kchunk, nchunk, kr, rho)
 cudaError_t launch_bessel_i8_aimg3(const BesselI8& p, uint8_t* A0, uint8_t* A1, uint8_t* A2, cudaStream_t s);
+int bessel_i8_arows(long stages);                // J image rows per block: stages = tiles x 64-node stages of the launch
+long bessel_i8_aimg_blocks(const BesselI8& p);  // its blocks for one item
 size_t bessel_i8_stage_bytes_a();
 size_t bessel_i8_stage_bytes_b(int Np);
 size_t bessel_i8_smem(int Np);
