@@ -1962,12 +1962,15 @@ static int green_impl(ytf_ctx* ctx, const ytf_cache* c, int obs_layer, double zs
           if (herr) return fail(ctx, YTF_ERR_CUDA, "closed_form_G: a tensor-core pipeline wait timed out");
         }
       } else {
-        long tiles = ((npix + 63) / 64) * ((ncol + 31) / 32);
-        long want = (4L * nsm + tiles - 1) / tiles;
-        int splits = (int)std::max(1L, std::min(want, std::max(1L, c->n / 512)));
-        splits = lateral_splits(c->n, splits);
+        Lateral64 lp;
+        std::memset(&lp, 0, sizeof(lp));
+        lp.npix = npix; lp.n = c->n; lp.nx = nx; lp.ncol = ncol; lp.S = S;
+        const int splits = lateral64_plan(lp);
+        WS(Ex, double2, "g_ex", (size_t)c->n * nx);
+        WS(Ey, double2, "g_ey", (size_t)c->n * ny);
         WS(Gp, double2, "g_partial2", (size_t)splits * npix * ncol);
-        CK(LAUNCH("k_lateral", launch_lateral(v, nx, ny, dxs, dys, ncol, S, Gp, splits, ctx->stream)));
+        lp.Ex = Ex; lp.Ey = Ey; lp.partial = Gp;
+        CK(LAUNCH("k_lateral", launch_lateral64(lp, v, dxs, dys, ctx->stream)));
         CK(LAUNCH("k_reduce_splits2", launch_reduce_splits2(npix * ncol, splits, Gp, G, ctx->stream)));
       }
     }

@@ -201,6 +201,19 @@ cudaError_t launch_strengths2d(const SynthParams& p, double2* S, cudaStream_t s,
 int lateral_splits(long n, int splits);  // effective split count of launch_lateral
 cudaError_t launch_lateral(const CacheView& c, int nx, int ny, const double* xs, const double* ys, int ncol, const double2* S,
                            double2* partial, int splits, cudaStream_t s);
+// the lateral sum on FP64 tensor-core instructions, with phase tables
+struct Lateral64 {
+  long npix, n;
+  int nx, ncol;
+  double2* Ex;        // [nx][n] scratch
+  double2* Ey;        // [npix / nx][n] scratch
+  const double2* S;   // [ncol][n]
+  double2* partial;   // [splits][npix * ncol]
+  long kchunk;
+  int splits;
+};
+int lateral64_plan(Lateral64& p);  // kchunk and splits from npix, n, ncol
+cudaError_t launch_lateral64(const Lateral64& p, const CacheView& c, const double* xs, const double* ys, cudaStream_t s);
 cudaError_t launch_reduce_splits2(long len, int splits, const double2* partial, double2* G, cudaStream_t s);
 
 // batched synthesis of small observation sets (uneven batches): per item the partial sums

@@ -1022,7 +1022,8 @@ cudaError_t launch_strengths2d(const SynthParams& p, double2* S, cudaStream_t s,
 }
 
 // ------------------------------------------------------------------------------------
-// 2D lateral sum: G[pix][col] = Σ_n e^{i(kx_n x_i + ky_n y_j)} S[col][n] (complex FP64)
+// 2D lateral sum: G[pix][col] = Σ_n e^{i(kx_n x_i + ky_n y_j)} S[col][n] (complex FP64), for callers
+// without room for phase tables (ytf_green_noalloc)
 // Tile: 64 pixels x 32 columns, 16 nodes per stage; 256 threads, 4 pixels x 2 columns each.
 // The phase operand is generated per stage in shared memory (sincos per node and
 // coordinate, then one complex product per (node, pixel)).
@@ -1106,6 +1107,167 @@ __global__ void __launch_bounds__(256) k_lateral(CacheView c, int nx, int ny, co
       if (col < ncol) G[pix + npix * col] = acc[a][b];
     }
   }
+}
+
+// ------------------------------------------------------------------------------------
+// The same sum on the FP64 tensor-core instructions, for callers with room for the phase tables
+// Ex[i][n] = e^{i kx_n x_i}, Ey[j][n] = e^{i ky_n y_j} (k_phase_tables64, one sincos per node and
+// coordinate): real form G[pix][2c + part] = Σ_k A[pix][k] B[k][2c + part] over k = 2 n + {0, 1}, A =
+// (Re P, Im P) with P = Ex Ey formed once per stage of 8 nodes, B = (Sr, -Si) for the real and (Si, Sr)
+// for the imaginary column, read from the strengths themselves with the sign flipped on load. A CTA
+// of four warps takes 64 pixels x 8 F real columns (F <= 12: all 4 F columns of most calls, so P is
+// formed once per pixel), one node slice; a warp 16 pixels x all columns.
+//   Bound: the FP64 pipe. 576 pixels x 36 columns x 49152 nodes: 307 us (26.6 TFLOP/s); k_lateral, which
+// takes two sincos per (node, pixel, 32 columns) and 6 shared loads per 8 products, 1189 us.
+// ------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(128) k_phase_tables64(CacheView c, int nx, int ny, const double* __restrict__ xs,
+                                                        const double* __restrict__ ys, double2* __restrict__ Ex,
+                                                        double2* __restrict__ Ey) {
+  const long nn = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (nn >= c.n) return;
+  double sp, cp;
+  sincos(c.phi[nn / c.Nk], &sp, &cp);
+  const double k = c.kr[nn % c.Nk];
+  // rows of each axis split over blockIdx.y
+  for (int e = blockIdx.y; e < nx + ny; e += gridDim.y) {
+    double s, co;
+    sincos(e < nx ? k * cp * xs[e] : k * sp * ys[e - nx], &s, &co);
+    (e < nx ? Ex + (long)e * c.n : Ey + (long)(e - nx) * c.n)[nn] = make_double2(co, s);
+  }
+}
+
+constexpr int L64_P = 64, L64_N = 8, L64_LD = 2 * L64_N + 4;
+
+template <int F>
+__global__ void __launch_bounds__(128, F <= 9 ? 3 : 2) k_lateral64(const __grid_constant__ Lateral64 p) {
+  constexpr int NC = 4 * F;  // complex columns
+  __shared__ __align__(16) double As[2][L64_P * L64_LD];
+  __shared__ __align__(16) double Bs[2][NC * L64_LD];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const long p0 = (long)blockIdx.x * L64_P;
+  const int c0 = blockIdx.y * NC;
+  const long k0 = (long)blockIdx.z * p.kchunk, k1 = min(p.n, k0 + p.kchunk);
+  const int nst = (int)((k1 - k0 + L64_N - 1) / L64_N);
+  // the phase products of this thread: node tid & 7 of pixels (tid >> 3) + 16 e
+  const double2 *ex[4], *ey[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const long pix = min(p0 + (tid >> 3) + 16 * e, p.npix - 1);  // a pixel past the set repeats the last
+    ex[e] = p.Ex + (pix % p.nx) * p.n;
+    ey[e] = p.Ey + (pix / p.nx) * p.n;
+  }
+  double2 px[4], py[4];
+  auto load_phases = [&](int st) {
+    const long nn = min(k0 + (long)st * L64_N + (tid & 7), p.n - 1);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      px[e] = __ldg(ex[e] + nn);
+      py[e] = __ldg(ey[e] + nn);
+    }
+  };
+  auto store_phases = [&](int st) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      *reinterpret_cast<double2*>(&As[st & 1][((tid >> 3) + 16 * e) * L64_LD + 2 * (tid & 7)]) =
+          make_double2(px[e].x * py[e].x - px[e].y * py[e].y, px[e].x * py[e].y + px[e].y * py[e].x);
+  };
+  // strengths of 8 nodes per column, zero past the slice and the columns (so that what A holds there
+  // does not count)
+  auto load_strengths = [&](int st) {
+    for (int t = tid; t < NC * L64_N; t += 128) {
+      const int c = t >> 3, j = t & 7;
+      const long nn = k0 + (long)st * L64_N + j;
+      const bool in = c0 + c < p.ncol && nn < k1;
+      cp16((uint32_t)__cvta_generic_to_shared(&Bs[st & 1][c * L64_LD + 2 * j]),
+           reinterpret_cast<const double*>(p.S + (in ? (long)(c0 + c) * p.n + nn : 0)), in ? 16 : 0);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  double acc[2][F][2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < F; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  // B fragment of a lane: column (lane >> 2) of 8 real ones = complex column >> 1, part & 1; k = lane & 3
+  const int part = (lane >> 2) & 1, kp = lane & 1;
+  const int flip = (part == 0 && kp == 1) ? (int)0x80000000 : 0;
+  const int boff = (lane >> 3) * L64_LD + 2 * ((lane & 3) >> 1) + (part ^ kp);
+  const int aoff = (16 * warp + (lane >> 2)) * L64_LD + (lane & 3);
+  if (nst > 0) {
+    load_phases(0);
+    load_strengths(0);
+    store_phases(0);
+  }
+  for (int st = 0; st < nst; ++st) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    if (st + 1 < nst) {
+      load_phases(st + 1);
+      load_strengths(st + 1);
+    }
+    const double* A = As[st & 1] + aoff;
+    const double* B = Bs[st & 1] + boff;
+#pragma unroll
+    for (int q = 0; q < 2 * L64_N; q += 4) {
+      const double a0 = A[q], a1 = A[8 * L64_LD + q];
+#pragma unroll
+      for (int j = 0; j < F; ++j) {
+        const double v = B[4 * j * L64_LD + q];
+        const double b = __hiloint2double(__double2hiint(v) ^ flip, __double2loint(v));
+        mma_f64(acc[0][j][0], acc[0][j][1], a0, b);
+        mma_f64(acc[1][j][0], acc[1][j][1], a1, b);
+      }
+    }
+    if (st + 1 < nst) store_phases(st + 1);
+  }
+  double2* G = p.partial + (long)blockIdx.z * p.npix * p.ncol;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const long pix = p0 + 16 * warp + 8 * i + (lane >> 2);
+    if (pix >= p.npix) continue;
+#pragma unroll
+    for (int j = 0; j < F; ++j) {
+      const int c = c0 + 4 * j + (lane & 3);
+      if (c < p.ncol) G[pix + p.npix * c] = make_double2(acc[i][j][0], acc[i][j][1]);
+    }
+  }
+}
+
+// balanced column tiles of at most 48 complex columns
+static int lateral64_f(int ncol) {
+  const int tiles = (ncol + 47) / 48;
+  return ((ncol + tiles - 1) / tiles + 3) / 4;
+}
+
+int lateral64_plan(Lateral64& p) {
+  const int nc = 4 * lateral64_f(p.ncol);
+  const long tiles = ((p.npix + L64_P - 1) / L64_P) * ((p.ncol + nc - 1) / nc);
+  // node slices for three CTAs per SM, at least 64 nodes each
+  const long want = std::max(1L, std::min(148L * 3 / tiles, p.n / 64));
+  p.kchunk = ((p.n + want - 1) / want + L64_N - 1) / L64_N * L64_N;
+  p.splits = (int)((p.n + p.kchunk - 1) / p.kchunk);
+  return p.splits;
+}
+
+template <int F>
+static void lateral64_run(const Lateral64& p, cudaStream_t s) {
+  if constexpr (F >= 1) {
+    if (lateral64_f(p.ncol) != F) return lateral64_run<F - 1>(p, s);
+    const dim3 grid((unsigned)((p.npix + L64_P - 1) / L64_P), (unsigned)((p.ncol + 4 * F - 1) / (4 * F)),
+                    (unsigned)p.splits);
+    k_lateral64<F><<<grid, 128, 0, s>>>(p);
+  }
+}
+
+cudaError_t launch_lateral64(const Lateral64& p, const CacheView& c, const double* xs, const double* ys, cudaStream_t s) {
+  if (p.npix <= 0 || p.ncol <= 0 || p.n <= 0) return cudaSuccess;
+  const int ny = (int)(p.npix / p.nx);
+  k_phase_tables64<<<dim3((unsigned)((p.n + 127) / 128), (unsigned)std::min(p.nx + ny, 8)), 128, 0, s>>>(
+      c, p.nx, ny, xs, ys, p.Ex, p.Ey);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  lateral64_run<12>(p, s);
+  return cudaGetLastError();
 }
 
 __global__ void k_reduce_splits2(long len, int splits, const double2* __restrict__ P, double2* __restrict__ C) {
