@@ -2886,6 +2886,17 @@ extern "C" int ytf_plan_retune(ytf_plan* P, const ytf_tune* tune_in) {
     for (int st : stages) {
       std::vector<int> prob;
       std::vector<long> a, b;
+      // t.tile units per tile at most: a stage with few units takes smaller tiles, down to one unit
+      // per thread, until each CTA of the grid has four (at 1024 units a tile the scan stage of 96
+      // stacks, 266k nodes, had 310 tiles for 592 CTAs and eight serial units per thread: 408 us
+      // against 262 us)
+      long all = 0;
+      for (const TransferParams& q : pp) {
+        const bool fast = only_source_observed(q);
+        all += st <= 1 ? (long)q.nL * q.n : st == 3 ? (fast ? 0 : q.n) : !fast ? 0 : st == 6 ? (long)(q.nL - 1) * q.n : q.n;
+      }
+      const long ctas = 4L * t.ctas_per_sm * P->nsm;
+      const long tile = std::min<long>(t.tile, ((all + ctas - 1) / ctas + t.block - 1) / t.block * t.block);
       for (int j = 0; j < (int)pass.size(); ++j) {
         const TransferParams& q = pp[j];
         const bool fast = only_source_observed(q);
@@ -2894,10 +2905,10 @@ extern "C" int ytf_plan_retune(ytf_plan* P, const ytf_tune* tune_in) {
         else if (st == 3) units = fast ? 0 : q.n;
         else if (st == 6) units = fast ? (long)(q.nL - 1) * q.n : 0;
         else units = fast ? q.n : 0;
-        for (long u = 0; u < units; u += t.tile) {
+        for (long u = 0; u < units; u += tile) {
           prob.push_back(j);
           a.push_back(u);
-          b.push_back(std::min(units, u + (long)t.tile));
+          b.push_back(std::min(units, u + tile));
         }
       }
       if (prob.empty()) continue;
@@ -2917,6 +2928,16 @@ extern "C" int ytf_plan_retune(ytf_plan* P, const ytf_tune* tune_in) {
   std::vector<long> woff{0}, foff{0};
   std::vector<int> item_of;
   size_t npart = 0, syn_smem = 0;
+  // t.chunk nodes per work unit at most, fewer (in steps of a sub-batch) until each resident CTA has
+  // four units: 2048-node units of 266k nodes are 180 for 444 CTAs
+  int chunk = t.chunk;
+  {
+    long all = 0;
+    for (int i = 0; i < nb; ++i)
+      if (!P->large[i] && (long)P->gr[i].nx * P->gr[i].ny * P->gr[i].nz > 0) all += P->cs[i]->n;
+    const long units = 4L * 3 * P->nsm;
+    chunk = (int)std::min<long>(t.chunk, std::max(1L, ((all + units - 1) / units + 63) / 64) * 64);
+  }
   for (int i = 0; i < nb; ++i) {
     const ytf_green_desc& g = P->gr[i];
     const long npix = (long)g.nx * g.ny;
@@ -2934,7 +2955,7 @@ extern "C" int ytf_plan_retune(ytf_plan* P, const ytf_tune* tune_in) {
     it.rmap = it.is2d ? nullptr : P->d_rmap + P->rmap_off[i];
     it.nr = P->nr[i];
     const long n = P->cs[i]->n;
-    it.nw = (int)((n + t.chunk - 1) / t.chunk);
+    it.nw = (int)((n + chunk - 1) / chunk);
     it.G = P->g_off[i] >= 0 ? P->d_G + P->g_off[i] : (double2*)g.out;
     items.push_back(it);
     item_of.push_back(i);
@@ -3007,7 +3028,7 @@ extern "C" int ytf_plan_retune(ytf_plan* P, const ytf_tune* tune_in) {
     const long* df = reinterpret_cast<const long*>(P->tb + o_foff);
     if (woff.back() > 0) {
       const int grid = (int)std::min<long>(woff.back(), (long)t.synth_ctas_per_sm * nsm);
-      step(launch_synth_small(di, (int)items.size(), dw, woff.back(), ctr + synth_counter, t.chunk, grid, syn_smem, s));
+      step(launch_synth_small(di, (int)items.size(), dw, woff.back(), ctr + synth_counter, chunk, grid, syn_smem, s));
       P->kcount["k_synth_small"] += 1;
     }
     step(launch_synth_finish(di, (int)items.size(), df, foff.back(), s));
