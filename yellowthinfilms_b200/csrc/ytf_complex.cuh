@@ -22,7 +22,12 @@ __host__ __device__ __forceinline__ cd& operator+=(cd& a, cd b) { a.x += b.x; a.
 __host__ __device__ __forceinline__ cd& operator-=(cd& a, cd b) { a.x -= b.x; a.y -= b.y; return a; }
 __host__ __device__ __forceinline__ cd conj(cd a) { return cd{a.x, -a.y}; }
 __host__ __device__ __forceinline__ double norm2(cd a) { return a.x * a.x + a.y * a.y; }
-__host__ __device__ __forceinline__ double cabs(cd a) { return hypot(a.x, a.y); }
+// |a|: the plain root where the squares neither overflow nor lose bits to underflow, hypot elsewhere
+// (a zero, an infinity or a NaN included)
+__host__ __device__ __forceinline__ double cabs(cd a) {
+  const double m = a.x * a.x + a.y * a.y;
+  return m > 1e-280 && m < 1e280 ? sqrt(m) : hypot(a.x, a.y);
+}
 __host__ __device__ __forceinline__ double cabs1(cd a) { return fabs(a.x) + fabs(a.y); }
 __host__ __device__ __forceinline__ bool isfin(cd a) { return isfinite(a.x) && isfinite(a.y); }
 __host__ __device__ __forceinline__ bool iszero(cd a) { return a.x == 0.0 && a.y == 0.0; }
@@ -40,8 +45,14 @@ __host__ __device__ __forceinline__ cd operator/(cd a, cd b) {
   return cd{(a.x * r + a.y) / den, (a.y * r - a.x) / den};
 }
 __host__ __device__ __forceinline__ cd operator/(cd a, double s) { return cd{a.x / s, a.y / s}; }
-// 1 / b by Smith's scaling with two real divisions
+// 1 / b: conj(b) / |b|² (one real division) where |b|² is far from overflow and underflow, Smith's
+// scaling with two real divisions elsewhere
 __host__ __device__ __forceinline__ cd recip(cd b) {
+  const double m = b.x * b.x + b.y * b.y;
+  if (m > 1e-280 && m < 1e280) {
+    const double t = 1.0 / m;
+    return cd{b.x * t, -b.y * t};
+  }
   if (fabs(b.x) >= fabs(b.y)) {
     if (b.x == 0.0 && b.y == 0.0) return cd{1.0 / b.x, 0.0 / b.x};
     const double r = b.y / b.x, t = 1.0 / (b.x + b.y * r);
@@ -54,7 +65,7 @@ __host__ __device__ __forceinline__ cd recip(cd b) {
 // principal square root, signed-zero aware (branch cut on the negative real axis)
 __host__ __device__ __forceinline__ cd csqrt(cd z) {
   if (z.x == 0.0 && z.y == 0.0) return cd{0.0, z.y};
-  double t = sqrt(0.5 * (fabs(z.x) + hypot(z.x, z.y)));
+  double t = sqrt(0.5 * (fabs(z.x) + cabs(z)));
   if (z.x >= 0.0) return cd{t, z.y / (2.0 * t)};
   return cd{fabs(z.y) / (2.0 * t), copysign(t, z.y)};
 }

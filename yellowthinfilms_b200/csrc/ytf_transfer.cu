@@ -311,9 +311,10 @@ __device__ void closed_modes(const LayerDev& L, double w, cd kx, cd ky, cd Q[4],
   double s, c;
   cd kr2;
   if (kx.y == 0.0 && ky.y == 0.0) {
+    // cos and sin of the in-plane direction (φ = 0 at the origin), without the angle itself
     const double kr = hypot(kx.x, ky.x);
-    const double phi = kr == 0 ? 0.0 : atan2(ky.x, kx.x);
-    sincos(phi, &s, &c);
+    c = kr == 0 ? 1.0 : kx.x / kr;
+    s = kr == 0 ? 0.0 : ky.x / kr;
     kr2 = cd{kr * kr, 0.0};
   } else {  // complex 1D node on a deformed contour: direction (1, 0), kt² = kx²
     s = 0.0;
@@ -354,7 +355,8 @@ __device__ bool block_modes(const LayerDev& L, double w, cd kx, cd ky, cd Q[4], 
   cd disc = csqrt(hd * hd + m12 * m21);
   cd mid = (m11 + m22) * 0.5;
   cd mu[2] = {mid + disc, mid - disc};
-  double scale = fmax(fmax(cabs(m11), cabs(m22)), fmax(cabs(m12), cabs(m21)));
+  // the largest entry (1-norms: within √2 of the moduli) sets the scale of q² below
+  const double scale = fmax(fmax(cabs1(m11), cabs1(m22)), fmax(cabs1(m12), cabs1(m21)));
   if (!(scale > 0) || !isfinite(scale)) return false;
   if (cabs(mu[0] - mu[1]) <= 1e-6 * fmax(cabs(mu[0]), cabs(mu[1]))) return false;
   int col = 0;
@@ -706,7 +708,11 @@ __device__ __forceinline__ bool interface_matrix(const Mode4& A, const Mode4& B,
   cd L[4][4], R[4][4];
   interface_lhs_rhs(A, B, L, R);
   if (!lu_solve4<4>(L, R)) {
-    interface_qr(A, B, S);
+    // copies: an operand whose address went to the call would live in local memory on the LU path too
+    const Mode4 a = A, b = B;
+    S4 s;
+    interface_qr(a, b, s);
+    S = s;
     return true;
   }
   S.b11 = M2{R[0][0], R[0][1], R[1][0], R[1][1]};
@@ -1048,12 +1054,14 @@ __device__ __forceinline__ void chain_body(const TransferParams& p, long node) {
 // and the projection's status travel in the layer status bytes, which k_scan reads and
 // translates.
 // ------------------------------------------------------------------------------------
-// largest singular value of a 2x2 complex matrix: √ of the larger eigenvalue of A^H A
+// largest singular value of a 2x2 complex matrix: √ of the larger eigenvalue of A^H A, its discriminant
+// as (g00 - g11)² + 4 |g01|² (t² - 4 det cancels to √eps where the two singular values are equal,
+// e.g. where nothing comes back: F⁺ = I)
 __device__ __forceinline__ double sigma_max2(const M2& A) {
   const double g00 = norm2(A.a00) + norm2(A.a10), g11 = norm2(A.a01) + norm2(A.a11);
   const cd g01 = conj(A.a00) * A.a01 + conj(A.a10) * A.a11;
-  const double t = g00 + g11, dt = g00 * g11 - norm2(g01);
-  return sqrt(fmax((t + sqrt(fmax(t * t - 4.0 * dt, 0.0))) / 2.0, 0.0));
+  const double d = g00 - g11;
+  return sqrt(0.5 * (g00 + g11 + sqrt(d * d + 4.0 * norm2(g01))));
 }
 
 struct ModeV {  // one layer's mode vectors: Vf, Vb (4x2)
@@ -1170,21 +1178,46 @@ __device__ __forceinline__ void seeds_body(const TransferParams& p, long node) {
   if (f) p.lstat[(long)layer * p.n + node] |= f;
 }
 
+// the singular case of iface_body, from the stored modes: no register array of the LU path has its
+// address taken (the modes, and the result, then stay out of local memory: see iface_body)
+__device__ __noinline__ void iface_singular(const TransferParams& p, int a, long node, S4& X) {
+  Mode4 A, B;
+  load_modes(p, a, node, A);
+  load_modes(p, a + 1, node, B);
+  interface_qr(A, B, X);
+}
+
+// One thread per (node, interface); bound by the latency of its 36 loads and of the LU chain. With the
+// modes passed to the out-of-line QR by reference they lived in local memory (1.8 KB a thread, L1 60%
+// busy): 65536 nodes x 7 interfaces 100 us against 69 us.
 __device__ __forceinline__ void iface_body(const TransferParams& p, int j, long node) {
   const int a = j - 2, b = j - 1;
   S4 X;
   {
-    ModeV va, vb;
-    load_v(p, a, node, 0, va);
-    load_v(p, b, node, 0, vb);
-    p.dec[(long)a * p.n + node] = (uint8_t)(match_decision(va.vf, vb.vf) | match_decision(va.vb, vb.vb) << 2);
-    Mode4 A, B;
-    for (int i = 0; i < 4; ++i)
-      for (int m = 0; m < 2; ++m) {
-        A.vf[i][m] = va.vf[i][m]; A.vb[i][m] = va.vb[i][m];
-        B.vf[i][m] = vb.vf[i][m]; B.vb[i][m] = vb.vb[i][m];
-      }
-    if (!interface_matrix(A, B, X)) p.lstat[(long)b * p.n + node] |= ST_SINGULAR;
+    cd L[4][4], R[4][4];
+    {
+      ModeV va, vb;
+      load_v(p, a, node, 0, va);
+      load_v(p, b, node, 0, vb);
+      p.dec[(long)a * p.n + node] = (uint8_t)(match_decision(va.vf, vb.vf) | match_decision(va.vb, vb.vb) << 2);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+          L[i][m] = -vb.vf[i][m]; L[i][2 + m] = va.vb[i][m];
+          R[i][m] = -va.vf[i][m]; R[i][2 + m] = vb.vb[i][m];
+        }
+    }
+    if (lu_solve4<4>(L, R)) {
+      X.b11 = M2{R[0][0], R[0][1], R[1][0], R[1][1]};
+      X.b12 = M2{R[0][2], R[0][3], R[1][2], R[1][3]};
+      X.b21 = M2{R[2][0], R[2][1], R[3][0], R[3][1]};
+      X.b22 = M2{R[2][2], R[2][3], R[3][2], R[3][3]};
+    } else {
+      S4 s;
+      iface_singular(p, a, node, s);
+      X = s;
+    }
   }
   {  // layer a's propagation, in its raw column order as X
     cd qf[2], qb[2];
