@@ -374,14 +374,14 @@ int alloc_cache(ytf_ctx* ctx, ytf_cache* c, bool upload_nodes = true) {
   return YTF_OK;
 }
 
-// which SLeft/SRight slots the walk to the observation layers reads (k_chain)
-// the forward-only chain applies when every observation layer is the source layer
+// no walk to other layers when every observation layer is the source layer (k_scan)
 bool only_source_observed(const TransferParams& p) {
   for (int i = 0; i < p.nobs; ++i)
     if (p.obs[i] != p.src) return false;
   return true;
 }
 
+// which SLeft/SRight slots the walk to the observation layers reads (k_walk)
 void need_masks(int N, int src, const int* obs, int nobs, uint32_t& needL, uint32_t& needR) {
   needL = needR = 0;
   for (int i = 0; i < nobs; ++i) {
@@ -425,6 +425,7 @@ void fill_params(TransferParams& p, const ytf_stack* st, const ytf_cache* c) {
   p.nobs = c->nobs;
   for (int i = 0; i < c->nobs; ++i) p.obs[i] = c->obs[i];
   need_masks(st->nL, c->src, c->obs, c->nobs, p.needL, p.needR);
+  p.xrec = only_source_observed(p) ? 16 : 24;
   p.omega = c->omega;
   p.Nk = c->Nk;
   p.Np = c->Np;
@@ -441,37 +442,40 @@ void fill_params(TransferParams& p, const ytf_stack* st, const ytf_cache* c) {
   p.basis = c->d_basis;
 }
 
-// the forward-only chain (every observation layer is the source layer)
-int launch_forward_chain(ytf_ctx* ctx, const TransferParams& p) {
+// the solve behind the modes (launch_chain_part)
+int launch_chain(ytf_ctx* ctx, const TransferParams& p) {
   CK(LAUNCH("k_iface", launch_chain_part(0, p, ctx->stream)));
   CK(LAUNCH("k_seeds", launch_chain_part(1, p, ctx->stream)));
-  CK(LAUNCH("k_scan", launch_chain_part(2, p, ctx->stream)));
+  if (only_source_observed(p)) {
+    CK(LAUNCH("k_scan", launch_chain_part(2, p, ctx->stream)));
+  } else {
+    CK(LAUNCH("k_basis", launch_chain_part(3, p, ctx->stream)));
+    CK(LAUNCH("k_walk", launch_chain_part(4, p, ctx->stream)));
+  }
   return YTF_OK;
 }
 
 // per-node scratch bytes of the transfer kernels
-size_t scratch_per_node(int N, uint32_t needL, uint32_t needR) {
-  size_t b = (size_t)N * 20 * 16 + (size_t)std::max(N - 1, 1) * 16 * 16 + (size_t)N;
-  if (needL) b += (size_t)N * 16 * 16;
-  if (needR) b += (size_t)N * 16 * 16;
-  return b;
+size_t scratch_per_node(const TransferParams& p) {
+  const size_t N = p.nL, I = std::max(p.nL - 1, 1);
+  return N * 20 * 16 + N + I * (p.xrec * 16 + 1) + (p.needL ? N * 8 * 16 : 0) + (p.needR ? N * 8 * 16 : 0);
 }
 
-// run k_layer_modes + k_chain over [0, total) in chunks that fit the scratch budget
+// the node solve over [0, total) in chunks that fit the scratch budget
 int run_transfer(ytf_ctx* ctx, TransferParams p, long total) {
   const int N = p.nL;
-  size_t per = scratch_per_node(N, p.needL, p.needR);
+  size_t per = scratch_per_node(p);
   const size_t budget = (size_t)6 << 30;  // 6 GiB of scratch per pass
   long chunk = (long)std::max<size_t>(1024, budget / per);
   chunk = std::min(chunk, total);
   WS(modes, double2, "tr_modes", (size_t)N * 20 * chunk);
   WS(lstat, uint8_t, "tr_lstat", (size_t)N * chunk);
-  WS(sint, double2, "tr_sint", (size_t)std::max(N - 1, 1) * 16 * chunk);
+  WS(sint, double2, "tr_sint", (size_t)std::max(N - 1, 1) * p.xrec * chunk);
   WS(dec, uint8_t, "tr_dec", (size_t)std::max(N - 1, 1) * chunk);
   double2* sleft = nullptr;
   double2* sright = nullptr;
-  if (p.needL) { WS(sl, double2, "tr_sleft", (size_t)N * 16 * chunk); sleft = sl; }
-  if (p.needR) { WS(sr, double2, "tr_sright", (size_t)N * 16 * chunk); sright = sr; }
+  if (p.needL) { WS(sl, double2, "tr_sleft", (size_t)N * 8 * chunk); sleft = sl; }
+  if (p.needR) { WS(sr, double2, "tr_sright", (size_t)N * 8 * chunk); sright = sr; }
   p.modes = modes;
   p.lstat = lstat;
   p.sint = sint;
@@ -483,10 +487,7 @@ int run_transfer(ytf_ctx* ctx, TransferParams p, long total) {
     p.n = std::min(chunk, total - off);
     CK(LAUNCH("k_layer_modes", launch_layer_modes(p, ctx->stream)));
     CK(LAUNCH("k_layer_modes_qr", launch_layer_modes_qr(p, ctx->stream)));
-    if (only_source_observed(p)) {
-      if (int rc = launch_forward_chain(ctx, p)) return rc;
-    }
-    else CK(LAUNCH("k_chain", launch_chain(p, ctx->stream)));
+    if (int rc = launch_chain(ctx, p)) return rc;
   }
   return YTF_OK;
 }
@@ -714,7 +715,7 @@ int solve_rotation(ytf_ctx* ctx, const ytf_stack* st, ytf_cache* c, const Transf
   int N = st->nL;
   WS(modes, double2, "tr_modes", (size_t)N * 20 * nb);
   WS(lstat, uint8_t, "tr_lstat", (size_t)N * nb);
-  WS(sint, double2, "tr_sint", (size_t)std::max(N - 1, 1) * 16 * nb);
+  WS(sint, double2, "tr_sint", (size_t)std::max(N - 1, 1) * p.xrec * nb);
   WS(bstat, uint8_t, "tr_bstatus", (size_t)nb);
   WS(btv, uint8_t, "tr_btvalid", (size_t)nb * c->nobs);
   WS(bT, double2, "tr_bT", (size_t)16 * nb * c->nobs);
@@ -728,17 +729,14 @@ int solve_rotation(ytf_ctx* ctx, const ytf_stack* st, ytf_cache* c, const Transf
   b.sint = sint;
   WS(bdec, uint8_t, "tr_dec", (size_t)std::max(N - 1, 1) * nb);
   b.dec = bdec;
-  if (b.needL) { WS(sl, double2, "tr_sleft", (size_t)N * 16 * nb); b.sleft = sl; }
-  if (b.needR) { WS(sr, double2, "tr_sright", (size_t)N * 16 * nb); b.sright = sr; }
+  if (b.needL) { WS(sl, double2, "tr_sleft", (size_t)N * 8 * nb); b.sleft = sl; }
+  if (b.needR) { WS(sr, double2, "tr_sright", (size_t)N * 8 * nb); b.sright = sr; }
   b.status = bstat;
   b.tvalid = btv;
   b.Tout = bT;
   CK(LAUNCH("k_layer_modes", launch_layer_modes(b, ctx->stream)));
   CK(LAUNCH("k_layer_modes_qr", launch_layer_modes_qr(b, ctx->stream)));
-  if (only_source_observed(b)) {
-    if (int rc = launch_forward_chain(ctx, b)) return rc;
-  }
-  else CK(LAUNCH("k_chain", launch_chain(b, ctx->stream)));
+  if (int rc = launch_chain(ctx, b)) return rc;
   TransferParams f = p;
   f.mode = 1;
   f.n = nb;
@@ -829,6 +827,7 @@ int ytf_cavity_response(ytf_ctx* ctx, const ytf_stack* st, double omega, int sou
   p.src = source_layer;
   p.nobs = 1;
   p.obs[0] = source_layer;
+  p.xrec = 16;
   p.omega = omega;
   p.mode = 1;
   p.Nk = (int)n;
@@ -888,6 +887,7 @@ int ytf_cavity_response_batch(ytf_ctx* ctx, int nitems, const ytf_stack* const* 
     p.src = source_layer[i];
     p.nobs = 1;
     p.obs[0] = source_layer[i];
+    p.xrec = 16;
     p.omega = omega[i];
     p.mode = 1;
     p.Nk = (int)n;
@@ -900,7 +900,7 @@ int ytf_cavity_response_batch(ytf_ctx* ctx, int nitems, const ytf_stack* const* 
     p.status = dstat + off;
     p.resp = dresp + off;
     ps.push_back(p);
-    scr.push_back(scratch_per_node(p.nL, 0, 0) * (size_t)n + 4 * 256);
+    scr.push_back(scratch_per_node(p) * (size_t)n + 4 * 256);
     off += n;
   }
   size_t first = 0;
@@ -1336,15 +1336,10 @@ int ytf_transfer_batch(ytf_ctx* ctx, int nb, const ytf_transfer_desc* d, ytf_cac
     ps[i].n = cs[i]->n;
     ps[i].off = 0;
     ps[i].nout = cs[i]->n;
-    const int N = ps[i].nL;
-    const bool fast = only_source_observed(ps[i]);
-    size_t per = (size_t)N * 20 * 16 + (size_t)N;
-    if (fast) per += (size_t)std::max(N - 1, 1) * (16 * 16 + 1);
-    if (!fast) per = scratch_per_node(N, ps[i].needL, ps[i].needR);
-    scratch[i] = per * (size_t)cs[i]->n + 5 * 256;
+    scratch[i] = scratch_per_node(ps[i]) * (size_t)cs[i]->n + 6 * 256;
   }
-  // per pass: every item's block, then the forward-only and general subsets, 3 offset arrays
-  size_t pbytes = 2 * (size_t)nb * sizeof(TransferParams) + 4 * (size_t)(nb + 1) * sizeof(long);
+  // per pass: every item's block, then the scan's and the walk's subsets, 5 offset arrays
+  size_t pbytes = 2 * (size_t)nb * sizeof(TransferParams) + 5 * (size_t)(nb + 1) * sizeof(long);
   char* h = (char*)pinned_staging(ctx, 8 * std::max<size_t>(stage, 1) + pbytes + 64);
   if (!h) return abort_all(fail(ctx, YTF_ERR_NOMEM, "build_cavity_transfer: page-locked staging allocation failed"));
   {
@@ -1408,43 +1403,39 @@ int ytf_transfer_batch(ytf_ctx* ctx, int nb, const ytf_transfer_desc* d, ytf_cac
     long* offs = offm + (m + 1);
     long* offg = offs + (m + 1);
     long* offi = offg + (m + 1);
+    long* offa = offi + (m + 1);
     std::vector<int> fast_ids, gen_ids;
-    offm[0] = 0;
+    offm[0] = offi[0] = offa[0] = 0;
     for (int j = 0; j < m; ++j) {
       TransferParams& q = ps[items[j]];
       const int N = q.nL;
       const long n = q.n;
       q.modes = (double2*)carve((size_t)N * 20 * 16 * n);
       q.lstat = (uint8_t*)carve((size_t)N * n);
-      if (only_source_observed(q)) {
-        q.sint = (double2*)carve((size_t)std::max(N - 1, 1) * 16 * 16 * n);
-        q.dec = (uint8_t*)carve((size_t)std::max(N - 1, 1) * n);
-        fast_ids.push_back(j);
-      } else {
-        q.sint = (double2*)carve((size_t)std::max(N - 1, 1) * 16 * 16 * n);
-        q.sleft = q.needL ? (double2*)carve((size_t)N * 16 * 16 * n) : nullptr;
-        q.sright = q.needR ? (double2*)carve((size_t)N * 16 * 16 * n) : nullptr;
-        gen_ids.push_back(j);
-      }
+      q.sint = (double2*)carve((size_t)std::max(N - 1, 1) * q.xrec * 16 * n);
+      q.dec = (uint8_t*)carve((size_t)std::max(N - 1, 1) * n);
+      q.sleft = q.needL ? (double2*)carve((size_t)N * 8 * 16 * n) : nullptr;
+      q.sright = q.needR ? (double2*)carve((size_t)N * 8 * 16 * n) : nullptr;
+      (only_source_observed(q) ? fast_ids : gen_ids).push_back(j);
+      offa[j + 1] = offa[j] + n;
+      offi[j + 1] = offi[j] + (long)(N - 1) * n;
       offm[j + 1] = offm[j] + (long)N * n;
     }
-    // parameter blocks: all items (mode kernels), then the forward-only and general subsets
+    // parameter blocks: all items (modes, interfaces, seeds), then the scan's and the walk's subsets
     const int nf = (int)fast_ids.size(), ng = (int)gen_ids.size();
     std::vector<TransferParams> all(m);
     for (int j = 0; j < m; ++j) all[j] = ps[items[j]];
     std::memcpy(hp, all.data(), sizeof(TransferParams) * m);
     offs[0] = 0;
     offg[0] = 0;
-    offi[0] = 0;
     std::vector<TransferParams> pf, pg;
     for (int j = 0; j < nf; ++j) {
       const TransferParams& q = all[fast_ids[j]];
       pf.push_back(q);
       offs[j + 1] = offs[j] + q.n;
-      offi[j + 1] = offi[j] + (long)(q.nL - 1) * q.n;
     }
     for (int j = 0; j < ng; ++j) { pg.push_back(all[gen_ids[j]]); offg[j + 1] = offg[j] + all[gen_ids[j]].n; }
-    const size_t blk = sizeof(TransferParams) * m + 4 * sizeof(long) * (m + 1);
+    const size_t blk = sizeof(TransferParams) * m + 5 * sizeof(long) * (m + 1);
     TransferParams* hpf = (TransferParams*)(h + blk);
     TransferParams* hpg = hpf + nf;
     if (nf) std::memcpy(hpf, pf.data(), sizeof(TransferParams) * nf);
@@ -1460,16 +1451,18 @@ int ytf_transfer_batch(ytf_ctx* ctx, int nb, const ytf_transfer_desc* d, ytf_cac
     const long* doffs = doffm + (m + 1);
     const long* doffg = doffs + (m + 1);
     const long* doffi = doffg + (m + 1);
+    const long* doffa = doffi + (m + 1);
     const TransferParams* dpf = (const TransferParams*)(dpar + blk);
     const TransferParams* dpg = dpf + nf;
     CK(LAUNCH("k_layer_modes", launch_transfer_batch(0, dp, doffm, m, offm[m], ctx->stream)));
     CK(LAUNCH("k_layer_modes_qr", launch_transfer_batch(1, dp, doffm, m, offm[m], ctx->stream)));
-    if (nf) {
-      if (offi[nf]) CK(LAUNCH("k_iface", launch_transfer_batch(6, dpf, doffi, nf, offi[nf], ctx->stream)));
-      CK(LAUNCH("k_seeds", launch_transfer_batch(5, dpf, doffs, nf, offs[nf], ctx->stream)));
-      CK(LAUNCH("k_scan", launch_transfer_batch(7, dpf, doffs, nf, offs[nf], ctx->stream)));
+    if (offi[m]) CK(LAUNCH("k_iface", launch_transfer_batch(6, dp, doffi, m, offi[m], ctx->stream)));
+    CK(LAUNCH("k_seeds", launch_transfer_batch(5, dp, doffa, m, offa[m], ctx->stream)));
+    if (nf) CK(LAUNCH("k_scan", launch_transfer_batch(7, dpf, doffs, nf, offs[nf], ctx->stream)));
+    if (ng) {
+      CK(LAUNCH("k_basis", launch_transfer_batch(4, dpg, doffg, ng, offg[ng], ctx->stream)));
+      CK(LAUNCH("k_walk", launch_transfer_batch(3, dpg, doffg, ng, offg[ng], ctx->stream)));
     }
-    if (ng) CK(LAUNCH("k_chain", launch_transfer_batch(3, dpg, doffg, ng, offg[ng], ctx->stream)));
   }
   cudaError_t e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) return abort_all(fail(ctx, YTF_ERR_CUDA, cudaGetErrorString(e)));
@@ -2485,7 +2478,7 @@ static int gl_rule_batch_impl(ytf_ctx* ctx, int nsets, const int* npanels, const
 // weights, coordinates, 1D radii) and one of host outputs, and groups the node solves into
 // passes that share one scratch arena; ytf_plan_retune builds the tile tables and records
 // the graph: H2D of the inputs, counter reset, per pass the persistent stage kernels
-// (modes, QR pass, forward-only match/seeds/iface/scan or the general chain), the batched
+// (modes, QR pass, iface, seeds, then scan or basis and walk), the batched
 // synthesis and its chunk sums, D2H of the host outputs.
 // =====================================================================================
 struct ytf_plan {
@@ -2774,9 +2767,9 @@ int plan_build(ytf_plan* P) {
     const int N = q.nL;
     const long n = q.n;
     auto r256 = [](size_t b) { return (b + 255) & ~size_t(255); };
-    size_t b = r256((size_t)N * 20 * 16 * n) + r256((size_t)N * n) + r256((size_t)std::max(N - 1, 1) * 16 * 16 * n);
-    if (only_source_observed(q)) b += r256((size_t)std::max(N - 1, 1) * n);
-    else b += (q.needL ? r256((size_t)N * 16 * 16 * n) : 0) + (q.needR ? r256((size_t)N * 16 * 16 * n) : 0);
+    size_t b = r256((size_t)N * 20 * 16 * n) + r256((size_t)N * n) + r256((size_t)std::max(N - 1, 1) * q.xrec * 16 * n);
+    b += r256((size_t)std::max(N - 1, 1) * n);
+    b += (q.needL ? r256((size_t)N * 8 * 16 * n) : 0) + (q.needR ? r256((size_t)N * 8 * 16 * n) : 0);
     need[i] = b;
   }
   {
@@ -2812,13 +2805,10 @@ int plan_build(ytf_plan* P) {
       const long n = q.n;
       q.modes = (double2*)carve((size_t)N * 20 * 16 * n);
       q.lstat = (uint8_t*)carve((size_t)N * n);
-      q.sint = (double2*)carve((size_t)std::max(N - 1, 1) * 16 * 16 * n);
-      if (only_source_observed(q)) {
-        q.dec = (uint8_t*)carve((size_t)std::max(N - 1, 1) * n);
-      } else {
-        q.sleft = q.needL ? (double2*)carve((size_t)N * 16 * 16 * n) : nullptr;
-        q.sright = q.needR ? (double2*)carve((size_t)N * 16 * 16 * n) : nullptr;
-      }
+      q.sint = (double2*)carve((size_t)std::max(N - 1, 1) * q.xrec * 16 * n);
+      q.dec = (uint8_t*)carve((size_t)std::max(N - 1, 1) * n);
+      q.sleft = q.needL ? (double2*)carve((size_t)N * 8 * 16 * n) : nullptr;
+      q.sright = q.needR ? (double2*)carve((size_t)N * 8 * 16 * n) : nullptr;
     }
   }
   CK(cudaStreamCreateWithFlags(&P->cap, cudaStreamNonBlocking));
@@ -2882,7 +2872,7 @@ extern "C" int ytf_plan_retune(ytf_plan* P, const ytf_tune* tune_in) {
     std::vector<TransferParams> pp;
     for (int i : pass) pp.push_back(P->ps[i]);
     const size_t po = put(pp.data(), sizeof(TransferParams) * pp.size());
-    const int stages[] = {0, 1, 6, 5, 7, 3};
+    const int stages[] = {0, 1, 6, 5, 7, 4, 3};
     for (int st : stages) {
       std::vector<int> prob;
       std::vector<long> a, b;
@@ -2893,7 +2883,7 @@ extern "C" int ytf_plan_retune(ytf_plan* P, const ytf_tune* tune_in) {
       long all = 0;
       for (const TransferParams& q : pp) {
         const bool fast = only_source_observed(q);
-        all += st <= 1 ? (long)q.nL * q.n : st == 3 ? (fast ? 0 : q.n) : !fast ? 0 : st == 6 ? (long)(q.nL - 1) * q.n : q.n;
+        all += st <= 1 ? (long)q.nL * q.n : st == 6 ? (long)(q.nL - 1) * q.n : st == 5 || (st == 7) == fast ? q.n : 0;
       }
       const long ctas = 4L * t.ctas_per_sm * P->nsm;
       const long tile = std::min<long>(t.tile, ((all + ctas - 1) / ctas + t.block - 1) / t.block * t.block);
@@ -2902,9 +2892,8 @@ extern "C" int ytf_plan_retune(ytf_plan* P, const ytf_tune* tune_in) {
         const bool fast = only_source_observed(q);
         long units;
         if (st == 0 || st == 1) units = (long)q.nL * q.n;
-        else if (st == 3) units = fast ? 0 : q.n;
-        else if (st == 6) units = fast ? (long)(q.nL - 1) * q.n : 0;
-        else units = fast ? q.n : 0;
+        else if (st == 6) units = (long)(q.nL - 1) * q.n;
+        else units = st == 5 || (st == 7) == fast ? q.n : 0;
         for (long u = 0; u < units; u += tile) {
           prob.push_back(j);
           a.push_back(u);
@@ -3009,7 +2998,7 @@ extern "C" int ytf_plan_retune(ytf_plan* P, const ytf_tune* tune_in) {
   if (P->in_count) step(cudaMemcpyAsync(P->d_in, P->h_in, 8 * P->in_count, cudaMemcpyHostToDevice, s));
   step(cudaMemsetAsync(ctr, 0, 4 * (size_t)ncounter, s));
   step(cudaMemsetAsync(P->d_err, 0, sizeof(unsigned), s));
-  static const char* names[] = {"k_persist_modes", "k_persist_qr", "", "k_persist_chain", "",
+  static const char* names[] = {"k_persist_modes", "k_persist_qr", "", "k_persist_walk", "k_persist_basis",
                                 "k_persist_seeds", "k_persist_iface", "k_persist_scan"};
   for (auto& L : launches) {
     TileQueue q;

@@ -30,10 +30,12 @@ struct TransferParams {
   const LayerDev* layers;  // device, nL entries
   int nL, src, nobs;       // src, obs[] are 1-based
   int obs[MAXL];
-  uint32_t needL, needR;   // layers (bit l-1) whose SLeft / SRight are kept in scratch
+  uint32_t needL, needR;   // layers (bit l-1) whose SLeft / SRight blocks are kept in scratch
+  int xrec;                // complex values per interface record: 16, or 24 with the unpropagated b21, b22
+                           // that other observation layers than the source's need
   double omega;
   int mode;                // 0: 1D nodes; 1: 2D full solve; 2: 2D rotation base (φ = 0)
-  long n;                  // nodes solved by k_layer_modes / k_chain (this chunk)
+  long n;                  // nodes solved in this chunk
   long off;                // global index of the chunk's first node
   long nout;               // nodes of the output cache (== n except the rotation fill)
   int Nk, Np;
@@ -43,10 +45,10 @@ struct TransferParams {
   // scratch
   double2* modes;          // [nL][20][n]
   uint8_t* lstat;          // [nL][n]
-  double2* sint;           // [nL-1][16][n]
-  double2* sleft;          // [nL][16][n]
-  double2* sright;         // [nL][16][n]
-  uint8_t* dec;            // [nL-1][n] matching decisions per interface (forward-only chain)
+  double2* sint;           // [nL-1][xrec][n]
+  double2* sleft;          // [nL][8][n]: b12, b22
+  double2* sright;         // [nL][8][n]: b11, b21
+  uint8_t* dec;            // [nL-1][n] matching decisions per interface
   // outputs
   uint8_t* status;         // [nout] (rotation base: [n])
   uint8_t* valid;          // [nout]
@@ -64,13 +66,12 @@ struct TransferParams {
 
 cudaError_t launch_layer_modes(const TransferParams& p, cudaStream_t stream);
 cudaError_t launch_layer_modes_qr(const TransferParams& p, cudaStream_t stream);
-cudaError_t launch_chain(const TransferParams& p, cudaStream_t stream);
-// k_chain when every observation layer is the source layer, as three kernels: part 0..2 =
-// k_iface, k_seeds, k_scan, launched in that order (needs the sint and dec scratch)
+// the solve behind the modes as kernels of their own: part 0 = k_iface, 1 = k_seeds, then 2 = k_scan
+// where every observation layer is the source layer, else 3 = k_basis and 4 = k_walk
 cudaError_t launch_chain_part(int part, const TransferParams& p, cudaStream_t stream);
 // batched transfer kernels over nb problems (device arrays probs[nb], off[nb + 1]; total =
-// off[nb]): kernel 0 = layer modes, 1 = general QR pass, 3 = chain, 5-7 = the forward-only
-// chain (seeds, iface (off over (nL - 1) n interface-node pairs), scan; iface first)
+// off[nb]): kernel 0 = layer modes, 1 = general QR pass, 6 = iface (off over (nL - 1) n
+// interface-node pairs), 5 = seeds, 7 = scan, 4 = basis, 3 = walk (in launch_chain_part's order)
 cudaError_t launch_transfer_batch(int kernel, const TransferParams* probs, const long* off, int nb, long total,
                                   cudaStream_t stream);
 cudaError_t launch_rotate_fill(const TransferParams& p, const uint8_t* base_status, const uint8_t* base_tvalid,
@@ -84,8 +85,8 @@ struct TileQueue {
   int ntiles;
   unsigned* counter;  // next tile; zero before the launch
 };
-// stage: 0 modes, 1 QR pass, 3 general chain, 6 iface, 5 seeds, 7 scan (units as the batched
-// kernels, iface before seeds); block 128 or 256 threads; grid CTAs (persistent)
+// stage: 0 modes, 1 QR pass, 6 iface, 5 seeds, 7 scan, 4 basis, 3 walk (units as the batched
+// kernels, in launch_chain_part's order); block 128 or 256 threads; grid CTAs (persistent)
 cudaError_t launch_persist(int stage, int block, int grid, const TransferParams* probs, const TileQueue& q,
                            cudaStream_t s);
 

@@ -14,9 +14,9 @@
 //                   eigen, then split forward/backward by Poynting flux. Layer-major
 //                   indexing keeps one layer (one material kind) per warp: no divergence
 //                   between the closed-form and the general path.
-//   k_chain       : one thread per node. Mode matching through the stack, interface
-//                   matrices, forward/backward Redheffer scans, cavity resummation, the
-//                   stack walk reduced to the observation layers, T^o, seeds and basis.
+//   k_iface, k_seeds, k_scan (or k_basis and k_walk): interface matrices and mode matching per (node,
+//                   interface), source projection, cavity resummation, the stack walk reduced to the
+//                   observation layers, T^o, seeds and basis per node.
 //   k_rotate_fill : one thread per (kρ, φ) node of an azimuthally symmetric 2D grid: the
 //                   φ = 0 solve rotated exactly (mod_ModeSolver.jl:471-482).
 // Per-(node, layer) intermediates live in a global scratch arena, structure-of-arrays
@@ -530,17 +530,6 @@ __device__ __forceinline__ void load_modes(const TransferParams& p, int layer, l
     M.qb[m] = ld(rec, 18 + m, p.n, node);
   }
 }
-__device__ __forceinline__ void store_modes(const TransferParams& p, int layer, long node, const Mode4& M) {
-  double2* rec = p.modes + (long)layer * 20 * p.n;
-  for (int m = 0; m < 2; ++m) {
-    for (int i = 0; i < 4; ++i) {
-      st(rec, i + 4 * m, p.n, node, M.vf[i][m]);
-      st(rec, 8 + i + 4 * m, p.n, node, M.vb[i][m]);
-    }
-    st(rec, 16 + m, p.n, node, M.qf[m]);
-    st(rec, 18 + m, p.n, node, M.qb[m]);
-  }
-}
 // W = R4s V row map: W0 = V3, W1 = -V2, W2 = -V1, W3 = V0
 __device__ __forceinline__ cd Wof(const cd v[4][2], int i, int m) {
   switch (i) {
@@ -550,23 +539,6 @@ __device__ __forceinline__ cd Wof(const cd v[4][2], int i, int m) {
     default: return v[0][m];
   }
 }
-// _match_modes (mod_ModeSolver.jl:333-349) for one direction: swap b's columns if needed
-__device__ __forceinline__ void match_dir(const cd wa_src[4][2], cd vb[4][2], cd qb[2]) {
-  cd C[2][2];
-  for (int a = 0; a < 2; ++a)
-    for (int b = 0; b < 2; ++b) {
-      cd s = conj(Wof(wa_src, 0, a)) * vb[0][b];
-      for (int i = 1; i < 4; ++i) s += conj(Wof(wa_src, i, a)) * vb[i][b];
-      C[a][b] = s;
-    }
-  double sid = norm2(C[0][0]) + norm2(C[1][1]);
-  double ssw = norm2(C[0][1]) + norm2(C[1][0]);
-  if (ssw > sid) {
-    for (int i = 0; i < 4; ++i) { cd t = vb[i][0]; vb[i][0] = vb[i][1]; vb[i][1] = t; }
-    cd t = qb[0]; qb[0] = qb[1]; qb[1] = t;
-  }
-}
-
 // 4x4 LU solve with partial pivoting, NR right-hand sides; false on an exact zero pivot.
 // Every array index is a compile-time constant (the pivot row swap is a predicated exchange
 // with each candidate row), so the matrices stay in registers.
@@ -727,14 +699,6 @@ __device__ __forceinline__ void st_s4(double2* base, long slot, long n, long nod
   const cd* v = reinterpret_cast<const cd*>(&S);
   for (int e = 0; e < 16; ++e) st(b, e, n, node, v[e]);
 }
-__device__ __forceinline__ S4 ld_s4(const double2* base, long slot, long n, long node) {
-  S4 S;
-  cd* v = reinterpret_cast<cd*>(&S);
-  const double2* b = base + slot * 16 * n;
-  for (int e = 0; e < 16; ++e) v[e] = ld(b, e, n, node);
-  return S;
-}
-
 // Source_projection_Berreman_xyz (mod_SourceProj.jl:34-60); returns (sif, sib) 2x3 each
 __device__ bool source_projection(cd kx, cd ky, double w, const LayerDev& L, const Mode4& M, cd sif[2][3], cd sib[2][3]) {
   cd etz1 = E(L, 1, 3), etz2 = E(L, 2, 3), ezz = E(L, 3, 3);
@@ -840,199 +804,8 @@ __device__ __forceinline__ void write_T(const TransferParams& p, int oi, long id
 }
 
 // ------------------------------------------------------------------------------------
-// K2: per-node chain
-// ------------------------------------------------------------------------------------
-__device__ __forceinline__ void chain_body(const TransferParams& p, long node) {
-  const long n = p.n;
-  const int N = p.nL, src = p.src;
-  const bool base = p.mode == 2;  // rotation base: seeds/basis are filled per φ later
-  const long nT = base ? n : p.nout;
-  const long gnode = base ? node : p.off + node;  // index into the outputs
-  uint8_t stat = 0;
-  for (int l = 0; l < N; ++l) stat |= p.lstat[(long)l * n + node];
-  cd kx, ky;
-  node_k(p, p.off + node, kx, ky);
-  const cd z{0.0, 0.0};
-  // outputs default to "invalid"
-  if (!base) p.valid[gnode] = 0;
-  for (int oi = 0; oi < p.nobs; ++oi) p.tvalid[(long)oi * nT + gnode] = 0;
-  if (stat & (ST_EIGEN | ST_SORT)) {
-    p.status[gnode] = stat;
-    return;
-  }
-  // forward pass: matching, interfaces, SLeft prefix scan
-  Mode4 prev;
-  load_modes(p, 0, node, prev);
-  S4 S0 = s4_diag(expi(prev.qf[0], p.layers[0].d), expi(prev.qf[1], p.layers[0].d), expi(-prev.qb[0], p.layers[0].d),
-                  expi(-prev.qb[1], p.layers[0].d));
-  S4 SLsrc = s4_identity();
-  if ((p.needL >> 0) & 1u) st_s4(p.sleft, 0, n, node, s4_identity());
-  bool seeds_ok = true;
-  cd sif[2][3], sib[2][3];
-  if (src == 1 && !base) {
-    seeds_ok = source_projection(kx, ky, p.omega, p.layers[0], prev, sif, sib);
-  }
-  for (int oi = 0; oi < p.nobs; ++oi)
-    if (p.obs[oi] == 1 && !base) write_basis(p, oi, gnode, p.nout, p.layers[0], prev, kx, ky);
-  if (src == 1 && !base) write_seeds(p, gnode, p.nout, prev, sif, sib);
-  for (int j = 2; j <= N; ++j) {
-    Mode4 cur;
-    load_modes(p, j - 1, node, cur);
-    {
-      cd wf[4][2], wb[4][2];
-      for (int i = 0; i < 4; ++i)
-        for (int m = 0; m < 2; ++m) { wf[i][m] = prev.vf[i][m]; wb[i][m] = prev.vb[i][m]; }
-      match_dir(wf, cur.vf, cur.qf);
-      match_dir(wb, cur.vb, cur.qb);
-    }
-    store_modes(p, j - 1, node, cur);
-    S4 Si;
-    if (!interface_matrix(prev, cur, Si)) stat |= ST_SINGULAR;
-    st_s4(p.sint, j - 2, n, node, Si);
-    S4 SL = redheffer(S0, Si);
-    if ((p.needL >> (j - 1)) & 1u) st_s4(p.sleft, j - 1, n, node, SL);
-    if (j == src) SLsrc = SL;
-    const double d = p.layers[j - 1].d;
-    cd pf0 = expi(cur.qf[0], d), pf1 = expi(cur.qf[1], d), pb0 = expi(-cur.qb[0], d), pb1 = expi(-cur.qb[1], d);
-    // Redheffer(SL, diag(pf0, pf1, pb0, pb1))
-    S0.b11 = dl(pf0, pf1, SL.b11);
-    S0.b12 = dl(pf0, pf1, dr(SL.b12, pb0, pb1));
-    S0.b21 = SL.b21;
-    S0.b22 = dr(SL.b22, pb0, pb1);
-    if (!base) {
-      if (j == src) {
-        seeds_ok = source_projection(kx, ky, p.omega, p.layers[j - 1], cur, sif, sib);
-        write_seeds(p, gnode, p.nout, cur, sif, sib);
-      }
-      for (int oi = 0; oi < p.nobs; ++oi)
-        if (p.obs[oi] == j) write_basis(p, oi, gnode, p.nout, p.layers[j - 1], cur, kx, ky);
-    }
-    prev = cur;
-  }
-  if (stat & ST_SINGULAR) {
-    p.status[gnode] = stat;
-    return;
-  }
-  // backward pass: SRight suffix scan down to the source layer
-  S4 SR = s4_identity();
-  if (N >= 1 && ((p.needR >> (N - 1)) & 1u)) st_s4(p.sright, N - 1, n, node, SR);
-  for (int k = N - 1; k >= src; --k) {
-    // Q of layer k (1-based) from the matched records
-    const double2* rec = p.modes + (long)(k - 1) * 20 * n;
-    cd qf0 = ld(rec, 16, n, node), qf1 = ld(rec, 17, n, node), qb0 = ld(rec, 18, n, node), qb1 = ld(rec, 19, n, node);
-    const double d = p.layers[k - 1].d;
-    S4 Si = ld_s4(p.sint, k - 1, n, node);
-    S4 eff = redheffer_diag_left(expi(qf0, d), expi(qf1, d), expi(-qb0, d), expi(-qb1, d), Si);
-    SR = redheffer(eff, SR);
-    if ((p.needR >> (k - 1)) & 1u) st_s4(p.sright, k - 1, n, node, SR);
-  }
-  // cavity at the source layer (_R_cavity, _cavity_resummation)
-  const double2* srec = p.modes + (long)(src - 1) * 20 * n;
-  cd Qf0 = ld(srec, 16, n, node), Qf1 = ld(srec, 17, n, node), Qb0 = ld(srec, 18, n, node), Qb1 = ld(srec, 19, n, node);
-  const double ds = p.layers[src - 1].d;
-  M2 RL = SLsrc.b12;
-  M2 RR = M2{z, z, z, z};
-  S4 RRr = s4_identity();
-  M24 Fp, Fm;
-  const M2 I2 = M2{cd{1, 0}, z, z, cd{1, 0}}, Z2 = M2{z, z, z, z};
-  if (src < N) {
-    // SΦ = diag(e^{iQf(-d)}, e^{iQb d}) ⋆ SRight[src]
-    RRr = redheffer_diag_left(expi(Qf0, -ds), expi(Qf1, -ds), expi(Qb0, ds), expi(Qb1, ds), SR);
-    RR = RRr.b21;
-    cd PF0 = expi(Qf0, ds), PF1 = expi(Qf1, ds), PB0 = expi(Qb0, -ds), PB1 = expi(Qb1, -ds);
-    M2 Mx = mul(dr(dl(PF0, PF1, RL), PB0, PB1), RR);
-    M2 D = imin(Mx);
-    // RHS = S₊ + ΦF (RL S₋) = [I, ΦF RL]
-    Fp.L = solve(D, I2);
-    Fp.R = solve(D, dl(PF0, PF1, RL));
-    // F⁻ = S₋ + ΦB (RR F⁺)
-    Fm.L = dl(PB0, PB1, mul(RR, Fp.L));
-    Fm.R = add(I2, dl(PB0, PB1, mul(RR, Fp.R)));
-  } else {
-    Fp = M24{Z2, Z2};
-    Fm = M24{Z2, I2};
-  }
-  // T^o per observation layer
-  bool any_tbad = false;
-  for (int oi = 0; oi < p.nobs; ++oi) {
-    const int o = p.obs[oi];
-    M24 Ef, Eb;
-    if (o == src) {
-      Ef = mul24(RL, Fm);
-      Eb = mul24(RR, Fp);
-    } else if (o > src) {
-      M24 cp = mul24(RRr.b11, Fp);
-      if (o == N) {
-        Ef = flush24(cp);
-        Eb = M24{Z2, Z2};
-      } else {
-        S4 SRo = ld_s4(p.sright, o - 1, n, node);
-        M24 bp = cond2x2_eq(SRo.b11) > 1e8 ? M24{Z2, Z2} : M24{solve(SRo.b11, cp.L), solve(SRo.b11, cp.R)};
-        Ef = flush24(bp);
-        M24 Ebn;
-        if (o + 1 == N) {
-          Ebn = M24{Z2, Z2};
-        } else {
-          S4 SRn = ld_s4(p.sright, o, n, node);
-          M24 bn = cond2x2_eq(SRn.b11) > 1e8 ? M24{Z2, Z2} : M24{solve(SRn.b11, cp.L), solve(SRn.b11, cp.R)};
-          Ebn = flush24(mul24(SRn.b21, bn));
-        }
-        const double2* orec = p.modes + (long)(o - 1) * 20 * n;
-        const double dO = p.layers[o - 1].d;
-        cd f0 = expi(ld(orec, 16, n, node), dO), f1 = expi(ld(orec, 17, n, node), dO);
-        S4 Si = ld_s4(p.sint, o - 1, n, node);
-        Eb = flush24(add24(mul24(Si.b21, dl24(f0, f1, Ef)), mul24(Si.b22, Ebn)));
-      }
-    } else {  // o < src
-      M2 S22 = SLsrc.b22;
-      M24 am = mul24(S22, Fm);
-      auto bminus = [&](int k) -> M24 {  // b₋ of walk-left layer k (2 ≤ k ≤ src-1)
-        S4 SLk = ld_s4(p.sleft, k - 1, n, node);
-        return cond2x2_eq(SLk.b22) > 1e8 ? M24{Z2, Z2} : M24{solve(SLk.b22, am.L), solve(SLk.b22, am.R)};
-      };
-      if (o == 1) {
-        Ef = M24{Z2, Z2};
-      } else {
-        S4 SLo = ld_s4(p.sleft, o - 1, n, node);
-        M24 bm = cond2x2_eq(SLo.b22) > 1e8 ? M24{Z2, Z2} : M24{solve(SLo.b22, am.L), solve(SLo.b22, am.R)};
-        Ef = flush24(mul24(SLo.b12, bm));
-      }
-      M24 Ebn = (o == src - 1) ? Fm : flush24(bminus(o + 1));
-      const double2* orec = p.modes + (long)(o - 1) * 20 * n;
-      const double dO = p.layers[o - 1].d;
-      cd f0 = expi(ld(orec, 16, n, node), dO), f1 = expi(ld(orec, 17, n, node), dO);
-      S4 Si = ld_s4(p.sint, o - 1, n, node);
-      Eb = flush24(add24(mul24(Si.b21, dl24(f0, f1, Ef)), mul24(Si.b22, Ebn)));
-    }
-    bool fin = fin2(Ef.L) && fin2(Ef.R) && fin2(Eb.L) && fin2(Eb.R);
-    if (!fin) any_tbad = true;
-    if (fin) write_T(p, oi, gnode, nT, Ef, Eb);
-    else write_T(p, oi, gnode, nT, M24{Z2, Z2}, M24{Z2, Z2});
-    p.tvalid[(long)oi * nT + gnode] = fin ? 1 : 0;
-  }
-  if (any_tbad) stat |= ST_TNONFINITE;
-  if (!base) {
-    bool sfin = seeds_ok;
-    for (int m = 0; m < 2 && sfin; ++m)
-      for (int q = 0; q < 3; ++q) sfin = sfin && isfin(sif[m][q]) && isfin(sib[m][q]);
-    if (!seeds_ok) stat |= ST_SINGULAR;
-    if (!sfin) {
-      stat |= ST_SEEDS;
-      for (int oi = 0; oi < p.nobs; ++oi) p.tvalid[(long)oi * p.nout + gnode] = 0;
-      p.valid[gnode] = 0;
-    } else {
-      p.valid[gnode] = 1;
-      stat |= ST_VALID;
-    }
-  } else {
-    stat |= ST_VALID;  // the base solve succeeded; seeds are checked per φ
-  }
-  p.status[gnode] = stat;
-}
-
-// ------------------------------------------------------------------------------------
-// K2': the same solve when every observation layer is the source layer (needL = needR = 0):
-// no walk to other layers, so of SLeft[src] only the reflection block b12 enters T^o and of
+// K2: from the modes to T^o, seeds and basis. Where every observation layer is the source layer there
+// is no walk to other layers, so of SLeft[src] only the reflection block b12 enters T^o and of
 // SRight[src] only b21. Each block follows a recursion of its own through the star product (the
 // other blocks of the partial products never enter it): from the left
 //   R <- X12 + X11 (I - R X21)^-1 R X22,   and from the right   R <- X21 + X22 (I - R X12)^-1 R X11,
@@ -1048,6 +821,11 @@ __device__ __forceinline__ void chain_body(const TransferParams& p, long node) {
 //   k_scan   (per node)             the swap mask of the stack, then the two reflections over the
 //                                   interfaces (each X_j read in the matched columns' order),
 //                                   cavity, T^o
+// Other observation layers take k_basis (per node, observation layer) and k_walk in k_scan's place: the
+// same recursions carry one more block each (SLeft's b22, SRight's b11, off the same solve), the
+// blocks of the layers next to an observation layer are kept, and T^o walks from the cavity. 14364
+// nodes x 5 layers, all observed: iface, seeds, basis and walk 84 us; one thread per node for the
+// whole chain (2.6 KB of local memory each) took 162 us.
 // 65536 nodes x 8 layers: k_scan 37 us against 71 us with the full products.
 // Reading in another order is exact; only the LU's pivot order differs from a solve on matched columns.
 // The interface matrices live in the `sint` scratch, the decisions in `dec`; the LU failures
@@ -1141,7 +919,7 @@ __device__ __forceinline__ M2 ld_m2(const double2* base, int blk, int sr, int sc
             ld(base, e + r1 + 1 - sc, n, node)};
 }
 __device__ __forceinline__ S4 ld_x(const TransferParams& p, int j, long node, uint64_t swaps) {
-  const double2* base = p.sint + (long)(j - 2) * 16 * p.n;
+  const double2* base = p.sint + (long)(j - 2) * p.xrec * p.n;
   const uint32_t m = (uint32_t)(swaps >> (2 * (j - 2)));  // layer a's bits, then layer b's
   const int saf = m & 1, sab = (m >> 1) & 1, sbf = (m >> 2) & 1, sbb = (m >> 3) & 1;
   return S4{ld_m2(base, 0, sbf, saf, p.n, node), ld_m2(base, 1, sbf, sbb, p.n, node), ld_m2(base, 2, sab, saf, p.n, node),
@@ -1171,11 +949,23 @@ __device__ __forceinline__ void seeds_body(const TransferParams& p, long node) {
   for (int m = 0; m < 2; ++m)
     for (int q = 0; q < 3; ++q) fin = fin && isfin(sif[m][q]) && isfin(sib[m][q]);
   write_seeds(p, gnode, p.nout, M, sif, sib);
-  for (int oi = 0; oi < p.nobs; ++oi) write_basis(p, oi, gnode, p.nout, p.layers[layer], M, kx, ky);
+  for (int oi = 0; oi < p.nobs; ++oi)
+    if (p.obs[oi] == p.src) write_basis(p, oi, gnode, p.nout, p.layers[layer], M, kx, ky);
   uint8_t f = 0;
   if (!ok) f |= ST_PROJ_SINGULAR;
   if (!(ok && fin)) f |= ST_SEEDS;
   if (f) p.lstat[(long)layer * p.n + node] |= f;
+}
+
+// the mode basis of an observation layer other than the source layer
+__device__ __forceinline__ void basis_body(const TransferParams& p, int oi, long node) {
+  const int layer = p.obs[oi] - 1;
+  if (p.mode == 2 || layer == p.src - 1 || (node_status(p, node) & (ST_EIGEN | ST_SORT))) return;
+  cd kx, ky;
+  node_k(p, p.off + node, kx, ky);
+  Mode4 M;
+  load_matched(p, layer, node, swaps_upto(p, node, layer + 1), M);
+  write_basis(p, oi, p.off + node, p.nout, p.layers[layer], M, kx, ky);
 }
 
 // the singular case of iface_body, from the stored modes: no register array of the LU path has its
@@ -1219,13 +1009,42 @@ __device__ __forceinline__ void iface_body(const TransferParams& p, int j, long 
       X = s;
     }
   }
+  if (p.xrec > 16) {  // an observation layer's own interface, before the propagation (k_walk)
+    bool seen = false;
+    for (int oi = 0; oi < p.nobs; ++oi) seen = seen || (p.obs[oi] == j - 1 && j - 1 != p.src);
+    if (seen) {
+      double2* raw = p.sint + ((long)(j - 2) * p.xrec + 16) * p.n;
+      const cd v[8] = {X.b21.a00, X.b21.a01, X.b21.a10, X.b21.a11, X.b22.a00, X.b22.a01, X.b22.a10, X.b22.a11};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) st(raw, e, p.n, node, v[e]);
+    }
+  }
   {  // layer a's propagation, in its raw column order as X
     cd qf[2], qb[2];
     load_q(p, a, node, 0, qf, qb);
     const double d = p.layers[a].d;
     X = redheffer_diag_left(expi(qf[0], d), expi(qf[1], d), expi(-qb[0], d), expi(-qb[1], d), X);
   }
-  st_s4(p.sint, j - 2, p.n, node, X);
+  st_s4(p.sint + (long)(j - 2) * p.xrec * p.n, 0, p.n, node, X);
+}
+
+// rotation base: the source and observation layers' stored columns in the matched order, which
+// k_rotate_fill reads
+__device__ __forceinline__ void settle_columns(const TransferParams& p, long node, uint64_t swaps) {
+  for (int i = -1; i < p.nobs; ++i) {
+    const int layer = (i < 0 ? p.src : p.obs[i]) - 1;
+    if (i >= 0 && layer == p.src - 1) continue;
+    double2* rec = p.modes + (long)layer * 20 * p.n;
+    for (int dirb = 0; dirb < 2; ++dirb) {
+      if (!((swaps >> (2 * layer + dirb)) & 1)) continue;
+      for (int e = 0; e < 5; ++e) {
+        const int e0 = e < 4 ? 8 * dirb + e : 16 + 2 * dirb, e1 = e < 4 ? e0 + 4 : e0 + 1;
+        const cd a = ld(rec, e0, p.n, node), b = ld(rec, e1, p.n, node);
+        st(rec, e0, p.n, node, b);
+        st(rec, e1, p.n, node, a);
+      }
+    }
+  }
 }
 
 __device__ __forceinline__ void scan_body(const TransferParams& p, long node) {
@@ -1317,6 +1136,151 @@ __device__ __forceinline__ void scan_body(const TransferParams& p, long node) {
     }
   } else {
     stat |= ST_VALID;
+    settle_columns(p, node, swaps);
+  }
+  p.status[gnode] = stat;
+}
+
+// two 2x2 blocks of a partial product: SLeft[k] b12, b22 or SRight[k] b11, b21 (k 1-based)
+__device__ __forceinline__ void st_pair(double2* base, int k, long n, long node, const M2& A, const M2& B) {
+  double2* b = base + (long)(k - 1) * 8 * n;
+  const cd v[8] = {A.a00, A.a01, A.a10, A.a11, B.a00, B.a01, B.a10, B.a11};
+#pragma unroll
+  for (int e = 0; e < 8; ++e) st(b, e, n, node, v[e]);
+}
+__device__ __forceinline__ M2 ld_pair(const double2* base, int k, int which, long n, long node) {
+  const double2* b = base + ((long)(k - 1) * 8 + 4 * which) * n;
+  return M2{ld(b, 0, n, node), ld(b, 1, n, node), ld(b, 2, n, node), ld(b, 3, n, node)};
+}
+// A \ (X.L, X.R) unless A is ill-conditioned (_walk_stack's guard: zero)
+__device__ __forceinline__ M24 guarded_solve(const M2& A, const M24& X) {
+  const cd z{0.0, 0.0};
+  if (cond2x2_eq(A) > 1e8) return M24{M2{z, z, z, z}, M2{z, z, z, z}};
+  return M24{solve(A, X.L), solve(A, X.R)};
+}
+
+// the general form of scan_body (mod_FieldSolver.jl:72-341): T^o of every observation layer
+__device__ __forceinline__ void walk_body(const TransferParams& p, long node) {
+  const long n = p.n;
+  const int N = p.nL, src = p.src;
+  const bool base = p.mode == 2;
+  const long nT = base ? n : p.nout;
+  const long gnode = base ? node : p.off + node;
+  uint8_t stat = node_status(p, node);
+  const bool seeds_ok = !(stat & ST_PROJ_SINGULAR), seeds_fin = !(stat & ST_SEEDS);
+  stat &= (uint8_t)~(ST_PROJ_SINGULAR | ST_SEEDS);
+  const cd z{0.0, 0.0};
+  if (!base) p.valid[gnode] = 0;
+  for (int oi = 0; oi < p.nobs; ++oi) p.tvalid[(long)oi * nT + gnode] = 0;
+  if ((stat & (ST_EIGEN | ST_SORT)) || (stat & ST_SINGULAR)) {
+    p.status[gnode] = stat;
+    return;
+  }
+  const uint64_t swaps = swaps_upto(p, node, N);
+  const M2 I2 = M2{cd{1, 0}, z, z, cd{1, 0}}, Z2 = M2{z, z, z, z};
+  // SLeft[j] b12 and b22, left to right
+  M2 RL = Z2, S22 = I2;
+#pragma unroll 1
+  for (int j = 2; j <= src; ++j) {
+    const S4 X = ld_x(p, j, node, swaps);
+    const M2 Y = solve(imin(mul(X.b21, RL)), X.b22);
+    RL = add(X.b12, mul(X.b11, mul(RL, Y)));
+    S22 = mul(S22, Y);
+    if (j < src && ((p.needL >> (j - 1)) & 1u)) st_pair(p.sleft, j, n, node, RL, S22);
+  }
+  // SRight[j - 1] b21 and b11, right to left
+  M2 SR = Z2, S11 = I2;
+#pragma unroll 1
+  for (int j = N; j > src; --j) {
+    const S4 X = ld_x(p, j, node, swaps);
+    const M2 Y = solve(imin(mul(X.b12, SR)), X.b11);
+    SR = add(X.b21, mul(X.b22, mul(SR, Y)));
+    S11 = mul(S11, Y);
+    if (j - 1 > src && ((p.needR >> (j - 2)) & 1u)) st_pair(p.sright, j - 1, n, node, S11, SR);
+  }
+  // cavity at the source layer (_R_cavity, _cavity_resummation)
+  const double ds = p.layers[src - 1].d;
+  M24 Fp, Fm;
+  M2 RR = Z2;
+  {
+    cd Qs[4];
+    load_q(p, src - 1, node, swaps, Qs, Qs + 2);
+    if (src < N) {
+      const cd n0 = expi(Qs[0], -ds), n1 = expi(Qs[1], -ds);
+      RR = dr(dl(expi(Qs[2], ds), expi(Qs[3], ds), SR), n0, n1);
+      S11 = dr(S11, n0, n1);
+      const cd PB0 = expi(Qs[2], -ds), PB1 = expi(Qs[3], -ds);
+      const M2 PRL = dl(expi(Qs[0], ds), expi(Qs[1], ds), RL);
+      const M2 D = imin(mul(dr(PRL, PB0, PB1), RR));
+      Fp.L = solve(D, I2);
+      Fp.R = solve(D, PRL);
+      Fm.L = dl(PB0, PB1, mul(RR, Fp.L));
+      Fm.R = add(I2, dl(PB0, PB1, mul(RR, Fp.R)));
+    } else {
+      Fp = M24{Z2, Z2};
+      Fm = M24{Z2, I2};
+    }
+  }
+  // T^o per observation layer
+  bool any_tbad = false;
+#pragma unroll 1
+  for (int oi = 0; oi < p.nobs; ++oi) {
+    const int o = p.obs[oi];
+    M24 Ef, Eb;
+    if (o == src) {
+      Ef = mul24(RL, Fm);
+      Eb = mul24(RR, Fp);
+    } else {
+      M24 Ebn;  // the backward wave entering from the layer above
+      if (o > src) {
+        const M24 cp = mul24(S11, Fp);
+        if (o == N) {
+          Ef = flush24(cp);
+        } else {
+          Ef = flush24(guarded_solve(ld_pair(p.sright, o, 0, n, node), cp));
+          if (o + 1 == N) Ebn = M24{Z2, Z2};
+          else Ebn = flush24(mul24(ld_pair(p.sright, o + 1, 1, n, node),
+                                   guarded_solve(ld_pair(p.sright, o + 1, 0, n, node), cp)));
+        }
+      } else {
+        const M24 am = mul24(S22, Fm);
+        if (o == 1) Ef = M24{Z2, Z2};
+        else Ef = flush24(mul24(ld_pair(p.sleft, o, 0, n, node), guarded_solve(ld_pair(p.sleft, o, 1, n, node), am)));
+        if (o == src - 1) Ebn = Fm;
+        else Ebn = flush24(guarded_solve(ld_pair(p.sleft, o + 1, 1, n, node), am));
+      }
+      if (o == N) {
+        Eb = M24{Z2, Z2};
+      } else {
+        cd qf[2], qb[2];
+        load_q(p, o - 1, node, swaps, qf, qb);
+        const double dO = p.layers[o - 1].d;
+        const double2* raw = p.sint + ((long)(o - 1) * p.xrec + 16) * n;
+        const uint32_t m = (uint32_t)(swaps >> (2 * (o - 1)));
+        const M2 b21 = ld_m2(raw, 0, (m >> 1) & 1, m & 1, n, node), b22 = ld_m2(raw, 1, (m >> 1) & 1, (m >> 3) & 1, n, node);
+        Eb = flush24(add24(mul24(b21, dl24(expi(qf[0], dO), expi(qf[1], dO), Ef)), mul24(b22, Ebn)));
+      }
+    }
+    const bool fin = fin2(Ef.L) && fin2(Ef.R) && fin2(Eb.L) && fin2(Eb.R);
+    if (!fin) any_tbad = true;
+    if (fin) write_T(p, oi, gnode, nT, Ef, Eb);
+    else write_T(p, oi, gnode, nT, M24{Z2, Z2}, M24{Z2, Z2});
+    p.tvalid[(long)oi * nT + gnode] = fin ? 1 : 0;
+  }
+  if (any_tbad) stat |= ST_TNONFINITE;
+  if (!base) {
+    if (!seeds_ok) stat |= ST_SINGULAR;
+    if (!(seeds_ok && seeds_fin)) {
+      stat |= ST_SEEDS;
+      for (int oi = 0; oi < p.nobs; ++oi) p.tvalid[(long)oi * p.nout + gnode] = 0;
+      p.valid[gnode] = 0;
+    } else {
+      p.valid[gnode] = 1;
+      stat |= ST_VALID;
+    }
+  } else {
+    stat |= ST_VALID;  // the base solve succeeded; seeds are checked per φ
+    settle_columns(p, node, swaps);
   }
   p.status[gnode] = stat;
 }
@@ -1338,9 +1302,13 @@ __global__ void __launch_bounds__(128, 4) k_scan(TransferParams p) {
   if (node < p.n) scan_body(p, node);
 }
 
-__global__ void __launch_bounds__(128) k_chain(TransferParams p) {
+__global__ void __launch_bounds__(128, 2) k_walk(TransferParams p) {
   const long node = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (node < p.n) chain_body(p, node);
+  if (node < p.n) walk_body(p, node);
+}
+__global__ void __launch_bounds__(128) k_basis(TransferParams p) {
+  const long node = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (node < p.n) basis_body(p, blockIdx.y, node);
 }
 
 // ------------------------------------------------------------------------------------
@@ -1379,12 +1347,19 @@ __global__ void __launch_bounds__(128) k_layer_modes_qr_batch(const TransferPara
   const int layer = (int)(lt / p.n);
   layer_modes_qr_body(p, layer, lt - (long)layer * p.n);
 }
-__global__ void __launch_bounds__(128) k_chain_batch(const TransferParams* __restrict__ probs,
-                                                     const long* __restrict__ off, int nb) {
+__global__ void __launch_bounds__(128, 2) k_walk_batch(const TransferParams* __restrict__ probs,
+                                                       const long* __restrict__ off, int nb) {
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= off[nb]) return;
   const int i = find_problem(off, nb, t);
-  chain_body(probs[i], t - off[i]);
+  walk_body(probs[i], t - off[i]);
+}
+__global__ void __launch_bounds__(128) k_basis_batch(const TransferParams* __restrict__ probs, const long* __restrict__ off,
+                                                     int nb) {
+  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= off[nb]) return;
+  const int i = find_problem(off, nb, t);
+  for (int oi = 0; oi < probs[i].nobs; ++oi) basis_body(probs[i], oi, t - off[i]);
 }
 
 // ------------------------------------------------------------------------------------
@@ -1392,7 +1367,7 @@ __global__ void __launch_bounds__(128) k_chain_batch(const TransferParams* __res
 // graph): a fixed grid of CTAs pulls tiles (problem, unit range) from a device counter until
 // the queue is empty, so CTAs that drew short problems take more tiles instead of idling
 // behind the longest one; a tile's units go to the CTA's threads in a block-stride loop.
-// Units per stage: 0 modes and 1 QR = (layer, node) pairs, layer-major; 3 chain, 4 match,
+// Units per stage: 0 modes and 1 QR = (layer, node) pairs, layer-major; 3 walk, 4 basis,
 // 5 seeds, 7 scan = nodes; 6 iface = (interface, node) pairs. The counter is zeroed before
 // each launch (a memset node of the same graph). No CTA waits on another.
 // ------------------------------------------------------------------------------------
@@ -1405,7 +1380,9 @@ __device__ __forceinline__ void stage_unit(const TransferParams& p, long u) {
     if constexpr (STAGE == 0) layer_modes_body(p, layer, u - (long)layer * p.n);
     else layer_modes_qr_body(p, layer, u - (long)layer * p.n);
   } else if constexpr (STAGE == 3) {
-    chain_body(p, u);
+    walk_body(p, u);
+  } else if constexpr (STAGE == 4) {
+    for (int oi = 0; oi < p.nobs; ++oi) basis_body(p, oi, u);
   } else if constexpr (STAGE == 5) {
     seeds_body(p, u);
   } else if constexpr (STAGE == 6) {
@@ -1440,6 +1417,7 @@ cudaError_t launch_persist_b(int stage, int grid, const TransferParams* probs, c
     case 0: k_persist<0, BLOCK><<<grid, BLOCK, 0, s>>>(probs, q); break;
     case 1: k_persist<1, BLOCK><<<grid, BLOCK, 0, s>>>(probs, q); break;
     case 3: k_persist<3, BLOCK><<<grid, BLOCK, 0, s>>>(probs, q); break;
+    case 4: k_persist<4, BLOCK><<<grid, BLOCK, 0, s>>>(probs, q); break;
     case 5: k_persist<5, BLOCK><<<grid, BLOCK, 0, s>>>(probs, q); break;
     case 6: k_persist<6, BLOCK><<<grid, BLOCK, 0, s>>>(probs, q); break;
     case 7: k_persist<7, BLOCK><<<grid, BLOCK, 0, s>>>(probs, q); break;
@@ -1527,12 +1505,6 @@ cudaError_t launch_layer_modes_qr(const TransferParams& p, cudaStream_t stream) 
   return cudaGetLastError();
 }
 
-cudaError_t launch_chain(const TransferParams& p, cudaStream_t stream) {
-  if (p.n <= 0) return cudaSuccess;
-  k_chain<<<(unsigned)((p.n + 127) / 128), 128, 0, stream>>>(p);
-  return cudaGetLastError();
-}
-
 __global__ void __launch_bounds__(128) k_seeds_batch(const TransferParams* __restrict__ probs, const long* __restrict__ off,
                                                      int nb) {
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1567,6 +1539,8 @@ cudaError_t launch_chain_part(int part, const TransferParams& p, cudaStream_t st
       if (p.nL > 1) k_iface<<<(unsigned)((p.n * (p.nL - 1) + 127) / 128), 128, 0, stream>>>(p);
       break;
     case 1: k_seeds<<<g, 128, 0, stream>>>(p); break;
+    case 3: k_basis<<<dim3(g, (unsigned)p.nobs), 128, 0, stream>>>(p); break;
+    case 4: k_walk<<<g, 128, 0, stream>>>(p); break;
     default: k_scan<<<g, 128, 0, stream>>>(p); break;
   }
   return cudaGetLastError();
@@ -1582,7 +1556,8 @@ cudaError_t launch_transfer_batch(int kernel, const TransferParams* probs, const
     case 5: k_seeds_batch<<<grid, 128, 0, stream>>>(probs, off, nb); break;
     case 6: k_iface_batch<<<grid, 128, 0, stream>>>(probs, off, nb); break;
     case 7: k_scan_batch<<<grid, 128, 0, stream>>>(probs, off, nb); break;
-    default: k_chain_batch<<<grid, 128, 0, stream>>>(probs, off, nb); break;
+    case 4: k_basis_batch<<<grid, 128, 0, stream>>>(probs, off, nb); break;
+    default: k_walk_batch<<<grid, 128, 0, stream>>>(probs, off, nb); break;
   }
   return cudaGetLastError();
 }
