@@ -210,6 +210,9 @@ class CavityTransferCache2D(_Cache):
 
 
 def _f64(x):
+    # the usual case without the conversions' call overhead
+    if type(x) is np.ndarray and x.dtype == np.float64 and x.ndim == 1 and x.flags.c_contiguous:
+        return x
     return np.ascontiguousarray(np.atleast_1d(np.asarray(x, dtype=np.float64)))
 
 

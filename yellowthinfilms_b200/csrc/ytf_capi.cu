@@ -292,6 +292,15 @@ void* pinned_staging(ytf_ctx* ctx, size_t bytes) {
   return ctx->pinned;
 }
 
+// φ and n nodes to the device in one copy from page-locked memory (freed by the caller's synchronisation)
+int upload_k(ytf_ctx* ctx, double* dst, double phi, const double* kr, long n) {
+  double* h = (double*)pinned_staging(ctx, 8 * (size_t)(n + 1));
+  if (!h) return fail(ctx, YTF_ERR_NOMEM, "_cavity_response: page-locked staging allocation failed");
+  h[0] = phi;
+  std::memcpy(h + 1, kr, 8 * (size_t)n);
+  return upload(ctx, dst, h, 8 * (size_t)(n + 1));
+}
+
 // state shared by the items of one ytf_green_batch call: pre-uploaded coordinates, one
 // tensor-core error word, no per-item synchronisation
 struct GreenBatch {
@@ -301,27 +310,38 @@ struct GreenBatch {
   unsigned* err;
   const double* drho = nullptr;  // 1D: the distinct radii (radii_map), pre-uploaded
   const int* drmap = nullptr;    // 1D: pixel -> radius index
+  int nr = 0;                    // 1D: distinct radii
 };
 
 // distinct radii hypot(x_i, y_j) in first-occurrence order over (i fastest, j), as the
-// reference, and each pixel's index into them
+// reference, and each pixel's index into them (open addressing by the radius' bits: a node-based map
+// cost 40 ns a pixel, half of a 32-item batch's host time before its first launch)
 void radii_map(int nx, const double* xs, int ny, const double* ys, std::vector<double>& ur, std::vector<int>& rmap) {
   const long npix = (long)nx * ny;
   ur.clear();
   rmap.assign(npix, 0);
-  std::unordered_map<double, int> idx;
-  idx.reserve(npix * 2);
+  size_t cap = 16;
+  while (cap < 2 * (size_t)npix) cap *= 2;
+  std::vector<int> slot(cap, -1);
   for (int j = 0; j < ny; ++j)
     for (int i = 0; i < nx; ++i) {
-      double r = std::hypot(xs[i], ys[j]);
-      auto it = idx.find(r);
-      if (it == idx.end()) { idx.emplace(r, (int)ur.size()); rmap[i + (long)nx * j] = (int)ur.size(); ur.push_back(r); }
-      else rmap[i + (long)nx * j] = it->second;
+      const double r = std::hypot(xs[i], ys[j]);
+      uint64_t h;
+      std::memcpy(&h, &r, 8);
+      h *= 0x9E3779B97F4A7C15ull;
+      size_t q = (size_t)(h >> 20) & (cap - 1);
+      while (slot[q] >= 0 && ur[slot[q]] != r) q = (q + 1) & (cap - 1);  // a NaN is a radius of its own
+      if (slot[q] < 0) {
+        slot[q] = (int)ur.size();
+        ur.push_back(r);
+      }
+      rmap[i + (long)nx * j] = slot[q];
     }
 }
 
 // allocate the cache's arrays in one block
-int alloc_cache(ytf_ctx* ctx, ytf_cache* c, bool upload_nodes = true) {
+// (`clear`: zero-filled; a build writes every value of its own, zeros for nodes that fail)
+int alloc_cache(ytf_ctx* ctx, ytf_cache* c, bool upload_nodes = true, bool clear = false) {
   long n = c->n;
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -352,25 +372,17 @@ int alloc_cache(ytf_ctx* ctx, ytf_cache* c, bool upload_nodes = true) {
   c->d_status = (uint8_t*)(b + o_status); c->d_valid = (uint8_t*)(b + o_valid); c->d_tvalid = (uint8_t*)(b + o_tvalid);
   c->d_T = (double2*)(b + o_T); c->d_Qf = (double2*)(b + o_Qf); c->d_Qb = (double2*)(b + o_Qb);
   c->d_sf = (double2*)(b + o_sf); c->d_sb = (double2*)(b + o_sb); c->d_basis = (double2*)(b + o_basis);
-  CK(cudaMemsetAsync(c->block, 0, off, ctx->stream));
-  (void)o_status;
-  int rc;
+  if (clear) CK(cudaMemsetAsync(c->block, 0, off, ctx->stream));
   if (!upload_nodes) return YTF_OK;
-  if (c->src_kr) {
-    CK(cudaMemcpyAsync(c->d_kr, c->src_kr, 8 * (size_t)c->Nk, cudaMemcpyDeviceToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(c->d_wr, c->src_wr, 8 * (size_t)c->Nk, cudaMemcpyDeviceToDevice, ctx->stream));
-  } else {
-    if ((rc = upload(ctx, c->d_kr, c->kr.data(), 8 * c->kr.size()))) return rc;
-    if ((rc = upload(ctx, c->d_wr, c->wr.data(), 8 * c->wr.size()))) return rc;
-  }
-  if (!c->kri.empty()) {
-    if ((rc = upload(ctx, c->d_kri, c->kri.data(), 8 * c->kri.size()))) return rc;
-    if ((rc = upload(ctx, c->d_wri, c->wri.data(), 8 * c->wri.size()))) return rc;
-  }
-  if (!c->phi.empty()) {
-    if ((rc = upload(ctx, c->d_phi, c->phi.data(), 8 * c->phi.size()))) return rc;
-    if ((rc = upload(ctx, c->d_wphi, c->wphi.data(), 8 * c->wphi.size()))) return rc;
-  }
+  // the node arrays lie at the front of the block: one copy from page-locked memory, which the build's
+  // synchronisation frees
+  char* h = (char*)pinned_staging(ctx, o_status);
+  if (!h) return fail(ctx, YTF_ERR_NOMEM, "build_cavity_transfer: page-locked staging allocation failed");
+  auto put = [&](size_t o, const std::vector<double>& v) {
+    if (!v.empty()) std::memcpy(h + o, v.data(), 8 * v.size());
+  };
+  put(o_kr, c->kr); put(o_wr, c->wr); put(o_phi, c->phi); put(o_wphi, c->wphi); put(o_kri, c->kri); put(o_wri, c->wri);
+  CK(cudaMemcpyAsync(c->block, h, o_status, cudaMemcpyHostToDevice, ctx->stream));
   return YTF_OK;
 }
 
@@ -394,6 +406,13 @@ void need_masks(int N, int src, const int* obs, int nobs, uint32_t& needL, uint3
         if (k >= src + 1 && k <= N - 1) needR |= 1u << (k - 1);
     }
   }
+}
+
+// every layer has closed-form modes: no (node, layer) pair needs the general QR pass
+bool all_closed(const ytf_stack* st) {
+  for (auto& L : st->host)
+    if (!closed_form(L)) return false;
+  return true;
 }
 
 int common_checks(ytf_ctx* ctx, const ytf_stack* st, const char* fn, int src, int nobs, const int* obs_in, std::vector<int>& obs) {
@@ -426,6 +445,7 @@ void fill_params(TransferParams& p, const ytf_stack* st, const ytf_cache* c) {
   for (int i = 0; i < c->nobs; ++i) p.obs[i] = c->obs[i];
   need_masks(st->nL, c->src, c->obs, c->nobs, p.needL, p.needR);
   p.xrec = only_source_observed(p) ? 16 : 24;
+  p.closed = all_closed(st);
   p.omega = c->omega;
   p.Nk = c->Nk;
   p.Np = c->Np;
@@ -486,7 +506,7 @@ int run_transfer(ytf_ctx* ctx, TransferParams p, long total) {
     p.off = off;
     p.n = std::min(chunk, total - off);
     CK(LAUNCH("k_layer_modes", launch_layer_modes(p, ctx->stream)));
-    CK(LAUNCH("k_layer_modes_qr", launch_layer_modes_qr(p, ctx->stream)));
+    if (!p.closed) CK(LAUNCH("k_layer_modes_qr", launch_layer_modes_qr(p, ctx->stream)));
     if (int rc = launch_chain(ctx, p)) return rc;
   }
   return YTF_OK;
@@ -640,7 +660,7 @@ namespace {
 int prepare_cache(ytf_ctx* ctx, const ytf_stack* st, bool is2d, double omega, int source_layer, int nk,
                   const double* k_nodes, const double* k_weights, int nphi, const double* phi_nodes,
                   const double* phi_weights, int nobs, const int* obs_layers, int check_symmetry, int rotation,
-                  bool upload_nodes, ytf_cache** out, bool* use_rot, bool nodes_dev = false) {
+                  bool upload_nodes, ytf_cache** out, bool* use_rot, bool nodes_dev = false, bool clear = false) {
   *out = nullptr;
   *use_rot = false;
   const char* fn = is2d ? "build_cavity_transfer_2d" : "build_cavity_transfer_1d";
@@ -704,7 +724,7 @@ int prepare_cache(ytf_ctx* ctx, const ytf_stack* st, bool is2d, double omega, in
   }
   for (auto& L : st->host) c->d_layer.push_back(L.d);
   c->d_src = st->host[source_layer - 1].d;
-  if ((rc = alloc_cache(ctx, c, upload_nodes))) { ytf_cache_destroy(c); return rc; }
+  if ((rc = alloc_cache(ctx, c, upload_nodes, clear))) { ytf_cache_destroy(c); return rc; }
   *out = c;
   return YTF_OK;
 }
@@ -735,7 +755,6 @@ int solve_rotation(ytf_ctx* ctx, const ytf_stack* st, ytf_cache* c, const Transf
   b.tvalid = btv;
   b.Tout = bT;
   CK(LAUNCH("k_layer_modes", launch_layer_modes(b, ctx->stream)));
-  CK(LAUNCH("k_layer_modes_qr", launch_layer_modes_qr(b, ctx->stream)));
   if (int rc = launch_chain(ctx, b)) return rc;
   TransferParams f = p;
   f.mode = 1;
@@ -813,13 +832,12 @@ int ytf_cavity_response(ytf_ctx* ctx, const ytf_stack* st, double omega, int sou
   if (n == 0) return YTF_OK;
   CK(cudaSetDevice(ctx->device));
   // a (kρ, φ) grid of n x 1 nodes solved by the forward-only chain in response mode
-  WS(dk, double, "cr_k", n);
-  WS(dphi, double, "cr_phi", 1);
+  WS(dphi, double, "cr_k", n + 1);  // φ, then the nodes
   WS(dresp, double, "cr_out", n);
   WS(dstat, uint8_t, "cr_status", n);
   int rc;
-  if ((rc = upload(ctx, dk, kr, 8 * (size_t)n))) return rc;
-  if ((rc = upload(ctx, dphi, &phi, 8))) return rc;
+  double* dk = dphi + 1;
+  if ((rc = upload_k(ctx, dphi, phi, kr, n))) return rc;
   TransferParams p;
   std::memset(&p, 0, sizeof(p));
   p.layers = st->dev;
@@ -828,6 +846,7 @@ int ytf_cavity_response(ytf_ctx* ctx, const ytf_stack* st, double omega, int sou
   p.nobs = 1;
   p.obs[0] = source_layer;
   p.xrec = 16;
+  p.closed = all_closed(st);
   p.omega = omega;
   p.mode = 1;
   p.Nk = (int)n;
@@ -862,13 +881,12 @@ int ytf_cavity_response_batch(ytf_ctx* ctx, int nitems, const ytf_stack* const* 
   if (total == 0) return YTF_OK;
   if (!kr || !out) return YTF_ERR_ARG;
   CK(cudaSetDevice(ctx->device));
-  WS(dk, double, "crb_k", total);
-  WS(dphi, double, "crb_phi", 1);
+  WS(dphi, double, "crb_k", total + 1);  // φ, then the nodes
   WS(dresp, double, "crb_out", total);
   WS(dstat, uint8_t, "crb_status", total);
   int rc;
-  if ((rc = upload(ctx, dk, kr, 8 * (size_t)total))) return rc;
-  if ((rc = upload(ctx, dphi, &phi, 8))) return rc;
+  double* dk = dphi + 1;
+  if ((rc = upload_k(ctx, dphi, phi, kr, total))) return rc;
   // each item is its own (kρ, φ) grid of counts[i] x 1 nodes, solved by the forward-only
   // chain in response mode; all items of a pass share the same five batched launches (the
   // batched kernels map a flat index to (item, node) and run the single-item per-node code),
@@ -876,6 +894,7 @@ int ytf_cavity_response_batch(ytf_ctx* ctx, int nitems, const ytf_stack* const* 
   const size_t budget = (size_t)6 << 30;
   std::vector<TransferParams> ps;
   std::vector<size_t> scr;
+  bool open = false;  // some item needs the general QR pass
   long off = 0;
   for (int i = 0; i < nitems; ++i) {
     const long n = counts[i];
@@ -888,6 +907,8 @@ int ytf_cavity_response_batch(ytf_ctx* ctx, int nitems, const ytf_stack* const* 
     p.nobs = 1;
     p.obs[0] = source_layer[i];
     p.xrec = 16;
+    p.closed = all_closed(stacks[i]);
+    open = open || !p.closed;
     p.omega = omega[i];
     p.mode = 1;
     p.Nk = (int)n;
@@ -947,7 +968,7 @@ int ytf_cavity_response_batch(ytf_ctx* ctx, int nitems, const ytf_stack* const* 
     const long* doffs = doffm + (m + 1);
     const long* doffi = doffs + (m + 1);
     CK(LAUNCH("k_layer_modes", launch_transfer_batch(0, dp, doffm, m, offm[m], ctx->stream)));
-    CK(LAUNCH("k_layer_modes_qr", launch_transfer_batch(1, dp, doffm, m, offm[m], ctx->stream)));
+    if (open) CK(LAUNCH("k_layer_modes_qr", launch_transfer_batch(1, dp, doffm, m, offm[m], ctx->stream)));
     if (offi[m]) CK(LAUNCH("k_iface", launch_transfer_batch(6, dp, doffi, m, offi[m], ctx->stream)));
     CK(LAUNCH("k_seeds", launch_transfer_batch(5, dp, doffs, m, offs[m], ctx->stream)));
     CK(LAUNCH("k_scan", launch_transfer_batch(7, dp, doffs, m, offs[m], ctx->stream)));
@@ -1340,32 +1361,44 @@ int ytf_transfer_batch(ytf_ctx* ctx, int nb, const ytf_transfer_desc* d, ytf_cac
   }
   // per pass: every item's block, then the scan's and the walk's subsets, 5 offset arrays
   size_t pbytes = 2 * (size_t)nb * sizeof(TransferParams) + 5 * (size_t)(nb + 1) * sizeof(long);
-  char* h = (char*)pinned_staging(ctx, 8 * std::max<size_t>(stage, 1) + pbytes + 64);
+  char* h = (char*)pinned_staging(ctx, 8 * std::max<size_t>(stage, 1) + 4 * (size_t)nb * sizeof(CopySeg) + pbytes + 128);
   if (!h) return abort_all(fail(ctx, YTF_ERR_NOMEM, "build_cavity_transfer: page-locked staging allocation failed"));
+  // every item's node arrays in one upload and one scatter launch (device-resident nodes: read where
+  // they lie, on the same stream)
   {
     double* hd = (double*)h;
     size_t k = 0;
+    std::vector<CopySeg> segs;
+    WS(dnodes, double, "tb_nodes", std::max<size_t>(stage, 1) + (size_t)4 * nb * sizeof(CopySeg) / 8);
+    long most = 0;
     for (int i = 0; i < nb; ++i) {
       ytf_cache* c = cs[i];
-      auto put = [&](double* dst, const std::vector<double>& v) -> int {
-        if (v.empty()) return YTF_OK;
+      auto put = [&](double* dst, const std::vector<double>& v) {
+        if (v.empty()) return;
         std::memcpy(hd + k, v.data(), 8 * v.size());
-        cudaError_t e = cudaMemcpyAsync(dst, hd + k, 8 * v.size(), cudaMemcpyHostToDevice, ctx->stream);
+        segs.push_back({dnodes + k, dst, (long)v.size()});
+        most = std::max(most, (long)v.size());
         k += v.size();
-        return e == cudaSuccess ? YTF_OK : fail(ctx, YTF_ERR_CUDA, cudaGetErrorString(e));
       };
-      int rc;
-      if ((rc = put(c->d_kr, c->kr)) || (rc = put(c->d_wr, c->wr)) || (rc = put(c->d_phi, c->phi)) ||
-          (rc = put(c->d_wphi, c->wphi)))
-        return abort_all(rc);
-      if (c->src_kr && c->Nk > 0) {  // device-resident nodes: device to device, on the same stream
-        cudaError_t e = cudaMemcpyAsync(c->d_kr, c->src_kr, 8 * (size_t)c->Nk, cudaMemcpyDeviceToDevice, ctx->stream);
-        if (e == cudaSuccess)
-          e = cudaMemcpyAsync(c->d_wr, c->src_wr, 8 * (size_t)c->Nk, cudaMemcpyDeviceToDevice, ctx->stream);
-        if (e != cudaSuccess) return abort_all(fail(ctx, YTF_ERR_CUDA, cudaGetErrorString(e)));
+      put(c->d_kr, c->kr);
+      put(c->d_wr, c->wr);
+      put(c->d_phi, c->phi);
+      put(c->d_wphi, c->wphi);
+      if (c->src_kr && c->Nk > 0) {
+        segs.push_back({c->src_kr, c->d_kr, c->Nk});
+        segs.push_back({c->src_wr, c->d_wr, c->Nk});
+        most = std::max(most, (long)c->Nk);
       }
     }
-    h += ((8 * k + 63) / 64) * 64;
+    if (!segs.empty()) {
+      std::memcpy(hd + k, segs.data(), sizeof(CopySeg) * segs.size());
+      const size_t nbytes = 8 * k + sizeof(CopySeg) * segs.size();
+      cudaError_t e = cudaMemcpyAsync(dnodes, hd, nbytes, cudaMemcpyHostToDevice, ctx->stream);
+      if (e == cudaSuccess)
+        e = LAUNCH("k_copy_segments", launch_copy_segments((const CopySeg*)(dnodes + k), (int)segs.size(), most, ctx->stream));
+      if (e != cudaSuccess) return abort_all(fail(ctx, YTF_ERR_CUDA, cudaGetErrorString(e)));
+      h += (nbytes + 63) / 64 * 64;
+    }
   }
   // rotation items and items too large for one pass take the single-problem paths
   for (int i = 0; i < nb; ++i) {
@@ -1405,6 +1438,8 @@ int ytf_transfer_batch(ytf_ctx* ctx, int nb, const ytf_transfer_desc* d, ytf_cac
     long* offi = offg + (m + 1);
     long* offa = offi + (m + 1);
     std::vector<int> fast_ids, gen_ids;
+    bool open = false;
+    for (int i2 : items) open = open || !ps[i2].closed;
     offm[0] = offi[0] = offa[0] = 0;
     for (int j = 0; j < m; ++j) {
       TransferParams& q = ps[items[j]];
@@ -1455,7 +1490,7 @@ int ytf_transfer_batch(ytf_ctx* ctx, int nb, const ytf_transfer_desc* d, ytf_cac
     const TransferParams* dpf = (const TransferParams*)(dpar + blk);
     const TransferParams* dpg = dpf + nf;
     CK(LAUNCH("k_layer_modes", launch_transfer_batch(0, dp, doffm, m, offm[m], ctx->stream)));
-    CK(LAUNCH("k_layer_modes_qr", launch_transfer_batch(1, dp, doffm, m, offm[m], ctx->stream)));
+    if (open) CK(LAUNCH("k_layer_modes_qr", launch_transfer_batch(1, dp, doffm, m, offm[m], ctx->stream)));
     if (offi[m]) CK(LAUNCH("k_iface", launch_transfer_batch(6, dp, doffi, m, offi[m], ctx->stream)));
     CK(LAUNCH("k_seeds", launch_transfer_batch(5, dp, doffa, m, offa[m], ctx->stream)));
     if (nf) CK(LAUNCH("k_scan", launch_transfer_batch(7, dpf, doffs, nf, offs[nf], ctx->stream)));
@@ -1644,12 +1679,7 @@ static int synth1d_parts(ytf_ctx* ctx, const SynthParams& sp, int nz, double dz,
   // accumulation per node slice. Real nodes: J digits relative to an envelope, straight from the
   // Bessel evaluation; a deformed contour: from the FP64 tables of complex J_n, relative to the
   // slice's largest real or imaginary part.
-  unsigned* err = gb ? gb->err : nullptr;
-  if (!err) {
-    WS(e1, unsigned, "g_tc_err", 1);
-    err = e1;
-    CK(cudaMemsetAsync(err, 0, sizeof(unsigned), ctx->stream));
-  }
+  unsigned* err = gb->err;
   WS(Cf, float, "g_Cf", ncol * ld);
   CK(LAUNCH("k_coef1d", launch_coef1d_amp(sp, amp1, Cf, ld, dz, ctx->stream)));
   // one node slicing for the three orders: its length sets the digits' scales, and follows the
@@ -1717,12 +1747,6 @@ static int synth1d_parts(ytf_ctx* ctx, const SynthParams& sp, int nz, double dz,
   }
   CK(LAUNCH("k_bessel_i8", launch_bimg(be, 3, ctx->stream)));
   CK(LAUNCH("k_bessel_i8", launch_gemm_i8(be, 3 * np, ctx->stream)));
-  if (!gb) {
-    unsigned herr = 0;
-    CK(cudaMemcpyAsync(&herr, err, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
-    if (herr) return fail(ctx, YTF_ERR_CUDA, "closed_form_G: a tensor-core pipeline wait timed out");
-  }
   return YTF_OK;
 }
 
@@ -1773,19 +1797,39 @@ static int green_impl(ytf_ctx* ctx, const ytf_cache* c, int obs_layer, double zs
   long nout = npix * nz * 9;
   if (nout == 0) return YTF_OK;
   CacheView& v = sp.c;
-  const double *dzo, *dxs, *dys;
   int rc;
-  if (gb) {
-    dzo = gb->dzo; dxs = gb->dxs; dys = gb->dys;
-  } else {
-    WS(uzo, double, "g_zo", nz);
-    WS(uxs, double, "g_xs", nx);
-    WS(uys, double, "g_ys", ny);
-    if ((rc = upload(ctx, uzo, z_obs, 8 * (size_t)nz))) return rc;
-    if ((rc = upload(ctx, uxs, xs, 8 * (size_t)nx))) return rc;
-    if ((rc = upload(ctx, uys, ys, 8 * (size_t)ny))) return rc;
-    dzo = uzo; dxs = uxs; dys = uys;
+  // a call of its own: the coordinates (and a 1D call's distinct radii and pixel map) in one copy from
+  // page-locked memory, one error word read back with the one synchronisation at the end
+  const bool single = gb == nullptr;
+  GreenBatch own{};
+  int nr1 = 0;
+  unsigned* herr = nullptr;
+  if (single) {
+    std::vector<double> ur;
+    std::vector<int> rmap;
+    if (!c->is2d && c->n > 0) radii_map(nx, xs, ny, ys, ur, rmap);
+    nr1 = (int)ur.size();
+    const size_t nd = (size_t)nz + nx + ny + ur.size(), bytes = 8 * nd + 4 * rmap.size();
+    const size_t eoff = (bytes + 63) / 64 * 64;
+    char* h = (char*)pinned_staging(ctx, eoff + 64);
+    if (!h) return fail(ctx, YTF_ERR_NOMEM, "closed_form_G: page-locked staging allocation failed");
+    double* hd = (double*)h;
+    std::memcpy(hd, z_obs, 8 * (size_t)nz);
+    std::memcpy(hd + nz, xs, 8 * (size_t)nx);
+    std::memcpy(hd + nz + nx, ys, 8 * (size_t)ny);
+    if (nr1) std::memcpy(hd + nz + nx + ny, ur.data(), 8 * ur.size());
+    if (!rmap.empty()) std::memcpy(hd + nd, rmap.data(), 4 * rmap.size());
+    herr = (unsigned*)(h + eoff);
+    *herr = 0;
+    WS(dc, char, "g_coords", eoff + 64);
+    if ((rc = upload(ctx, dc, h, eoff + 64))) return rc;  // the error word (0) behind the coordinates
+    const double* dd = (const double*)dc;
+    own.dzo = dd; own.dxs = dd + nz; own.dys = dd + nz + nx;
+    own.err = (unsigned*)(dc + eoff);
+    if (nr1) { own.drho = dd + nz + nx + ny; own.drmap = (const int*)(dd + nd); }
+    gb = &own;
   }
+  const double *dzo = gb->dzo, *dxs = gb->dxs, *dys = gb->dys;
   sp.zo = dzo;
   double2* G;
   if (out_is_device) {
@@ -1802,24 +1846,11 @@ static int green_impl(ytf_ctx* ctx, const ytf_cache* c, int obs_layer, double zs
   if (c->n == 0) {  // an empty rule integrates to zero
     CK(cudaMemsetAsync(G, 0, sizeof(double2) * nout, ctx->stream));
   } else if (!c->is2d) {
-    std::vector<double> ur;
-    std::vector<int> rmap;
-    radii_map(nx, xs, ny, ys, ur, rmap);
-    int nr = (int)ur.size();
+    int nr = nr1;
+    const double* drho = gb->drho;
+    const int* drmap = gb->drmap;
+    if (!single) nr = gb->nr;
     long nk = c->n;
-    const double* drho;
-    const int* drmap;
-    if (gb && gb->drho) {
-      drho = gb->drho;
-      drmap = gb->drmap;
-    } else {
-      WS(urho, double, "g_rho", nr);
-      WS(urmap, int, "g_rmap", npix);
-      if ((rc = upload(ctx, urho, ur.data(), 8 * (size_t)nr))) return rc;
-      if ((rc = upload(ctx, urmap, rmap.data(), 4 * (size_t)npix))) return rc;
-      drho = urho;
-      drmap = urmap;
-    }
     Asm1D as;
     std::memset(&as, 0, sizeof(as));
     as.sym = sp.sym;
@@ -1901,22 +1932,11 @@ static int green_impl(ytf_ctx* ctx, const ytf_cache* c, int obs_layer, double zs
       CK(cudaMemsetAsync(cmax, 0, sizeof(unsigned long long) * lp.nchunk * ncol, ctx->stream));
       CK(LAUNCH("k_strengths2d", launch_strengths2d(sp, S, ctx->stream, cmax, kchunk, amp)));
       WS(Gp, double2, "g_partial2", (size_t)lp.nchunk * npix * ncol);
-      unsigned* err = gb ? gb->err : nullptr;
-      if (!err) {
-        WS(e1, unsigned, "g_tc_err", 1);
-        err = e1;
-        CK(cudaMemsetAsync(err, 0, sizeof(unsigned), ctx->stream));
-      }
+      unsigned* err = gb->err;
       lp.Bq = Bq; lp.colmax = cmax; lp.partial = Gp; lp.err = err;
       lp.wait_limit = ctx->wait_limit;
       CK(LAUNCH("k_lateral_i8", launch_lateral_i8(lp, ctx->stream)));
       CK(LAUNCH("k_reduce_splits2", launch_reduce_splits2(npix * ncol, lp.nchunk, Gp, G, ctx->stream)));
-      if (!gb) {
-        unsigned herr = 0;
-        CK(cudaMemcpyAsync(&herr, err, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        if (herr) return fail(ctx, YTF_ERR_CUDA, "closed_form_G: a tensor-core pipeline wait timed out");
-      }
     } else {
       CK(LAUNCH("k_strengths2d", launch_strengths2d(sp, S, ctx->stream, nullptr, 0, amp)));
       if (precision == YTF_PREC_SPLIT_BF16) {
@@ -1938,22 +1958,11 @@ static int green_impl(ytf_ctx* ctx, const ytf_cache* c, int obs_layer, double zs
         int splits = (int)((c->n + kchunk - 1) / kchunk);
         lp.kchunk = kchunk;
         WS(Gp, double2, "g_partial2", (size_t)splits * npix * ncol);
-        unsigned* err = gb ? gb->err : nullptr;
-        if (!err) {
-          WS(e1, unsigned, "g_tc_err", 1);
-          err = e1;
-          CK(cudaMemsetAsync(err, 0, sizeof(unsigned), ctx->stream));
-        }
+        unsigned* err = gb->err;
         lp.partial = Gp;
         lp.err = err;
         CK(LAUNCH("k_lateral_tc", launch_lateral_tc(lp, splits, ctx->stream)));
         CK(LAUNCH("k_reduce_splits2", launch_reduce_splits2(npix * ncol, splits, Gp, G, ctx->stream)));
-        if (!gb) {
-          unsigned herr = 0;
-          CK(cudaMemcpyAsync(&herr, err, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
-          CK(cudaStreamSynchronize(ctx->stream));
-          if (herr) return fail(ctx, YTF_ERR_CUDA, "closed_form_G: a tensor-core pipeline wait timed out");
-        }
       } else {
         Lateral64 lp;
         std::memset(&lp, 0, sizeof(lp));
@@ -1968,11 +1977,12 @@ static int green_impl(ytf_ctx* ctx, const ytf_cache* c, int obs_layer, double zs
       }
     }
   }
-synthesis_done:
   if (!out_is_device) CK(cudaMemcpyAsync(out, G, sizeof(double2) * nout, cudaMemcpyDeviceToHost, ctx->stream));
-  if (!gb) {
+  if (single) {
+    if (precision != YTF_PREC_FP64) CK(cudaMemcpyAsync(herr, gb->err, sizeof(unsigned), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     prof_collect(ctx);
+    if (*herr) return fail(ctx, YTF_ERR_CUDA, "closed_form_G: a tensor-core pipeline wait timed out");
   }
   return YTF_OK;
 }
@@ -2333,6 +2343,7 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
     if (!ur[i].empty()) {
       gb.drho = dc + tot + orho[i];
       gb.drmap = dm + omap[i];
+      gb.nr = (int)ur[i].size();
     }
     if (nslot) {
       ctx->stream = ctx->slot_streams[i % nslot];
@@ -2566,26 +2577,6 @@ void plan_free(ytf_plan* P) {
   delete P;
 }
 
-// distinct radii of a pixel set in first-occurrence order over (i fastest, j), as the 1D
-// synthesis of closed_form_G
-void radius_map(int nx, int ny, const double* xs, const double* ys, std::vector<double>& ur, std::vector<int>& rm) {
-  ur.clear();
-  rm.assign((size_t)nx * ny, 0);
-  std::unordered_map<double, int> idx;
-  for (int j = 0; j < ny; ++j)
-    for (int i = 0; i < nx; ++i) {
-      const double r = std::hypot(xs[i], ys[j]);
-      auto it = idx.find(r);
-      if (it == idx.end()) {
-        idx.emplace(r, (int)ur.size());
-        rm[i + (size_t)nx * j] = (int)ur.size();
-        ur.push_back(r);
-      } else {
-        rm[i + (size_t)nx * j] = it->second;
-      }
-    }
-}
-
 int plan_fail(ytf_ctx* ctx, int rc, int item) {
   ctx->err += " (plan item " + std::to_string(item) + ")";
   return rc;
@@ -2696,7 +2687,7 @@ int plan_build(ytf_plan* P) {
       P->nout_syn[i] = P->large[i] ? 0 : npix * 9 * g.nz;
     } else {
       std::vector<double> ur;
-      radius_map(g.nx, g.ny, g.xs, g.ys, ur, P->rmap[i]);
+      radii_map(g.nx, g.xs, g.ny, g.ys, ur, P->rmap[i]);
       P->nr[i] = (int)ur.size();
       if (P->nr[i] > SYN_MAXR || (long)P->nr[i] * 13 * g.nz > SYN_MAXOUT)
         return plan_fail(ctx, fail(ctx, YTF_ERR_ARG, "ytf_plan_create: 1D items need at most " + std::to_string(SYN_MAXR) +
@@ -2883,7 +2874,7 @@ extern "C" int ytf_plan_retune(ytf_plan* P, const ytf_tune* tune_in) {
       long all = 0;
       for (const TransferParams& q : pp) {
         const bool fast = only_source_observed(q);
-        all += st <= 1 ? (long)q.nL * q.n : st == 6 ? (long)(q.nL - 1) * q.n : st == 5 || (st == 7) == fast ? q.n : 0;
+        all += st <= 1 ? (st == 1 && q.closed ? 0 : (long)q.nL * q.n) : st == 6 ? (long)(q.nL - 1) * q.n : st == 5 || (st == 7) == fast ? q.n : 0;
       }
       const long ctas = 4L * t.ctas_per_sm * P->nsm;
       const long tile = std::min<long>(t.tile, ((all + ctas - 1) / ctas + t.block - 1) / t.block * t.block);
@@ -2891,7 +2882,7 @@ extern "C" int ytf_plan_retune(ytf_plan* P, const ytf_tune* tune_in) {
         const TransferParams& q = pp[j];
         const bool fast = only_source_observed(q);
         long units;
-        if (st == 0 || st == 1) units = (long)q.nL * q.n;
+        if (st == 0 || st == 1) units = st == 1 && q.closed ? 0 : (long)q.nL * q.n;
         else if (st == 6) units = (long)(q.nL - 1) * q.n;
         else units = st == 5 || (st == 7) == fast ? q.n : 0;
         for (long u = 0; u < units; u += tile) {
@@ -3113,7 +3104,7 @@ extern "C" int ytf_plan_run(ytf_plan* P) {
     if (!c->is2d && P->nr[i]) {
       std::vector<double> ur;
       std::vector<int> rm;
-      radius_map(g.nx, g.ny, g.xs, g.ys, ur, rm);
+      radii_map(g.nx, g.xs, g.ny, g.ys, ur, rm);
       if (rm != P->rmap[i]) return plan_fail(ctx, fail(ctx, YTF_ERR_ARG, "ytf_plan_run: the pattern of equal radii changed"), i);
       std::memcpy(hc + g.nz + g.nx + g.ny, ur.data(), 8 * ur.size());
     }

@@ -33,6 +33,7 @@ struct TransferParams {
   uint32_t needL, needR;   // layers (bit l-1) whose SLeft / SRight blocks are kept in scratch
   int xrec;                // complex values per interface record: 16, or 24 with the unpropagated b21, b22
                            // that other observation layers than the source's need
+  int closed;              // every layer has closed-form modes (no general QR pass)
   double omega;
   int mode;                // 0: 1D nodes; 1: 2D full solve; 2: 2D rotation base (φ = 0)
   long n;                  // nodes solved in this chunk
@@ -76,6 +77,14 @@ cudaError_t launch_transfer_batch(int kernel, const TransferParams* probs, const
                                   cudaStream_t stream);
 cudaError_t launch_rotate_fill(const TransferParams& p, const uint8_t* base_status, const uint8_t* base_tvalid,
                                const double2* Tbase, cudaStream_t stream);
+
+// dst[0 .. n - 1] = src[0 .. n - 1] of every segment (device array segs[ns]; most: the largest n)
+struct CopySeg {
+  const double* src;
+  double* dst;
+  long n;
+};
+cudaError_t launch_copy_segments(const CopySeg* segs, int ns, long most, cudaStream_t s);
 
 // persistent transfer kernels: tiles of units of one problem each, pulled from a counter
 struct TileQueue {

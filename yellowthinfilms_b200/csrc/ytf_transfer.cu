@@ -934,10 +934,26 @@ __device__ __forceinline__ uint8_t node_status(const TransferParams& p, long nod
   return stat;
 }
 
+// a failed node's outputs are zeros (cache blocks are not cleared before the build)
+__device__ __forceinline__ void zero_rows(double2* b, int rows, long n, long node) {
+  for (int e = 0; e < rows; ++e) st(b, e, n, node, cd{0.0, 0.0});
+}
+__device__ __forceinline__ void zero_seeds(const TransferParams& p, long node) {
+  zero_rows(p.Qf, 2, p.nout, node);
+  zero_rows(p.Qb, 2, p.nout, node);
+  zero_rows(p.sf, 6, p.nout, node);
+  zero_rows(p.sb, 6, p.nout, node);
+}
+
 __device__ __forceinline__ void seeds_body(const TransferParams& p, long node) {
   if (p.mode == 2 || p.resp) return;
-  if (node_status(p, node) & (ST_EIGEN | ST_SORT)) return;
   const long gnode = p.off + node;
+  if (node_status(p, node) & (ST_EIGEN | ST_SORT)) {
+    zero_seeds(p, gnode);
+    for (int oi = 0; oi < p.nobs; ++oi)
+      if (p.obs[oi] == p.src) zero_rows(p.basis + (long)oi * 16 * p.nout, 16, p.nout, gnode);
+    return;
+  }
   const int layer = p.src - 1;
   cd kx, ky;
   node_k(p, p.off + node, kx, ky);
@@ -960,7 +976,11 @@ __device__ __forceinline__ void seeds_body(const TransferParams& p, long node) {
 // the mode basis of an observation layer other than the source layer
 __device__ __forceinline__ void basis_body(const TransferParams& p, int oi, long node) {
   const int layer = p.obs[oi] - 1;
-  if (p.mode == 2 || layer == p.src - 1 || (node_status(p, node) & (ST_EIGEN | ST_SORT))) return;
+  if (p.mode == 2 || layer == p.src - 1) return;
+  if (node_status(p, node) & (ST_EIGEN | ST_SORT)) {
+    zero_rows(p.basis + (long)oi * 16 * p.nout, 16, p.nout, p.off + node);
+    return;
+  }
   cd kx, ky;
   node_k(p, p.off + node, kx, ky);
   Mode4 M;
@@ -1064,6 +1084,7 @@ __device__ __forceinline__ void scan_body(const TransferParams& p, long node) {
   if (stat & (ST_EIGEN | ST_SORT)) {
     p.status[gnode] = stat;
     if (p.resp) p.resp[gnode] = 0.0;
+    else zero_rows(p.Tout, 16 * p.nobs, nT, gnode);
     return;
   }
   const uint64_t swaps = swaps_upto(p, node, N);
@@ -1086,6 +1107,7 @@ __device__ __forceinline__ void scan_body(const TransferParams& p, long node) {
   if (stat & ST_SINGULAR) {
     p.status[gnode] = stat;
     if (p.resp) p.resp[gnode] = 0.0;
+    else zero_rows(p.Tout, 16 * p.nobs, nT, gnode);
     return;
   }
   // cavity at the source layer (_R_cavity, _cavity_resummation), as k_chain
@@ -1172,8 +1194,9 @@ __device__ __forceinline__ void walk_body(const TransferParams& p, long node) {
   const cd z{0.0, 0.0};
   if (!base) p.valid[gnode] = 0;
   for (int oi = 0; oi < p.nobs; ++oi) p.tvalid[(long)oi * nT + gnode] = 0;
-  if ((stat & (ST_EIGEN | ST_SORT)) || (stat & ST_SINGULAR)) {
+  if (stat & (ST_EIGEN | ST_SORT | ST_SINGULAR)) {
     p.status[gnode] = stat;
+    zero_rows(p.Tout, 16 * p.nobs, nT, gnode);
     return;
   }
   const uint64_t swaps = swaps_upto(p, node, N);
@@ -1450,7 +1473,13 @@ __global__ void __launch_bounds__(128) k_rotate_fill(TransferParams p, const uin
   p.valid[idx] = 0;
   for (int oi = 0; oi < p.nobs; ++oi) p.tvalid[(long)oi * nout + idx] = 0;
   uint8_t bst = base_status[k];
-  if (!(bst & ST_VALID)) { p.status[idx] = bst; return; }
+  auto failed = [&](uint8_t st_) {
+    p.status[idx] = st_;
+    zero_seeds(p, idx);
+    zero_rows(p.Tout, 16 * p.nobs, nout, idx);
+    zero_rows(p.basis, 16 * p.nobs, nout, idx);
+  };
+  if (!(bst & ST_VALID)) return failed(bst);
   auto rot = [&](Mode4& M) {
     for (int m = 0; m < 2; ++m) {
       cd a0 = M.vf[0][m], a1 = M.vf[1][m], a2 = M.vf[2][m], a3 = M.vf[3][m];
@@ -1471,7 +1500,7 @@ __global__ void __launch_bounds__(128) k_rotate_fill(TransferParams p, const uin
   for (int m = 0; m < 2 && ok; ++m)
     for (int qq = 0; qq < 3; ++qq) ok = ok && isfin(sif[m][qq]) && isfin(sib[m][qq]);
   uint8_t stat = bst & ~ST_VALID;
-  if (!ok) { p.status[idx] = stat | ST_SEEDS; return; }
+  if (!ok) return failed(stat | ST_SEEDS);
   for (int oi = 0; oi < p.nobs; ++oi) {
     uint8_t tv = base_tvalid[(long)oi * nb + k];
     const double2* tb = Tbase + (long)oi * 16 * nb;
@@ -1488,9 +1517,22 @@ __global__ void __launch_bounds__(128) k_rotate_fill(TransferParams p, const uin
   p.status[idx] = stat | ST_VALID;
 }
 
+__global__ void __launch_bounds__(256) k_copy_segments(const CopySeg* __restrict__ segs) {
+  const CopySeg g = segs[blockIdx.y];
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < g.n; i += (long)gridDim.x * blockDim.x) g.dst[i] = g.src[i];
+}
+
 // ------------------------------------------------------------------------------------
 // launchers
 // ------------------------------------------------------------------------------------
+cudaError_t launch_copy_segments(const CopySeg* segs, int ns, long most, cudaStream_t s) {
+  for (int i = 0; i < ns; i += 65535) {  // the grid's y limit
+    const long b = (most + 1023) / 1024;
+    k_copy_segments<<<dim3((unsigned)(b < 1 ? 1 : b > 64 ? 64 : b), (unsigned)(ns - i < 65535 ? ns - i : 65535)), 256, 0, s>>>(segs + i);
+  }
+  return cudaGetLastError();
+}
+
 cudaError_t launch_layer_modes(const TransferParams& p, cudaStream_t stream) {
   long tot = (long)p.n * p.nL;
   if (tot <= 0) return cudaSuccess;
