@@ -465,11 +465,11 @@ void fill_params(TransferParams& p, const ytf_stack* st, const ytf_cache* c) {
 // the solve behind the modes (launch_chain_part)
 int launch_chain(ytf_ctx* ctx, const TransferParams& p) {
   CK(LAUNCH("k_iface", launch_chain_part(0, p, ctx->stream)));
-  CK(LAUNCH("k_seeds", launch_chain_part(1, p, ctx->stream)));
+  if (!p.resp && p.mode != 2) CK(LAUNCH("k_seeds", launch_chain_part(1, p, ctx->stream)));
   if (only_source_observed(p)) {
     CK(LAUNCH("k_scan", launch_chain_part(2, p, ctx->stream)));
   } else {
-    CK(LAUNCH("k_basis", launch_chain_part(3, p, ctx->stream)));
+    if (p.mode != 2) CK(LAUNCH("k_basis", launch_chain_part(3, p, ctx->stream)));
     CK(LAUNCH("k_walk", launch_chain_part(4, p, ctx->stream)));
   }
   return YTF_OK;
@@ -970,7 +970,6 @@ int ytf_cavity_response_batch(ytf_ctx* ctx, int nitems, const ytf_stack* const* 
     CK(LAUNCH("k_layer_modes", launch_transfer_batch(0, dp, doffm, m, offm[m], ctx->stream)));
     if (open) CK(LAUNCH("k_layer_modes_qr", launch_transfer_batch(1, dp, doffm, m, offm[m], ctx->stream)));
     if (offi[m]) CK(LAUNCH("k_iface", launch_transfer_batch(6, dp, doffi, m, offi[m], ctx->stream)));
-    CK(LAUNCH("k_seeds", launch_transfer_batch(5, dp, doffs, m, offs[m], ctx->stream)));
     CK(LAUNCH("k_scan", launch_transfer_batch(7, dp, doffs, m, offs[m], ctx->stream)));
     // the host block is read by the copy above before the next pass reuses it
     CK(cudaStreamSynchronize(ctx->stream));

@@ -512,6 +512,25 @@ __global__ void __launch_bounds__(128) k_layer_modes_qr(TransferParams p) {
   layer_modes_qr_body(p, layer, t - (long)layer * p.n);
 }
 
+// the propagation of a layer's forward and backward waves over d: pf[m] = e^{i qf[m] d}, pb[m] =
+// e^{-i qb[m] d}. Modes without a preferred direction come as q and -q (every closed-form and block
+// layer, in either order of the two): then pb repeats pf's exponentials.
+__device__ __forceinline__ bool neg_of(cd a, cd b) { return a.x == -b.x && a.y == -b.y; }
+__device__ __forceinline__ void propagation(const cd qf[2], const cd qb[2], double d, cd pf[2], cd pb[2]) {
+  pf[0] = expi(qf[0], d);
+  pf[1] = expi(qf[1], d);
+  if (neg_of(qb[0], qf[0]) && neg_of(qb[1], qf[1])) {
+    pb[0] = pf[0];
+    pb[1] = pf[1];
+  } else if (neg_of(qb[0], qf[1]) && neg_of(qb[1], qf[0])) {
+    pb[0] = pf[1];
+    pb[1] = pf[0];
+  } else {
+    pb[0] = expi(-qb[0], d);
+    pb[1] = expi(-qb[1], d);
+  }
+}
+
 // ------------------------------------------------------------------------------------
 // K2 helpers
 // ------------------------------------------------------------------------------------
@@ -714,30 +733,17 @@ __device__ bool source_projection(cd kx, cd ky, double w, const LayerDev& L, con
     J[2][q] = jty - etz2 * z * rezz;
     J[3][q] = -jtx - (-etz1) * z * rezz;
   }
-  cd V[4][4], W[4][4];
+  // s = V^-1 J: the reference solves (W^H V) s = W^H J with W = R4s V, the same system multiplied by the
+  // (non-singular where V is) W^H, at the square of V's condition number and twice the arithmetic
+  cd V[4][4];
+#pragma unroll
   for (int i = 0; i < 4; ++i) {
     V[i][0] = M.vf[i][0]; V[i][1] = M.vf[i][1]; V[i][2] = M.vb[i][0]; V[i][3] = M.vb[i][1];
   }
-  for (int j = 0; j < 4; ++j) {
-    W[0][j] = V[3][j]; W[1][j] = -V[2][j]; W[2][j] = -V[1][j]; W[3][j] = V[0][j];
-  }
-  cd WV[4][4], WJ[4][3];
-  for (int a = 0; a < 4; ++a) {
-    for (int b = 0; b < 4; ++b) {
-      cd s = conj(W[0][a]) * V[0][b];
-      for (int i = 1; i < 4; ++i) s += conj(W[i][a]) * V[i][b];
-      WV[a][b] = s;
-    }
-    for (int q = 0; q < 3; ++q) {
-      cd s = conj(W[0][a]) * J[0][q];
-      for (int i = 1; i < 4; ++i) s += conj(W[i][a]) * J[i][q];
-      WJ[a][q] = s;
-    }
-  }
-  if (!lu_solve4<3>(WV, WJ)) return false;
+  if (!lu_solve4<3>(V, J)) return false;
   for (int q = 0; q < 3; ++q) {
-    sif[0][q] = WJ[0][q]; sif[1][q] = WJ[1][q];
-    sib[0][q] = WJ[2][q]; sib[1][q] = WJ[3][q];
+    sif[0][q] = J[0][q]; sif[1][q] = J[1][q];
+    sib[0][q] = J[2][q]; sib[1][q] = J[3][q];
   }
   return true;
 }
@@ -1042,8 +1048,9 @@ __device__ __forceinline__ void iface_body(const TransferParams& p, int j, long 
   {  // layer a's propagation, in its raw column order as X
     cd qf[2], qb[2];
     load_q(p, a, node, 0, qf, qb);
-    const double d = p.layers[a].d;
-    X = redheffer_diag_left(expi(qf[0], d), expi(qf[1], d), expi(-qb[0], d), expi(-qb[1], d), X);
+    cd pf[2], pb[2];
+    propagation(qf, qb, p.layers[a].d, pf, pb);
+    X = redheffer_diag_left(pf[0], pf[1], pb[0], pb[1], X);
   }
   st_s4(p.sint + (long)(j - 2) * p.xrec * p.n, 0, p.n, node, X);
 }
@@ -1116,8 +1123,11 @@ __device__ __forceinline__ void scan_body(const TransferParams& p, long node) {
   M24 Fp, Fm;
   const M2 I2 = M2{cd{1, 0}, z, z, cd{1, 0}}, Z2 = M2{z, z, z, z};
   if (src < N) {
-    RR = dr(dl(expi(Qs[2], ds), expi(Qs[3], ds), SR), expi(Qs[0], -ds), expi(Qs[1], -ds));
-    const cd PF0 = expi(Qs[0], ds), PF1 = expi(Qs[1], ds), PB0 = expi(Qs[2], -ds), PB1 = expi(Qs[3], -ds);
+    cd P[2], B[2], nP[2], nB[2];
+    propagation(Qs, Qs + 2, ds, P, B);
+    propagation(Qs, Qs + 2, -ds, nP, nB);
+    RR = dr(dl(nB[0], nB[1], SR), nP[0], nP[1]);
+    const cd PF0 = P[0], PF1 = P[1], PB0 = B[0], PB1 = B[1];
     const M2 PRL = dl(PF0, PF1, RL);
     const M2 D = imin(mul(dr(PRL, PB0, PB1), RR));
     Fp.L = solve(D, I2);
@@ -1229,11 +1239,13 @@ __device__ __forceinline__ void walk_body(const TransferParams& p, long node) {
     cd Qs[4];
     load_q(p, src - 1, node, swaps, Qs, Qs + 2);
     if (src < N) {
-      const cd n0 = expi(Qs[0], -ds), n1 = expi(Qs[1], -ds);
-      RR = dr(dl(expi(Qs[2], ds), expi(Qs[3], ds), SR), n0, n1);
-      S11 = dr(S11, n0, n1);
-      const cd PB0 = expi(Qs[2], -ds), PB1 = expi(Qs[3], -ds);
-      const M2 PRL = dl(expi(Qs[0], ds), expi(Qs[1], ds), RL);
+      cd P[2], B[2], nP[2], nB[2];
+      propagation(Qs, Qs + 2, ds, P, B);
+      propagation(Qs, Qs + 2, -ds, nP, nB);
+      RR = dr(dl(nB[0], nB[1], SR), nP[0], nP[1]);
+      S11 = dr(S11, nP[0], nP[1]);
+      const cd PB0 = B[0], PB1 = B[1];
+      const M2 PRL = dl(P[0], P[1], RL);
       const M2 D = imin(mul(dr(PRL, PB0, PB1), RR));
       Fp.L = solve(D, I2);
       Fp.R = solve(D, PRL);
