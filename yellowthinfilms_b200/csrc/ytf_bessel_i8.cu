@@ -33,7 +33,7 @@ constexpr double BI_SCALE = 8355000.0;
 size_t bessel_i8_stage_bytes_a() { return 3ul * BI_M * 64; }
 size_t bessel_i8_stage_bytes_b(int Np) { return 3ul * (size_t)Np * 64; }
 size_t bessel_i8_smem(int Np) {
-  return (size_t)BI_STAGES * (bessel_i8_stage_bytes_a() + bessel_i8_stage_bytes_b(Np)) + 128;
+  return (size_t)BI_STAGES * (bessel_i8_stage_bytes_a() + bessel_i8_stage_bytes_b(Np)) + 8 * BI_ACC_STRIDE + 128;
 }
 int bessel_i8_ctile(int N) {
   int nt = (N + 159) / 160;
@@ -397,6 +397,7 @@ cudaError_t launch_bessel_i8_aimg3(const BesselI8& p, uint8_t* A0, uint8_t* A1, 
 }
 
 struct BiShared {
+  double fac[BI_ACC_STRIDE];  // per column: what one unit of the combined digits is worth
   uint64_t full[BI_STAGES], empty[BI_STAGES], done;
   uint32_t tmem;
   int abort_flag;
@@ -500,7 +501,17 @@ __device__ __forceinline__ void gemm_i8_img_body(const BesselI8& p, int mt, int 
       if (*abort_flag) bi_drain_wait(smem_u32(&sh->done), 0);
     }
   } else {
-    // epilogue: warp w reads tensor-memory lanes 32 (w % 4) .. +31 (rows of the radius tile)
+    // epilogue: warp w reads tensor-memory lanes 32 (w % 4) .. +31 (rows of the radius tile). The
+    // columns' factors are formed once per CTA while the MMAs run: two FP64 divisions per value in the
+    // drain took more than the MMAs of a short slice (440 CTAs of 3 stages each: 115 -> 44 us; 32 film
+    // stacks 466 -> 310 us; 1536 radii x 1025 heights 2.95 -> 2.66 ms)
+    const unsigned long long* cmax = p.colmax + (long)z * p.N;
+    for (int c = tid - 64; c < nct; c += 128) {
+      const unsigned long long bits = cmax[c0 + c];
+      const double m = __longlong_as_double((long long)bits);
+      sh->fac[c] = !isfinite(m) ? __longlong_as_double(0x7ff8000000000000LL) : m > 0.0 ? 65536.0 / (BI_SCALE * col_scale(bits)) : 0.0;
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");
     bool ok = bi_wait(smem_u32(&sh->done), 0, abort_flag, p.err, p.wait_limit);
     ok = __all_sync(0xffffffffu, ok) && !*abort_flag;
     if (ok && nst > 0) {
@@ -511,7 +522,6 @@ __device__ __forceinline__ void gemm_i8_img_body(const BesselI8& p, int mt, int 
       const double eA = r >= p.M ? 1.0 : p.rowscale ? p.rowscale[(long)z * p.M + r]
                                                      : j_env(p.kmin[z] * p.rho[r]);  // the row's J digit scale
       double* out = p.partial + (long)z * p.N * p.M;
-      const unsigned long long* cmax = p.colmax + (long)z * p.N;
       for (int e0 = 0; e0 < p.Np; e0 += 8) {
         uint32_t v0[8], v1[8], v2[8];
         tmem_ld8(tmem + lanebase + e0, v0);
@@ -523,12 +533,7 @@ __device__ __forceinline__ void gemm_i8_img_body(const BesselI8& p, int mt, int 
           const int cl = e0 + e;
           if (cl < nct && r < p.M) {
             const long long v = (long long)(int)v0[e] * 65536 + (long long)(int)v1[e] * 256 + (long long)(int)v2[e];
-            const unsigned long long bits = cmax[c0 + cl];
-            const double m = __longlong_as_double((long long)bits);
-            double f;
-            if (!isfinite(m)) f = __longlong_as_double(0x7ff8000000000000LL);
-            else f = m > 0.0 ? 65536.0 / (BI_SCALE * col_scale(bits)) : 0.0;
-            out[(long)(c0 + cl) * p.M + r] = (double)v * f * eA;
+            out[(long)(c0 + cl) * p.M + r] = (double)v * sh->fac[cl] * eA;
           }
         }
       }
