@@ -100,3 +100,17 @@ def test_bessel_pair_of_the_images():
     x = np.concatenate([np.linspace(25, 60, 3001), np.geomspace(60, 1e5, 3001)])
     a, b = api.bessel_j01(x)
     assert np.abs(a - j0(x)).max() <= 1e-12 and np.abs(b - j1(x)).max() <= 1e-12
+
+
+@pytest.mark.parametrize("im", [0.0, 1e-3, 0.4, 0.41, 3.0, 30.0])
+def test_complex_bessel_ranges(im):
+    """J_0, J_1, J_2 of z = x ± i im on both sides of every range: Taylor rows (0 <= x < 25 up to
+    |im| = 0.4, row edges at whole x), series (|z| <= 8), recurrence, asymptotic expansion (|z| >= 25).
+    The series' largest term is e^8 / √(16π) ≈ 4e2 of 2^-53 each: 1e-13 relative to e^|im| covers it."""
+    from scipy.special import jv
+    from yellowthinfilms_b200 import api
+    x = np.concatenate([np.linspace(0.0, 60.0, 1201), np.arange(1, 27) - 1e-9, [24.9999999, 25.0000001, 180.3]])
+    for sign in (1, -1):
+        z = x + 1j * sign * im
+        for n in (0, 1, 2):
+            assert np.abs(api.bessel_j(n, z) - jv(n, z)).max() < 1e-13 * np.exp(im)

@@ -1,22 +1,26 @@
 // ytf_bessel.cuh -- Bessel functions J_0, J_1, J_2 of a complex argument (device), for the
-// synthesis on a deformed kρ contour (kρ ρ complex). Three regimes, each a published method:
+// synthesis on a deformed kρ contour (kρ ρ complex, close to the real axis for most radii). Published
+// methods by range:
+//   0 <= Re z < 25, |Im z| <= 0.4 : the Taylor rows of J_0 about i + 1/2 (ytf_bessel_tab.cuh) at the
+//                   complex distance d, |d| <= 0.65: one complex Horner pass for the value and the
+//                   derivative -J_1, |error| < 1e-15;
+//   |z| >= 25     : the Hankel asymptotic expansion J_n(z) = √(2/(πz)) (P cos χ - Q sin χ),
+//                   χ = z - nπ/2 - π/4 (A&S 9.2.5, 9.2.9-10), P and Q as polynomials in 1/z² up to
+//                   the 19th term (the next is below 1e-17 at |z| = 25), both orders from one phase;
 //   |z| <= 8      : the power series J_n(z) = (z/2)^n Σ_m (-z²/4)^m / (m! (m+n)!)
 //                   (A&S 9.1.10); the largest term is ~1e2, so ~1e-14 absolute accuracy;
 //   8 < |z| < 25  : Miller's backward recurrence J_{k-1} = (2k/z) J_k - J_{k+1} from an order
 //                   N = |z| + 32 with the normalisation J_0 + 2 Σ_{k≥1} J_{2k} = 1 (A&S 9.1.27,
-//                   9.1.46), valid for complex z;
-//   |z| >= 25     : the Hankel asymptotic expansion J_n(z) = √(2/(πz)) (P cos χ - Q sin χ),
-//                   χ = z - nπ/2 - π/4 (A&S 9.2.5, 9.2.9-10), 24 terms (the terms fall below
-//                   1e-16 of the first well before the expansion's smallest term at k ~ 2|z|).
+//                   9.1.46), valid for complex z.
 // J_2 from the recurrence 2J_1/z - J_0 above |z| = 1, from its series below. Principal
-// branches (Re z > 0 on the contour).
+// branches (Re z > 0 on the contour). Bound by FP64 issue: 256 radii x 4096 contour nodes with
+// the slice maxima took 98 + 40 us with series, Miller and a 24-term complex loop per order and a pass
+// over the tables for the maxima; 31 us with the Taylor rows, the polynomials and the maxima per warp.
 #pragma once
+#include "ytf_bessel_tab.cuh"
 #include "ytf_complex.cuh"
 
 namespace ytf {
-
-__device__ __forceinline__ cd ccos(cd z) { return cd{cos(z.x) * cosh(z.y), -sin(z.x) * sinh(z.y)}; }
-__device__ __forceinline__ cd csin(cd z) { return cd{sin(z.x) * cosh(z.y), cos(z.x) * sinh(z.y)}; }
 
 // (z/2)^n Σ_m (-z²/4)^m / (m! (m+n)!), n = 0, 1, 2
 __device__ inline cd bessel_series(int n, cd z) {
@@ -37,7 +41,47 @@ __device__ inline cd bessel_series(int n, cd z) {
   return s * p;
 }
 
+// Hankel's coefficients a_k(n) = Π_{j<=k} (4n² - (2j - 1)²) / (k! 8^k)
+struct HankelCoef {
+  double a[2][20];
+};
+__host__ __device__ constexpr HankelCoef hankel_coef() {
+  HankelCoef h{};
+  for (int n = 0; n < 2; ++n) {
+    h.a[n][0] = 1.0;
+    for (int k = 1; k < 20; ++k) h.a[n][k] = h.a[n][k - 1] * (4.0 * n * n - (2.0 * k - 1) * (2.0 * k - 1)) / (8.0 * k);
+  }
+  return h;
+}
+// Σ_{k = first, first + 2, ... <= 19} ± a_k w^{(k - first) / 2}, signs alternating from +
+template <int N, int FIRST>
+__device__ __forceinline__ cd hankel_sum(cd w) {
+  constexpr HankelCoef h = hankel_coef();
+  cd s{(9 % 2 ? -1.0 : 1.0) * h.a[N][FIRST + 18], 0.0};
+#pragma unroll
+  for (int i = 8; i >= 0; --i) {
+    s = s * w;
+    s.x += (i % 2 ? -1.0 : 1.0) * h.a[N][FIRST + 2 * i];
+  }
+  return s;
+}
+
 __device__ inline void bessel_j01_c(cd z, cd& J0, cd& J1) {
+  if (z.x >= 0.0 && z.x < (double)JTAB_N && fabs(z.y) <= 0.4) {
+    const int i = (int)z.x;
+    const cd d{z.x - ((double)i + 0.5), z.y};
+    const double* c = JTAB + i * JTAB_M;
+    cd p{c[JTAB_M - 1], 0.0}, q{0.0, 0.0};
+#pragma unroll
+    for (int m = JTAB_M - 2; m >= 0; --m) {
+      q = q * d + p;
+      p = p * d;
+      p.x += c[m];
+    }
+    J0 = p;
+    J1 = -q;
+    return;
+  }
   const double az = cabs(z);
   if (az <= 8.0) {
     J0 = bessel_series(0, z);
@@ -57,7 +101,7 @@ __device__ inline void bessel_j01_c(cd z, cd& J0, cd& J1) {
       if (km1 > 0 && (km1 % 2) == 0) sum += jk * 2.0;
       if (km1 == 1) j1v = jk;
       if (km1 == 0) j0v = jk;
-      if (cabs(jk) > 1e200) {  // rescale on growth
+      if (cabs1(jk) > 1e200) {  // rescale on growth
         jk = jk * 1e-200; jp1 = jp1 * 1e-200; sum = sum * 1e-200; j1v = j1v * 1e-200;
       }
     }
@@ -68,28 +112,23 @@ __device__ inline void bessel_j01_c(cd z, cd& J0, cd& J1) {
     return;
   }
   // Hankel asymptotic expansion
-  const cd iz = recip(z);
+  const cd iz = recip(z), w = iz * iz;
   const cd sq = csqrt(iz * (2.0 / 3.14159265358979323846));
-  for (int n = 0; n <= 1; ++n) {
-    const double mu = 4.0 * n * n;
-    cd P{1.0, 0.0}, Q{0.0, 0.0};
-    cd term{1.0, 0.0};
-    for (int k = 1; k <= 24; ++k) {
-      const double a = (mu - (2.0 * k - 1) * (2.0 * k - 1)) / (8.0 * k);
-      term = term * iz * a;
-      if (k % 2 == 1) Q += ((k / 2) % 2 == 0 ? term : -term);
-      else P += ((k / 2) % 2 == 0 ? term : -term);
-    }
-    const cd chi = z - cd{n * 3.14159265358979323846 / 2 + 3.14159265358979323846 / 4, 0.0};
-    const cd J = sq * (P * ccos(chi) - Q * csin(chi));
-    if (n == 0) J0 = J;
-    else J1 = J;
-  }
+  const cd P0 = hankel_sum<0, 0>(w), Q0 = iz * hankel_sum<0, 1>(w);
+  const cd P1 = hankel_sum<1, 0>(w), Q1 = iz * hankel_sum<1, 1>(w);
+  // cos z and sin z, then χ_0 = z - π/4, χ_1 = χ_0 - π/2
+  double sx, cx;
+  sincos(z.x, &sx, &cx);
+  const double sh = sinh(z.y), ch = fabs(sh) < 1e150 ? sqrt(fma(sh, sh, 1.0)) : fabs(sh);
+  const cd cz{cx * ch, -sx * sh}, sz{sx * ch, cx * sh};
+  const cd c0 = (cz + sz) * 0.70710678118654752440, s0 = (sz - cz) * 0.70710678118654752440;
+  J0 = sq * (P0 * c0 - Q0 * s0);
+  J1 = sq * (P1 * s0 + Q1 * c0);
 }
 
 __device__ inline void bessel_j012_c(cd z, cd& J0, cd& J1, cd& J2) {
   bessel_j01_c(z, J0, J1);
-  if (cabs(z) < 1.0) J2 = bessel_series(2, z);
+  if (norm2(z) < 1.0) J2 = bessel_series(2, z);
   else J2 = recip(z) * J1 * 2.0 - J0;
 }
 

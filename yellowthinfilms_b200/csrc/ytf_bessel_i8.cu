@@ -396,6 +396,9 @@ cudaError_t launch_bessel_i8_aimg3(const BesselI8& p, uint8_t* A0, uint8_t* A1, 
   return cudaGetLastError();
 }
 
+// a row's digit scale from its slice maximum
+__device__ __forceinline__ double row_scale(double m) { return m > 0.0 && isfinite(m) ? m : 1.0; }
+
 struct BiShared {
   double fac[BI_ACC_STRIDE];  // per column: what one unit of the combined digits is worth
   uint64_t full[BI_STAGES], empty[BI_STAGES], done;
@@ -504,7 +507,7 @@ __device__ __forceinline__ void gemm_i8_img_body(const BesselI8& p, int mt, int 
     // epilogue: warp w reads tensor-memory lanes 32 (w % 4) .. +31 (rows of the radius tile). The
     // columns' factors are formed once per CTA while the MMAs run: two FP64 divisions per value in the
     // drain took more than the MMAs of a short slice (440 CTAs of 3 stages each: 115 -> 44 us; 32 film
-    // stacks 466 -> 310 us; 1536 radii x 1025 heights 2.95 -> 2.66 ms)
+    // stacks 466 -> 310 us; 4096 radii x 256 heights 2.95 -> 2.66 ms)
     const unsigned long long* cmax = p.colmax + (long)z * p.N;
     for (int c = tid - 64; c < nct; c += 128) {
       const unsigned long long bits = cmax[c0 + c];
@@ -519,7 +522,7 @@ __device__ __forceinline__ void gemm_i8_img_body(const BesselI8& p, int mt, int 
       const int q = warp & 3;
       const uint32_t lanebase = (uint32_t)(32 * q) << 16;
       const int r = mt * BI_M + 32 * q + lane;
-      const double eA = r >= p.M ? 1.0 : p.rowscale ? p.rowscale[(long)z * p.M + r]
+      const double eA = r >= p.M ? 1.0 : p.rowscale ? row_scale(p.rowscale[(long)z * p.M + r])
                                                      : j_env(p.kmin[z] * p.rho[r]);  // the row's J digit scale
       double* out = p.partial + (long)z * p.N * p.M;
       for (int e0 = 0; e0 < p.Np; e0 += 8) {
@@ -573,25 +576,6 @@ __global__ void __launch_bounds__(256) k_bimg_real(const __grid_constant__ Besse
   bimg_slice_body(set.e[i], blockIdx.x - set.first[i]);
 }
 
-// per (order, slice, radius): max(|Re J|, |Im J|) over the slice's nodes (1 where it is 0)
-__global__ void __launch_bounds__(256) k_jtab_max(BesselI8 p, const double* __restrict__ J, double* __restrict__ rs) {
-  const int z = blockIdx.x, r = blockIdx.y, o = blockIdx.z;
-  const long plane = (long)p.M * p.K;
-  const double* re = J + (2L * o) * plane + (long)r * p.K;
-  const double* im = re + plane;
-  const long k0 = (long)z * p.kchunk, k1 = min(p.K, k0 + p.kchunk);
-  double m = 0.0;
-  for (long k = k0 + threadIdx.x; k < k1; k += blockDim.x) m = fmax(m, fmax(fabs(re[k]), fabs(im[k])));
-  __shared__ double red[256];
-  red[threadIdx.x] = m;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + w]);
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) rs[((long)o * p.nchunk + z) * p.M + r] = red[0] > 0.0 && isfinite(red[0]) ? red[0] : 1.0;
-}
-
 // one thread per (image, radius tile, row, slice, 4-node word): the digits of Re or Im J_o
 // relative to the row's slice maximum, written as one 32-bit word of each digit plane
 struct Img6 {
@@ -614,7 +598,7 @@ __global__ void __launch_bounds__(256) k_jtab_img(BesselI8 p, const double* __re
   const int r = mt * BI_M + row;
   const bool rv = r < p.M;
   const int o = im / 2;
-  const double sA = rv ? BI_SCALE / rs[((long)o * p.nchunk + z) * p.M + r] : 0.0;
+  const double sA = rv ? BI_SCALE / row_scale(rs[((long)o * p.nchunk + z) * p.M + r]) : 0.0;
   const double* tab = J + (long)im * p.M * p.K + (long)(rv ? r : 0) * p.K;
   const long g = wq / 4;
   const int q = (int)(wq % 4);
@@ -638,12 +622,9 @@ __global__ void __launch_bounds__(256) k_jtab_img(BesselI8 p, const double* __re
     *reinterpret_cast<uint32_t*>(blk + (size_t)pl * BI_M * 64 + plane_off(row, kb) + 4 * q) = w[pl];
 }
 
-cudaError_t launch_jtable_images(const BesselI8& bp, const double* Jtab, double* rowscale, uint8_t* const img[6],
+cudaError_t launch_jtable_images(const BesselI8& bp, const double* Jtab, const double* rowscale, uint8_t* const img[6],
                                  cudaStream_t s) {
   if (bp.M <= 0 || bp.K <= 0) return cudaSuccess;
-  k_jtab_max<<<dim3((unsigned)bp.nchunk, (unsigned)bp.M, 3), 256, 0, s>>>(bp, Jtab, rowscale);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
   const long tot = 6L * bp.ntile_m * BI_M * bp.nchunk * (bp.kchunk / 4);
   Img6 im6;
   for (int i = 0; i < 6; ++i) im6.p[i] = img[i];

@@ -1727,8 +1727,10 @@ static int synth1d_parts(ytf_ctx* ctx, const SynthParams& sp, int nz, double dz,
   for (int o = 0; o < 3; ++o) be[o].Bimg = Bi + boff[o];
   if (cplx) {
     WS(Jc, double, "g_J", 6 * (size_t)nr * nk);
-    CK(LAUNCH("k_bessel_c", launch_bessel_c(sp.c.kr, sp.c.kri, nk, drho, nr, nk, Jc, ctx->stream)));
     WS(rs, double, "g_bic_rs", 3 * (size_t)nchunk * nr);
+    CK(cudaMemsetAsync(rs, 0, 8 * 3 * (size_t)nchunk * nr, ctx->stream));
+    CK(LAUNCH("k_bessel_c", launch_bessel_c(sp.c.kr, sp.c.kri, nk, drho, nr, nk, Jc, ctx->stream,
+                                            (unsigned long long*)rs, kchunk, nchunk)));
     uint8_t* imgs[6];
     for (int i = 0; i < 6; ++i) imgs[i] = Ai + i * abytes;
     CK(LAUNCH("k_bessel_i8", launch_jtable_images(be[0], Jc, rs, imgs, ctx->stream)));

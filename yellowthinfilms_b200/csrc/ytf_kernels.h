@@ -159,9 +159,9 @@ inline int c1d_amp_rows(int sym, int with_direct) { return !sym ? 12 : with_dire
 cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, double* C, long ldc, double dz, cudaStream_t s);
 // the same columns rounded to FP32 (the int8x3 contraction's input)
 cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, float* C, long ldc, double dz, cudaStream_t s);
-// J_n tables, rows ld apart
+// J_n tables, rows ld apart; rs (zeroed, [3][nchunk][nr]): the slices' largest |Re J|, |Im J| as bits
 cudaError_t launch_bessel_c(const double* kr, const double* kri, long nk, const double* rho, int nr, long ld, double* J,
-                            cudaStream_t s);
+                            cudaStream_t s, unsigned long long* rs = nullptr, long kchunk = 0, int nchunk = 0);
 cudaError_t launch_bessel_eval(long n, int order, const double* zr, const double* zi, double* outr, double* outi,
                                cudaStream_t s);
 cudaError_t launch_bessel(const double* kr, long nk, const double* rho, int nr, long ld, double* J0, double* J1,
@@ -325,14 +325,14 @@ struct BesselI8 {
   int arows;         // rows per block of the J image kernel (bessel_i8_arows)
   double* kmin;      // [nchunk] smallest node of each slice (the J digits' scale, launch_slice_kmin)
   const double* rowscale;  // [nchunk][M] the J digits' scale per (slice, radius) when set (digits
-                           // rint(J 8355000 / rowscale)); else j_env(kmin[z] ρ_r)
+                           // rint(J 8355000 / rowscale), 1 in place of 0 and non-finite values); else
+                           // j_env(kmin[z] ρ_r)
 };
-// complex J_n tables ([6][nr][nk]: Re J_0, Im J_0, Re J_1, ... from launch_bessel_c) into the
-// int8x3 layout: rowscale[o][z][r] = max over slice z of max(|Re J_o|, |Im J_o|) at radius r
-// (1 where it is 0), then for each order o and part (0 Re, 1 Im) the digit image
-// img[2 o + part] in bp's A layout (ntile_m x nchunk x stages); bp gives M, K, ntile_m, kchunk,
-// nchunk
-cudaError_t launch_jtable_images(const BesselI8& bp, const double* Jtab, double* rowscale, uint8_t* const img[6],
+// complex J_n tables ([6][nr][nk]: Re J_0, Im J_0, Re J_1, ... and their slice maxima rowscale from
+// launch_bessel_c) into the int8x3 layout: for each order o and part (0 Re, 1 Im) the digit image
+// img[2 o + part] in bp's A layout (ntile_m x nchunk x stages), relative to the row's slice maximum (to
+// 1 where that is 0 or not finite); bp gives M, K, ntile_m, kchunk, nchunk
+cudaError_t launch_jtable_images(const BesselI8& bp, const double* Jtab, const double* rowscale, uint8_t* const img[6],
                                  cudaStream_t s);
 // J_0(x), J_1(x) as the int8x3 1D synthesis evaluates them (Taylor rows below 25, asymptotic above)
 cudaError_t launch_bessel_j01(const double* x, long n, double* J0, double* J1, cudaStream_t s);

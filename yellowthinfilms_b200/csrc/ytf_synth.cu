@@ -239,29 +239,60 @@ __global__ void k_bessel(const double* kr, long nk, const double* rho, int nr, l
   J2[o] = a2;
 }
 
-// J_n(kρ ρ) of complex nodes (deformed contour): real and imaginary tables of each order
-__global__ void k_bessel_c(const double* kr, const double* kri, long nk, const double* rho, int nr, long ld, double* J) {
-  long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  int r = blockIdx.y;
-  if (k >= nk) return;
-  const cd z = cd{kr[k], kri[k]} * rho[r];
-  cd a0, a1, a2;
-  if (z.x == 0.0 && z.y == 0.0) {
-    a0 = cd{1.0, 0.0}; a1 = cd{0.0, 0.0}; a2 = cd{0.0, 0.0};
-  } else {
-    bessel_j012_c(z, a0, a1, a2);
+// largest of the warp's values max(|x|, |y|) as IEEE bits (non-negative doubles order as their bits),
+// Inf where either is not finite: the high words first, then the low words of the lanes that hold the
+// largest high one
+__device__ __forceinline__ unsigned long long warp_max_bits(cd v, bool live) {
+  unsigned hx = (unsigned)__double2hiint(v.x) & 0x7fffffffu, hy = (unsigned)__double2hiint(v.y) & 0x7fffffffu;
+  unsigned lx = (unsigned)__double2loint(v.x), ly = (unsigned)__double2loint(v.y);
+  const bool y = hy > hx || (hy == hx && ly > lx);
+  unsigned h = y ? hy : hx, l = y ? ly : lx;
+  if (h >= 0x7ff00000u) { h = 0x7ff00000u; l = 0; }
+  if (!live) h = l = 0;
+  const unsigned mh = __reduce_max_sync(0xffffffffu, h);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, h == mh ? l : 0u);
+  return (unsigned long long)mh << 32 | ml;
+}
+
+// J_n(kρ ρ) of complex nodes (deformed contour): real and imaginary tables of each order, rows ld apart.
+// With rs (zeroed by the caller; [order][slice][radius] IEEE bits, slices of kchunk nodes, a multiple of
+// 32) also each slice's largest |Re J| or |Im J|, reduced per warp.
+__global__ void __launch_bounds__(128) k_bessel_c(const double* kr, const double* kri, long nk, const double* rho, int nr,
+                                                  long ld, double* J, unsigned long long* rs, long kchunk, int nchunk) {
+  const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int r = blockIdx.y;
+  const bool live = k < nk;
+  if (!live && !rs) return;
+  cd a[3] = {cd{0.0, 0.0}, cd{0.0, 0.0}, cd{0.0, 0.0}};
+  if (live) {
+    const cd z = cd{kr[k], kri[k]} * rho[r];
+    if (z.x == 0.0 && z.y == 0.0) a[0] = cd{1.0, 0.0};
+    else bessel_j012_c(z, a[0], a[1], a[2]);
+    const long o = (long)r * ld + k, plane = (long)nr * ld;
+#pragma unroll
+    for (int n = 0; n < 3; ++n) {
+      J[2 * n * plane + o] = a[n].x;
+      J[(2 * n + 1) * plane + o] = a[n].y;
+    }
   }
-  const long o = (long)r * ld + k, plane = (long)nr * ld;
-  J[o] = a0.x; J[plane + o] = a0.y;
-  J[2 * plane + o] = a1.x; J[3 * plane + o] = a1.y;
-  J[4 * plane + o] = a2.x; J[5 * plane + o] = a2.y;
+  if (rs) {
+    const int z = (int)(((long)blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) / kchunk);
+#pragma unroll
+    for (int n = 0; n < 3; ++n) {
+      // a NaN counts as no maximum
+      const cd v{a[n].x == a[n].x ? a[n].x : 0.0, a[n].y == a[n].y ? a[n].y : 0.0};
+      const unsigned long long bits = warp_max_bits(v, live);
+      if ((threadIdx.x & 31) == 0 && z < nchunk) atomicMax(rs + ((long)n * nchunk + z) * nr + r, bits);
+    }
+  }
 }
 
 cudaError_t launch_bessel_c(const double* kr, const double* kri, long nk, const double* rho, int nr, long ld, double* J,
-                            cudaStream_t s) {
+                            cudaStream_t s, unsigned long long* rs, long kchunk, int nchunk) {
   if (nk <= 0 || nr <= 0) return cudaSuccess;
+  if (rs && (kchunk <= 0 || kchunk % 32 != 0)) return cudaErrorInvalidValue;
   dim3 grid((unsigned)((nk + 127) / 128), (unsigned)nr);
-  k_bessel_c<<<grid, 128, 0, s>>>(kr, kri, nk, rho, nr, ld, J);
+  k_bessel_c<<<grid, 128, 0, s>>>(kr, kri, nk, rho, nr, ld, J, rs, kchunk, nchunk);
   return cudaGetLastError();
 }
 
@@ -921,21 +952,6 @@ cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, double* C, lon
 
 cudaError_t launch_coef1d_amp(const SynthParams& p, double2* amp, float* C, long ldc, double dz, cudaStream_t s) {
   return coef1d_amp_impl<float>(p, amp, C, ldc, dz, s);
-}
-
-// largest of the warp's values max(|x|, |y|) as IEEE bits (non-negative doubles order as their bits),
-// Inf where either is not finite: the high words first, then the low words of the lanes that hold the
-// largest high one
-__device__ __forceinline__ unsigned long long warp_max_bits(cd v, bool live) {
-  unsigned hx = (unsigned)__double2hiint(v.x) & 0x7fffffffu, hy = (unsigned)__double2hiint(v.y) & 0x7fffffffu;
-  unsigned lx = (unsigned)__double2loint(v.x), ly = (unsigned)__double2loint(v.y);
-  const bool y = hy > hx || (hy == hx && ly > lx);
-  unsigned h = y ? hy : hx, l = y ? ly : lx;
-  if (h >= 0x7ff00000u) { h = 0x7ff00000u; l = 0; }
-  if (!live) h = l = 0;
-  const unsigned mh = __reduce_max_sync(0xffffffffu, h);
-  const unsigned ml = __reduce_max_sync(0xffffffffu, h == mh ? l : 0u);
-  return (unsigned long long)mh << 32 | ml;
 }
 
 // z rows zo[0 .. m - 1] evenly spaced (to 4 ulp of the progression); every lane of the warp calls it
