@@ -63,12 +63,13 @@ __host__ __device__ __forceinline__ cd recip(cd b) {
 }
 
 // principal square root, signed-zero aware (branch cut on the negative real axis)
-__host__ __device__ __forceinline__ cd csqrt(cd z) {
+__host__ __device__ __forceinline__ cd csqrt_m(cd z, double m) {  // m = |z|
   if (z.x == 0.0 && z.y == 0.0) return cd{0.0, z.y};
-  double t = sqrt(0.5 * (fabs(z.x) + cabs(z)));
+  double t = sqrt(0.5 * (fabs(z.x) + m));
   if (z.x >= 0.0) return cd{t, z.y / (2.0 * t)};
   return cd{fabs(z.y) / (2.0 * t), copysign(t, z.y)};
 }
+__host__ __device__ __forceinline__ cd csqrt(cd z) { return csqrt_m(z, cabs(z)); }
 
 __host__ __device__ __forceinline__ cd cexp(cd z) {
   double e = exp(z.x);

@@ -48,7 +48,8 @@ __device__ __forceinline__ void node_k(const TransferParams& p, long node, cd& k
     kx = cd{p.kr[node], p.kr_im ? p.kr_im[node] : 0.0};
     ky = cd{0.0, 0.0};
   } else if (p.mode == 1) {  // full 2D solve, node = k + Nk * q
-    long k = node % p.Nk, q = node / p.Nk;
+    const long q = (unsigned long)node <= 0xffffffffu ? (long)((unsigned)node / (unsigned)p.Nk) : node / p.Nk;
+    const long k = node - q * p.Nk;
     double s, c;
     sincos(p.phi[q], &s, &c);
     kx = cd{p.kr[k] * c, 0.0};
@@ -89,6 +90,18 @@ __device__ void berreman(const LayerDev& L, double w, cd kx, cd ky, cd B[4][4]) 
   B[3][0] = t32 * dm * t21 - (-w) * Se11; B[3][1] = t32 * dm * t22 - (-w) * Se12;
   B[2][2] = Rse1 * t21 - k1 * rm1; B[2][3] = Rse1 * t22 - k1 * rm2;
   B[3][2] = Rse2 * t21 - k2 * rm1; B[3][3] = Rse2 * t22 - k2 * rm2;
+}
+
+// the blocks B12 and B21 of the same matrix without xz/yz coupling (B11 = B22 = 0 there)
+__device__ __forceinline__ void berreman_blocks(const LayerDev& L, double w, cd kx, cd ky, cd B12[2][2], cd B21[2][2]) {
+  const cd de = recip(E(L, 3, 3)), dm = recip(U(L, 3, 3));
+  const double iw = 1.0 / w;
+  const cd t31 = iw * kx, t32 = iw * ky;
+  const cd e1 = t31 * de, e2 = t32 * de, u1 = t31 * dm, u2 = t32 * dm;
+  B12[0][0] = w * U(L, 2, 1) + e1 * ky; B12[0][1] = w * U(L, 2, 2) - e1 * kx;
+  B12[1][0] = e2 * ky - w * U(L, 1, 1); B12[1][1] = -(w * U(L, 1, 2)) - e2 * kx;
+  B21[0][0] = -(u1 * ky) - w * E(L, 2, 1); B21[0][1] = u1 * kx - w * E(L, 2, 2);
+  B21[1][0] = w * E(L, 1, 1) - u2 * ky; B21[1][1] = u2 * kx + w * E(L, 1, 2);
 }
 
 // ------------------------------------------------------------------------------------
@@ -312,7 +325,7 @@ __device__ void closed_modes(const LayerDev& L, double w, cd kx, cd ky, cd Q[4],
   cd kr2;
   if (kx.y == 0.0 && ky.y == 0.0) {
     // cos and sin of the in-plane direction (φ = 0 at the origin), without the angle itself
-    const double kr = hypot(kx.x, ky.x);
+    const double kr = ky.x == 0.0 ? fabs(kx.x) : cabs(cd{kx.x, ky.x});
     c = kr == 0 ? 1.0 : kx.x / kr;
     s = kr == 0 ? 0.0 : ky.x / kr;
     kr2 = cd{kr * kr, 0.0};
@@ -345,21 +358,24 @@ __device__ __forceinline__ bool no_z_coupling(const LayerDev& L) {
          iszero(U(L, 2, 3)) && iszero(U(L, 3, 1)) && iszero(U(L, 3, 2));
 }
 
-__device__ bool block_modes(const LayerDev& L, double w, cd kx, cd ky, cd Q[4], cd V[4][4]) {
-  cd B[4][4];
-  berreman(L, w, kx, ky, B);
-  // M = B12 B21 (B12 = rows 0-1, cols 2-3; B21 = rows 2-3, cols 0-1)
-  cd m11 = B[0][2] * B[2][0] + B[0][3] * B[3][0], m12 = B[0][2] * B[2][1] + B[0][3] * B[3][1];
-  cd m21 = B[1][2] * B[2][0] + B[1][3] * B[3][0], m22 = B[1][2] * B[2][1] + B[1][3] * B[3][1];
+// The pairs come as Q[2i + 1] = -Q[2i], V[.][2i + 1] the same vector with (a; b) -> (a; -b) or (-a; b),
+// unsorted. Each μ takes one normalisation, one square root and one reciprocal for its two vectors.
+__device__ __forceinline__ bool block_modes(const LayerDev& L, double w, cd kx, cd ky, cd Q[4], cd V[4][4]) {
+  cd P[2][2], R[2][2];  // B12, B21
+  berreman_blocks(L, w, kx, ky, P, R);
+  // M = B12 B21
+  cd m11 = P[0][0] * R[0][0] + P[0][1] * R[1][0], m12 = P[0][0] * R[0][1] + P[0][1] * R[1][1];
+  cd m21 = P[1][0] * R[0][0] + P[1][1] * R[1][0], m22 = P[1][0] * R[0][1] + P[1][1] * R[1][1];
   cd hd = (m11 - m22) * 0.5;
   cd disc = csqrt(hd * hd + m12 * m21);
   cd mid = (m11 + m22) * 0.5;
   cd mu[2] = {mid + disc, mid - disc};
+  const double am[2] = {cabs(mu[0]), cabs(mu[1])};
   // the largest entry (1-norms: within √2 of the moduli) sets the scale of q² below
   const double scale = fmax(fmax(cabs1(m11), cabs1(m22)), fmax(cabs1(m12), cabs1(m21)));
   if (!(scale > 0) || !isfinite(scale)) return false;
-  if (cabs(mu[0] - mu[1]) <= 1e-6 * fmax(cabs(mu[0]), cabs(mu[1]))) return false;
-  int col = 0;
+  if (cabs(mu[0] - mu[1]) <= 1e-6 * fmax(am[0], am[1])) return false;
+  bool fin = true;
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     // eigenvector of M for mu_i: (m12, mu_i - m11) or (mu_i - m22, m21), the larger one;
@@ -370,49 +386,54 @@ __device__ bool block_modes(const LayerDev& L, double w, cd kx, cd ky, cd Q[4], 
     double n1 = norm2(a1x) + norm2(a1y), n2 = norm2(a2x) + norm2(a2y);
     cd ax = n1 >= n2 ? a1x : a2x, ay = n1 >= n2 ? a1y : a2y;
     if (!(fmax(n1, n2) > 0)) return false;
-    cd q = csqrt(mu[i]);
-    if (!(cabs(q) > 1e-12 * sqrt(scale))) return false;
+    if (!(am[i] > 1e-24 * scale)) return false;  // |q| > 1e-12 √scale
+    cd q = csqrt_m(mu[i], am[i]);
     // b = B21 a / q
     const cd rq = recip(q);
-    cd bx = (B[2][0] * ax + B[2][1] * ay) * rq, by = (B[3][0] * ax + B[3][1] * ay) * rq;
+    cd bx = (R[0][0] * ax + R[0][1] * ay) * rq, by = (R[1][0] * ax + R[1][1] * ay) * rq;
+    // unit 2-norm, largest component real (ZGEEVX)
+    const cd v[4] = {ax, ay, bx, by};
+    double nn = 0.0, best = -1.0;
+    cd vb{1.0, 0.0};
+    bool low = false;  // the largest component is in b
 #pragma unroll
-    for (int sgn = 0; sgn < 2; ++sgn) {
-      cd v[4] = {ax, ay, sgn ? -bx : bx, sgn ? -by : by};
-      double nn = 0.0, best = -1.0;
-      cd vb{1.0, 0.0};
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        double a2 = norm2(v[r]);
-        nn += a2;
-        if (a2 > best) { best = a2; vb = v[r]; }
-      }
-      const double inv = rsqrt(nn);  // unit 2-norm, largest component real (ZGEEVX)
-      const cd ph = conj(vb) * rsqrt(best);
-#pragma unroll
-      for (int r = 0; r < 4; ++r) V[r][col] = (v[r] * ph) * inv;
-      Q[col] = sgn ? -q : q;
-      ++col;
+    for (int r = 0; r < 4; ++r) {
+      const double a2 = norm2(v[r]);
+      nn += a2;
+      if (a2 > best) { best = a2; vb = v[r]; low = r >= 2; }
     }
+    const double inv = rsqrt(nn);
+    const cd ph = conj(vb) * rsqrt(best);
+    fin = fin && isfin(q);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const cd u = (v[r] * ph) * inv;
+      fin = fin && isfin(u);
+      V[r][2 * i] = u;
+      V[r][2 * i + 1] = (r >= 2) == low ? u : -u;
+    }
+    Q[2 * i] = q;
+    Q[2 * i + 1] = -q;
   }
-#pragma unroll
-  for (int c = 0; c < 4; ++c)
-    if (!isfin(Q[c]) || !isfin(V[0][c]) || !isfin(V[1][c]) || !isfin(V[2][c]) || !isfin(V[3][c])) return false;
-  // sort eigenpairs by (real, imag) (Julia's eigsortby): a 4-input sorting network
-  auto cswap = [&](int x, int y) {
-    bool sw = Q[y].x < Q[x].x || (Q[y].x == Q[x].x && Q[y].y < Q[x].y);
-    if (sw) {
-      cd t = Q[x]; Q[x] = Q[y]; Q[y] = t;
-#pragma unroll
-      for (int r = 0; r < 4; ++r) { cd u = V[r][x]; V[r][x] = V[r][y]; V[r][y] = u; }
-    }
-  };
-  cswap(0, 1); cswap(2, 3); cswap(0, 2); cswap(1, 3); cswap(1, 2);
-  return true;
+  return fin;
+}
+
+// Poynting flux Pz = ¼ Re(V_j · W_j) of mode j, W = R4s V = (V3, -V2, -V1, V0)
+__device__ __forceinline__ double mode_flux(const cd V[4][4], int j) {
+  cd s = conj(V[0][j]) * V[3][j];
+  s += conj(V[1][j]) * (-V[2][j]);
+  s += conj(V[2][j]) * (-V[1][j]);
+  s += conj(V[3][j]) * V[0][j];
+  return 0.25 * s.x;
 }
 
 // Forward/backward split of one layer's four eigenpairs (mod_ModeSolver.jl:274-326) and
 // the scratch record: Vf[4x2] (8), Vb[4x2] (8), Qf (2), Qb (2); column-major. Each
 // eigenpair is written straight to its slot, so no register array is indexed at run time.
+// PAIRS: V and Q hold ± pairs (2i, 2i + 1), whose fluxes differ in sign alone. SORT: the pairs are
+// taken in the order of (Re Q, Im Q) (Julia's eigsortby), by rank: the vectors themselves stay put
+// (a sorting network moved 40 doubles through 5 exchanges).
+template <bool PAIRS, bool SORT>
 __device__ __forceinline__ uint8_t classify_store(const TransferParams& p, int layer, long node, const cd Q[4],
                                                   const cd V[4][4]) {
   const long n = p.n;
@@ -424,33 +445,34 @@ __device__ __forceinline__ uint8_t classify_store(const TransferParams& p, int l
   // half-space's light line). On the real axis and below it the two rules agree.
   const bool proper = p.kr_im && (layer == 0 || layer == p.nL - 1);
   int cls[4];  // 0 forward, 1 backward, 2 degenerate
+  double Pz = 0.0;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    // Poynting flux Pz = ¼ Re(V_j · W_j), W = R4s V = (V3, -V2, -V1, V0)
-    cd s = conj(V[0][j]) * V[3][j];
-    s += conj(V[1][j]) * (-V[2][j]);
-    s += conj(V[2][j]) * (-V[1][j]);
-    s += conj(V[3][j]) * V[0][j];
-    double Pz = 0.25 * s.x;
+    Pz = PAIRS && (j & 1) ? -Pz : mode_flux(V, j);
     if (proper && fabs(Q[j].y) > tol * cabs(Q[j])) cls[j] = Q[j].y > 0 ? 0 : 1;
     else if (fabs(Pz) > tol) cls[j] = Pz > 0 ? 0 : 1;
     else if (fabs(Q[j].y) > tol) cls[j] = Q[j].y > tol ? 0 : 1;
     else cls[j] = 2;
   }
   // slots in eigen order; the degenerate ones then fill forward first (the reference's order)
-  int nf = 0, nb = 0, slot[4];
+  int cnt[2] = {0, 0}, rank[4] = {0, 0, 0, 0}, slot[4];  // rank: earlier modes of the same class
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    if (cls[j] == 0) slot[j] = nf++;
-    else if (cls[j] == 1) slot[j] = 2 + nb++;
-  }
-  if (nf > 2 || nb > 2) return ST_SORT;
+    cnt[0] += cls[j] == 0;
+    cnt[1] += cls[j] == 1;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    if (cls[j] == 2) {
-      if (nf < 2) slot[j] = nf++;
-      else slot[j] = 2 + nb++;
+    for (int i = 0; i < j; ++i) {
+      const bool jfirst = SORT && (Q[j].x < Q[i].x || (Q[j].x == Q[i].x && Q[j].y < Q[i].y));
+      const int same = cls[i] == cls[j];
+      rank[i] += jfirst ? same : 0;
+      rank[j] += jfirst ? 0 : same;
     }
+  }
+  if (cnt[0] > 2 || cnt[1] > 2) return ST_SORT;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int d = cnt[0] + rank[j];
+    slot[j] = cls[j] == 0 ? rank[j] : cls[j] == 1 ? 2 + rank[j] : d < 2 ? d : cnt[1] + d;
   }
   double2* rec = p.modes + (long)layer * 20 * n;
 #pragma unroll
@@ -474,14 +496,14 @@ __device__ __forceinline__ void layer_modes_body(const TransferParams& p, int la
   node_k(p, p.off + node, kx, ky);
   const LayerDev& L = p.layers[layer];
   cd Q[4], V[4][4];
-  bool done;
+  uint8_t stat = ST_NEED_QR;
   if ((L.ekind == 0 || L.ekind == 1) && L.mkind == 0) {
     closed_modes(L, p.omega, kx, ky, Q, V);
-    done = true;
-  } else {
-    done = no_z_coupling(L) && block_modes(L, p.omega, kx, ky, Q, V);
+    stat = classify_store<true, false>(p, layer, node, Q, V);
+  } else if (no_z_coupling(L) && block_modes(L, p.omega, kx, ky, Q, V)) {
+    stat = classify_store<true, true>(p, layer, node, Q, V);
   }
-  p.lstat[(long)layer * n + node] = done ? classify_store(p, layer, node, Q, V) : ST_NEED_QR;
+  p.lstat[(long)layer * n + node] = stat;
 }
 __global__ void __launch_bounds__(128) k_layer_modes(TransferParams p) {
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -501,7 +523,7 @@ __device__ __forceinline__ void layer_modes_qr_body(const TransferParams& p, int
   berreman(L, p.omega, kx, ky, B);
   uint8_t stat = 0;
   if (!eig4(B, Q, V)) stat = ST_EIGEN;
-  else stat = classify_store(p, layer, node, Q, V);
+  else stat = classify_store<false, false>(p, layer, node, Q, V);
   p.lstat[(long)layer * n + node] = stat;
 }
 __global__ void __launch_bounds__(128) k_layer_modes_qr(TransferParams p) {
