@@ -114,3 +114,17 @@ def test_complex_bessel_ranges(im):
         z = x + 1j * sign * im
         for n in (0, 1, 2):
             assert np.abs(api.bessel_j(n, z) - jv(n, z)).max() < 1e-13 * np.exp(im)
+
+
+@pytest.mark.parametrize("edge", [0.0, 1e-9, 0.5, 1.0, 2.0, 24.0, 25.0, 500.0])
+def test_real_bessel_ranges_of_the_fp64_tables(oracle, edge):
+    """FP64 1D synthesis with k ρ on both sides of an edge of the J_n ranges (series below 1, Taylor rows
+    at whole arguments, Hankel's expansion from 25), at the tolerance of the shapes above."""
+    from yellowthinfilms_b200 import api
+    st = config1_like_stack()
+    k, w = _rule(8)
+    gc = api.build_cavity_transfer_1d(st, W, 1, k, w, obs_layers=[1])
+    oc = oracle.build_cavity_transfer_1d(st, W, 1, k, w, obs_layers=[1])
+    rho = edge / k[3] * np.array([1 - 1e-12, 1.0, 1 + 1e-12])
+    Go = oracle.closed_form_G(oc, 1, 0.03, [0.05, 0.1], rho, [0.0])
+    assert relerr(api.closed_form_G(gc, 1, 0.03, [0.05, 0.1], rho, [0.0]), Go) < 1e-10

@@ -66,6 +66,15 @@ __device__ __forceinline__ cd hankel_sum(cd w) {
   return s;
 }
 
+template <int N, int FIRST>
+__device__ __forceinline__ double hankel_sum(double w) {
+  constexpr HankelCoef h = hankel_coef();
+  double s = (9 % 2 ? -1.0 : 1.0) * h.a[N][FIRST + 18];
+#pragma unroll
+  for (int i = 8; i >= 0; --i) s = fma(s, w, (i % 2 ? -1.0 : 1.0) * h.a[N][FIRST + 2 * i]);
+  return s;
+}
+
 __device__ inline void bessel_j01_c(cd z, cd& J0, cd& J1) {
   if (z.x >= 0.0 && z.x < (double)JTAB_N && fabs(z.y) <= 0.4) {
     const int i = (int)z.x;
