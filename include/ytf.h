@@ -393,11 +393,13 @@ typedef struct ytf_plan ytf_plan;
 typedef struct {
   int block;             /* threads per CTA of the persistent node-solve kernels: 128 or 256 */
   int ctas_per_sm;       /* node-solve grid: ctas_per_sm x SM count (1..32) */
-  int tile;              /* units per node-solve tile (nodes; (node, layer) pairs for the mode solve) */
-  int chunk;             /* nodes per synthesis work unit (multiple of 16) */
+  int tile;              /* units per node-solve tile at most (nodes; (node, layer) pairs for the mode solve);
+                            fewer until the tiles fill the grid */
+  int chunk;             /* nodes per synthesis work unit at most (multiple of 16); fewer until each resident
+                            CTA has four units */
   int synth_ctas_per_sm; /* synthesis grid: synth_ctas_per_sm x SM count (1..8) */
 } ytf_tune;
-/* tune NULL: block 128, 4 CTAs per SM, tile 1024, chunk 2048, 2 synthesis CTAs per SM */
+/* tune NULL: block 128, 4 CTAs per SM, tile 1024, chunk 2048, 3 synthesis CTAs per SM */
 int ytf_plan_create(ytf_ctx* ctx, int nb, const ytf_transfer_desc* tr, const ytf_green_desc* gr,
                     const ytf_tune* tune, ytf_plan** out);
 /* re-record the graph with other tiles (the caches, scratch and staging are kept) */

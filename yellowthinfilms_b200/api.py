@@ -843,7 +843,7 @@ class BatchPlan:
 
     @staticmethod
     def _tune_dict(tune):
-        t = dict(block=128, ctas_per_sm=4, tile=1024, chunk=2048, synth_ctas_per_sm=2)
+        t = dict(block=128, ctas_per_sm=4, tile=1024, chunk=2048, synth_ctas_per_sm=3)
         t.update(tune or {})
         return t
 

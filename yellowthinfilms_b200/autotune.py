@@ -22,9 +22,9 @@ import math
 import os
 from typing import Callable, Optional
 
-DEFAULT = dict(block=128, ctas_per_sm=4, tile=1024, chunk=2048, synth_ctas_per_sm=2)
+DEFAULT = dict(block=128, ctas_per_sm=4, tile=1024, chunk=2048, synth_ctas_per_sm=3)
 CANDIDATES = dict(ctas_per_sm=(1, 2, 4, 8), block=(128, 256), tile=(256, 1024, 4096), chunk=(512, 2048, 8192),
-                  synth_ctas_per_sm=(1, 2, 4))
+                  synth_ctas_per_sm=(1, 2, 3, 4))
 ORDER = ("ctas_per_sm", "block", "tile", "chunk", "synth_ctas_per_sm")
 
 

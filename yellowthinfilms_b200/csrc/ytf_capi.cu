@@ -2693,7 +2693,7 @@ int plan_build(ytf_plan* P) {
       if (P->nr[i] > SYN_MAXR || (long)P->nr[i] * 13 * g.nz > SYN_MAXOUT)
         return plan_fail(ctx, fail(ctx, YTF_ERR_ARG, "ytf_plan_create: 1D items need at most " + std::to_string(SYN_MAXR) +
                                                          " distinct radii and 13*nz*radii <= " + std::to_string(SYN_MAXOUT)), i);
-      P->nout_syn[i] = (long)P->nr[i] * 13 * g.nz;
+      P->nout_syn[i] = (long)P->nr[i] * (P->sps[i].sym ? 5 : 13) * g.nz;
       P->rmap_off[i] = rmap_count;
       rmap_count += (size_t)npix;
     }
@@ -2828,7 +2828,7 @@ int plan_build(ytf_plan* P) {
 extern "C" int ytf_plan_retune(ytf_plan* P, const ytf_tune* tune_in) {
   if (!P) return YTF_ERR_ARG;
   ytf_ctx* ctx = P->ctx;
-  ytf_tune t{128, 4, 1024, 2048, 2};
+  ytf_tune t{128, 4, 1024, 2048, 3};
   if (tune_in) t = *tune_in;
   if (!(t.block == 128 || t.block == 256) || t.ctas_per_sm < 1 || t.ctas_per_sm > 32 || t.tile < 1 || t.chunk < 16 ||
       t.chunk % 16 != 0 || t.synth_ctas_per_sm < 1 || t.synth_ctas_per_sm > 8)
@@ -2940,7 +2940,7 @@ extern "C" int ytf_plan_retune(ytf_plan* P, const ytf_tune* tune_in) {
     it.G = P->g_off[i] >= 0 ? P->d_G + P->g_off[i] : (double2*)g.out;
     items.push_back(it);
     item_of.push_back(i);
-    syn_smem = std::max(syn_smem, synth_small_smem(it.is2d, (int)npix, it.nr, g.nz));
+    syn_smem = std::max(syn_smem, synth_small_smem(it.is2d, it.sp.sym, (int)npix, it.nr, g.nz));
     npart += (size_t)it.nw * P->nout_syn[i];
     woff.push_back(woff.back() + it.nw);
     foff.push_back(foff.back() + (it.is2d ? npix * 9 * g.nz : npix * g.nz));

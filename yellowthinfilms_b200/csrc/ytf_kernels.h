@@ -242,11 +242,11 @@ struct SynthItem {
   const int* rmap;         // 1D: [nx ny] pixel -> radius (device)
   int nr;
   int nw;                  // node chunks of this item
-  double2* partial;        // [nw][outputs]
+  double2* partial;        // [nw][outputs] (1D: real columns, 10 nz or 26 nz of nr each)
   double2* G;              // [nx ny nz 9] Julia layout (device)
 };
 size_t synth_small_smem();                                      // the largest item's
-size_t synth_small_smem(int is2d, int npix, int nr, int nz);    // one item's
+size_t synth_small_smem(int is2d, int sym, int npix, int nr, int nz);  // one item's
 cudaError_t synth_small_init();  // shared-memory attribute of k_synth_small (before any capture)
 // w_off[nitems + 1]: prefix of the items' chunk counts; counter zeroed before the launch;
 // smem: the largest synth_small_smem(item) of the batch

@@ -1504,33 +1504,53 @@ cudaError_t launch_gl_nodes(int npanels, const double* pa, const double* pb, con
 
 // ------------------------------------------------------------------------------------
 // Batched synthesis of many small observation sets (uneven batches, one graph launch).
-// Work unit = (item, chunk of nodes), pulled by persistent CTAs from a counter. Per
-// sub-batch of SYN_SB = 64 nodes, threads 0-63 take one node each and form in shared memory
-//   2D: its strengths S[node][col] (col = zi + nz (cc + 3 q)), reflected amplitudes first;
-//   1D: its coefficient columns C[node][zi 13 + m] (m: 5 of order 0, 4 of order 1, 4 of
-//       order 2);
-// while threads 64-127 form for the same nodes
-//   2D: the phases P[node][pix] = e^{i kx x} e^{i ky y} (one sincos per x and per y);
-//   1D: the tables J_n(kρ ρ_r), n = 0, 1, 2;
-// then all threads accumulate the outputs o = row + nrow col of the item's partial sum (2D
-// rows: pixels; 1D rows: distinct radii) in shared memory, a strided set of outputs each,
-// over the sub-batch's nodes in registers. The shared arrays are laid out with the item's own
-// sizes. k_synth_finish sums the chunks of each output in chunk order (2D) or sums them and
-// assembles the pixel (1D).
+// Work unit = (item, chunk of nodes), pulled by persistent CTAs from a counter. Per sub-batch of
+// SYN_SB = 32 nodes (one per lane) the CTA's four warps form in shared memory
+//   first the phases of every z row (mode, forward / backward, direct) and of the source, rows and
+//   exponentials dealt out over the warps;
+//   then 2D: the strengths S[node][col] (col = zi + nz (cc + 3 q)), one source orientation q per warp,
+//   and the pixels' phases e^{i kx x} e^{i ky y} (one sincos per x and per y) on the fourth;
+//   or 1D: the real coefficient columns C[col][node], one group of columns per warp where TE and TM
+//   decouple (5 complex columns per row: c1s), every fourth row per warp otherwise (13 per row), and
+//   the tables J_n(kρ ρ_r), n = 0, 1, 2;
+// then the outputs o = row + nrow col of the item's partial sum (2D rows: pixels, complex columns; 1D
+// rows: distinct radii, real columns) take the sub-batch in register tiles of 4 rows x 3 (2D) or 1 (1D)
+// columns, small sets with the nodes split over 2 or 4 groups of warps. k_synth_finish sums the chunks
+// of each output in chunk order (2D) or sums them and assembles the pixel (1D).
+// Bound by FP64 latency and issue. 96 uneven items, 266k nodes, 16 pixels x 4 rows each: 487 us with 64 nodes
+// on two of the four warps (one thread through all of a node's strengths), 13 columns and one output
+// per thread, two CTAs per SM; 245 us (349 with two CTAs per SM and no prefetch).
 // ------------------------------------------------------------------------------------
-constexpr int SYN_SB = 64;
+constexpr int SYN_SB = 32, SYN_LD = SYN_SB + 1;
 
-// shared bytes of one item's work unit
-__host__ __device__ __forceinline__ size_t synth_item_smem(int is2d, int npix, int nr, int nz) {
-  const size_t nout = is2d ? (size_t)npix * 9 * nz : (size_t)nr * 13 * nz;
-  if (is2d) return 16 * nout + (size_t)SYN_SB * (npix + 9 * nz) * 16;
-  return 16 * nout + (size_t)SYN_SB * 3 * nr * 8 + (size_t)SYN_SB * 13 * nz * 16;
+// the shared arrays of one item's work unit (bytes from the start), laid out with the item's own sizes
+struct SynLayout {
+  int nrow, ncol, units, groups;  // outputs, register tiles, node groups
+  int acc, cols, tab, ph, bytes;
+};
+__host__ __device__ __forceinline__ SynLayout syn_layout(int is2d, int sym, int npix, int nr, int nz) {
+  SynLayout L;
+  L.nrow = is2d ? npix : nr;
+  L.ncol = is2d ? 9 * nz : (sym ? 10 : 26) * nz;
+  L.units = (L.nrow + 3) / 4 * (is2d ? (L.ncol + 2) / 3 : L.ncol);
+  L.groups = L.units <= 32 ? 4 : L.units <= 64 ? 2 : 1;
+  L.acc = 0;
+  L.cols = L.groups * L.nrow * L.ncol * (is2d ? 16 : 8);
+  L.cols = (L.cols + 15) / 16 * 16;
+  L.tab = L.cols + (is2d ? SYN_SB * (L.ncol | 1) * 16 : L.ncol * SYN_LD * 8);
+  L.tab = (L.tab + 15) / 16 * 16;
+  L.ph = L.tab + (is2d ? SYN_SB * (npix | 1) * 16 : 3 * nr * SYN_LD * 8);
+  L.ph = (L.ph + 15) / 16 * 16;
+  L.bytes = L.ph + (6 * nz + 4) * SYN_SB * 16;
+  return L;
 }
 
-size_t synth_small_smem(int is2d, int npix, int nr, int nz) { return synth_item_smem(is2d, npix, nr, nz); }
+size_t synth_small_smem(int is2d, int sym, int npix, int nr, int nz) {
+  return (size_t)syn_layout(is2d, sym, npix, nr, nz).bytes;
+}
 
 size_t synth_small_smem() {
-  const size_t a = synth_item_smem(1, SYN_MAXPIX, 0, SYN_MAXZ), b = synth_item_smem(0, 0, SYN_MAXR, SYN_MAXZ);
+  const size_t a = synth_small_smem(1, 0, SYN_MAXPIX, 0, SYN_MAXZ), b = synth_small_smem(0, 0, 0, SYN_MAXR, SYN_MAXZ);
   return a > b ? a : b;
 }
 
@@ -1544,12 +1564,215 @@ __device__ __forceinline__ int find_item(const long* __restrict__ off, int nb, l
   return lo;
 }
 
+// reflected amplitudes of source orientation q (reflected_amp, the source phases P: f 0, f 1, b 0, b 1)
+__device__ __forceinline__ void reflected_amp_q(const SynthParams& p, long k, int q, const cd P[4], cd Af[2], cd Ab[2]) {
+  const CacheView& c = p.c;
+  Af[0] = Af[1] = Ab[0] = Ab[1] = cd{0.0, 0.0};
+  if (!(c.valid[k] && c.tvalid[k])) return;
+  const cd sf0 = ldc(c.sf, 2 * q, c.n, k) * P[0], sf1 = ldc(c.sf, 1 + 2 * q, c.n, k) * P[1];
+  const cd sb0 = ldc(c.sb, 2 * q, c.n, k) * P[2], sb1 = ldc(c.sb, 1 + 2 * q, c.n, k) * P[3];
+  const cd uF[4] = {p.uf_F * sf0, p.uf_F * sf1, p.ub_F * sb0, p.ub_F * sb1};
+  const cd uB[4] = {p.uf_B * sf0, p.uf_B * sf1, p.ub_B * sb0, p.ub_B * sb1};
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      Af[m] += ldc(c.T, m + 4 * i, c.n, k) * uF[i];
+      Ab[m] += ldc(c.T, 2 + m + 4 * i, c.n, k) * uB[i];
+    }
+}
+
+// phases of one sub-batch, [row][lane]: 6 zi + 2 m + (0 forward, 1 backward) of mode m, 6 zi + 4 + m the
+// direct term's (forward above the source, backward below); 6 nz + i the source's P[i]
+__device__ __forceinline__ void syn_phases(const SynthParams& p, long node, int warp, int lane, double2* ph) {
+  const CacheView& c = p.c;
+  const long n = c.n;
+  for (int zi = warp; zi < p.nz; zi += 4) {
+    const double z = p.zo[zi], zeta = z - p.zpos;
+#pragma unroll 1
+    for (int e = 0; e < 6; ++e) {
+      if (e >= 4 && (!p.with_direct || zeta == 0.0)) continue;
+      const int m = e >= 4 ? e - 4 : e >> 1;
+      const bool b = e >= 4 ? zeta < 0.0 : (e & 1) != 0;
+      const cd kz = e >= 4 ? ldc(b ? c.Qb : c.Qf, m, n, node) : ldc(c.basis, (b ? 14 : 12) + m, n, node);
+      const double d = e >= 4 ? zeta : b ? z - p.d_obs : z;
+      const cd v = phase_cl(kz, d);
+      ph[(6 * zi + e) * SYN_SB + lane] = make_double2(v.x, v.y);
+    }
+  }
+  const int m = warp & 1;
+  const cd q = warp < 2 ? mul_i(ldc(c.Qf, m, n, node)) * (c.d_src - p.zpos) : mul_i(-ldc(c.Qb, m, n, node)) * p.zpos;
+  const cd v = cexp(q);
+  ph[(6 * p.nz + warp) * SYN_SB + lane] = make_double2(v.x, v.y);
+}
+
+// the next sub-batch's node data into L2 (48 rows, four 128-byte lines each of 32 nodes)
+__device__ __forceinline__ void syn_prefetch(const CacheView& c, long node0, int tid) {
+  for (int e = tid; e < 48 * 4; e += 128) {
+    const int f = e >> 2;
+    const long node = min(node0 + 8 * (e & 3), c.n - 1);
+    const double2* src = f < 16 ? c.T + f * c.n : f < 32 ? c.basis + (f - 16) * c.n : f < 38 ? c.sf + (f - 32) * c.n
+                       : f < 44 ? c.sb + (f - 38) * c.n : f < 46 ? c.Qf + (f - 44) * c.n : c.Qb + (f - 46) * c.n;
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(src + node));
+  }
+}
+
+// one orientation q of strengths_row at every z row of the node
+__device__ __forceinline__ void syn_strengths(const SynthParams& p, long node, int lane, int q, const double2* ph, cd* S) {
+  const CacheView& c = p.c;
+  const long n = c.n;
+  auto gp = [&](int f) { const double2 v = ph[f * SYN_SB + lane]; return cd{v.x, v.y}; };
+  const int nz = p.nz;
+  cd Af[2], Ab[2];
+  {
+    const cd P[4] = {gp(6 * nz), gp(6 * nz + 1), gp(6 * nz + 2), gp(6 * nz + 3)};
+    reflected_amp_q(p, node, q, P, Af, Ab);
+  }
+  const long pp = n <= 0x7fffffffL ? (long)((unsigned)node / (unsigned)c.Nk) : node / c.Nk, k = node - pp * c.Nk;
+  const double W = c.kr[k] * c.wr[k] * c.wphi[pp] / (4.0 * 3.14159265358979323846 * 3.14159265358979323846);
+  const bool dir = p.with_direct && c.valid[node];
+  cd ef[2][3], eb[2][3], sf[2], sb[2];
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      ef[m][a] = ldc(c.basis, 2 * a + m, n, node);
+      eb[m][a] = ldc(c.basis, 6 + 2 * a + m, n, node);
+    }
+    sf[m] = sb[m] = cd{0.0, 0.0};
+    if (dir) {
+      sf[m] = ldc(c.sf, m + 2 * q, n, node);
+      sb[m] = ldc(c.sb, m + 2 * q, n, node);
+    }
+  }
+  for (int zi = 0; zi < nz; ++zi) {
+    const double zeta = p.zo[zi] - p.zpos;
+    cd s[3] = {cd{0.0, 0.0}, cd{0.0, 0.0}, cd{0.0, 0.0}};
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      cd tf = Af[m] * gp(6 * zi + 2 * m), tb = Ab[m] * gp(6 * zi + 2 * m + 1);
+      if (dir && zeta > 0.0) tf += sf[m] * gp(6 * zi + 4 + m);
+      if (dir && zeta < 0.0) tb += sb[m] * gp(6 * zi + 4 + m);
+      const cd af = fin0(cd{W, 0.0} * tf), ab = fin0(cd{W, 0.0} * tb);
+#pragma unroll
+      for (int a = 0; a < 3; ++a) s[a] += ef[m][a] * af + eb[m][a] * ab;
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) S[zi + nz * (a + 3 * q)] = s[a];
+  }
+}
+
+// decoupled TE / TM: the columns of one warp at every z row (coef1d_row's xx of orders 0 and 2 on warp 0,
+// zx, xz, zz on warps 1, 2, 3), real and imaginary parts in rows of C
+__device__ __forceinline__ void syn_columns_sym(const SynthParams& p, long node, int warp, int lane, const double2* ph,
+                                                double* C) {
+  const CacheView& c = p.c;
+  const long n = c.n;
+  auto gp = [&](int f) { const double2 v = ph[f * SYN_SB + lane]; return cd{v.x, v.y}; };
+  const int nz = p.nz;
+  const cd W = cd{0.0, 1.0 / (2.0 * 3.14159265358979323846)} * cd{c.wr[node], c.wri ? c.wri[node] : 0.0};
+  const cd kx{c.kr[node], c.kri ? c.kri[node] : 0.0};
+  // which of the two modes is TE: the one with the larger E_y (the other's is zero)
+  const bool te1 = norm2(ldc(c.basis, 3, n, node)) + norm2(ldc(c.basis, 9, n, node)) >
+                   norm2(ldc(c.basis, 2, n, node)) + norm2(ldc(c.basis, 8, n, node));
+  const bool dir = p.with_direct && c.valid[node];
+  const cd P[4] = {gp(6 * nz), gp(6 * nz + 1), gp(6 * nz + 2), gp(6 * nz + 3)};
+  const cd half{0.0, -0.5};
+  // term t: 0 TE of y, 1 TM of x or z; amplitudes, field factors kx e and direct seeds
+  cd A[2][2], e[2][2], sd[2][2];
+  int md[2];
+  const int nt = warp == 0 ? 2 : 1;
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    if (t >= nt) break;
+    const bool teterm = warp == 0 && t == 0;
+    const int q = teterm ? 1 : warp < 2 ? 0 : 2;
+    md[t] = teterm == te1 ? 1 : 0;
+    cd Af[2], Ab[2];
+    reflected_amp_q(p, node, q, P, Af, Ab);
+    A[t][0] = md[t] ? Af[1] : Af[0];
+    A[t][1] = md[t] ? Ab[1] : Ab[0];
+    const int comp = teterm ? 2 : warp == 0 || warp == 2 ? 0 : 4;  // E_y, E_x or E_z of the mode
+    const cd f = warp == 0 ? half * kx : warp == 3 ? cd{0.0, -1.0} * kx : kx;
+#pragma unroll
+    for (int br = 0; br < 2; ++br) {
+      e[t][br] = f * ldc(c.basis, 6 * br + comp + md[t], n, node);
+      sd[t][br] = dir ? ldc(br ? c.sb : c.sf, md[t] + 2 * q, n, node) : cd{0.0, 0.0};
+    }
+  }
+  for (int zi = 0; zi < nz; ++zi) {
+    const double zeta = p.zo[zi] - p.zpos;
+    cd v[2];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      if (t >= nt) break;
+      const cd gf = gp(6 * zi + 2 * md[t]), gb = gp(6 * zi + 2 * md[t] + 1);
+      if (p.with_direct) {
+        cd tf = A[t][0] * gf, tb = A[t][1] * gb;
+        if (dir && zeta > 0.0) tf += sd[t][0] * gp(6 * zi + 4 + md[t]);
+        if (dir && zeta < 0.0) tb += sd[t][1] * gp(6 * zi + 4 + md[t]);
+        v[t] = fin0(W * tf) * e[t][0] + fin0(W * tb) * e[t][1];
+      } else {
+        v[t] = (fin0(W * A[t][0]) * gf) * e[t][0] + (fin0(W * A[t][1]) * gb) * e[t][1];
+      }
+    }
+    auto put = [&](int m, cd x) {
+      C[(10 * zi + 2 * m) * SYN_LD + lane] = x.x;
+      C[(10 * zi + 2 * m + 1) * SYN_LD + lane] = x.y;
+    };
+    if (warp == 0) {
+      put(0, v[0] + v[1]);
+      put(4, v[0] - v[1]);
+    } else {
+      put(warp == 1 ? 2 : warp == 2 ? 3 : 1, v[0]);
+    }
+  }
+}
+
+// acc (rows x cols of tile u; tw columns per tile) += the nodes t0 .. t1 - 1
+template <int TW, class Row, class Col, class T>
+__device__ __forceinline__ void syn_tile(int u, int nrow, int ncol, int t0, int t1, const Row& row, const Col& col, T* acc) {
+  const int nrt = (nrow + 3) / 4;
+  const int nct = (ncol + TW - 1) / TW;
+  // real columns run over the lanes, complex tiles keep a column's row tiles together
+  const int rt = TW == 1 ? u / nct : u % nrt, ct = TW == 1 ? u % nct : u / nrt;
+  const int r0 = 4 * rt, c0 = TW * ct;
+  T a[4][TW];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < TW; ++j) a[i][j] = acc[min(r0 + i, nrow - 1) + nrow * min(c0 + j, ncol - 1)];
+  for (int t = t0; t < t1; ++t) {
+    T x[4], y[TW];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) x[i] = row(t, min(r0 + i, nrow - 1), c0);
+#pragma unroll
+    for (int j = 0; j < TW; ++j) y[j] = col(t, min(c0 + j, ncol - 1));
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < TW; ++j) {
+        if constexpr (TW == 1) {
+          a[i][j] = fma(x[i], y[j], a[i][j]);
+        } else {
+          a[i][j].x = fma(x[i].x, y[j].x, fma(-x[i].y, y[j].y, a[i][j].x));
+          a[i][j].y = fma(x[i].x, y[j].y, fma(x[i].y, y[j].x, a[i][j].y));
+        }
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < TW; ++j)
+      if (r0 + i < nrow && c0 + j < ncol) acc[r0 + i + nrow * (c0 + j)] = a[i][j];
+}
+
 __global__ void __launch_bounds__(128, 3) k_synth_small(const SynthItem* __restrict__ items, int nitems,
                                                       const long* __restrict__ w_off, long nwork, unsigned* counter,
                                                       int chunk) {
   extern __shared__ __align__(16) unsigned char syn_smem[];
   __shared__ long wsh;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (;;) {
     if (tid == 0) wsh = (long)atomicAdd(counter, 1u);
     __syncthreads();
@@ -1564,103 +1787,96 @@ __global__ void __launch_bounds__(128, 3) k_synth_small(const SynthItem* __restr
     const long k0 = cid * chunk, k1 = min(c.n, k0 + chunk);
     const int nz = p.nz, npix = I.nx * I.ny;
     const bool two = I.is2d != 0;
-    const int ncol = two ? 9 * nz : 13 * nz;
-    const int nrow = two ? npix : I.nr;
-    const int nout = nrow * ncol;
-    cd* acc = reinterpret_cast<cd*>(syn_smem);                      // [nout]
-    cd* Ss = acc + nout;                                            // 2D [SB][ncol]
-    cd* Ps = Ss + SYN_SB * ncol;                                    // 2D [SB][npix]
-    cd* Cs = acc + nout;                                            // 1D [SB][ncol]
-    double* Js = reinterpret_cast<double*>(Cs + SYN_SB * ncol);     // 1D [SB][3][nr]
-    for (int o = tid; o < nout; o += 128) acc[o] = cd{0.0, 0.0};
+    const SynLayout L = syn_layout(two, p.sym, npix, I.nr, nz);
+    const int nout = L.nrow * L.ncol, nreal = two ? 2 * nout : nout;
+    double* acc = reinterpret_cast<double*>(syn_smem + L.acc);     // [groups][ncol][nrow], 2D complex
+    cd* Ss = reinterpret_cast<cd*>(syn_smem + L.cols);             // 2D [SB][ncol | 1]
+    cd* Ps = reinterpret_cast<cd*>(syn_smem + L.tab);              // 2D [SB][npix | 1]
+    double* Cs = reinterpret_cast<double*>(syn_smem + L.cols);     // 1D [ncol][SB + 1]
+    double* Js = reinterpret_cast<double*>(syn_smem + L.tab);      // 1D [3][nr][SB + 1]
+    double2* ph = reinterpret_cast<double2*>(syn_smem + L.ph);     // [6 nz + 4][SB]
+    for (int o = tid; o < L.groups * nreal; o += 128) acc[o] = 0.0;
     for (long b0 = k0; b0 < k1; b0 += SYN_SB) {
       const int nb = (int)min((long)SYN_SB, k1 - b0);
-      const int j = tid & (SYN_SB - 1);
-      const long node = b0 + j;
-      if (j < nb) {
-        if (tid < SYN_SB) {
-          cd Af[2][3], Ab[2][3];
-          reflected_amp(p, node, Af, Ab);
-          if (two) {
-            const long k = node % c.Nk, pp = node / c.Nk;
-            const double wt = c.kr[k] * c.wr[k] * c.wphi[pp] / (4.0 * 3.14159265358979323846 * 3.14159265358979323846);
-            cd kzf[2], kzb[2], ef[2][3], eb[2][3];
-            load_obs_basis(c, node, kzf, kzb, ef, eb);
-            for (int zi = 0; zi < nz; ++zi) {
-              cd sv[3][3];
-              strengths_row(p, node, p.zo[zi], cd{wt, 0.0}, Af, Ab, kzf, kzb, ef, eb, sv);
-              for (int q = 0; q < 3; ++q)
-                for (int cc = 0; cc < 3; ++cc) Ss[j * ncol + zi + nz * (cc + 3 * q)] = sv[cc][q];
-            }
-          } else {
-            for (int zi = 0; zi < nz; ++zi) {
-              cd c0[5], c1[4], c2[4];
-              coef1d_row(p, node, p.zo[zi], Af, Ab, c0, c1, c2);
-              cd* dst = Cs + j * ncol + 13 * zi;
-              for (int m = 0; m < 5; ++m) dst[m] = c0[m];
-              for (int m = 0; m < 4; ++m) { dst[5 + m] = c1[m]; dst[9 + m] = c2[m]; }
-            }
-          }
-        } else if (two) {
-          const long k = node % c.Nk, pp = node / c.Nk;
+      const long node = min(b0 + lane, k1 - 1);  // lanes past the end repeat the last node, and are not summed
+      if (b0 + SYN_SB < k1) syn_prefetch(c, b0 + SYN_SB, tid);
+      syn_phases(p, node, warp, lane, ph);
+      __syncthreads();  // the phases are in, the last sub-batch is summed
+      if (two) {
+        if (warp < 3) {
+          syn_strengths(p, node, lane, warp, ph, Ss + lane * (L.ncol | 1));
+        } else {
+          const long pp = c.n <= 0x7fffffffL ? (long)((unsigned)node / (unsigned)c.Nk) : node / c.Nk, k = node - pp * c.Nk;
           double sn, cs;
           sincos(c.phi[pp], &sn, &cs);
           const double kx = c.kr[k] * cs, ky = c.kr[k] * sn;
-          double sy[8], cy[8];
-          const int ny8 = min(I.ny, 8);
-          for (int jj = 0; jj < ny8; ++jj) sincos(ky * I.ys[jj], &sy[jj], &cy[jj]);
+          cd* P = Ps + lane * (npix | 1);
+          for (int jj = 0; jj < I.ny; ++jj) {  // e^{i ky y} in the row's last pixel, read before it is written
+            double s2, c2;
+            sincos(ky * I.ys[jj], &s2, &c2);
+            P[I.nx * jj + I.nx - 1] = cd{c2, s2};
+          }
           for (int i = 0; i < I.nx; ++i) {
             double sx, cx;
             sincos(kx * I.xs[i], &sx, &cx);
             for (int jj = 0; jj < I.ny; ++jj) {
-              double s2, c2;
-              if (jj < 8) { s2 = sy[jj]; c2 = cy[jj]; }
-              else sincos(ky * I.ys[jj], &s2, &c2);
-              Ps[j * npix + i + I.nx * jj] = cd{cx * c2 - sx * s2, cx * s2 + sx * c2};
+              const cd y = P[I.nx * jj + I.nx - 1];
+              P[i + I.nx * jj] = cd{cx * y.x - sx * y.y, cx * y.y + sx * y.x};
             }
           }
-        } else {
-          const double kx = c.kr[node];
-          double* dst = Js + j * 3 * I.nr;
-          for (int r = 0; r < I.nr; ++r) {
-            double a0, a1, a2;
-            bessel_j012(kx * I.rho[r], a0, a1, a2);
-            dst[r] = a0;
-            dst[I.nr + r] = a1;
-            dst[2 * I.nr + r] = a2;
+        }
+      } else {
+        if (p.sym) {
+          syn_columns_sym(p, node, warp, lane, ph, Cs);
+        } else if (warp < nz) {
+          cd Af[2][3], Ab[2][3];
+          reflected_amp(p, node, Af, Ab);
+          for (int zi = warp; zi < nz; zi += 4) {
+            cd cc[13];
+            coef1d_row(p, node, p.zo[zi], Af, Ab, cc, cc + 5, cc + 9);
+#pragma unroll
+            for (int m = 0; m < 13; ++m) {
+              Cs[(26 * zi + 2 * m) * SYN_LD + lane] = cc[m].x;
+              Cs[(26 * zi + 2 * m + 1) * SYN_LD + lane] = cc[m].y;
+            }
           }
+        }
+        const double kx = c.kr[node];
+        for (int r = 3 - warp; r < I.nr; r += 4) {  // warp 0 has the most columns: it comes last
+          double a0, a1, a2;
+          bessel_j012(kx * I.rho[r], a0, a1, a2);
+          Js[r * SYN_LD + lane] = a0;
+          Js[(I.nr + r) * SYN_LD + lane] = a1;
+          Js[(2 * I.nr + r) * SYN_LD + lane] = a2;
         }
       }
       __syncthreads();
-      for (int o = tid; o < nout; o += 128) {
-        const int row = o % nrow, cidx = o / nrow;
-        cd a = acc[o];
+      // groups of nodes: 4 of 32 threads, 2 of 64 or all 128 threads on all nodes
+      const int gt = 128 / L.groups, g = tid / gt, per = SYN_SB / L.groups;
+      const int t0 = g * per, t1 = min(nb, t0 + per);
+      for (int u = tid - g * gt; u < L.units; u += gt) {
         if (two) {
-          const cd* pp = Ps + row;
-          const cd* sp = Ss + cidx;
-          for (int t = 0; t < nb; ++t) {
-            const cd pv = pp[t * npix], sv = sp[t * ncol];
-            a.x = fma(pv.x, sv.x, fma(-pv.y, sv.y, a.x));
-            a.y = fma(pv.x, sv.y, fma(pv.y, sv.x, a.y));
-          }
+          const int pld = npix | 1, sld = L.ncol | 1;
+          syn_tile<3>(u, L.nrow, L.ncol, t0, t1, [&](int t, int r, int) { return Ps[t * pld + r]; },
+                      [&](int t, int cidx) { return Ss[t * sld + cidx]; }, reinterpret_cast<cd*>(acc) + g * nout);
         } else {
-          const int m = cidx % 13;
-          const int ord = m < 5 ? 0 : (m < 9 ? 1 : 2);
-          const double* jp = Js + ord * I.nr + row;
-          const cd* cp = Cs + cidx;
-          for (int t = 0; t < nb; ++t) {
-            const double jv = jp[t * 3 * I.nr];
-            const cd cv = cp[t * ncol];
-            a.x = fma(jv, cv.x, a.x);
-            a.y = fma(jv, cv.y, a.y);
-          }
+          const int R = p.sym ? 10 : 26, h1 = p.sym ? 4 : 10, h2 = p.sym ? 8 : 18, nr = I.nr;
+          syn_tile<1>(u, L.nrow, L.ncol, t0, t1,
+                      [&](int t, int r, int cidx) {
+                        const int h = cidx % R;
+                        return Js[((h < h1 ? 0 : h < h2 ? nr : 2 * nr) + r) * SYN_LD + t];
+                      },
+                      [&](int t, int cidx) { return Cs[cidx * SYN_LD + t]; }, acc + g * nout);
         }
-        acc[o] = a;
       }
-      __syncthreads();
     }
-    double2* out = I.partial + cid * (long)nout;
-    for (int o = tid; o < nout; o += 128) out[o] = make_double2(acc[o].x, acc[o].y);
+    __syncthreads();
+    double* out = reinterpret_cast<double*>(I.partial) + cid * (long)nreal;
+    for (int o = tid; o < nreal; o += 128) {
+      double v = acc[o];
+      for (int g = 1; g < L.groups; ++g) v += acc[g * nreal + o];
+      out[o] = v;
+    }
     __syncthreads();
   }
 }
@@ -1688,17 +1904,25 @@ __global__ void __launch_bounds__(128) k_synth_finish(const SynthItem* __restric
   const long pix = u % npix;
   const int zi = (int)(u / npix);
   const int r = I.rmap[pix];
-  const long nout = (long)I.nr * 13 * nz;
+  const int R = I.sp.sym ? 10 : 26;
+  const long nout = (long)I.nr * R * nz;
+  const double* part = reinterpret_cast<const double*>(I.partial) + r + (long)I.nr * R * zi;
+  double x[26];
+#pragma unroll
+  for (int m = 0; m < 26; ++m) x[m] = 0.0;
+  for (int k = 0; k < I.nw; ++k, part += nout)
+#pragma unroll
+    for (int m = 0; m < 26; ++m)
+      if (m < R) x[m] += part[(long)I.nr * m];
   cd g[13];
-  for (int m = 0; m < 13; ++m) {
-    cd s{0.0, 0.0};
-    const long o = r + (long)I.nr * (13 * zi + m);
-    for (int k = 0; k < I.nw; ++k) {
-      const double2 v = I.partial[(long)k * nout + o];
-      s.x += v.x;
-      s.y += v.y;
-    }
-    g[m] = s;
+  if (I.sp.sym) {
+    const cd z{0.0, 0.0}, c0{x[0], x[1]}, c4{x[8], x[9]};
+    g[0] = g[3] = c0; g[1] = g[2] = z; g[4] = cd{x[2], x[3]};
+    g[5] = cd{x[4], x[5]}; g[7] = cd{x[6], x[7]}; g[6] = g[8] = z;
+    g[9] = c4; g[12] = -c4; g[10] = g[11] = z;
+  } else {
+#pragma unroll
+    for (int m = 0; m < 13; ++m) g[m] = cd{x[2 * m], x[2 * m + 1]};
   }
   const int i = (int)(pix % I.nx), j = (int)(pix / I.nx);
   assemble1d_pixel(I.xs[i], I.ys[j], g, g + 5, g + 9, pix, npix, zi, nz, I.G);
