@@ -128,3 +128,15 @@ def test_real_bessel_ranges_of_the_fp64_tables(oracle, edge):
     rho = edge / k[3] * np.array([1 - 1e-12, 1.0, 1 + 1e-12])
     Go = oracle.closed_form_G(oc, 1, 0.03, [0.05, 0.1], rho, [0.0])
     assert relerr(api.closed_form_G(gc, 1, 0.03, [0.05, 0.1], rho, [0.0]), Go) < 1e-10
+
+
+@pytest.mark.parametrize("n", [450, 6001, 11003])
+def test_int8_slices_of_every_length(n):
+    """The coefficient images' blocks by slice length (up to 512 nodes, 10000, above) with a ragged last
+    stage: int8x3 against the FP64 synthesis of the same cache, at the shapes' 1e-6."""
+    from yellowthinfilms_b200 import api
+    k = 6 * W * (np.arange(n) + 0.5) / n
+    c = api.build_cavity_transfer_1d(config1_like_stack(), W, 1, k, np.full(n, 6 * W / n), obs_layers=[1])
+    z, x = np.linspace(0.0, 0.3, 256), np.geomspace(0.01, 3.0, 2048)
+    G = api.closed_form_G(c, 1, 0.03, z, x, [0.0], terms="scattered", precision="int8x3")
+    assert relerr(G, api.closed_form_G(c, 1, 0.03, z, x, [0.0], terms="scattered")) < 1e-6

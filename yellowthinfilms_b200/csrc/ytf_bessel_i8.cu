@@ -2,13 +2,13 @@
 //
 // closed_form_G for 1D caches (mod_ClosedFormField.jl:435-487) contracts, per Bessel order n,
 //   P_n[r][c] = Σ_k J_n(k_k ρ_r) C_n[c][k]
-// (C_n: the real and imaginary parts of the order's coefficient columns, k_coef1d). Both
+// (C_n: the real and imaginary parts of the order's coefficient columns, k_coef_sym or k_coef1d_amp). Both
 // operands are fixed point in three signed base-256 digits, as in the 2D lateral kernel:
 //   J: X = rint(8355000 J / j_env(k_min ρ))   per (radius, node slice): |J_n| ≤ j_env
 //   C: Y = rint(8355000 C / max|C|)   per (node slice, column)
 // and the six digit products of weight ≥ 256² are summed exactly in INT32 in tensor memory.
 // Unlike the lateral kernel, both operands are prepared once per launch as the exact shared-
-// memory image of each 64-node stage (k_aimg_bessel evaluates J_n straight into digits; no
+// memory image of each 64-node stage (k_aimg_bessel3 evaluates J_n straight into digits; no
 // FP64 table), so the contraction kernel only streams images: warp 0 issues the two bulk
 // copies of a stage (one mbarrier, byte-counted), one thread of warp 1 issues the 12 MMAs
 // (6 digit products x 2 K-halves; M=128 radii, N ≤ 160 columns, K=32), warps 2-5 read the
@@ -178,10 +178,17 @@ cudaError_t launch_slice_kmin(const double* kr, long K, long kchunk, int nchunk,
   return cudaGetLastError();
 }
 
-__device__ __forceinline__ void digits3b(int Y, uint32_t& d0, uint32_t& d1, uint32_t& d2) {
-  d2 = (uint32_t)Y & 255u;
-  d1 = (uint32_t)((Y + 128) >> 8) & 255u;
-  d0 = (uint32_t)((Y + 32896) >> 16) & 255u;
+// 1.5 2^52 + 0x808080: the low word of fma(v, scale, AI_MAGIC) is rint(v scale) + 0x808080, whose bytes are
+// the balanced digits + 128
+constexpr double AI_MAGIC = 6755399441055744.0 + 8421504.0;
+// the digit planes (most significant first) of four such words, one byte each: seven byte permutes in
+// place of the shifts, masks and additions of every digit by itself
+__device__ __forceinline__ void digit_words(const uint32_t u[4], uint32_t& d0, uint32_t& d1, uint32_t& d2) {
+  const uint32_t l01 = __byte_perm(u[0], u[1], 0x5140), l23 = __byte_perm(u[2], u[3], 0x5140);
+  const uint32_t h01 = __byte_perm(u[0], u[1], 0x0062), h23 = __byte_perm(u[2], u[3], 0x0062);
+  d0 = __byte_perm(h01, h23, 0x5410) ^ 0x80808080u;
+  d1 = __byte_perm(l01, l23, 0x7632) ^ 0x80808080u;
+  d2 = __byte_perm(l01, l23, 0x5410) ^ 0x80808080u;
 }
 
 __device__ __forceinline__ double col_scale(unsigned long long bits) {
@@ -189,30 +196,25 @@ __device__ __forceinline__ double col_scale(unsigned long long bits) {
   return (m > 0.0 && isfinite(m)) ? BI_SCALE / m : 0.0;
 }
 
-// the coefficient digit images and their (slice, column) maxima: one block of 256 threads per (column tile, 8-slot row group, node slice). Thread (j, r8) = (tid >> 3,
-// tid & 7) takes column slot 8 rg + r8 and the slice's 16-node groups j, j + 32, ...: a first
-// pass reduces max |C| (IEEE bits into colmax: a non-finite entry counts as Inf),
-// a second pass reads the same bytes again (from L2) and writes the digits. Each thread reads
-// 64 consecutive bytes of its column per group; a warp (four groups x eight slots) writes each
-// digit plane's 512-byte block of a stage whole. Blocks: ntile_n x (Np / 8) x nchunk.
-// 16 entries c[k0 .. k0 + 15] (k0 a multiple of 16, c's rows on 16 bytes), zero at k >= K: four
-// 16-byte loads when the group lies wholly below K
-__device__ __forceinline__ void load16(const float* c, long k0, long K, float v[16]) {
-  if (k0 + 16 <= K) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float4 f = __ldg(reinterpret_cast<const float4*>(c + k0) + q);
-      v[4 * q] = f.x; v[4 * q + 1] = f.y; v[4 * q + 2] = f.z; v[4 * q + 3] = f.w;
-    }
-  } else {
-#pragma unroll
-    for (int h = 0; h < 16; ++h) v[h] = k0 + h < K ? c[k0 + h] : 0.0f;
-  }
+// entries c[k .. k + 3] (k a multiple of 4, c's rows on 16 bytes), zero at k >= K
+__device__ __forceinline__ float4 load4(const float* c, long k, long K) {
+  if (k + 4 <= K) return __ldg(reinterpret_cast<const float4*>(c + k));
+  return make_float4(k < K ? c[k] : 0.0f, k + 1 < K ? c[k + 1] : 0.0f, k + 2 < K ? c[k + 2] : 0.0f, 0.0f);
 }
 
+// the coefficient digit images and their (slice, column) maxima: one block per (column tile, 8-slot row
+// group, node slice), its warps taking the slice's 64-node stages in turn, lane (r8, t) = (lane >> 2,
+// lane & 3) column slot 8 rg + r8 and nodes 16 i + 4 t .. + 3, i < 4, of a stage: every load takes 64
+// consecutive bytes of eight columns, every store one whole 128-byte line of a digit plane. A first pass
+// reduces max |C| (IEEE bits into colmax: a non-finite entry counts as Inf), a second reads the same
+// bytes again (from L2) and writes the digits. Blocks: ntile_n x (Np / 8) x nchunk.
+// Bound by the loads in flight: two stages' in the first pass, the next stage's in the second. 32 film
+// stacks x 64 heights (237M values) 349 us with 64 bytes of a column per thread (16 lines touched by each load, one
+// stage in flight) and the digits by conversions and shifts; 334 us. 65536 nodes x 2560 columns 367 -> 302 us.
 __device__ __forceinline__ void bimg_slice_body(const BesselI8& p, long b) {
-  __shared__ float wmax[8][8];
-  const int tid = threadIdx.x, r8 = tid & 7, j = tid >> 3;
+  __shared__ float wmax[32][8];
+  const int tid = threadIdx.x, lane = tid & 31, r8 = lane >> 2, t4 = 4 * (lane & 3);
+  const int warp = tid >> 5, nwarp = blockDim.x >> 5;
   const int rgroups = p.Np / 8;
   const int rg = (int)(b % rgroups);
   const long rest = b / rgroups;
@@ -222,52 +224,59 @@ __device__ __forceinline__ void bimg_slice_body(const BesselI8& p, long b) {
   const int col = ct * p.ctile + slot;
   const bool cv = slot < p.ctile && col < p.N;
   const float* c = p.C + (long)(cv ? col : 0) * p.ldc;
-  const long kbase = (long)z * p.kchunk;
-  const int groups = (int)(p.kchunk / 16);
-  float m = 0.0f;
-  for (int g = j; g < groups; g += 32) {
-    float v[16];
-    load16(c, kbase + 16L * g, cv ? p.K : 0, v);
+  const long K = cv ? p.K : 0, kbase = (long)z * p.kchunk + t4;
+  const int nstage = (int)(p.kchunk / BI_NODES);
+  int mi = 0;  // |C| orders as its bits; NaN above Inf
+  for (int s = warp; s < nstage; s += 2 * nwarp) {  // two stages' loads in flight
+    float4 f[8];
 #pragma unroll
-    for (int h = 0; h < 16; ++h) m = isfinite(v[h]) ? fmaxf(m, fabsf(v[h])) : __int_as_float(0x7f800000);
+    for (int i = 0; i < 8; ++i) {
+      const int st = s + (i >> 2) * nwarp;
+      f[i] = load4(c, kbase + 64L * st + 16 * (i & 3), st < nstage ? K : 0);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      mi = max(max(mi, __float_as_int(f[i].x) & 0x7fffffff), __float_as_int(f[i].y) & 0x7fffffff);
+      mi = max(max(mi, __float_as_int(f[i].z) & 0x7fffffff), __float_as_int(f[i].w) & 0x7fffffff);
+    }
   }
-  // lanes 8 apart share a slot: reduce over them, then over the block's eight warps
-  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
-  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
-  if ((tid & 31) < 8) wmax[tid >> 5][r8] = m;
+  // the four lanes of a slot, then the block's warps
+  float m = __int_as_float(min(mi, 0x7f800000));
+  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+  if (t4 == 0) wmax[warp][r8] = m;
   __syncthreads();
   float mm = wmax[0][r8];
-#pragma unroll
-  for (int w = 1; w < 8; ++w) mm = fmaxf(mm, wmax[w][r8]);
+  for (int w = 1; w < nwarp; ++w) mm = fmaxf(mm, wmax[w][r8]);
   const unsigned long long bits = (unsigned long long)__double_as_longlong((double)mm);
-  if (j == 0 && cv) p.colmax[(long)z * p.N + col] = bits;
+  if (warp == 0 && t4 == 0 && cv) p.colmax[(long)z * p.N + col] = bits;
   const double sB = cv ? col_scale(bits) : 0.0;
-  const long nstage = p.kchunk / BI_NODES;
-  const size_t sbytes = 3ul * (size_t)p.Np * 64;
-  uint8_t* base = p.Bimg + ((size_t)ct * p.nchunk + z) * nstage * sbytes;
-  for (int g = j; g < groups; g += 32) {
-    float v16[16];
-    load16(c, kbase + 16L * g, cv ? p.K : 0, v16);
-    uint32_t w[3][4];
+  const size_t plane = (size_t)p.Np * 64, sbytes = 3 * plane;
+  uint8_t* base = p.Bimg + ((size_t)ct * p.nchunk + z) * nstage * sbytes + t4;
+  float4 f[4], nx[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      uint32_t b0 = 0, b1 = 0, b2 = 0;
+  for (int i = 0; i < 4; ++i) nx[i] = load4(c, kbase + 64L * warp + 16 * i, warp < nstage ? K : 0);
+  for (int s = warp; s < nstage; s += nwarp) {
+    const int s1 = s + nwarp;
 #pragma unroll
-      for (int h = 0; h < 4; ++h) {
-        const double v = (double)v16[4 * q + h];
-        uint32_t d0, d1, d2;
-        digits3b(__double2int_rn(v * sB), d0, d1, d2);
-        b0 |= d0 << (8 * h);
-        b1 |= d1 << (8 * h);
-        b2 |= d2 << (8 * h);
-      }
-      w[0][q] = b0; w[1][q] = b1; w[2][q] = b2;
+    for (int i = 0; i < 4; ++i) {
+      f[i] = nx[i];
+      nx[i] = load4(c, kbase + 64L * s1 + 16 * i, s1 < nstage ? K : 0);
     }
-    uint8_t* blk = base + (size_t)(g / 4) * sbytes;
+    uint8_t* blk = base + (size_t)s * sbytes;
 #pragma unroll
-    for (int pl = 0; pl < 3; ++pl)
-      *reinterpret_cast<uint4*>(blk + (size_t)pl * p.Np * 64 + plane_off(slot, (g % 4) * 16)) =
-          make_uint4(w[pl][0], w[pl][1], w[pl][2], w[pl][3]);
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t u[4] = {(uint32_t)__double2loint(fma((double)f[i].x, sB, AI_MAGIC)),
+                             (uint32_t)__double2loint(fma((double)f[i].y, sB, AI_MAGIC)),
+                             (uint32_t)__double2loint(fma((double)f[i].z, sB, AI_MAGIC)),
+                             (uint32_t)__double2loint(fma((double)f[i].w, sB, AI_MAGIC))};
+      uint32_t d0, d1, d2;
+      digit_words(u, d0, d1, d2);
+      uint8_t* dst = blk + plane_off(slot, 16 * i);
+      *reinterpret_cast<uint32_t*>(dst) = d0;
+      *reinterpret_cast<uint32_t*>(dst + plane) = d1;
+      *reinterpret_cast<uint32_t*>(dst + 2 * plane) = d2;
+    }
   }
 }
 
@@ -285,7 +294,6 @@ __device__ __forceinline__ void bimg_slice_body(const BesselI8& p, long b) {
 // j1, a division and a root per pair and FP64-to-integer conversions, 1363 us; this form with 32-row
 // blocks and one pair after the other, 806 us.
 // ------------------------------------------------------------------------------------
-constexpr double AI_MAGIC = 6755399441055744.0 + 8421504.0;  // 1.5 2^52 + 0x808080
 
 // rows per block: a whole tile (the per-thread reciprocals then serve 32 pairs) once the stages alone
 // give each SM eight blocks, a quarter of it below
@@ -376,12 +384,12 @@ __device__ __forceinline__ void aimg_bessel3_body(const BesselI8& p, long b, uin
     const uint32_t at = plane_off(row, 4 * w);
 #pragma unroll
     for (int o = 0; o < 3; ++o) {
-      const uint32_t l01 = __byte_perm(U[o][0], U[o][1], 0x5140), l23 = __byte_perm(U[o][2], U[o][3], 0x5140);
-      const uint32_t h01 = __byte_perm(U[o][0], U[o][1], 0x0062), h23 = __byte_perm(U[o][2], U[o][3], 0x0062);
+      uint32_t d0, d1, d2;
+      digit_words(U[o], d0, d1, d2);
       uint8_t* dst = out[o] + at;
-      *reinterpret_cast<uint32_t*>(dst) = __byte_perm(h01, h23, 0x5410) ^ 0x80808080u;
-      *reinterpret_cast<uint32_t*>(dst + BI_M * 64) = __byte_perm(l01, l23, 0x7632) ^ 0x80808080u;
-      *reinterpret_cast<uint32_t*>(dst + 2 * BI_M * 64) = __byte_perm(l01, l23, 0x5410) ^ 0x80808080u;
+      *reinterpret_cast<uint32_t*>(dst) = d0;
+      *reinterpret_cast<uint32_t*>(dst + BI_M * 64) = d1;
+      *reinterpret_cast<uint32_t*>(dst + 2 * BI_M * 64) = d2;
     }
   }
 }
@@ -570,7 +578,7 @@ __global__ void __launch_bounds__(BI_THREADS, 1) k_gemm_i8_img(const __grid_cons
   const long rest = b / p.ntile_m;
   gemm_i8_img_body(p, mt, (int)(rest % p.ntile_n), (int)(rest / p.ntile_n), smem);
 }
-__global__ void __launch_bounds__(256) k_bimg_real(const __grid_constant__ BesselI8Set set) {
+__global__ void __launch_bounds__(1024) k_bimg_real(const __grid_constant__ BesselI8Set set) {
   int i = 0;
   while (i + 1 < set.n && set.first[i + 1] <= (long)blockIdx.x) ++i;
   bimg_slice_body(set.e[i], blockIdx.x - set.first[i]);
@@ -602,17 +610,14 @@ __global__ void __launch_bounds__(256) k_jtab_img(BesselI8 p, const double* __re
   const double* tab = J + (long)im * p.M * p.K + (long)(rv ? r : 0) * p.K;
   const long g = wq / 4;
   const int q = (int)(wq % 4);
-  uint32_t w[3] = {0u, 0u, 0u};
+  uint32_t v4[4], w[3];
 #pragma unroll
   for (int h = 0; h < 4; ++h) {
     const long k = (long)z * p.kchunk + 16 * g + 4 * q + h;
     const double v = (rv && k < p.K) ? tab[k] : 0.0;
-    uint32_t d0, d1, d2;
-    digits3b(__double2int_rn(v * sA), d0, d1, d2);
-    w[0] |= d0 << (8 * h);
-    w[1] |= d1 << (8 * h);
-    w[2] |= d2 << (8 * h);
+    v4[h] = (uint32_t)__double2int_rn(v * sA) + 0x808080u;  // digits 0 for a NaN
   }
+  digit_words(v4, w[0], w[1], w[2]);
   const long nstage = p.kchunk / BI_NODES;
   const int s = (int)(g / 4), kb = (int)(g % 4) * 16;
   const size_t sbytes = 3ul * BI_M * 64;
@@ -637,6 +642,14 @@ static bool entry_ok(const BesselI8& p) {
          p.Np <= BI_ACC_STRIDE && p.Np >= p.ctile && (long)p.nchunk * p.kchunk >= p.K && p.ldc % 4 == 0;
 }
 
+// threads of a block of the coefficient images (see bimg_slice_body). Long slices: the resident blocks'
+// slices, 32 bytes per node each, have to stay in L2 between the two passes (16384 nodes: 300 us at
+// 1024 threads, 360 us at 256); short ones: no warp without a stage (192 nodes: 10.2 us at 128, 14.5 us at
+// 256 threads).
+static unsigned bimg_threads(long kchunk) {
+  return kchunk > 10000 ? 1024 : kchunk > 5000 ? 512 : kchunk > 512 ? 256 : 128;
+}
+
 cudaError_t launch_bimg(const BesselI8* e, int n, cudaStream_t s) {
   BesselI8Set set;
   set.n = n;
@@ -648,7 +661,7 @@ cudaError_t launch_bimg(const BesselI8* e, int n, cudaStream_t s) {
     blocks += (long)e[i].ntile_n * (e[i].Np / 8) * e[i].nchunk;
   }
   if (blocks <= 0) return cudaSuccess;
-  k_bimg_real<<<(unsigned)blocks, 256, 0, s>>>(set);
+  k_bimg_real<<<(unsigned)blocks, bimg_threads(e[0].kchunk), 0, s>>>(set);
   return cudaGetLastError();
 }
 
@@ -693,7 +706,7 @@ __global__ void __launch_bounds__(256) k_slice_kmin_group(const BesselI8* __rest
 }
 
 // ntile_n x (Np / 8) x nchunk blocks per entry (bimg_slice_body)
-__global__ void __launch_bounds__(256) k_bimg_real_group(const BesselI8* __restrict__ bp, const long* __restrict__ first,
+__global__ void __launch_bounds__(1024) k_bimg_real_group(const BesselI8* __restrict__ bp, const long* __restrict__ first,
                                                        int ne) {
   const int e = group_entry(first, ne, blockIdx.x);
   bimg_slice_body(bp[e], blockIdx.x - first[e]);
@@ -725,7 +738,7 @@ cudaError_t launch_bessel_i8_group(const Synth1DGroup& g, int stage, cudaStream_
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   if (stage == 1 && g.grid[3] > 0) {
-    k_bimg_real_group<<<(unsigned)g.grid[3], 256, 0, s>>>(g.bp, g.first_bimg, ne);
+    k_bimg_real_group<<<(unsigned)g.grid[3], bimg_threads(g.kchunk), 0, s>>>(g.bp, g.first_bimg, ne);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   if (stage == 2 && g.grid[4] > 0) {

@@ -2068,7 +2068,7 @@ static Group1DLayout group1d_layout(int item, const SynthParams& sp, int nz, int
 struct Group1DDesc {
   size_t off_it, off_bp, off_first, bytes;
   int ni;
-  long grid[9];
+  long grid[9], kchunk;
 };
 
 static bool group1d_eligible(const ytf_ctx* ctx, const ytf_green_desc& g) {
@@ -2217,7 +2217,7 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
     long* f_csym = f_rsym + (ni + 1);
     long* f_bimg = f_csym + (ni + 1);
     long* f_gemm = f_bimg + (3 * ni + 1);
-    long nref = 0, ncoef = 0, naimg = 0, nasm = 0, nbimg = 0, ngemm = 0, nkmin = 0, nrsym = 0, ncsym = 0;
+    long longest = 0, nref = 0, ncoef = 0, naimg = 0, nasm = 0, nbimg = 0, ngemm = 0, nkmin = 0, nrsym = 0, ncsym = 0;
     long stages = 0;  // of the group's J images
     for (size_t j = groups[g].first; j < groups[g].second; ++j) stages += (long)lay[j].ntm * lay[j].nchunk * (lay[j].kchunk / 64);
     const int arows = bessel_i8_arows(stages);
@@ -2251,6 +2251,7 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
       f_csym[q] = ncsym; ncsym += sym ? nkb * ((L.nz + COEF_SYM_ZB - 1) / COEF_SYM_ZB) : 0;
       f_asm[q] = nasm; nasm += asm1d_blocks(it.a);
       f_kmin[q] = nkmin; nkmin += L.nchunk;
+      longest = std::max(longest, L.kchunk);
       const size_t coff[3] = {0, (size_t)L.N[0] * L.ldc, (size_t)(L.N[0] + L.N[1]) * L.ldc};
       for (int od = 0; od < 3; ++od) {
         BesselI8& bp = hbp[3 * q + od];
@@ -2283,6 +2284,7 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
     f_bimg[3 * ni] = nbimg; f_gemm[3 * ni] = ngemm;
     const long grid[9] = {nref, ncoef, naimg, nbimg, ngemm, nasm, nkmin, nrsym, ncsym};
     for (int k = 0; k < 9; ++k) D.grid[k] = grid[k];
+    D.kchunk = longest;
   }
   CK(cudaMemcpyAsync(dc, h, total_bytes, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemsetAsync(err, 0, sizeof(unsigned), ctx->stream));
@@ -2305,6 +2307,7 @@ int ytf_green_batch(ytf_ctx* ctx, int nb, const ytf_green_desc* d) {
     G.first_bimg = df + 7 * (ni + 1);
     G.first_gemm = G.first_bimg + (3 * ni + 1);
     for (int k = 0; k < 9; ++k) G.grid[k] = D.grid[k];
+    G.kchunk = D.kchunk;
     CK(LAUNCH("k_reflect2d", launch_reflect_coef_group(G, 0, ctx->stream)));
     CK(LAUNCH("k_coef1d", launch_reflect_coef_group(G, 1, ctx->stream)));
     CK(LAUNCH("k_aimg_bessel3", launch_bessel_i8_group(G, 0, ctx->stream)));

@@ -386,6 +386,7 @@ struct Synth1DGroup {
   const long* first_rsym;      // [ni + 1] symmetric items' factors and columns (first_reflect and
   const long* first_csym;      // [ni + 1] first_coef count the other items)
   long grid[9];
+  long kchunk;                 // the longest slice of the items
 };
 // the entry whose block range holds block b: the last e with first[e] <= b (first ascending)
 __device__ __forceinline__ int group_entry(const long* first, int ne, long b) {
