@@ -958,11 +958,11 @@ __device__ __forceinline__ void coef_sym_rows(const SynthParams& p, const double
 // 4081 x 61 in FP64 12.3 -> 9.1 us
 template <class T>
 __global__ void __launch_bounds__(128, 3) k_coef_sym(SynthParams p, const double2* __restrict__ amp, T* C0, T* C1, T* C2,
-                                                     long cst, double dz) {
+                                                     long cst, double dz, int zb) {
   const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= p.c.n) return;
-  const int z0 = blockIdx.y * COEF_SYM_ZB;
-  coef_sym_rows(p, amp, k, z0, min(p.nz, z0 + COEF_SYM_ZB), dz, C0, C1, C2, cst);
+  const int z0 = blockIdx.y * zb;
+  coef_sym_rows(p, amp, k, z0, min(p.nz, z0 + zb), dz, C0, C1, C2, cst);
 }
 
 // the order-0 rows at C, orders 1 and 2 behind them
@@ -973,8 +973,13 @@ static cudaError_t coef1d_amp_impl(const SynthParams& p, double2* amp, T* C, lon
     const unsigned nb = (unsigned)((p.c.n + 127) / 128);
     T* C1 = C + (size_t)C1S_R0 * p.nz * ldc;
     k_reflect_sym<<<nb, 128, 0, s>>>(p, amp);
-    k_coef_sym<T><<<dim3(nb, (unsigned)((p.nz + COEF_SYM_ZB - 1) / COEF_SYM_ZB)), 128, 0, s>>>(
-        p, amp, C, C1, C1 + (size_t)C1S_R1 * p.nz * ldc, ldc, dz);
+    // rows per thread: fewer where the grid fills less than a quarter of the SMs, whose time is the chain of
+    // one thread's rows (256 nodes x 4 rows: 6.8 us at 16 rows a thread, 5.4 us at one); beyond that the
+    // exponentials a split repeats cost more (4081 x 61: 9.1 us at 16 rows, 12.8 us at 8)
+    int zb = COEF_SYM_ZB;
+    while (zb > 1 && (long)nb * ((p.nz + zb - 1) / zb) < 37) zb /= 2;
+    k_coef_sym<T><<<dim3(nb, (unsigned)((p.nz + zb - 1) / zb)), 128, 0, s>>>(
+        p, amp, C, C1, C1 + (size_t)C1S_R1 * p.nz * ldc, ldc, dz, zb);
     return cudaGetLastError();
   }
   k_reflect2d<<<(unsigned)((p.c.n + 127) / 128), 128, 0, s>>>(p, amp);
