@@ -13,6 +13,19 @@ __device__ __forceinline__ uint32_t plane_off(int r, int kb) {
   return (uint32_t)((r >> 3) * 512 + (kb >> 4) * 128 + (r & 7) * 16 + (kb & 15));
 }
 
+// 1.5 2^52 + 0x808080: the low word of fma(v, scale, AI_MAGIC) is rint(v scale) + 0x808080, whose bytes are
+// the balanced digits + 128
+constexpr double AI_MAGIC = 6755399441055744.0 + 8421504.0;
+// the digit planes (most significant first) of four such words, one byte each: seven byte permutes in
+// place of the shifts, masks and additions of every digit by itself
+__device__ __forceinline__ void digit_words(const uint32_t u[4], uint32_t& d0, uint32_t& d1, uint32_t& d2) {
+  const uint32_t l01 = __byte_perm(u[0], u[1], 0x5140), l23 = __byte_perm(u[2], u[3], 0x5140);
+  const uint32_t h01 = __byte_perm(u[0], u[1], 0x0062), h23 = __byte_perm(u[2], u[3], 0x0062);
+  d0 = __byte_perm(h01, h23, 0x5410) ^ 0x80808080u;
+  d1 = __byte_perm(l01, l23, 0x7632) ^ 0x80808080u;
+  d2 = __byte_perm(l01, l23, 0x5410) ^ 0x80808080u;
+}
+
 // shared-memory matrix descriptor: start >> 4, LBO = 128 B (the two K-cores of one MMA),
 // SBO = 512 B (consecutive 8-row groups), descriptor version 1, no swizzle
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
