@@ -195,9 +195,10 @@ __device__ __forceinline__ float4 load4(const float* c, long k, long K) {
 // consecutive bytes of eight columns, every store one whole 128-byte line of a digit plane. A first pass
 // reduces max |C| (IEEE bits into colmax: a non-finite entry counts as Inf), a second reads the same
 // bytes again (from L2) and writes the digits. Blocks: ntile_n x (Np / 8) x nchunk.
-// Bound by the loads in flight: two stages' in the first pass, the next stage's in the second. 32 film
-// stacks x 64 heights (237M values) 349 us with 64 bytes of a column per thread (16 lines touched by each load, one
-// stage in flight) and the digits by conversions and shifts; 334 us. 65536 nodes x 2560 columns 367 -> 302 us.
+// Bound by the loads in flight: two stages' in the first pass, the next stage's in the second. 65536 nodes x
+// 2560 columns 367 us with 64 bytes of a column per thread (16 lines touched by each load, one stage in
+// flight, blocks of 256) and the digits by conversions and shifts; 303 us. 32 film stacks x 64 heights in
+// 4096-node slices (237M values) 349 us; 335-347 us.
 __device__ __forceinline__ void bimg_slice_body(const BesselI8& p, long b) {
   __shared__ float wmax[32][8];
   const int tid = threadIdx.x, lane = tid & 31, r8 = lane >> 2, t4 = 4 * (lane & 3);
@@ -253,10 +254,10 @@ __device__ __forceinline__ void bimg_slice_body(const BesselI8& p, long b) {
     uint8_t* blk = base + (size_t)s * sbytes;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const uint32_t u[4] = {(uint32_t)__double2loint(fma((double)f[i].x, sB, AI_MAGIC)),
-                             (uint32_t)__double2loint(fma((double)f[i].y, sB, AI_MAGIC)),
-                             (uint32_t)__double2loint(fma((double)f[i].z, sB, AI_MAGIC)),
-                             (uint32_t)__double2loint(fma((double)f[i].w, sB, AI_MAGIC))};
+      const uint32_t u[4] = {fixed_bits((double)f[i].x, sB),
+                             fixed_bits((double)f[i].y, sB),
+                             fixed_bits((double)f[i].z, sB),
+                             fixed_bits((double)f[i].w, sB)};
       uint32_t d0, d1, d2;
       digit_words(u, d0, d1, d2);
       uint8_t* dst = blk + plane_off(slot, 16 * i);

@@ -20,7 +20,7 @@
 // host keeps each CTA's node slice ≤ 16384 nodes (K ≤ 32768 real terms), so |acc| < 1.4e9.
 //
 // Kernels:
-//   (k_strengths2d reduces max|S| per (node slice, column) while it writes S)
+//   (k_strengths_rows reduces max|S| per (node slice, column) while it writes S)
 //   k_bslice : B' digits, written once per launch in the exact shared-memory image of each
 //              32-node stage (3 planes x Np rows x 64 B, canonical K-major core matrices)
 //   k_lateral_i8 : one CTA per (128-pixel tile, column tile, node slice); 8 producer warps
@@ -224,8 +224,8 @@ __global__ void __launch_bounds__(256) k_bslice(LateralI8 p) {
     uint32_t r[2], i[2], m[2];  // Re, Im, -Im digit words: those of -Y are 2 0x808080 - Y's
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      r[h] = (uint32_t)__double2loint(fma(v[u][h].x, sB, AI_MAGIC));
-      i[h] = (uint32_t)__double2loint(fma(v[u][h].y, sB, AI_MAGIC));
+      r[h] = fixed_bits(v[u][h].x, sB);
+      i[h] = fixed_bits(v[u][h].y, sB);
       m[h] = 0x1010100u - i[h];
     }
     // row 2c: (Sr, -Si); row 2c+1: (Si, Sr)

@@ -16,6 +16,10 @@ __device__ __forceinline__ uint32_t plane_off(int r, int kb) {
 // 1.5 2^52 + 0x808080: the low word of fma(v, scale, AI_MAGIC) is rint(v scale) + 0x808080, whose bytes are
 // the balanced digits + 128
 constexpr double AI_MAGIC = 6755399441055744.0 + 8421504.0;
+// the same of the rounded product: rint(fl(v scale)) + 0x808080
+__device__ __forceinline__ uint32_t fixed_bits(double v, double scale) {
+  return (uint32_t)__double2loint(__dadd_rn(__dmul_rn(v, scale), AI_MAGIC));
+}
 // the digit planes (most significant first) of four such words, one byte each: seven byte permutes in
 // place of the shifts, masks and additions of every digit by itself
 __device__ __forceinline__ void digit_words(const uint32_t u[4], uint32_t& d0, uint32_t& d1, uint32_t& d2) {
