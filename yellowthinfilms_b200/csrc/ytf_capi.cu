@@ -314,8 +314,8 @@ struct GreenBatch {
 };
 
 // distinct radii hypot(x_i, y_j) in first-occurrence order over (i fastest, j), as the
-// reference, and each pixel's index into them (open addressing by the radius' bits: a node-based map
-// cost 40 ns a pixel, half of a 32-item batch's host time before its first launch)
+// reference, and each pixel's index into them (open addressing by the radius' bits: no allocation per
+// radius, as a node-based map makes)
 void radii_map(int nx, const double* xs, int ny, const double* ys, std::vector<double>& ur, std::vector<int>& rmap) {
   const long npix = (long)nx * ny;
   ur.clear();
@@ -1626,7 +1626,7 @@ struct Parts1D {
 };
 
 // the order contractions of the 1D synthesis over the nodes of sp.c: the per-node coefficient columns
-// (k_coef1d), the Bessel tables or digit images, and one launch for every contraction (two per
+// (k_coef_sym, k_coef1d_amp), the Bessel tables or digit images, and one launch for every contraction (two per
 // order, Re J and Im J, on a deformed contour), in FP64 or on the int8 tensor cores
 static int synth1d_parts(ytf_ctx* ctx, const SynthParams& sp, int nz, double dz, int nr, const double* drho, int precision,
                          int nsm, const GreenBatch* gb, Parts1D& out) {
@@ -2874,7 +2874,7 @@ extern "C" int ytf_plan_retune(ytf_plan* P, const ytf_tune* tune_in) {
       // t.tile units per tile at most: a stage with few units takes smaller tiles, down to one unit
       // per thread, until each CTA of the grid has four (at 1024 units a tile the scan stage of 96
       // stacks, 266k nodes, had 310 tiles for 592 CTAs and eight serial units per thread: 408 us
-      // against 262 us)
+      // against 180 us)
       long all = 0;
       for (const TransferParams& q : pp) {
         const bool fast = only_source_observed(q);
@@ -2912,8 +2912,9 @@ extern "C" int ytf_plan_retune(ytf_plan* P, const ytf_tune* tune_in) {
   std::vector<long> woff{0}, foff{0};
   std::vector<int> item_of;
   size_t npart = 0, syn_smem = 0;
-  // t.chunk nodes per work unit at most, fewer (in steps of a sub-batch) until each resident CTA has
-  // four units: 2048-node units of 266k nodes are 180 for 444 CTAs
+  // t.chunk nodes per work unit at most, fewer (in steps of 64) until each resident CTA has four units:
+  // 2048-node units of 266k nodes are 180 for 444 CTAs (the synthesis stage's time with them 1371 us,
+  // with units of 192 nodes 485 us, in the form the kernel had then)
   int chunk = t.chunk;
   {
     long all = 0;

@@ -103,10 +103,6 @@ __host__ __device__ __forceinline__ M2 solve(const M2& A, const M2& B) {
   return M2{(A.a11 * B.a00 - A.a01 * B.a10) * r, (A.a11 * B.a01 - A.a01 * B.a11) * r,
             (A.a00 * B.a10 - A.a10 * B.a00) * r, (A.a00 * B.a11 - A.a10 * B.a01) * r};
 }
-__host__ __device__ __forceinline__ M2 inv(const M2& A) {
-  const cd r = recip(det(A));
-  return M2{A.a11 * r, -(A.a01 * r), -(A.a10 * r), A.a00 * r};
-}
 // diag(p) * A and A * diag(p)
 __host__ __device__ __forceinline__ M2 dl(cd p0, cd p1, const M2& A) { return M2{p0 * A.a00, p0 * A.a01, p1 * A.a10, p1 * A.a11}; }
 __host__ __device__ __forceinline__ M2 dr(const M2& A, cd p0, cd p1) { return M2{A.a00 * p0, A.a01 * p1, A.a10 * p0, A.a11 * p1}; }
@@ -115,30 +111,8 @@ __host__ __device__ __forceinline__ M2 dr(const M2& A, cd p0, cd p1) { return M2
 struct S4 {
   M2 b11, b12, b21, b22;
 };
-__host__ __device__ __forceinline__ S4 s4_identity() {
-  cd o{1.0, 0.0}, z{0.0, 0.0};
-  return S4{M2{o, z, z, o}, M2{z, z, z, z}, M2{z, z, z, z}, M2{o, z, z, o}};
-}
-__host__ __device__ __forceinline__ S4 s4_diag(cd p0, cd p1, cd p2, cd p3) {
-  cd z{0.0, 0.0};
-  return S4{M2{p0, z, z, p1}, M2{z, z, z, z}, M2{z, z, z, z}, M2{p2, z, z, p3}};
-}
-
-// Redheffer star product (mod_ScatteringMatrix.jl:65-85), regrouped around the two 2x2
-// inverses: E = B11 (I - A12 B21)^-1, F = A22 (I - B21 A12)^-1, then
-//   S11 = E A11, S12 = B12 + E A12 B22, S21 = A21 + F B21 A11, S22 = F B22
-// (two complex reciprocals instead of sixteen complex divisions)
-__host__ __device__ __forceinline__ S4 redheffer(const S4& A, const S4& B) {
-  const M2 E = mul(B.b11, inv(imin(mul(A.b12, B.b21))));
-  const M2 F = mul(A.b22, inv(imin(mul(B.b21, A.b12))));
-  S4 o;
-  o.b11 = mul(E, A.b11);
-  o.b12 = add(B.b12, mul(mul(E, A.b12), B.b22));
-  o.b21 = add(A.b21, mul(mul(F, B.b21), A.b11));
-  o.b22 = mul(F, B.b22);
-  return o;
-}
-// Redheffer with a diagonal left factor diag(p0,p1,p2,p3) (blocks 12 = 21 = 0)
+// Redheffer star product (mod_ScatteringMatrix.jl:65-85) with a diagonal left factor diag(p0,p1,p2,p3)
+// (blocks 12 = 21 = 0)
 __host__ __device__ __forceinline__ S4 redheffer_diag_left(cd p0, cd p1, cd p2, cd p3, const S4& B) {
   // A.b12 = 0 => D1 = D2 = I
   S4 o;

@@ -289,7 +289,7 @@ struct LateralI8 {
   const float2* Py;  // [n_pad][ny]
   const double2* S;  // [ncol][n]
   uint8_t* Bq;       // [ntile][nchunk][kchunk/32][3 planes][Np rows x 64 B] digit images
-  const unsigned long long* colmax;  // [nchunk][ncol] bits of max(|Re S|, |Im S|) (k_strengths2d)
+  const unsigned long long* colmax;  // [nchunk][ncol] bits of max(|Re S|, |Im S|) (k_strengths_rows)
   double2* partial;  // [nchunk][npix * ncol]
   unsigned* err;     // nonzero if a pipeline wait timed out
   long wait_limit;   // polls of each bounded pipeline wait before it gives up

@@ -6,14 +6,15 @@
 // radius and z-row it is the contraction
 //     R[ρ, col] = Σ_k J_n(k ρ) · C_n[k, col],   n = 0, 1, 2,
 // of a Bessel table with per-node coefficients (weighted amplitude × mode field × phase ×
-// k). k_coef1d builds C_n (13 complex columns per z-row), k_bessel the tables, a GEMM
-// does the contraction and k_assemble1d combines orders, rotates by the pixel azimuth
-// and writes Julia's (Nx, Ny, Nz, 3, 3) column-major layout.
+// k). k_coef_sym (5 complex columns per z-row, where TE and TM decouple) or k_coef1d_amp (9) build
+// C_n, k_bessel the tables, k_gemm64 does the contractions and k_assemble1d combines orders,
+// rotates by the pixel azimuth and writes Julia's (Nx, Ny, Nz, 3, 3) column-major layout.
 //
 // 2D (any stack; closed_form_G for CavityTransferCache2D, lateral=:direct, :711-753):
-// k_strengths2d forms the 9 strengths per (node, z-row) (_strengths_row!, :616-659) and
-// k_lateral evaluates G[pix, col] = Σ_n e^{i(kx_n x + ky_n y)} S[col, n] as a complex GEMM
-// whose A operand is generated in shared memory from the node's (kx, ky).
+// k_strengths_rows forms the 9 strengths per (node, z-row) (_strengths_row!, :616-659) and
+// k_lateral64 evaluates G[pix, col] = Σ_n e^{i(kx_n x + ky_n y)} S[col, n] as a complex GEMM
+// whose A operand is formed from the x and y phase tables (k_strengths2d and k_lateral: the
+// allocation-free entry point's forms of the two).
 #include "ytf_complex.cuh"
 #include "ytf_kernels.h"
 #include "ytf_bessel.cuh"
@@ -460,9 +461,9 @@ __global__ void __launch_bounds__(32 * (BM / WT) * (BN / WT)) k_gemm64(const __g
   }
 }
 
-// 128 x 64 tiles once they give 148 CTAs (2.0 against 2.4 us per GFLOP at 251 x 61 heights x 4081
-// nodes with 32 x 32 ones); below that 32 x 32 tiles, whose shorter warps and finer slices shorten
-// the k chain (8 radii x 4 heights x 256 nodes: 5 against 11 us)
+// 128 x 64 tiles once they give 148 CTAs (251 radii x 61 heights x 4081 nodes: 55 us, 90 us with 32 x 32
+// ones); below that 32 x 32 tiles, whose shorter warps and finer slices shorten the k chain (8 radii x 4
+// heights x 256 nodes: 4.3 us against 9.3 us)
 static bool gemm64_large(const Gemm64& p) {
   long t = 0;
   for (int i = 0; i < p.n; ++i) t += (long)((p.M + 127) / 128) * ((p.e[i].N + 63) / 64);
@@ -758,7 +759,7 @@ __global__ void __launch_bounds__(128, 4) k_reflect2d(SynthParams p, double2* __
 }
 
 // 1D coefficient columns from the reflected amplitudes k_reflect2d wrote once per node (the
-// amplitudes do not depend on the z row); the arithmetic per (node, row) is k_coef1d's
+// amplitudes do not depend on the z row); the arithmetic per (node, row) is coef1d_row's
 // heights per thread of k_coef1d_amp: a node's amplitudes are loaded once for COEF1D_ZB
 // z rows (the per-row arithmetic and outputs are those of one row per thread)
 constexpr int COEF1D_ZB = 4;

@@ -734,27 +734,6 @@ __device__ __noinline__ void interface_qr(const Mode4& A, const Mode4& B, S4& S)
   S.b22 = M2{x[2][2], x[2][3], x[3][2], x[3][3]};
 }
 
-// _S_Interface_Matrix (mod_ScatteringMatrix.jl:27-47): [-Vf_B Vb_A] \ [-Vf_A Vb_B] by LU with
-// partial pivoting, and by the pivoted-QR least-squares solve when a pivot is exactly zero;
-// always succeeds (a non-finite result is caught downstream as in the reference)
-__device__ __forceinline__ bool interface_matrix(const Mode4& A, const Mode4& B, S4& S) {
-  cd L[4][4], R[4][4];
-  interface_lhs_rhs(A, B, L, R);
-  if (!lu_solve4<4>(L, R)) {
-    // copies: an operand whose address went to the call would live in local memory on the LU path too
-    const Mode4 a = A, b = B;
-    S4 s;
-    interface_qr(a, b, s);
-    S = s;
-    return true;
-  }
-  S.b11 = M2{R[0][0], R[0][1], R[1][0], R[1][1]};
-  S.b12 = M2{R[0][2], R[0][3], R[1][2], R[1][3]};
-  S.b21 = M2{R[2][0], R[2][1], R[3][0], R[3][1]};
-  S.b22 = M2{R[2][2], R[2][3], R[3][2], R[3][3]};
-  return true;
-}
-
 __device__ __forceinline__ void st_s4(double2* base, long slot, long n, long node, const S4& S) {
   double2* b = base + slot * 16 * n;
   const cd* v = reinterpret_cast<const cd*>(&S);
@@ -1045,7 +1024,9 @@ __device__ __noinline__ void iface_singular(const TransferParams& p, int a, long
   interface_qr(A, B, X);
 }
 
-// One thread per (node, interface); bound by the latency of its 36 loads and of the LU chain. With the
+// _S_Interface_Matrix (mod_ScatteringMatrix.jl:27-47): [-Vf_B Vb_A] \ [-Vf_A Vb_B] by LU with partial
+// pivoting, and by the pivoted-QR least-squares solve when a pivot is exactly zero (a non-finite result is
+// caught downstream as in the reference). One thread per (node, interface); bound by the latency of its 36 loads and of the LU chain. With the
 // modes passed to the out-of-line QR by reference they lived in local memory (1.8 KB a thread, L1 60%
 // busy): 65536 nodes x 7 interfaces 100 us against 69 us.
 __device__ __forceinline__ void iface_body(const TransferParams& p, int j, long node) {
@@ -1159,7 +1140,7 @@ __device__ __forceinline__ void scan_body(const TransferParams& p, long node) {
     else zero_rows(p.Tout, 16 * p.nobs, nT, gnode);
     return;
   }
-  // cavity at the source layer (_R_cavity, _cavity_resummation), as k_chain
+  // cavity at the source layer (_R_cavity, _cavity_resummation)
   const double ds = p.layers[src - 1].d;
   M2 RR = M2{z, z, z, z};
   M24 Fp, Fm;
