@@ -287,7 +287,7 @@ CONFIG = {"workload": "batched spectral solve + full 3x3 G: 8-layer biaxial/gyro
 # --------------------------------------------------------------------------------------
 # DRAM bytes (read + write) per launch from one ncu capture of the kernel on this workload;
 # absent until captured
-TRAFFIC = {"k_lateral": 81.7e6}
+TRAFFIC = {}
 DTYPE = {"int8x3": "f64 solve, int8 x3-digit tensor-core synthesis (exact int32 accum)",
          "split_bf16": "f64 solve, split-bf16 x3 tensor-core synthesis (fp32 accum)",
          "fp64": "f64"}
@@ -308,10 +308,11 @@ def measured_peaks():
 
 # FP64 operations per node of the per-node solve kernels on this workload, from one ncu count
 # of their DFMA/DADD/DMUL instructions (2 per DFMA); absent until captured
-FP64_OPS_PER_NODE = {"k_iface": 8.99e3,  # 1.79e8 DFMA + 0.97e8 DADD + 1.33e8 DMUL per 65536 nodes
-                     "k_scan": 7.43e3,  # 1.59e8 DFMA + 0.57e8 DADD + 1.12e8 DMUL per 65536 nodes
-                     "k_layer_modes": 9.46e3,  # 1.98e8 DFMA + 0.59e8 DADD + 1.64e8 DMUL (8 layers)
-                     "k_strengths2d": 8.04e3}  # k_reflect2d + k_strengths_rows (8 z rows)  # 1.832e8 DFMA + 0.596e8 DADD + 1.009e8 DMUL (8 z rows)
+FP64_OPS_PER_NODE = {"k_iface": 8.74e3,  # 1.68e8 DFMA + 0.96e8 DADD + 1.40e8 DMUL per 65536 nodes
+                     "k_scan": 3.02e3,  # 0.60e8 DFMA + 0.26e8 DADD + 0.51e8 DMUL per 65536 nodes
+                     "k_layer_modes": 6.05e3,  # 1.28e8 DFMA + 0.42e8 DADD + 0.99e8 DMUL (8 layers)
+                     "k_strengths2d": 5.59e3}  # k_reflect2d + k_strengths_rows (8 z rows):
+#                                              1.11e8 DFMA + 0.53e8 DADD + 0.91e8 DMUL
 FP64_NOMINAL = 37.2  # TFLOP/s: 148 SM x 64 FP64 FMA/clk x 2 x 1.965 GHz (no measured FP64 peak)
 
 
@@ -671,20 +672,20 @@ def run_reference_learned(args):
     return 0
 
 
-# FP64 operations per (ρ, k) pair of k_aimg_bessel3 (J_0, J_1 by Hankel's asymptotic pair from
-# x = 25 and the CUDA math library below, J_2 by series or recurrence, digits): ncu's DFMA x 2 +
-# DMUL + DADD of one grouped launch divided by its (ρ, k) slots, 3.32e9 / 23.05e6
-AIMG_FP64_PER_PAIR = 144.0
+# FP64 operations per (ρ, k) pair of k_aimg_bessel3 (J_0, J_1 by Taylor rows below x = 25 and Hankel's
+# asymptotic pair above, J_2 by series or recurrence, digits): ncu's DFMA x 2 + DMUL + DADD of one
+# grouped launch divided by its (ρ, k) slots, 2.23e9 / 23.05e6
+AIMG_FP64_PER_PAIR = 97.0
 # DRAM bytes per node synthesised of the grouped kernels (dram__bytes_read + write of one ncu
 # capture of `--workload synth --stacks 8 --group-bytes 1073741824`, one group of 89,144 nodes;
 # traffic grows with the nodes of a launch), scaled to a launch's nodes
-TRAFFIC_PER_NODE = {"k_gemm_i8_img": 6316.0, "k_aimg_bessel3": 1748.0, "k_coef1d": 4581.0, "k_bimg_real": 10357.0}
+TRAFFIC_PER_NODE = {"k_gemm_i8_img": 4493.0, "k_aimg_bessel3": 1766.0, "k_coef1d": 2455.0, "k_bimg_real": 4472.0}
 
 
 def learned_roofline(name, prof, nodes_synth):
     """Roofline entry of one kernel of the learned step's synthesis from its CUDA-event time in
     the profiled step: the int8x3 contraction against the sustained bf16 tensor peak (its
-    algorithmic flops: 2 x radii x 1152 real coefficient columns per node synthesised), the
+    algorithmic flops: 2 x radii x 640 real coefficient columns per node synthesised), the
     J_n image kernel against the nominal FP64 peak (its counted FP64 operations)."""
     roof = {"kernel": name, "bound": None, "achieved": None, "peak": None, "unit": None, "frac": None,
             "traffic": TRAFFIC.get(name)}
@@ -696,11 +697,11 @@ def learned_roofline(name, prof, nodes_synth):
         roof["traffic_note"] = "bytes per launch: ncu bytes per node (89,144-node capture) x nodes per launch"
     peaks = measured_peaks()
     if name in ("k_gemm_i8_img", "k_bessel_i8"):
-        flops = 2.0 * N_RHO * (18 * N_ZOBS) * nodes_synth  # the 9 stored complex coefficient columns per height
+        flops = 2.0 * N_RHO * (10 * N_ZOBS) * nodes_synth  # the 5 stored complex coefficient columns per height
         peak, src = peaks["bf16_sustained"]
         roof.update(bound="tensor", achieved=flops / t_k / 1e12, peak=peak, unit="TFLOP/s",
                     frac=flops / t_k / 1e12 / peak, peak_source=src, launches=nl,
-                    work=f"2 x {N_RHO} radii x 1152 real coefficient columns x nodes synthesised "
+                    work=f"2 x {N_RHO} radii x 640 real coefficient columns x nodes synthesised "
                          f"({int(nodes_synth)} over the chunk's syntheses) = {flops:.3e} flop in {nl} launches")
     elif name == "k_aimg_bessel3":
         ops = AIMG_FP64_PER_PAIR * N_RHO * nodes_synth
@@ -1005,15 +1006,15 @@ def run_bessel(args):
     ms, prof, clocks, G = run(prec)
     ms64, prof64, _, G64 = run("fp64")
     entries = G.size
-    flops = 2.0 * 4096 * 65536 * 18 * 256  # the 9 stored complex coefficient columns (18 real) per height
+    flops = 2.0 * 4096 * 65536 * 10 * 256  # the 5 stored complex coefficient columns (TE and TM decouple) per height
     name = "k_bessel_i8" if prec == "int8x3" else "k_dgemm_nt"
-    t_k = prof[name][0] / prof[name][1] * 1e-3 if name in prof else None
+    t_k = prof[name][0] / args.steps * 1e-3 if name in prof else None
     peak, src = measured_peaks()["bf16_sustained"]
     roof = {"kernel": name, "bound": "tensor" if prec == "int8x3" else "fp64",
-            "achieved": flops / 3 / t_k / 1e12 if t_k else None, "unit": "TFLOP/s",
+            "achieved": flops / t_k / 1e12 if t_k else None, "unit": "TFLOP/s",
             "peak": peak if prec == "int8x3" else FP64_NOMINAL, "traffic": None,
-            "work": "2 x 4096 radii x 65536 nodes x 18 real columns x 256 heights = 2.47e12 flop over the 3 orders "
-                    "(one launch per order: a third each)",
+            "work": "2 x 4096 radii x 65536 nodes x 10 real columns x 256 heights = 1.37e12 flop over the 3 orders, "
+                    "in the time of every kernel of the label (int8: J images, coefficient images, contraction)",
             "peak_source": src if prec == "int8x3" else "nominal FP64"}
     if roof["achieved"]:
         roof["frac"] = roof["achieved"] / roof["peak"]
