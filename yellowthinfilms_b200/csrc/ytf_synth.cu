@@ -1440,16 +1440,29 @@ cudaError_t launch_lateral64(const Lateral64& p, const CacheView& c, const doubl
   return cudaGetLastError();
 }
 
-__global__ void k_reduce_splits2(long len, int splits, const double2* __restrict__ P, double2* __restrict__ C) {
-  long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= len) return;
+// Σ_k P[k len] in the order of k, eight values in flight together
+__device__ __forceinline__ double2 sum_in_order(const double2* __restrict__ P, long len, int n) {
   double2 s = make_double2(0.0, 0.0);
-  for (int k = 0; k < splits; ++k) {
-    double2 v = P[(long)k * len + i];
-    s.x += v.x;
-    s.y += v.y;
+  for (int k = 0; k < n; k += 8) {
+    double2 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (k + i < n) v[i] = __ldg(P + (long)(k + i) * len);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (k + i < n) {
+        s.x += v[i].x;
+        s.y += v[i].y;
+      }
   }
-  C[i] = s;
+  return s;
+}
+// One thread per output; bound by the chain of its loads: 12285 outputs 14.6 us with one load at a
+// time in blocks of 256, 7.6 us; 20736 outputs 8.0 -> 5.1 us
+__global__ void __launch_bounds__(64) k_reduce_splits2(long len, int splits, const double2* __restrict__ P,
+                                                       double2* __restrict__ C) {
+  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < len) C[i] = sum_in_order(P + i, len, splits);
 }
 
 int lateral_splits(long n, int splits) {
@@ -1472,7 +1485,7 @@ cudaError_t launch_lateral(const CacheView& c, int nx, int ny, const double* xs,
 
 cudaError_t launch_reduce_splits2(long len, int splits, const double2* partial, double2* G, cudaStream_t s) {
   if (len <= 0) return cudaSuccess;
-  k_reduce_splits2<<<(unsigned)((len + 255) / 256), 256, 0, s>>>(len, splits, partial, G);
+  k_reduce_splits2<<<(unsigned)((len + 63) / 64), 64, 0, s>>>(len, splits, partial, G);
   return cudaGetLastError();
 }
 
@@ -1889,7 +1902,29 @@ __global__ void __launch_bounds__(128, 3) k_synth_small(const SynthItem* __restr
   }
 }
 
-__global__ void __launch_bounds__(128) k_synth_finish(const SynthItem* __restrict__ items, int nitems,
+// x[m] = Σ_k part[k R nz nr + m nr], the chunks in order, four (R = 10) or two of them in flight together
+template <int R>
+__device__ __forceinline__ void sum_columns_in_order(const double* __restrict__ part, int nr, int nz, int nw, double x[R]) {
+  constexpr int U = R > 16 ? 2 : 4;
+  const long nout = (long)nr * R * nz;
+#pragma unroll
+  for (int m = 0; m < R; ++m) x[m] = 0.0;
+  for (int k = 0; k < nw; k += U) {
+    double v[U][R];
+#pragma unroll
+    for (int i = 0; i < U; ++i)
+#pragma unroll
+      for (int m = 0; m < R; ++m) v[i][m] = k + i < nw ? __ldg(part + (k + i) * nout + (long)m * nr) : 0.0;
+#pragma unroll
+    for (int i = 0; i < U; ++i)
+#pragma unroll
+      for (int m = 0; m < R; ++m) x[m] += v[i][m];
+  }
+}
+
+// One thread per output (2D) or pixel (1D); bound by the chain of its loads over the chunks: 96 items 30 us
+// with one chunk at a time, 10 us
+__global__ void __launch_bounds__(64) k_synth_finish(const SynthItem* __restrict__ items, int nitems,
                                                        const long* __restrict__ f_off, long nfin) {
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nfin) return;
@@ -1900,35 +1935,25 @@ __global__ void __launch_bounds__(128) k_synth_finish(const SynthItem* __restric
   const long npix = (long)I.nx * I.ny;
   if (I.is2d) {
     const long nout = npix * 9 * nz;
-    double2 s = make_double2(0.0, 0.0);
-    for (int k = 0; k < I.nw; ++k) {
-      const double2 v = I.partial[(long)k * nout + u];
-      s.x += v.x;
-      s.y += v.y;
-    }
-    I.G[u] = s;
+    I.G[u] = sum_in_order(I.partial + u, nout, I.nw);
     return;
   }
   const long pix = u % npix;
   const int zi = (int)(u / npix);
   const int r = I.rmap[pix];
   const int R = I.sp.sym ? 10 : 26;
-  const long nout = (long)I.nr * R * nz;
   const double* part = reinterpret_cast<const double*>(I.partial) + r + (long)I.nr * R * zi;
-  double x[26];
-#pragma unroll
-  for (int m = 0; m < 26; ++m) x[m] = 0.0;
-  for (int k = 0; k < I.nw; ++k, part += nout)
-#pragma unroll
-    for (int m = 0; m < 26; ++m)
-      if (m < R) x[m] += part[(long)I.nr * m];
   cd g[13];
   if (I.sp.sym) {
+    double x[10];
+    sum_columns_in_order<10>(part, I.nr, nz, I.nw, x);
     const cd z{0.0, 0.0}, c0{x[0], x[1]}, c4{x[8], x[9]};
     g[0] = g[3] = c0; g[1] = g[2] = z; g[4] = cd{x[2], x[3]};
     g[5] = cd{x[4], x[5]}; g[7] = cd{x[6], x[7]}; g[6] = g[8] = z;
     g[9] = c4; g[12] = -c4; g[10] = g[11] = z;
   } else {
+    double x[26];
+    sum_columns_in_order<26>(part, I.nr, nz, I.nw, x);
 #pragma unroll
     for (int m = 0; m < 13; ++m) g[m] = cd{x[2 * m], x[2 * m + 1]};
   }
@@ -1950,7 +1975,7 @@ cudaError_t launch_synth_small(const SynthItem* items, int nitems, const long* w
 
 cudaError_t launch_synth_finish(const SynthItem* items, int nitems, const long* f_off, long nfin, cudaStream_t s) {
   if (nfin <= 0) return cudaSuccess;
-  k_synth_finish<<<(unsigned)((nfin + 127) / 128), 128, 0, s>>>(items, nitems, f_off, nfin);
+  k_synth_finish<<<(unsigned)((nfin + 63) / 64), 64, 0, s>>>(items, nitems, f_off, nfin);
   return cudaGetLastError();
 }
 
