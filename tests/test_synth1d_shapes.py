@@ -140,3 +140,16 @@ def test_int8_slices_of_every_length(n):
     z, x = np.linspace(0.0, 0.3, 256), np.geomspace(0.01, 3.0, 2048)
     G = api.closed_form_G(c, 1, 0.03, z, x, [0.0], terms="scattered", precision="int8x3")
     assert relerr(G, api.closed_form_G(c, 1, 0.03, z, x, [0.0], terms="scattered")) < 1e-6
+
+
+@pytest.mark.parametrize("panels,nr", [(3, 1), (17, 9), (65, 131)])
+def test_int8_contour_shapes(panels, nr):
+    """The complex J digit images at ragged rows (row groups of 8 in tiles of 128) and node counts (stages of
+    64): int8x3 on the deformed contour against its FP64 synthesis, at the shapes' 1e-6."""
+    from yellowthinfilms_b200 import api
+    st = config1_like_stack()
+    k, w = api.contour_rule(W, npanels=panels)
+    c = api.build_cavity_transfer_1d_contour(st, W, 1, k, w, obs_layers=[1])
+    x, z = np.geomspace(0.01, 3.0, nr), np.linspace(0.05, 0.3, 5)
+    G = api.closed_form_G(c, 1, 0.03, z, x, [0.0], precision="int8x3")
+    assert relerr(G, api.closed_form_G(c, 1, 0.03, z, x, [0.0], precision="fp64")) < 1e-6
