@@ -802,17 +802,41 @@ __global__ void __launch_bounds__(128) k_coef1d_amp(SynthParams p, const double2
 // 325k nodes x 64 heights took 1083 us and take 278 us (bound by the 832 MB of columns written, 127 us
 // at the copy rate, and the FP64 pipe).
 // ------------------------------------------------------------------------------------
+// A_y of the TE mode, A_x and A_z of the TM one, as reflected_amp's entries: one orientation after the other,
+// the T rows of its mode alone. Bound by load latency: 65536 nodes 17.4 us with all twelve amplitudes (162
+// registers), 12.0 us at four CTAs per SM; 32 film stacks, 325k nodes, 84 -> 79 us.
 __device__ __forceinline__ void reflect_sym_body(const SynthParams& p, long k, double2* amp) {
   const CacheView& c = p.c;
   const long n = c.n;
-  cd Af[2][3], Ab[2][3];
-  reflected_amp(p, k, Af, Ab);
   const cd W = cd{0.0, 1.0 / (2.0 * 3.14159265358979323846)} * cd{c.wr[k], c.wri ? c.wri[k] : 0.0};
   const cd kx{c.kr[k], c.kri ? c.kri[k] : 0.0};
   // which of the two modes is TE: the one with the larger E_y (the other's is zero)
   const bool te1 = norm2(ldc(c.basis, 3, n, k)) + norm2(ldc(c.basis, 9, n, k)) >
                    norm2(ldc(c.basis, 2, n, k)) + norm2(ldc(c.basis, 8, n, k));
   const int te = te1 ? 1 : 0, tm = 1 - te;
+  cd A[2][3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) A[0][q] = A[1][q] = cd{0.0, 0.0};
+  if (c.valid[k] && c.tvalid[k]) {
+    cd P[4];
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      P[m] = cexp(mul_i(ldc(c.Qf, m, n, k)) * (c.d_src - p.zpos));
+      P[2 + m] = cexp(mul_i(-ldc(c.Qb, m, n, k)) * p.zpos);
+    }
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const int m = q == 1 ? te : tm;
+      cd s[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s[i] = ldc(i < 2 ? c.sf : c.sb, (i & 1) + 2 * q, n, k) * P[i];
+#pragma unroll
+      for (int br = 0; br < 2; ++br)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          A[br][q] += ldc(c.T, 2 * br + m + 4 * i, n, k) * ((i < 2 ? (br ? p.uf_B : p.uf_F) : (br ? p.ub_B : p.ub_F)) * s[i]);
+    }
+  }
   auto put = [&](int row, cd v) { amp[(long)row * n + k] = make_double2(v.x, v.y); };
   const cd half{0.0, -0.5};
 #pragma unroll
@@ -827,8 +851,7 @@ __device__ __forceinline__ void reflect_sym_body(const SynthParams& p, long k, d
       put(row + 6 + br, wz * ex);
       put(row + 8 + br, cd{0.0, -1.0} * (wz * ez));
     };
-    const cd(*A)[3] = br == 0 ? Af : Ab;
-    factors(0, te1 ? A[0][0] : A[1][0], te1 ? A[1][1] : A[0][1], te1 ? A[0][2] : A[1][2]);
+    factors(0, A[br][0], A[br][1], A[br][2]);
     if (p.with_direct) {
       const double2* sd = br == 0 ? c.sf : c.sb;
       const bool v = c.valid[k];
@@ -839,7 +862,7 @@ __device__ __forceinline__ void reflect_sym_body(const SynthParams& p, long k, d
     put(12 + br, ldc(c.basis, (br == 0 ? 12 : 14) + tm, n, k));
   }
 }
-__global__ void __launch_bounds__(128) k_reflect_sym(SynthParams p, double2* __restrict__ amp) {
+__global__ void __launch_bounds__(128, 4) k_reflect_sym(SynthParams p, double2* __restrict__ amp) {
   const long k = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k < p.c.n) reflect_sym_body(p, k, amp);
 }
@@ -2154,7 +2177,7 @@ __global__ void __launch_bounds__(128, 3) k_coef1d_group(const Synth1DItem* __re
   }
 }
 
-__global__ void __launch_bounds__(128) k_reflect_sym_group(const Synth1DItem* __restrict__ items,
+__global__ void __launch_bounds__(128, 4) k_reflect_sym_group(const Synth1DItem* __restrict__ items,
                                                            const long* __restrict__ first, int ni) {
   const int i = group_entry(first, ni, blockIdx.x);
   const long k = (long)(blockIdx.x - first[i]) * blockDim.x + threadIdx.x;
