@@ -772,8 +772,8 @@ class BatchPlan:
     without ``cache`` (item i synthesises from the cache of transfer item i). Small
     observation sets share one batched FP64 synthesis kernel; larger 2D sets (or another
     precision) run closed_form_G's own kernels inside the same graph; 1D items are FP64.
-    ``tune``: dict of ytf_tune fields (block, ctas_per_sm, tile, chunk, synth_ctas_per_sm)
-    or None for the defaults. Every ``run`` re-reads the node, weight and coordinate arrays
+    ``tune``: dict of ytf_tune fields (block, ctas_per_sm, tile, chunk, synth_ctas_per_sm;
+    tile and chunk are upper bounds) or None for the defaults. Every ``run`` re-reads the node, weight and coordinate arrays
     held by the plan (``inputs(i)`` returns them for in-place updates of the same sizes)."""
 
     def __init__(self, transfer_items, green_items, tune=None, ctx: Optional[Context] = None):

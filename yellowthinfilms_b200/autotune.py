@@ -3,8 +3,8 @@ reference, which runs one build and one synthesis per item on the host's threads
 
 The tunables are the fields of ytf_tune: threads per CTA of the persistent node-solve
 kernels (``block``), their grid in CTAs per SM (``ctas_per_sm``), units per node-solve tile
-(``tile``), nodes per synthesis work unit (``chunk``) and the synthesis grid
-(``synth_ctas_per_sm``). The tuner measures the device time of the plan's graph
+(``tile``) and nodes per synthesis work unit (``chunk``), both upper bounds (a stage with few
+units takes smaller ones until its grid is full), and the synthesis grid (``synth_ctas_per_sm``). The tuner measures the device time of the plan's graph
 (``BatchPlan.retune`` + ``run``/``wait``, CUDA events) for candidates in a coordinate
 descent from the defaults: one parameter at a time over its candidate values, keeping the
 best, in the order of ``ORDER``. The choice is persisted in a JSON file keyed by
