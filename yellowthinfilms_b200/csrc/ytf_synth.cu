@@ -1083,6 +1083,7 @@ __global__ void __launch_bounds__(128, 4) k_strengths_rows(SynthParams p, const 
   auto g = [&](int f) { const double2 v = sh[f][lane]; return cd{v.x, v.y}; };
   auto gp = [&](int f) { const double2 v = ph[f][lane]; return cd{v.x, v.y}; };
   auto kz = [&](int i) { return g(i & 1 ? 26 + (i >> 1) : 24 + (i >> 1)); };  // mode i >> 1, f (0) or b (1)
+  bool stepped = false;  // this node's steps are in ph (written by the first group that takes the recurrence)
   for (int zg = 0; zg < p.nz; zg += SR_ROWS) {
     const int ng = min(SR_ROWS, p.nz - zg);
     bool rec = false;
@@ -1115,7 +1116,7 @@ __global__ void __launch_bounds__(128, 4) k_strengths_rows(SynthParams p, const 
         for (int e = warp; e < 12; e += 4) {
           const int i = e < 8 ? e & 3 : e < 10 ? 2 * (e - 8) : 2 * (e - 10) + 1;
           const double at = e < 4 ? (i & 1 ? z0 - p.d_obs : z0) : e < 8 ? dz : e < 10 ? zu : zd;
-          if ((e >= 4 && e < 8 && zg > 0) || (e >= 8 && !p.with_direct)) continue;
+          if ((e >= 4 && e < 8 && stepped) || (e >= 8 && !p.with_direct)) continue;
           const cd v = phase_call(kz(i), at);
           ph[e][lane] = make_double2(v.x, v.y);
           if (e >= 4 && e < 8) {
@@ -1124,6 +1125,7 @@ __global__ void __launch_bounds__(128, 4) k_strengths_rows(SynthParams p, const 
             ph[8 + e][lane] = make_double2(q.x, q.y);
           }
         }
+        stepped = true;
       }
     }
     __syncthreads();
