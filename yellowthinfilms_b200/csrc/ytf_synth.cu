@@ -844,7 +844,8 @@ __device__ __forceinline__ void reflect_sym_body(const SynthParams& p, long k, d
     const cd ey = ldc(c.basis, (br == 0 ? 2 : 8) + te, n, k);
     const cd ex = ldc(c.basis, (br == 0 ? 0 : 6) + tm, n, k), ez = ldc(c.basis, (br == 0 ? 4 : 10) + tm, n, k);
     auto factors = [&](int row, cd ax, cd ay, cd az) {
-      const cd wx = fin0(W * ax) * kx, wy = fin0(W * ay) * kx, wz = fin0(W * az) * kx;
+      // not finite: coef_sym_rows leaves the node to the general columns and their clamps
+      const cd wx = W * ax * kx, wy = W * ay * kx, wz = W * az * kx;
       put(row + br, half * (wy * ey));
       put(row + 2 + br, half * (wx * ex));
       put(row + 4 + br, wx * ez);
@@ -910,8 +911,8 @@ __device__ __forceinline__ void coef_sym_rows(const SynthParams& p, const double
   for (int i = 0; i < 10; ++i) big += fabs(F[i].x) + fabs(F[i].y);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    big += fabs(kz[i].x) * (fabs(zlo) + fabs(zhi));
     const double s = i & 1 ? p.d_obs : 0.0;
+    big += fabs(kz[i].x) * (fabs(zlo) + fabs(zhi) + fabs(s));  // not finite for a layer of infinite thickness
     const double a = -kz[i].y * (zlo - s), b = -kz[i].y * (zhi - s);
     lo = fmin(lo, fmin(a, b));
     hi = fmax(hi, fmax(a, b));
@@ -1107,7 +1108,7 @@ __global__ void __launch_bounds__(128, 4) k_strengths_rows(SynthParams p, const 
           lo = fmin(lo, -k.y * far);
           hi = fmax(hi, -k.y * far);
         }
-        big += fabs(k.x) * (fabs(z0) + fabs(z1)) + fabs(k.y);
+        big += fabs(k.x) * (fabs(z0) + fabs(z1) + fabs(s)) + fabs(k.y);
       }
       rec = lo >= -600.0 && hi <= 80.0 && big < 1e200;  // false for any NaN
       if (rec) {
