@@ -1,9 +1,10 @@
-"""1D synthesis in a last layer of infinite thickness: its backward wave, counted from z - d, has amplitude 0
-and no finite phase. Against the oracle at the synthesis tests' bounds."""
+"""Layers of infinite thickness. The last one: its backward wave, counted from z - d, has amplitude 0 and no
+finite phase. The first one, unobserved: its thickness does not enter. Against the oracle at the parity tests'
+bounds."""
 import numpy as np
 import pytest
 
-from helpers import config1_like_stack, lay, relerr
+from helpers import FOUNDATION_STACKS, config1_like_stack, lay, relerr
 
 pytestmark = pytest.mark.gpu
 
@@ -32,3 +33,38 @@ def test_infinite_last_layer(oracle, z, terms):
     G8 = api.closed_form_G_batch([dict(cache=gc, obs_layer=3, zsrc_local=0.03, z_obs=z, xs=x, ys=[0.0], terms=terms)] * 2,
                                  precision="int8x3")
     assert relerr(G8[1], Go) < 1e-6
+
+
+def _first(d, aniso):
+    st = config1_like_stack() if not aniso else list(FOUNDATION_STACKS[4][1])
+    st[0] = lay(st[0].eps_material, d)
+    return st
+
+
+@pytest.mark.parametrize("d", [0.0, np.inf])
+@pytest.mark.parametrize("aniso", [False, True])
+@pytest.mark.parametrize("obs", [[2], [2, 3]])
+def test_first_layer_thickness_does_not_enter(oracle, d, aniso, obs):
+    """With source and field in other layers the first layer only reflects: any thickness gives the same
+    field, caches and response."""
+    from yellowthinfilms_b200 import api
+    st, ref = _first(d, aniso), _first(1.0, aniso)
+    k, w = _rule(72)
+    ph, wp = 2 * np.pi * np.arange(3) / 3, np.full(3, 2 * np.pi / 3)
+    x, z = np.array([-0.3, 0.0, 0.2]), np.linspace(0.01, 0.08, 3)
+    grid = dict(omega=W, source_layer=2, kr_nodes=k, kr_weights=w, phi_nodes=ph, phi_weights=wp, obs_layers=obs)
+    syn = dict(zsrc_local=0.03, z_obs=z, xs=x, ys=x[:2])
+    oc = oracle.build_cavity_transfer_2d(ref, W, 2, k, w, ph, wp, obs_layers=obs)
+    caches = [api.build_cavity_transfer_2d(st, W, 2, k, w, ph, wp, obs_layers=obs, rotation=r) for r in ("auto", False)]
+    caches += api.build_cavity_transfer_batch([dict(grid, stack=st, rotation=False)] * 2)
+    for o in obs:
+        Go = oracle.closed_form_G(oc, o, 0.03, z, x, x[:2])
+        for c in caches:
+            assert c.valid.all() and c.Tvalid[o].all()
+            assert relerr(api.closed_form_G(c, obs_layer=o, **syn), Go) < 1e-10
+        G = api.BatchPlan([dict(grid, stack=st)], [dict(syn, obs_layer=o)])()[0]
+        assert relerr(G, Go) < 1e-10
+    r = api.cavity_response(ref, W, 2, k)
+    # the response's singular values are held to 1e-9 of the oracle elsewhere
+    assert np.abs(api.cavity_response(st, W, 2, k) - r).max() <= 1e-9 * r.max()
+    assert np.abs(api.cavity_response_batch([(st, W, 2, k)])[0] - r).max() <= 1e-9 * r.max()

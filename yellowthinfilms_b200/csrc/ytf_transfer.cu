@@ -1119,11 +1119,14 @@ __device__ __forceinline__ void scan_body(const TransferParams& p, long node) {
   }
   const uint64_t swaps = swaps_upto(p, node, N);
   // RL = SLeft[src].b12: the interfaces above the source layer, left to right
+  // (the first of them alone as it is: layer 1's propagation, not finite where its thickness is not, is no
+  // factor of X12)
   M2 RL = M2{z, z, z, z};
 #pragma unroll 1
   for (int j = 2; j <= src; ++j) {
     const S4 X = ld_x(p, j, node, swaps);
-    RL = add(X.b12, mul(X.b11, solve(imin(mul(RL, X.b21)), mul(RL, X.b22))));
+    if (j == 2) RL = X.b12;
+    else RL = add(X.b12, mul(X.b11, solve(imin(mul(RL, X.b21)), mul(RL, X.b22))));
   }
   // SR = SRight[src].b21: the interfaces below it, right to left
   M2 SR = M2{z, z, z, z};
@@ -1239,9 +1242,14 @@ __device__ __forceinline__ void walk_body(const TransferParams& p, long node) {
 #pragma unroll 1
   for (int j = 2; j <= src; ++j) {
     const S4 X = ld_x(p, j, node, swaps);
-    const M2 Y = solve(imin(mul(X.b21, RL)), X.b22);
-    RL = add(X.b12, mul(X.b11, mul(RL, Y)));
-    S22 = mul(S22, Y);
+    if (j == 2) {  // as it is (see scan_body)
+      RL = X.b12;
+      S22 = X.b22;
+    } else {
+      const M2 Y = solve(imin(mul(X.b21, RL)), X.b22);
+      RL = add(X.b12, mul(X.b11, mul(RL, Y)));
+      S22 = mul(S22, Y);
+    }
     if (j < src && ((p.needL >> (j - 1)) & 1u)) st_pair(p.sleft, j, n, node, RL, S22);
   }
   // SRight[j - 1] b21 and b11, right to left
