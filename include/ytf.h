@@ -144,7 +144,8 @@ int ytf_transfer_1d_contour(ytf_ctx* ctx, const ytf_stack* stack, double omega, 
                             const int* obs_layers, ytf_cache** out);
 
 /* J_0(x) and J_1(x) of real x exactly as the int8x3 1D synthesis evaluates them for its J
- * digit images: Taylor rows below |x| = 25 (absolute error below 1e-15), Hankel's asymptotic
+ * digit images: Taylor rows below |x| = 25 (absolute error below 1e-15; J_1 below |x| = 1 by its
+ * series, within 1e-16 of the images' value and with its relative accuracy), Hankel's asymptotic
  * expansions with one shared phase above (absolute error below 1e-12). For tests and callers that want
  * the same values; no counterpart in the reference (SpecialFunctions.besselj). */
 int ytf_bessel_j01(ytf_ctx* ctx, long n, const double* x, double* j0, double* j1);

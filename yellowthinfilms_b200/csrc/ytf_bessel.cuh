@@ -3,7 +3,8 @@
 // methods by range:
 //   0 <= Re z < 25, |Im z| <= 0.4 : the Taylor rows of J_0 about i + 1/2 (ytf_bessel_tab.cuh) at the
 //                   complex distance d, |d| <= 0.65: one complex Horner pass for the value and the
-//                   derivative -J_1, |error| < 1e-15;
+//                   derivative -J_1, |error| < 1e-15; J_1 below |z| = 1 from its series, for its relative
+//                   accuracy;
 //   |z| >= 25     : the Hankel asymptotic expansion J_n(z) = √(2/(πz)) (P cos χ - Q sin χ),
 //                   χ = z - nπ/2 - π/4 (A&S 9.2.5, 9.2.9-10), P and Q as polynomials in 1/z² up to
 //                   the 19th term (the next is below 1e-17 at |z| = 25), both orders from one phase;
@@ -39,6 +40,26 @@ __device__ inline cd bessel_series(int n, cd z) {
   cd p{1.0, 0.0};
   for (int i = 0; i < n; ++i) p = p * h;
   return s * p;
+}
+
+// N! (2/z)^N J_N(z) = Σ_m (-h2)^m N! / (m! (m + N)!), h2 = z²/4, below |z| = 1 (A&S 9.1.10; 9 terms, the
+// first left out under 1e-17), of a real or complex argument
+template <int N>
+__device__ __forceinline__ double bessel_series_unit(double h2) {
+  double s = 1.0;
+#pragma unroll
+  for (int m = 8; m >= 1; --m) s = fma(-(h2 * (1.0 / (m * (m + N)))), s, 1.0);
+  return s;
+}
+template <int N>
+__device__ __forceinline__ cd bessel_series_unit(cd h2) {
+  cd s{1.0, 0.0};
+#pragma unroll
+  for (int m = 8; m >= 1; --m) {
+    s = (h2 * s) * (-1.0 / (m * (m + N)));
+    s.x += 1.0;
+  }
+  return s;
 }
 
 // Hankel's coefficients a_k(n) = Π_{j<=k} (4n² - (2j - 1)²) / (k! 8^k)
@@ -88,7 +109,8 @@ __device__ inline void bessel_j01_c(cd z, cd& J0, cd& J1) {
       p.x += c[m];
     }
     J0 = p;
-    J1 = -q;
+    // near 0 the derivative holds J_1 = z/2 to 1e-17 of 1, not of itself
+    J1 = norm2(z) < 1.0 ? z * 0.5 * bessel_series_unit<1>(z * z * 0.25) : -q;
     return;
   }
   const double az = cabs(z);

@@ -207,17 +207,6 @@ __device__ __forceinline__ void unpack_order_sums(F0 P0, F1 P1, F2 P2, cd g0[5],
   g2[3] = -g2[0];
 }
 
-// J_0, J_1, J_2 of a real argument: CUDA's j0/j1, J2 by its power series below |x| = 1 and the
-// three-term recurrence above
-// (h/2)^n-free part of J_N's power series, Σ_m (-h2)^m N! / (m! (m + N)!), h2 = x²/4 (A&S 9.1.10): below
-// x = 1 the first term left out is under 1e-17
-template <int N>
-__device__ __forceinline__ double bessel_series_real(double h2) {
-  double s = 1.0;
-#pragma unroll
-  for (int m = 8; m >= 1; --m) s = fma(-(h2 * (1.0 / (m * (m + N)))), s, 1.0);
-  return s;
-}
 // J_0, J_1, J_2 of a real argument: power series below 1 (relative accuracy down to x = 0), the Taylor rows
 // up to 25 (|error| <= 2e-16), Hankel's expansion with one phase for both orders above (the library past
 // 1e15); J_2 from the recurrence (A&S 9.1.27) from 1 on.
@@ -227,9 +216,9 @@ __device__ __forceinline__ void bessel_j012(double x, double& a0, double& a1, do
   const double ax = fabs(x);
   if (ax < 1.0) {
     const double h2 = 0.25 * x * x;
-    a0 = bessel_series_real<0>(h2);
-    a1 = 0.5 * x * bessel_series_real<1>(h2);
-    a2 = 0.5 * h2 * bessel_series_real<2>(h2);
+    a0 = bessel_series_unit<0>(h2);
+    a1 = 0.5 * x * bessel_series_unit<1>(h2);
+    a2 = 0.5 * h2 * bessel_series_unit<2>(h2);
     return;
   }
   if (ax < (double)JTAB_N) {
