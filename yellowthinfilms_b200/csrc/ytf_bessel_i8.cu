@@ -98,8 +98,9 @@ __device__ __forceinline__ void j01_large(double x, double y, double a, double& 
                             0.1171875), y2, 1.0);
   const double q1 = y * fma(fma(fma(fma(27.248827311268542, y2, -1.993531733751297), y2, 0.2775764465332031), y2,
                                 -0.1025390625), y2, 0.375);
-  // x - π/4 = n π/2 + r, |r| <= π/4; nm holds n in its low bits
-  const double nm = fma(x, 0.6366197723675814, 6755399441055744.0 - 0.5);
+  // x - π/4 = n π/2 + r, |r| <= π/4: n = floor(2 x / π), rounded down onto the whole numbers at 1.5 2^52,
+  // whose low bits hold it
+  const double nm = __fma_rd(x, 0.6366197723675814, 6755399441055744.0);
   const double m = (nm - 6755399441055744.0) + 0.5;
   double r = fma(-m, 1.5707963267341256, x);
   r = fma(-m, 6.077100506303966e-11, r);
