@@ -1967,14 +1967,23 @@ static int green_impl(ytf_ctx* ctx, const ytf_cache* c, int obs_layer, double zs
       } else {
         Lateral64 lp;
         std::memset(&lp, 0, sizeof(lp));
-        lp.npix = npix; lp.n = c->n; lp.nx = nx; lp.ncol = ncol; lp.S = S;
-        const int splits = lateral64_plan(lp);
-        WS(Ex, double2, "g_ex", (size_t)c->n * nx);
-        WS(Ey, double2, "g_ey", (size_t)c->n * ny);
-        WS(Gp, double2, "g_partial2", (size_t)splits * npix * ncol);
+        // the nodes in passes whose phase tables are bounded, their sums added in order
+        const long pass = lateral64_pass(c->n, nx, ny);
+        lp.npix = npix; lp.n = pass; lp.lds = c->n; lp.nx = nx; lp.ncol = ncol;
+        WS(Ex, double2, "g_ex", (size_t)pass * nx);
+        WS(Ey, double2, "g_ey", (size_t)pass * ny);
+        int most = lateral64_plan(lp);
+        lp.n = (c->n - 1) % pass + 1;  // the last pass
+        most = std::max(most, lateral64_plan(lp));
+        WS(Gp, double2, "g_partial2", (size_t)most * npix * ncol);
         lp.Ex = Ex; lp.Ey = Ey; lp.partial = Gp;
-        CK(LAUNCH("k_lateral", launch_lateral64(lp, v, dxs, dys, ctx->stream)));
-        CK(LAUNCH("k_reduce_splits2", launch_reduce_splits2(npix * ncol, splits, Gp, G, ctx->stream)));
+        for (lp.n0 = 0; lp.n0 < c->n; lp.n0 += pass) {
+          lp.n = std::min(pass, c->n - lp.n0);
+          lp.S = S + lp.n0;
+          const int splits = lateral64_plan(lp);
+          CK(LAUNCH("k_lateral", launch_lateral64(lp, v, dxs, dys, ctx->stream)));
+          CK(LAUNCH("k_reduce_splits2", launch_reduce_splits2(npix * ncol, splits, Gp, G, ctx->stream, lp.n0 > 0)));
+        }
       }
     }
   }

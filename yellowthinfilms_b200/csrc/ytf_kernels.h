@@ -213,18 +213,21 @@ cudaError_t launch_lateral(const CacheView& c, int nx, int ny, const double* xs,
                            double2* partial, int splits, cudaStream_t s);
 // the lateral sum on FP64 tensor-core instructions, with phase tables
 struct Lateral64 {
-  long npix, n;
+  long npix, n;       // pixels; nodes of this pass
+  long n0, lds;       // first node of the pass; row stride of S (every node)
   int nx, ncol;
   double2* Ex;        // [nx][n] scratch
   double2* Ey;        // [npix / nx][n] scratch
-  const double2* S;   // [ncol][n]
+  const double2* S;   // [ncol][lds], from the pass' first node on
   double2* partial;   // [splits][npix * ncol]
   long kchunk;
   int splits;
 };
+long lateral64_pass(long n, int nx, int ny);  // nodes per pass that bound the phase tables
 int lateral64_plan(Lateral64& p);  // kchunk and splits from npix, n, ncol
 cudaError_t launch_lateral64(const Lateral64& p, const CacheView& c, const double* xs, const double* ys, cudaStream_t s);
-cudaError_t launch_reduce_splits2(long len, int splits, const double2* partial, double2* G, cudaStream_t s);
+// G = (add ? G : 0) + the sum of the splits in order
+cudaError_t launch_reduce_splits2(long len, int splits, const double2* partial, double2* G, cudaStream_t s, int add = 0);
 
 // batched synthesis of small observation sets (uneven batches): per item the partial sums
 // of each node chunk, then a per-output sum over the chunks (2D) or sum and pixel assembly (1D)

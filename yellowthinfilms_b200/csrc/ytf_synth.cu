@@ -1307,17 +1307,17 @@ __global__ void __launch_bounds__(256) k_lateral(CacheView c, int nx, int ny, co
 // ------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(128) k_phase_tables64(CacheView c, int nx, int ny, const double* __restrict__ xs,
                                                         const double* __restrict__ ys, double2* __restrict__ Ex,
-                                                        double2* __restrict__ Ey) {
+                                                        double2* __restrict__ Ey, long n0, long n) {
   const long nn = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (nn >= c.n) return;
+  if (nn >= n) return;
   double sp, cp;
-  sincos(c.phi[nn / c.Nk], &sp, &cp);
-  const double k = c.kr[nn % c.Nk];
+  sincos(c.phi[(n0 + nn) / c.Nk], &sp, &cp);
+  const double k = c.kr[(n0 + nn) % c.Nk];
   // rows of each axis split over blockIdx.y
   for (int e = blockIdx.y; e < nx + ny; e += gridDim.y) {
     double s, co;
     sincos(e < nx ? k * cp * xs[e] : k * sp * ys[e - nx], &s, &co);
-    (e < nx ? Ex + (long)e * c.n : Ey + (long)(e - nx) * c.n)[nn] = make_double2(co, s);
+    (e < nx ? Ex + (long)e * n : Ey + (long)(e - nx) * n)[nn] = make_double2(co, s);
   }
 }
 
@@ -1364,7 +1364,7 @@ __global__ void __launch_bounds__(128, F <= 9 ? 3 : 2) k_lateral64(const __grid_
       const long nn = k0 + (long)st * L64_N + j;
       const bool in = c0 + c < p.ncol && nn < k1;
       cp16((uint32_t)__cvta_generic_to_shared(&Bs[st & 1][c * L64_LD + 2 * j]),
-           reinterpret_cast<const double*>(p.S + (in ? (long)(c0 + c) * p.n + nn : 0)), in ? 16 : 0);
+           reinterpret_cast<const double*>(p.S + (in ? (long)(c0 + c) * p.lds + nn : 0)), in ? 16 : 0);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -1418,6 +1418,12 @@ __global__ void __launch_bounds__(128, F <= 9 ? 3 : 2) k_lateral64(const __grid_
   }
 }
 
+// nodes per pass: phase tables of at most 1 GiB, or of one 8-node stage where the coordinates are that many
+long lateral64_pass(long n, int nx, int ny) {
+  const long fit = (1L << 30) / (16L * ((long)nx + ny)) / L64_N * L64_N;
+  return std::min(n, std::max(fit, (long)L64_N));
+}
+
 // balanced column tiles of at most 48 complex columns
 static int lateral64_f(int ncol) {
   const int tiles = (ncol + 47) / 48;
@@ -1448,7 +1454,7 @@ cudaError_t launch_lateral64(const Lateral64& p, const CacheView& c, const doubl
   if (p.npix <= 0 || p.ncol <= 0 || p.n <= 0) return cudaSuccess;
   const int ny = (int)(p.npix / p.nx);
   k_phase_tables64<<<dim3((unsigned)((p.n + 127) / 128), (unsigned)std::min(p.nx + ny, 8)), 128, 0, s>>>(
-      c, p.nx, ny, xs, ys, p.Ex, p.Ey);
+      c, p.nx, ny, xs, ys, p.Ex, p.Ey, p.n0, p.n);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   lateral64_run<12>(p, s);
@@ -1475,9 +1481,15 @@ __device__ __forceinline__ double2 sum_in_order(const double2* __restrict__ P, l
 // One thread per output; bound by the chain of its loads: 12285 outputs 14.6 us with one load at a
 // time in blocks of 256, 7.6 us; 20736 outputs 8.0 -> 5.1 us
 __global__ void __launch_bounds__(64) k_reduce_splits2(long len, int splits, const double2* __restrict__ P,
-                                                       double2* __restrict__ C) {
+                                                       double2* __restrict__ C, int add) {
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < len) C[i] = sum_in_order(P + i, len, splits);
+  if (i >= len) return;
+  double2 s = sum_in_order(P + i, len, splits);
+  if (add) {
+    const double2 c = C[i];
+    s = make_double2(c.x + s.x, c.y + s.y);
+  }
+  C[i] = s;
 }
 
 int lateral_splits(long n, int splits) {
@@ -1498,9 +1510,9 @@ cudaError_t launch_lateral(const CacheView& c, int nx, int ny, const double* xs,
   return cudaGetLastError();
 }
 
-cudaError_t launch_reduce_splits2(long len, int splits, const double2* partial, double2* G, cudaStream_t s) {
+cudaError_t launch_reduce_splits2(long len, int splits, const double2* partial, double2* G, cudaStream_t s, int add) {
   if (len <= 0) return cudaSuccess;
-  k_reduce_splits2<<<(unsigned)((len + 63) / 64), 64, 0, s>>>(len, splits, partial, G);
+  k_reduce_splits2<<<(unsigned)((len + 63) / 64), 64, 0, s>>>(len, splits, partial, G, add);
   return cudaGetLastError();
 }
 
