@@ -295,7 +295,7 @@ struct ytf_mlp {
   long cap = 0;
   std::vector<float*> Z, H, dZ, dH;
   float *T = nullptr, *lb = nullptr;
-  // inputs and outputs of the largest forward-only batch from host memory (fused networks)
+  // inputs and outputs of the largest forward-only batch that is copied (fused networks)
   long cap_io = 0;
   float *Xin = nullptr, *Yout = nullptr;
   unsigned* tc_err = nullptr;      // page-locked: set by a kernel whose tensor-core wait ran out
@@ -398,7 +398,7 @@ int ensure(ytf_mlp* net, long B) {
   return YTF_OK;
 }
 
-// staging of a forward-only batch from host memory
+// staging of a forward-only batch from host memory or with outputs over its inputs
 int ensure_io(ytf_mlp* net, long B) {
   if (B <= net->cap_io) return YTF_OK;
   cudaFree(net->Xin); cudaFree(net->Yout);
@@ -684,10 +684,16 @@ int ytf_mlp_forward(ytf_mlp* net, int B, const float* X, float* out, int on_devi
   int rc;
   const size_t xb = sizeof(float) * B * net->sizes[0];
   if (net->fused) {
-    if (!on_device && (rc = ensure_io(net, B))) return rc;
-    if (!on_device) MCK(cudaMemcpyAsync(net->Xin, X, xb, cudaMemcpyHostToDevice, net->stream));
+    // device inputs are read where they lie, unless the outputs lie over them: a CTA writes its rows'
+    // outputs while others still read
+    const uintptr_t x0 = (uintptr_t)X, y0 = (uintptr_t)out;
+    const bool overlap = x0 < y0 + sizeof(float) * 2 * B && y0 < x0 + xb;
+    const bool copied = !on_device || overlap;
+    if (copied && (rc = ensure_io(net, B))) return rc;
+    if (copied)
+      MCK(cudaMemcpyAsync(net->Xin, X, xb, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, net->stream));
     float* y = on_device ? out : net->Yout;
-    if ((rc = pack_weights(net, false)) || (rc = forward_fused(net, B, on_device ? X : net->Xin, y, false))) return rc;
+    if ((rc = pack_weights(net, false)) || (rc = forward_fused(net, B, copied ? net->Xin : X, y, false))) return rc;
     if (!on_device) MCK(cudaMemcpyAsync(out, y, sizeof(float) * 2 * B, cudaMemcpyDeviceToHost, net->stream));
     MCK(cudaStreamSynchronize(net->stream));
     return check_waits(net);
