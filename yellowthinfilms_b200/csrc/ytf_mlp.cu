@@ -410,6 +410,16 @@ int ensure_io(ytf_mlp* net, long B) {
   return YTF_OK;
 }
 
+// memory of another GPU, which a kernel of this one reaches only with peer access (a copy always does)
+bool other_device(int device, const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device != device;
+}
+
 int round16(int n) { return (n + 15) / 16 * 16; }
 
 // the weight images of the fused kernels from the current parameters
@@ -684,17 +694,20 @@ int ytf_mlp_forward(ytf_mlp* net, int B, const float* X, float* out, int on_devi
   int rc;
   const size_t xb = sizeof(float) * B * net->sizes[0];
   if (net->fused) {
-    // device inputs are read where they lie, unless the outputs lie over them: a CTA writes its rows'
-    // outputs while others still read
+    // device memory is used where it lies, unless it is another GPU's or the outputs lie over the inputs (a CTA
+    // writes its rows' outputs while others still read)
     const uintptr_t x0 = (uintptr_t)X, y0 = (uintptr_t)out;
     const bool overlap = x0 < y0 + sizeof(float) * 2 * B && y0 < x0 + xb;
-    const bool copied = !on_device || overlap;
-    if (copied && (rc = ensure_io(net, B))) return rc;
-    if (copied)
+    const bool xcopy = !on_device || overlap || other_device(net->device, X);
+    const bool ycopy = !on_device || other_device(net->device, out);
+    if ((xcopy || ycopy) && (rc = ensure_io(net, B))) return rc;
+    if (xcopy)
       MCK(cudaMemcpyAsync(net->Xin, X, xb, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, net->stream));
-    float* y = on_device ? out : net->Yout;
-    if ((rc = pack_weights(net, false)) || (rc = forward_fused(net, B, copied ? net->Xin : X, y, false))) return rc;
-    if (!on_device) MCK(cudaMemcpyAsync(out, y, sizeof(float) * 2 * B, cudaMemcpyDeviceToHost, net->stream));
+    float* y = ycopy ? net->Yout : out;
+    if ((rc = pack_weights(net, false)) || (rc = forward_fused(net, B, xcopy ? net->Xin : X, y, false))) return rc;
+    if (ycopy)
+      MCK(cudaMemcpyAsync(out, y, sizeof(float) * 2 * B, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
+                          net->stream));
     MCK(cudaStreamSynchronize(net->stream));
     return check_waits(net);
   }
