@@ -6,20 +6,22 @@
 // shared memory from the first layer to the last: 128 x 256 values as two BF16 terms (hi, lo) in
 // the tensor cores' K-major layout, 128 KB. The BF16 weights come as prepacked images of that
 // layout (k_mlp_pack, once per pass), 64 input columns per bulk copy into a 3-slot ring. One
-// thread copies and issues the MMAs (hi·W, lo·W per 16 columns, FP32 sums in tensor memory);
+// thread copies and issues the MMAs (hi·W, lo·W per 16 columns, FP32 sums of their own in tensor memory:
+// an MMA cuts its sum off at the accumulator's last bit, so the small products would cost a large sum as many
+// units as the large ones do. Gradients of 2048 rows 6.0e-6 from 64 bits with one sum, 2.7e-6 with two);
 // sixteen warps drain the accumulator, apply bias + GELU (or the GELU derivative), split the result
 // and write it over the tile in place. Only the input, the result and what the backward pass
 // needs touch global memory.
 //   What bounds it: MMAs and drain of a tile alternate (the tile is rewritten in place), about 25
 // instructions per value in the drain, and 128 B/clk of shared memory for the operands and the
-// weight copies together. 65536 rows of the 154 -> 256 x 4 -> 2 forward pass: 186 us; one launch per
+// weight copies together. 65536 rows of the 154 -> 256 x 4 -> 2 forward pass: 183 us; one launch per
 // layer with the operands converted by 128 threads between the MMAs took 2409 us.
 //
 // k_mlp_dw forms every layer's dW = dZ^T H and db = Σ dZ in one grid over (layer, 128-row tile of
 // dW, slice of the batch); k_mlp_dw_sum adds the slices in order. The batch index is the
 // contraction index, so a thread takes one column of dZ or H over 8 consecutive samples (coalesced
 // loads along the columns) and stores the 8 terms of one K-core as 16 bytes. The bias
-// gradient is the sum of the same loads. 8192 rows: 71 us; the GEMMs per layer took 341 us and one
+// gradient is the sum of the same loads. hi·hi and the two mixed products have sums of their own here too. 8192 rows: 67 us; the GEMMs per layer took 341 us and one
 // thread per bias column 961 us.
 #pragma once
 #include <cuda_bf16.h>
@@ -148,7 +150,7 @@ __global__ void __launch_bounds__(256) k_mlp_pack(Pack p) {
 // against the absolute error of Φ); past t = 6 the exponent keeps falling (below -30 at 6, to -inf). In FP32 |error| < 7e-8 (rms
 // 1.4e-8), as 0.5 (1 + erff) gives, and no cancellation for negative arguments. The library's erff
 // branches on its argument, which diverges within a warp and keeps a thread's columns apart: the
-// forward pass of 65536 rows took 270 us with it and takes 186 us with this.
+// forward pass of 65536 rows took 270 us with it and 186 us with this.
 __device__ __forceinline__ float norm_tail(float t) {
   float r = -3.5514208462927854e-08f;
   r = fmaf(r, t, 1.0132938541573822e-06f);
@@ -215,7 +217,7 @@ __global__ void __launch_bounds__(FDRAIN + 32, 1) k_mlp_chain(const __grid_const
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&sh->tmem)),
-                 "r"(FW)
+                 "r"(2 * FW)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -267,7 +269,7 @@ __global__ void __launch_bounds__(FDRAIN + 32, 1) k_mlp_chain(const __grid_const
               const uint32_t oa = (uint32_t)(q >> 1) * FPLANE + (q & 1) * 256u;
               const uint64_t bd = umma_desc(b0 + (uint32_t)((q >> 1) & 1) * planeB + (q & 1) * 256u);
               mma_f16(tmem, umma_desc(smem_u32(hi) + oa), bd, idesc, q > 0 ? 1u : 0u);
-              mma_f16(tmem, umma_desc(smem_u32(lo) + oa), bd, idesc, 1u);
+              mma_f16(tmem + FW, umma_desc(smem_u32(lo) + oa), bd, idesc, q > 0 ? 1u : 0u);
             }
             tc_commit(smem_u32(&sh->empty[slot]));
             if (issued < total) ok = copy_next();
@@ -359,9 +361,13 @@ __global__ void __launch_bounds__(FDRAIN + 32, 1) k_mlp_chain(const __grid_const
         constexpr int NG = FDRAIN / 128;
         for (int n0 = 8 * part; n0 < L.Np; n0 += 16 * NG) {
           const bool two = n0 + 8 * NG < L.Np;
-          uint32_t v[2][8];
+          uint32_t v[2][8], w[2][8];
           tmem_ld8(tmem + lanebase + n0, v[0]);
-          if (two) tmem_ld8(tmem + lanebase + n0 + 8 * NG, v[1]);
+          tmem_ld8(tmem + FW + lanebase + n0, w[0]);
+          if (two) {
+            tmem_ld8(tmem + lanebase + n0 + 8 * NG, v[1]);
+            tmem_ld8(tmem + FW + lanebase + n0 + 8 * NG, w[1]);
+          }
           float z[2][8], y[2][8];  // BACK: Z; forward: the bias, then Z
           const float* zrow = BACK ? L.Z + b * L.N : L.bias;
           load_row8(zrow, n0, L.N, BACK ? vec : bvec, BACK ? live : true, z[0]);
@@ -373,7 +379,7 @@ __global__ void __launch_bounds__(FDRAIN + 32, 1) k_mlp_chain(const __grid_const
             const int n = n0 + 8 * NG * g;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-              const float acc = __uint_as_float(v[g][j]);
+              const float acc = __uint_as_float(v[g][j]) + __uint_as_float(w[g][j]);
               if (BACK) {
                 // dZ = dH GELU'(Z), GELU'(z) = Φ(z) + z φ(z)
                 const float zz = z[g][j];
@@ -390,14 +396,14 @@ __global__ void __launch_bounds__(FDRAIN + 32, 1) k_mlp_chain(const __grid_const
             if (L.H) store_row8(L.H + b * L.N, n, L.N, vec, live, y[g]);
             if (!BACK && last) store_row8(p.out + b * L.N, n, L.N, false, live, y[g]);
             if (!last) {
-              uint4 h, w;
-              split2(y[g][0], y[g][1], h.x, w.x);
-              split2(y[g][2], y[g][3], h.y, w.y);
-              split2(y[g][4], y[g][5], h.z, w.z);
-              split2(y[g][6], y[g][7], h.w, w.w);
+              uint4 h, l4;
+              split2(y[g][0], y[g][1], h.x, l4.x);
+              split2(y[g][2], y[g][3], h.y, l4.y);
+              split2(y[g][4], y[g][5], h.z, l4.z);
+              split2(y[g][6], y[g][7], h.w, l4.w);
               const uint32_t off = (uint32_t)(n >> 5) * FPLANE + plane_off(r, 2 * (n & 31));
               *reinterpret_cast<uint4*>(hi + off) = h;
-              *reinterpret_cast<uint4*>(lo + off) = w;
+              *reinterpret_cast<uint4*>(lo + off) = l4;
             }
           }
         }
@@ -415,7 +421,7 @@ __global__ void __launch_bounds__(FDRAIN + 32, 1) k_mlp_chain(const __grid_const
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(FW) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * FW) : "memory");
   }
 }
 
@@ -479,7 +485,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) k_mlp_dw(const __grid_constant_
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_sh)), "r"(FW)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_sh)), "r"(2 * FW)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -529,8 +535,8 @@ __global__ void __launch_bounds__(DW_THREADS, 1) k_mlp_dw(const __grid_constant_
         const uint64_t dah = umma_desc(smem_u32(ah) + oa), dal = umma_desc(smem_u32(al) + oa);
         const uint64_t dbh = umma_desc(smem_u32(bh) + ob), dbl = umma_desc(smem_u32(bl) + ob);
         mma_f16(tmem, dah, dbh, idesc, kb > 0 || q > 0 ? 1u : 0u);
-        mma_f16(tmem, dah, dbl, idesc, 1u);
-        mma_f16(tmem, dal, dbh, idesc, 1u);
+        mma_f16(tmem + FW, dah, dbl, idesc, kb > 0 || q > 0 ? 1u : 0u);
+        mma_f16(tmem + FW, dal, dbh, idesc, 1u);
       }
       tc_commit(smem_u32(&bar[kb & 1]));
     }
@@ -547,15 +553,16 @@ __global__ void __launch_bounds__(DW_THREADS, 1) k_mlp_dw(const __grid_constant_
     const int q4 = warp & 3;
     const int m = mt * FM + 32 * q4 + lane;
     for (int n = 8 * (warp >> 2); n < L.Np; n += 8 * (DW_THREADS / 128)) {
-      uint32_t v[8];
+      uint32_t v[8], w[8];
       if (nkb > 0) {
         tmem_ld8(tmem + ((uint32_t)(32 * q4) << 16) + n, v);
+        tmem_ld8(tmem + FW + ((uint32_t)(32 * q4) << 16) + n, w);
         tmem_wait_ld();
       }
       if (m < L.M)
 #pragma unroll
         for (int j = 0; j < 8; ++j)
-          if (n + j < L.N) part[L.poff + (long)m * L.N + n + j] = nkb > 0 ? __uint_as_float(v[j]) : 0.f;
+          if (n + j < L.N) part[L.poff + (long)m * L.N + n + j] = nkb > 0 ? __uint_as_float(v[j]) + __uint_as_float(w[j]) : 0.f;
     }
   }
   dbs[tid] = db;
@@ -565,7 +572,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) k_mlp_dw(const __grid_constant_
   __syncthreads();
   if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(FW) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * FW) : "memory");
   }
 }
 
