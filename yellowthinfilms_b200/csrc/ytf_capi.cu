@@ -9,11 +9,11 @@
 #include <set>
 #include <string>
 #include <thread>
-#include <unordered_map>
 #include <vector>
 
 #include "../../include/ytf.h"
 #include "ytf_kernels.h"
+#include "ytf_radii.h"
 #include "ytf_grid.h"
 
 using namespace ytf;
@@ -312,32 +312,6 @@ struct GreenBatch {
   const int* drmap = nullptr;    // 1D: pixel -> radius index
   int nr = 0;                    // 1D: distinct radii
 };
-
-// distinct radii hypot(x_i, y_j) in first-occurrence order over (i fastest, j), as the
-// reference, and each pixel's index into them (open addressing by the radius' bits: no allocation per
-// radius, as a node-based map makes)
-void radii_map(int nx, const double* xs, int ny, const double* ys, std::vector<double>& ur, std::vector<int>& rmap) {
-  const long npix = (long)nx * ny;
-  ur.clear();
-  rmap.assign(npix, 0);
-  size_t cap = 16;
-  while (cap < 2 * (size_t)npix) cap *= 2;
-  std::vector<int> slot(cap, -1);
-  for (int j = 0; j < ny; ++j)
-    for (int i = 0; i < nx; ++i) {
-      const double r = std::hypot(xs[i], ys[j]);
-      uint64_t h;
-      std::memcpy(&h, &r, 8);
-      h *= 0x9E3779B97F4A7C15ull;
-      size_t q = (size_t)(h >> 20) & (cap - 1);
-      while (slot[q] >= 0 && ur[slot[q]] != r) q = (q + 1) & (cap - 1);  // a NaN is a radius of its own
-      if (slot[q] < 0) {
-        slot[q] = (int)ur.size();
-        ur.push_back(r);
-      }
-      rmap[i + (long)nx * j] = slot[q];
-    }
-}
 
 // allocate the cache's arrays in one block
 // (`clear`: zero-filled; a build writes every value of its own, zeros for nodes that fail)
