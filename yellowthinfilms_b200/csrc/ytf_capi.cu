@@ -1287,19 +1287,9 @@ int ytf_bessel_j01(ytf_ctx* ctx, long n, const double* x, double* j0, double* j1
   return YTF_OK;
 }
 
-int ytf_transfer_batch(ytf_ctx* ctx, int nb, const ytf_transfer_desc* d, ytf_cache** out) {
-  if (!ctx || nb < 0 || (nb > 0 && (!d || !out))) return YTF_ERR_ARG;
-  for (int i = 0; i < nb; ++i) out[i] = nullptr;
-  if (nb == 0) return YTF_OK;
-  CK(cudaSetDevice(ctx->device));
-  std::vector<ytf_cache*> cs(nb, nullptr);
+// the caches of a batch into cs; on an error those made so far are the caller's to destroy
+static int transfer_batch(ytf_ctx* ctx, int nb, const ytf_transfer_desc* d, std::vector<ytf_cache*>& cs) {
   std::vector<char> rot(nb, 0);
-  auto abort_all = [&](int rc) {
-    cudaStreamSynchronize(ctx->stream);
-    for (auto c : cs)
-      if (c) ytf_cache_destroy(c);
-    return rc;
-  };
   // 1. validate and create every cache; node arrays go up from one page-locked block
   size_t stage = 0;
   for (int i = 0; i < nb; ++i) {
@@ -1313,8 +1303,7 @@ int ytf_transfer_batch(ytf_ctx* ctx, int nb, const ytf_transfer_desc* d, ytf_cac
                          d[i].nphi, d[i].phi_nodes, d[i].phi_weights, d[i].nobs, d[i].obs_layers,
                          d[i].check_symmetry, d[i].rotation, false, &cs[i], &r, d[i].nodes_on_device != 0);
     if (rc) {
-      std::string m = ctx->err;
-      abort_all(rc);
+      const std::string m = ctx->err;
       return fail(ctx, rc, m + " (batch item " + std::to_string(i) + ")");
     }
     rot[i] = r;
@@ -1335,7 +1324,7 @@ int ytf_transfer_batch(ytf_ctx* ctx, int nb, const ytf_transfer_desc* d, ytf_cac
   // per pass: every item's block, then the scan's and the walk's subsets, 5 offset arrays
   size_t pbytes = 2 * (size_t)nb * sizeof(TransferParams) + 5 * (size_t)(nb + 1) * sizeof(long);
   char* h = (char*)pinned_staging(ctx, 8 * std::max<size_t>(stage, 1) + 4 * (size_t)nb * sizeof(CopySeg) + pbytes + 128);
-  if (!h) return abort_all(fail(ctx, YTF_ERR_NOMEM, "build_cavity_transfer: page-locked staging allocation failed"));
+  if (!h) return fail(ctx, YTF_ERR_NOMEM, "build_cavity_transfer: page-locked staging allocation failed");
   // every item's node arrays in one upload and one scatter launch (device-resident nodes: read where
   // they lie, on the same stream)
   {
@@ -1369,7 +1358,7 @@ int ytf_transfer_batch(ytf_ctx* ctx, int nb, const ytf_transfer_desc* d, ytf_cac
       cudaError_t e = cudaMemcpyAsync(dnodes, hd, nbytes, cudaMemcpyHostToDevice, ctx->stream);
       if (e == cudaSuccess)
         e = LAUNCH("k_copy_segments", launch_copy_segments((const CopySeg*)(dnodes + k), (int)segs.size(), most, ctx->stream));
-      if (e != cudaSuccess) return abort_all(fail(ctx, YTF_ERR_CUDA, cudaGetErrorString(e)));
+      if (e != cudaSuccess) return fail(ctx, YTF_ERR_CUDA, cudaGetErrorString(e));
       h += (nbytes + 63) / 64 * 64;
     }
   }
@@ -1377,7 +1366,7 @@ int ytf_transfer_batch(ytf_ctx* ctx, int nb, const ytf_transfer_desc* d, ytf_cac
   for (int i = 0; i < nb; ++i) {
     if (cs[i]->n == 0 || !(rot[i] || scratch[i] > budget)) continue;
     int rc = rot[i] ? solve_rotation(ctx, d[i].stack, cs[i], ps[i]) : run_transfer(ctx, ps[i], cs[i]->n);
-    if (rc) return abort_all(rc);
+    if (rc) return rc;
   }
   int first = 0;
   bool staged = false;
@@ -1472,9 +1461,26 @@ int ytf_transfer_batch(ytf_ctx* ctx, int nb, const ytf_transfer_desc* d, ytf_cac
       CK(LAUNCH("k_walk", launch_transfer_batch(3, dpg, doffg, ng, offg[ng], ctx->stream)));
     }
   }
-  cudaError_t e = cudaStreamSynchronize(ctx->stream);
-  if (e != cudaSuccess) return abort_all(fail(ctx, YTF_ERR_CUDA, cudaGetErrorString(e)));
+  CK(cudaStreamSynchronize(ctx->stream));
   prof_collect(ctx);
+  return YTF_OK;
+}
+
+int ytf_transfer_batch(ytf_ctx* ctx, int nb, const ytf_transfer_desc* d, ytf_cache** out) {
+  if (!ctx || nb < 0 || (nb > 0 && (!d || !out))) return YTF_ERR_ARG;
+  for (int i = 0; i < nb; ++i) out[i] = nullptr;
+  if (nb == 0) return YTF_OK;
+  CK(cudaSetDevice(ctx->device));
+  std::vector<ytf_cache*> cs(nb, nullptr);
+  const int rc = transfer_batch(ctx, nb, d, cs);
+  if (rc) {
+    const std::string m = ctx->err;
+    cudaStreamSynchronize(ctx->stream);
+    for (auto c : cs)
+      if (c) ytf_cache_destroy(c);
+    ctx->err = m;
+    return rc;
+  }
   for (int i = 0; i < nb; ++i) out[i] = cs[i];
   return YTF_OK;
 }
