@@ -1,6 +1,6 @@
 """Layers of infinite thickness. The last one: its backward wave, counted from z - d, has amplitude 0 and no
-finite phase. The first one, unobserved: its thickness does not enter. Against the oracle at the parity tests'
-bounds."""
+finite phase. The first one, unobserved: its thickness does not enter. And heights that are not numbers, whose
+phases count as 0. Against the oracle at the parity tests' bounds."""
 import numpy as np
 import pytest
 
@@ -68,3 +68,27 @@ def test_first_layer_thickness_does_not_enter(oracle, d, aniso, obs):
     # the response's singular values are held to 1e-9 of the oracle elsewhere
     assert np.abs(api.cavity_response(st, W, 2, k) - r).max() <= 1e-9 * r.max()
     assert np.abs(api.cavity_response_batch([(st, W, 2, k)])[0] - r).max() <= 1e-9 * r.max()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("at", [0, 1, 16, 20])
+@pytest.mark.parametrize("terms", ["all", "scattered"])
+def test_a_height_that_is_not_a_number(oracle, bad, at, terms):
+    """Its field is 0, and the other heights' are as without it."""
+    from yellowthinfilms_b200 import api
+    st = config1_like_stack()
+    k, w = _rule(72)
+    z = np.sort(np.random.default_rng(1).uniform(0.0, 0.3, 21))
+    gc = api.build_cavity_transfer_1d(st, W, 1, k, w, obs_layers=[1, 2])
+    oc = oracle.build_cavity_transfer_1d(st, W, 1, k, w, obs_layers=[1, 2])
+    x = np.geomspace(0.01, 2.0, 5)
+    for o in (1, 2):
+        ok = np.arange(21) != at
+        Go = oracle.closed_form_G(oc, o, 0.03, z[ok], x, [0.0], terms=terms)
+        zb = np.where(ok, z, bad)
+        item = dict(cache=gc, obs_layer=o, zsrc_local=0.03, z_obs=zb, xs=x, ys=[0.0], terms=terms)
+        for G, tol in ((api.closed_form_G(gc, o, 0.03, zb, x, [0.0], terms=terms), 1e-10),
+                       (api.closed_form_G(gc, o, 0.03, zb, x, [0.0], terms=terms, precision="int8x3"), 1e-6),
+                       (api.closed_form_G_batch([item] * 2, precision="int8x3")[0], 1e-6)):
+            assert (G[:, :, at] == 0).all()
+            assert relerr(G[:, :, ok], Go) < tol

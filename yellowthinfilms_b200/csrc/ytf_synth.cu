@@ -893,9 +893,12 @@ __device__ __forceinline__ void coef_sym_rows(const SynthParams& p, const double
   for (int i = 0; i < 10; ++i) F[i] = ldc(amp, i, n, k);
 #pragma unroll
   for (int i = 0; i < 4; ++i) kz[i] = ldc(amp, 10 + i, n, k);
-  double zlo = p.zo[z0], zhi = zlo;
-  for (int zi = z0 + 1; zi < z1; ++zi) { zlo = fmin(zlo, p.zo[zi]); zhi = fmax(zhi, p.zo[zi]); }
-  double big = 0.0, lo = 0.0, hi = 0.0;
+  double zlo = p.zo[z0], zhi = zlo, big = fabs(zlo), lo = 0.0, hi = 0.0;
+  for (int zi = z0 + 1; zi < z1; ++zi) {
+    zlo = fmin(zlo, p.zo[zi]);
+    zhi = fmax(zhi, p.zo[zi]);
+    big += fabs(p.zo[zi]);  // the extremes pass over a NaN
+  }
 #pragma unroll
   for (int i = 0; i < 10; ++i) big += fabs(F[i].x) + fabs(F[i].y);
 #pragma unroll
