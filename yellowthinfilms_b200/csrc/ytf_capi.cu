@@ -2909,7 +2909,7 @@ extern "C" int ytf_plan_retune(ytf_plan* P, const ytf_tune* tune_in) {
     long all = 0;
     for (int i = 0; i < nb; ++i)
       if (!P->large[i] && (long)P->gr[i].nx * P->gr[i].ny * P->gr[i].nz > 0) all += P->cs[i]->n;
-    const long units = 4L * 3 * P->nsm;
+    const long units = 4L * std::min(3, t.synth_ctas_per_sm) * P->nsm;  // three CTAs fit an SM
     chunk = (int)std::min<long>(t.chunk, std::max(1L, ((all + units - 1) / units + 63) / 64) * 64);
   }
   for (int i = 0; i < nb; ++i) {
