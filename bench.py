@@ -343,7 +343,7 @@ def roofline(name, prof, steps=1):
             roof.update(split_multiplier=6, int8_ops_executed_per_launch=ex,
                         executed_frac_of_int8_peak=ex / t / 1e12 / (2 * peak),
                         int8_peak_note="int8 peak taken as 2 x the measured bf16 figure (nominal ratio)")
-    elif name == "k_lateral":
+    elif name == "k_lateral64":
         achieved = 8.0 * cmacs / t / 1e12
         roof.update(bound="fp64", achieved=achieved, peak=FP64_NOMINAL, unit="TFLOP/s", frac=achieved / FP64_NOMINAL,
                     peak_source="nominal FP64; no measured FP64 peak", work=work)
@@ -467,7 +467,7 @@ def run_ours(args):
     # roofline of the dominant kernel (and of the lateral contraction), from the CUDA-event
     # profile of the timed region
     top = max(prof.items(), key=lambda kv: kv[1][0])[0] if prof else None
-    lateral = next((k for k in ("k_lateral_i8", "k_lateral_tc", "k_lateral") if k in prof), None)
+    lateral = next((k for k in ("k_lateral_i8", "k_lateral_tc", "k_lateral64") if k in prof), None)
     roof = roofline(top, prof, args.steps)
     if lateral and lateral != top:
         roof["lateral"] = roofline(lateral, prof, args.steps)
@@ -1007,7 +1007,7 @@ def run_bessel(args):
     ms64, prof64, _, G64 = run("fp64")
     entries = G.size
     flops = 2.0 * 4096 * 65536 * 10 * 256  # the 5 stored complex coefficient columns (TE and TM decouple) per height
-    name = "k_bessel_i8" if prec == "int8x3" else "k_dgemm_nt"
+    name = "k_bessel_i8" if prec == "int8x3" else "k_gemm64"
     t_k = prof[name][0] / args.steps * 1e-3 if name in prof else None
     peak, src = measured_peaks()["bf16_sustained"]
     roof = {"kernel": name, "bound": "tensor" if prec == "int8x3" else "fp64",

@@ -314,8 +314,8 @@ struct GreenBatch {
 };
 
 // allocate the cache's arrays in one block
-// (`clear`: zero-filled; a build writes every value of its own, zeros for nodes that fail)
-int alloc_cache(ytf_ctx* ctx, ytf_cache* c, bool upload_nodes = true, bool clear = false) {
+// (not cleared: a build writes every value, zeros for nodes that fail)
+int alloc_cache(ytf_ctx* ctx, ytf_cache* c, bool upload_nodes = true) {
   long n = c->n;
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -346,7 +346,6 @@ int alloc_cache(ytf_ctx* ctx, ytf_cache* c, bool upload_nodes = true, bool clear
   c->d_status = (uint8_t*)(b + o_status); c->d_valid = (uint8_t*)(b + o_valid); c->d_tvalid = (uint8_t*)(b + o_tvalid);
   c->d_T = (double2*)(b + o_T); c->d_Qf = (double2*)(b + o_Qf); c->d_Qb = (double2*)(b + o_Qb);
   c->d_sf = (double2*)(b + o_sf); c->d_sb = (double2*)(b + o_sb); c->d_basis = (double2*)(b + o_basis);
-  if (clear) CK(cudaMemsetAsync(c->block, 0, off, ctx->stream));
   if (!upload_nodes) return YTF_OK;
   // the node arrays lie at the front of the block: one copy from page-locked memory, which the build's
   // synchronisation frees
@@ -634,7 +633,7 @@ namespace {
 int prepare_cache(ytf_ctx* ctx, const ytf_stack* st, bool is2d, double omega, int source_layer, int nk,
                   const double* k_nodes, const double* k_weights, int nphi, const double* phi_nodes,
                   const double* phi_weights, int nobs, const int* obs_layers, int check_symmetry, int rotation,
-                  bool upload_nodes, ytf_cache** out, bool* use_rot, bool nodes_dev = false, bool clear = false) {
+                  bool upload_nodes, ytf_cache** out, bool* use_rot, bool nodes_dev = false) {
   *out = nullptr;
   *use_rot = false;
   const char* fn = is2d ? "build_cavity_transfer_2d" : "build_cavity_transfer_1d";
@@ -698,7 +697,7 @@ int prepare_cache(ytf_ctx* ctx, const ytf_stack* st, bool is2d, double omega, in
   }
   for (auto& L : st->host) c->d_layer.push_back(L.d);
   c->d_src = st->host[source_layer - 1].d;
-  if ((rc = alloc_cache(ctx, c, upload_nodes, clear))) { ytf_cache_destroy(c); return rc; }
+  if ((rc = alloc_cache(ctx, c, upload_nodes))) { ytf_cache_destroy(c); return rc; }
   *out = c;
   return YTF_OK;
 }
@@ -1651,7 +1650,7 @@ static int synth1d_parts(ytf_ctx* ctx, const SynthParams& sp, int nz, double dz,
     carve(Pp, out.nchunk);
     for (int q = 0; q < np; ++q)
       for (int o = 0; o < 3; ++o) g.e[3 * q + o].out = (q ? out.part_im : out.part)[o];
-    CK(LAUNCH("k_dgemm_nt", launch_gemm64(g, ctx->stream)));
+    CK(LAUNCH("k_gemm64", launch_gemm64(g, ctx->stream)));
     return YTF_OK;
   }
   // int8 tensor cores: J_n and the coefficient columns as fixed-point digit images, exact INT32
@@ -1961,7 +1960,7 @@ static int green_impl(ytf_ctx* ctx, const ytf_cache* c, int obs_layer, double zs
           lp.n = std::min(pass, c->n - lp.n0);
           lp.S = S + lp.n0;
           const int splits = lateral64_plan(lp);
-          CK(LAUNCH("k_lateral", launch_lateral64(lp, v, dxs, dys, ctx->stream)));
+          CK(LAUNCH("k_lateral64", launch_lateral64(lp, v, dxs, dys, ctx->stream)));
           CK(LAUNCH("k_reduce_splits2", launch_reduce_splits2(npix * ncol, splits, Gp, G, ctx->stream, lp.n0 > 0)));
         }
       }
@@ -2800,9 +2799,9 @@ int plan_build(ytf_plan* P) {
   CK(cudaEventCreate(&P->e0));
   CK(cudaEventCreate(&P->e1));
   CK(synth_small_init());
-  CK(cudaStreamSynchronize(ctx->stream));  // cache blocks cleared before the first run
-  // one eager pass of the large items' synthesis (on the zeroed inputs) records the largest
-  // size of each workspace it asks for; the plan then owns buffers of those sizes
+  CK(cudaStreamSynchronize(ctx->stream));
+  // one eager pass of the large items' synthesis records the largest size of each workspace it asks for; the
+  // plan then owns buffers of those sizes. What it computes, on caches no build has written yet, is not read.
   std::map<std::string, size_t> rec;
   int rc = plan_large_synthesis(P, &rec, nullptr);
   if (rc) return rc;

@@ -1137,12 +1137,6 @@ __device__ __forceinline__ void scan_body(const TransferParams& p, long node) {
   }
   cd Qs[4];
   load_q(p, src - 1, node, swaps, Qs, Qs + 2);
-  if (stat & ST_SINGULAR) {
-    p.status[gnode] = stat;
-    if (p.resp) p.resp[gnode] = 0.0;
-    else zero_rows(p.Tout, 16 * p.nobs, nT, gnode);
-    return;
-  }
   // cavity at the source layer (_R_cavity, _cavity_resummation)
   const double ds = p.layers[src - 1].d;
   M2 RR = M2{z, z, z, z};
@@ -1230,7 +1224,7 @@ __device__ __forceinline__ void walk_body(const TransferParams& p, long node) {
   const cd z{0.0, 0.0};
   if (!base) p.valid[gnode] = 0;
   for (int oi = 0; oi < p.nobs; ++oi) p.tvalid[(long)oi * nT + gnode] = 0;
-  if (stat & (ST_EIGEN | ST_SORT | ST_SINGULAR)) {
+  if (stat & (ST_EIGEN | ST_SORT)) {
     p.status[gnode] = stat;
     zero_rows(p.Tout, 16 * p.nobs, nT, gnode);
     return;
@@ -1355,7 +1349,7 @@ __global__ void __launch_bounds__(128) k_seeds(TransferParams p) {
   const long node = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (node < p.n) seeds_body(p, node);
 }
-// at most 170 registers: three 128-thread CTAs per SM (16 B of spills)
+// at most 170 registers: three 128-thread CTAs per SM (32 B of spills)
 __global__ void __launch_bounds__(128, 3) k_iface(TransferParams p) {
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const long n = p.n;
