@@ -277,13 +277,15 @@ int upload(ytf_ctx* ctx, void* dst, const void* src, size_t bytes) {
 
 // page-locked staging buffer of at least `bytes` (the stream is idle when it is replaced:
 // every entry point that fills it synchronises before returning)
+constexpr size_t STAGE_BYTES = (size_t)2 << 20;
 void* pinned_staging(ytf_ctx* ctx, size_t bytes) {
   if (ctx->pinned_bytes >= bytes) return ctx->pinned;
+  const size_t grown = ctx->pinned_bytes + ctx->pinned_bytes / 2;  // slowly rising sizes share allocations
   cudaStreamSynchronize(ctx->stream);
   if (ctx->pinned) cudaFreeHost(ctx->pinned);
   ctx->pinned = nullptr;
   ctx->pinned_bytes = 0;
-  size_t want = std::max(bytes, (size_t)1 << 20);
+  const size_t want = std::max(std::max(bytes, STAGE_BYTES), grown);
   if (cudaHostAlloc(&ctx->pinned, want, cudaHostAllocDefault) != cudaSuccess) {
     ctx->pinned = nullptr;
     return nullptr;
@@ -292,10 +294,20 @@ void* pinned_staging(ytf_ctx* ctx, size_t bytes) {
   return ctx->pinned;
 }
 
-// φ and n nodes to the device in one copy from page-locked memory (freed by the caller's synchronisation)
+// the same for the arrays of one problem, NULL where they are larger than what is there: page-locking costs more
+// than it saves them (builds of 0.1 to 1 million nodes in 20 steps: 0.28 s with a buffer for each, 0.10 s
+// from the arrays themselves), so the caller then uploads each array from where it lies
+void* small_staging(ytf_ctx* ctx, size_t bytes) {
+  return bytes <= std::max(STAGE_BYTES, ctx->pinned_bytes) ? pinned_staging(ctx, bytes) : nullptr;
+}
+
+// φ and n nodes to the device, in one copy where they can be staged (freed by the caller's synchronisation)
 int upload_k(ytf_ctx* ctx, double* dst, double phi, const double* kr, long n) {
-  double* h = (double*)pinned_staging(ctx, 8 * (size_t)(n + 1));
-  if (!h) return fail(ctx, YTF_ERR_NOMEM, "_cavity_response: page-locked staging allocation failed");
+  double* h = (double*)small_staging(ctx, 8 * (size_t)(n + 1));
+  if (!h) {
+    if (int rc = upload(ctx, dst, &phi, 8)) return rc;
+    return upload(ctx, dst + 1, kr, 8 * (size_t)n);
+  }
   h[0] = phi;
   std::memcpy(h + 1, kr, 8 * (size_t)n);
   return upload(ctx, dst, h, 8 * (size_t)(n + 1));
@@ -347,16 +359,17 @@ int alloc_cache(ytf_ctx* ctx, ytf_cache* c, bool upload_nodes = true) {
   c->d_T = (double2*)(b + o_T); c->d_Qf = (double2*)(b + o_Qf); c->d_Qb = (double2*)(b + o_Qb);
   c->d_sf = (double2*)(b + o_sf); c->d_sb = (double2*)(b + o_sb); c->d_basis = (double2*)(b + o_basis);
   if (!upload_nodes) return YTF_OK;
-  // the node arrays lie at the front of the block: one copy from page-locked memory, which the build's
-  // synchronisation frees
-  char* h = (char*)pinned_staging(ctx, o_status);
-  if (!h) return fail(ctx, YTF_ERR_NOMEM, "build_cavity_transfer: page-locked staging allocation failed");
-  auto put = [&](size_t o, const std::vector<double>& v) {
-    if (!v.empty()) std::memcpy(h + o, v.data(), 8 * v.size());
-  };
-  put(o_kr, c->kr); put(o_wr, c->wr); put(o_phi, c->phi); put(o_wphi, c->wphi); put(o_kri, c->kri); put(o_wri, c->wri);
-  CK(cudaMemcpyAsync(c->block, h, o_status, cudaMemcpyHostToDevice, ctx->stream));
-  return YTF_OK;
+  // the node arrays lie at the front of the block: one copy where they can be staged (the build's
+  // synchronisation frees the buffer)
+  char* h = (char*)small_staging(ctx, o_status);
+  const std::pair<size_t, const std::vector<double>*> parts[] = {{o_kr, &c->kr},     {o_wr, &c->wr},   {o_phi, &c->phi},
+                                                                 {o_wphi, &c->wphi}, {o_kri, &c->kri}, {o_wri, &c->wri}};
+  for (auto& q : parts) {
+    if (q.second->empty()) continue;
+    if (h) std::memcpy(h + q.first, q.second->data(), 8 * q.second->size());
+    else if (int rc = upload(ctx, b + q.first, q.second->data(), 8 * q.second->size())) return rc;
+  }
+  return h ? upload(ctx, c->block, h, o_status) : YTF_OK;
 }
 
 // no walk to other layers when every observation layer is the source layer (k_scan)
@@ -1778,12 +1791,12 @@ static int green_impl(ytf_ctx* ctx, const ytf_cache* c, int obs_layer, double zs
   if (nout == 0) return YTF_OK;
   CacheView& v = sp.c;
   int rc;
-  // a call of its own: the coordinates (and a 1D call's distinct radii and pixel map) in one copy from
-  // page-locked memory, one error word read back with the one synchronisation at the end
+  // a call of its own: the coordinates (and a 1D call's distinct radii and pixel map) in one copy where they can
+  // be staged, one error word read back with the one synchronisation at the end
   const bool single = gb == nullptr;
   GreenBatch own{};
   int nr1 = 0;
-  unsigned* herr = nullptr;
+  unsigned no_err = 0, *herr = &no_err;
   if (single) {
     std::vector<double> ur;
     std::vector<int> rmap;
@@ -1791,18 +1804,22 @@ static int green_impl(ytf_ctx* ctx, const ytf_cache* c, int obs_layer, double zs
     nr1 = (int)ur.size();
     const size_t nd = (size_t)nz + nx + ny + ur.size(), bytes = 8 * nd + 4 * rmap.size();
     const size_t eoff = (bytes + 63) / 64 * 64;
-    char* h = (char*)pinned_staging(ctx, eoff + 64);
-    if (!h) return fail(ctx, YTF_ERR_NOMEM, "closed_form_G: page-locked staging allocation failed");
-    double* hd = (double*)h;
-    std::memcpy(hd, z_obs, 8 * (size_t)nz);
-    std::memcpy(hd + nz, xs, 8 * (size_t)nx);
-    std::memcpy(hd + nz + nx, ys, 8 * (size_t)ny);
-    if (nr1) std::memcpy(hd + nz + nx + ny, ur.data(), 8 * ur.size());
-    if (!rmap.empty()) std::memcpy(hd + nd, rmap.data(), 4 * rmap.size());
-    herr = (unsigned*)(h + eoff);
-    *herr = 0;
     WS(dc, char, "g_coords", eoff + 64);
-    if ((rc = upload(ctx, dc, h, eoff + 64))) return rc;  // the error word (0) behind the coordinates
+    char* h = (char*)small_staging(ctx, eoff + 64);
+    auto put = [&](size_t at, const void* src, size_t n) -> int {
+      if (!h) return n ? upload(ctx, dc + at, src, n) : YTF_OK;
+      if (n) std::memcpy(h + at, src, n);
+      return YTF_OK;
+    };
+    if ((rc = put(0, z_obs, 8 * (size_t)nz)) || (rc = put(8 * (size_t)nz, xs, 8 * (size_t)nx)) ||
+        (rc = put(8 * ((size_t)nz + nx), ys, 8 * (size_t)ny)) ||
+        (rc = put(8 * ((size_t)nz + nx + ny), ur.data(), 8 * ur.size())) ||
+        (rc = put(8 * nd, rmap.data(), 4 * rmap.size())) || (rc = put(eoff, &no_err, 4)))
+      return rc;
+    if (h) {
+      if ((rc = upload(ctx, dc, h, eoff + 64))) return rc;
+      herr = (unsigned*)(h + eoff);  // the error word (0) behind the coordinates
+    }
     const double* dd = (const double*)dc;
     own.dzo = dd; own.dxs = dd + nz; own.dys = dd + nz + nx;
     own.err = (unsigned*)(dc + eoff);
