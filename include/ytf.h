@@ -429,7 +429,8 @@ int ytf_plan_destroy(ytf_plan* plan);
  * error of output 0 plus the logistic loss of output 1 (targets T: [B][2]). Inputs X: [B][n0]
  * row-major float. ytf_mlp_train takes DEVICE pointers to a resident training set (n
  * samples) and runs `steps` Adam steps (β = 0.9, 0.999) on mini-batches drawn on the device
- * from a seeded hash; losses[steps] (optional) receives the mini-batch losses. */
+ * from a seeded hash; losses[steps] (optional) receives the mini-batch losses.
+ * ytf_mlp_forward with on_device: X and out may overlap and may lie on another GPU (both are then copied). */
 typedef struct ytf_mlp ytf_mlp;
 int ytf_mlp_create(int device, int nlayers, const int* sizes, unsigned long long seed, ytf_mlp** out);
 int ytf_mlp_destroy(ytf_mlp* net);
